@@ -949,16 +949,12 @@ def main(argv=None):
     # ---- roofline of the distance kernel ----
     peak = sgemm_peak(torch)
     stage(f"SGEMM peak {peak:.1f} TFLOP/s")
-    # as executed (terms a lane shares between its cells counted once), and the previous counting
-    # that charges every cell for them (box 11, plane 9, rectangle 16, full test 31 flops)
+    # as executed (terms a lane shares between its cells counted once)
     flops = float(cst.flops_distance)
-    flops_count = (cst.box_tests * 11.0 + cst.plane_tests * 9.0 + cst.rect_tests * 16.0 + cst.tri_tests * 31.0)
     mean_dist_ms = statistics.mean(dist_ms)
     achieved = flops / (mean_dist_ms * 1e-3) / 1e12
     roofline = {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                 "traffic": None, "kernel": "k_distance (+ k_distance_deferred)", "flops_per_launch": flops,
-                "flops_per_launch_per_cell_count": flops_count,
-                "frac_per_cell_count": flops_count / (mean_dist_ms * 1e-3) / 1e12 / peak,
                 "box_tests": int(cst.box_tests), "tri_tests": int(cst.tri_tests),
                 "plane_tests": int(cst.plane_tests), "rect_tests": int(cst.rect_tests),
                 "tiles_deferred": int(cst.tiles_deferred), "tile_used": int(cst.tile_used),
@@ -967,7 +963,7 @@ def main(argv=None):
                 "algorithmic_bytes_per_launch": total_cells * 4}
     # the memory side beside it: distance writes plus one read of every mesh's hierarchy
     hbm_peak, hbm_src = hbm_peak_gbs()
-    bvh_bytes = sum(len(i) * (80 + 64) for _, i, _ in meshes)  # 80-byte triangle records + 64-byte nodes
+    bvh_bytes = sum(len(i) * (80 + 32) for _, i, _ in meshes)  # 80-byte triangle records, boxes of two-triangle blocks
     moved = total_cells * 4 + bvh_bytes
     roofline["hbm"] = {"bytes_per_launch": moved, "achieved_gbs": moved / (mean_dist_ms * 1e-3) / 1e9,
                        "peak_gbs": hbm_peak, "frac": moved / (mean_dist_ms * 1e-3) / 1e9 / hbm_peak,

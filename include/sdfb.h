@@ -72,16 +72,19 @@ typedef struct sdfb_opts {
   uint32_t struct_size;
   int32_t sign_mode;      /* sdfb_sign_mode, default AUTO */
   float band_voxels;      /* GWN: width in voxels of the FP64 band around the surface, default 1 */
-  int32_t leaf_size;      /* BVH leaf size 1..16, default: autotuned table */
+  int32_t leaf_size;      /* 1..16: the tree's blocks hold the largest of 2, 4, 8 triangles not above
+                             it, at least 2; default: autotuned table */
   int32_t tile;           /* distance tile shape 1..6 (4x4x2, 8x4x1, 4x4x4, 8x4x2, 4x4x8, 8x4x4
                              cells per warp), 0: autotuned table */
   int32_t no_occupancy;   /* 1: skip occupancy (occ_out may be NULL) */
   int32_t no_distance;    /* 1: occupancy only (dist_out may be NULL) */
   int32_t count_work;     /* 1: count traversal work into stats (a slower, instrumented kernel) */
-  int32_t stack_depth;    /* traversal stack entries, 32 or 64, 0: autotuned table */
-  int32_t step_budget;    /* a distance tile's walk checks every this many steps whether all tiles
-                             are handed out, and if so leaves its tile to a second pass where a
-                             whole block finishes it; 0: autotuned table, -1: never */
+  int32_t stack_depth;    /* 32 or 64, 0: autotuned table. The traversal stack holds any tree either
+                             way; 32 is what SDFB_FAULT_SHALLOW_STACK shrinks */
+  int32_t step_budget;    /* a distance tile's walk checks every this many steps (about 8 warp
+                             instructions each) whether all tiles are handed out, and if so leaves
+                             its tile to a second pass where a whole block finishes it; 0: autotuned
+                             table, -1: never */
   int32_t fault_inject;   /* testing only, 0 in normal use: SDFB_FAULT_* bits that make a bounded
                              device wait or limit run out on purpose (the bake then fails with the
                              status that limit maps to, and the context stays usable) */
@@ -94,7 +97,7 @@ typedef struct sdfb_opts {
  * kernels already bound run out early, so the error path behind it can be tested. */
 #define SDFB_FAULT_DISPATCH 1      /* no warp hands its block a new chunk of distance tiles: the
                                       other warps' bounded wait for one runs out -> INTERNAL */
-#define SDFB_FAULT_STEP_LIMIT 2    /* a traversal walk may take only 8 steps -> INTERNAL */
+#define SDFB_FAULT_STEP_LIMIT 2    /* a traversal walk may visit only one node -> INTERNAL */
 #define SDFB_FAULT_SHALLOW_STACK 4 /* a 32-entry traversal stack holds 2 entries: the walk
                                       overflows and the bake reruns with 64 entries */
 #define SDFB_FAULT_STACK_ALL 8     /* every traversal stack holds 2 entries -> OVERFLOW */
@@ -118,8 +121,8 @@ typedef struct sdfb_stats {
   uint64_t triangles;
   uint64_t sat_tests;      /* triangle/box tests run by the occupancy kernel */
   uint64_t crossings;      /* parity crossings found */
-  uint64_t box_tests;      /* count_work: point-box tests, one per cell */
-  uint64_t tri_tests;      /* count_work: full point-triangle tests, one per cell */
+  uint64_t box_tests;      /* count_work: tree children measured against a whole tile */
+  uint64_t tri_tests;      /* count_work: exact point-triangle distances */
   double flops_distance;   /* count_work: FP32 flops of the distance tests as executed, terms a lane
                               shares between its cells counted once (FMA = 2) */
   uint64_t kernel_launches; /* kernels this call launched */
@@ -127,9 +130,8 @@ typedef struct sdfb_stats {
   uint64_t graph_replayed;  /* 1 when the launch sequence was replayed from a CUDA graph */
   uint64_t tiles_deferred;  /* distance tiles that exceeded the step budget and were finished by a
                                whole block in the second distance pass */
-  uint64_t plane_tests;     /* count_work: cell-plane lower-bound tests that screen triangles, per cell */
-  uint64_t rect_tests;      /* count_work: in-plane bounding-rectangle tests after the plane screen,
-                               per cell */
+  uint64_t plane_tests;     /* count_work: blocks' oriented boxes measured against a whole tile */
+  uint64_t rect_tests;      /* count_work: oriented boxes measured against single cells */
   uint64_t gwn_direct_cells; /* GWN: cells whose sign needed the direct FP64 sum over every cap */
 } sdfb_stats;
 

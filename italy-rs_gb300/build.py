@@ -21,7 +21,7 @@ LIB = os.path.join(LIB_DIR, "libsdfb.so")
 INCLUDE = os.path.join(ROOT, "include")
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-CU_SOURCES = ["primitives.cu", "lbvh.cu", "occupancy.cu", "parity.cu", "distance.cu", "sparse.cu", "gwn.cu",
+CU_SOURCES = ["primitives.cu", "ptree.cu", "lbvh.cu", "occupancy.cu", "parity.cu", "distance.cu", "sparse.cu", "gwn.cu",
               "orchestrate.cu", "server.cu", "noalloc.cu", "materials.cu",
               "consumer.cu", "weld.cu", "caps.cu", "api.cu"]
 CPP_SOURCES = ["host_mesh.cpp"]

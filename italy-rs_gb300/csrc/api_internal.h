@@ -56,11 +56,11 @@ struct PinBuf {
   void release();
 };
 
-// A mesh hierarchy resident in device memory (built once, reused by later bakes).
+// A mesh's hierarchies resident in device memory (built once, reused by later bakes).
 struct ResidentBvh {
-  const sdfb::Node *nodes = nullptr;
-  const sdfb::DistTri *dtris = nullptr;  // distance hierarchy
-  const sdfb::TriRec *tris = nullptr;    // winding-number hierarchy
+  sdfb::PTreeRec tree{};              // distance
+  const sdfb::Node *nodes = nullptr;  // winding number: the caps
+  const sdfb::TriRec *tris = nullptr;
   const uint32_t *leaf_order = nullptr;
   const float4 *node_moment = nullptr;
   int num_nodes = 0, num_inner = 0, num_tris = 0, root = 0;
@@ -102,8 +102,8 @@ struct GwnInput {
 // counter at 64, work counters at 128 (box, triangle, SAT, plane tests), the deferral counters at
 // 160.
 constexpr size_t kMiscDeferOffset = 192;
-// Traversal steps a distance tile may take before it is deferred to the block-per-tile pass.
-constexpr int kDefaultStepBudget = 1024;
+// Steps of work between a distance tile's looks at whether it should go to the block-per-tile pass.
+constexpr int kDefaultStepBudget = 2048;
 
 // Device workspace of one bake in flight. The context owns one; the serving loop owns one per
 // stream so consecutive waves overlap.
@@ -195,7 +195,7 @@ sdfb_status run_batch(sdfb_ctx *ctx, cudaStream_t st, std::vector<PlanMesh> &mes
                       bool use_graph, sdfb_stats *stats);
 // Builds the hierarchy of one mesh (and of its caps when cT > 0) into `mem` / `cap_mem`, which
 // must hold resident_bytes(T) / resident_bytes(cT, true). Enqueued on st with ws's temporaries.
-size_t resident_bytes(uint64_t tris, bool winding = false);
+size_t resident_bytes(uint32_t tris, bool winding = false);
 sdfb_status build_resident(sdfb_ctx *ctx, Workspace &ws, cudaStream_t st, const PlanMesh &mesh, void *mem,
                            ResidentBvh &out, void *cap_mem, ResidentBvh &cap_out);
 

@@ -208,7 +208,7 @@ struct TriRec {
 __device__ __forceinline__ float inv_or_zero(float x) { return x > 0.0f ? 1.0f / x : 0.0f; }
 
 // ---------------------------------------------------------------------------------------------
-// Triangle record for distance queries: 80 bytes, five float4s, in BVH leaf order. Each triangle
+// Triangle record for distance queries: 80 bytes, five float4s (kept in planes by ptree.cu). Each triangle
 // is stored in its own orthonormal frame: origin at vertex A, u along the longest edge AB, v in
 // the triangle's plane towards C, h along the unit normal. In that frame the triangle is
 // A = (0, 0), B = (b, 0), C = (c1, c2) with c2 >= 0 and 0 <= c1 <= b.
@@ -223,10 +223,6 @@ __device__ __forceinline__ float inv_or_zero(float x) { return x > 0.0f ? 1.0f /
 // edges count, and with c2 = 0 those are pieces of the u axis. The frame is computed in FP64 from
 // the FP32 vertices and then rounded; A is the exact input vertex.
 //
-// The frame makes a query cheap where the traversal spends its time: a lane holds several cells
-// of one (x, y) column, so the x and y parts of u, v and h are formed once per lane and each cell
-// adds its z term with one FMA; the plane bound h^2 used to skip a triangle is the first step of
-// the full test rather than extra work.
 struct DistTri {
   float4 q0, q1, q2, q3, q4;
 };
@@ -301,25 +297,20 @@ __device__ inline DistTri make_dist_tri(float3 fa, float3 fb, float3 fc) {
   return t;
 }
 
-// FP32 arithmetic of the distance tests as the kernel executes it, counted as flops (add / sub /
-// mul = 1, FMA = 2; min, max, saturate and compares are not counted), for the roofline figure.
-// The work counters count every test per cell; a lane forms some terms once for its VPL cells (the
-// x and y parts of a box distance, of the plane height and of the in-plane coordinates), so those
-// are spread over them. Per cell and test, each stage on top of the ones before whose values it
-// reuses:
-//   box         shared: dx 2 + dy 2 + dx^2 + dy^2 3;  per cell: dz 2 + fma 2     = 4 + 7 / VPL
-//   plane       shared: x, y offsets 2 + height 3;   per cell: z offset 1 + height 2 + h^2 1
-//                                                                                  = 4 + 5 / VPL
-//   rectangle   shared: u, v 6;  per cell: u, v 4 + range offsets 2 + sum of squares 4
-//                                                                                  = 10 + 6 / VPL
-//   full test   edge AB 3 + edge AC 10 + edge BC 11 + inside 6 + sum 1             = 31
-__host__ __device__ inline double distance_flops(int vpl, double box, double plane, double rect, double full) {
+// FP32 arithmetic of the distance walk as it executes it, counted as flops (add / sub / mul = 1,
+// FMA = 2; min, max, absolute value and compares are not counted), for the roofline figure:
+//   child box, whole tile    offset 3, extent 6, squares 10, the two bounds 34           = 53
+//   oriented box, whole tile offset 3, frame 15, extent 6, squares 10, world 15, bounds 34 = 83
+//   oriented box, one cell   shared by a lane's cells: offset 2, frame 9
+//                            per cell: offset 1, frame 6, extent 3, squares 5            = 15 + 11 / VPL
+//   exact distance           offset 3, frame 15, range 1, edges 24, inside 6, sum 2      = 51
+__host__ __device__ inline double distance_flops(int vpl, double box, double block, double cell, double exact) {
   const double k = vpl > 0 ? 1.0 / vpl : 1.0;
-  return (4.0 + 7.0 * k) * box + (4.0 + 5.0 * k) * plane + (10.0 + 6.0 * k) * rect + 31.0 * full;
+  return 53.0 * box + 83.0 * block + (15.0 + 11.0 * k) * cell + 51.0 * exact;
 }
 
 // ---------------------------------------------------------------------------------------------
-// BVH node (64 bytes): the boxes of both children plus their references, so one 64-byte read
+// Node of the caps' binary hierarchy (64 bytes): both children's boxes and references: one 64-byte read
 // yields everything a traversal step needs. A child box is stored as its centre c and half
 // extent e, rounded outward so that [c - e, c + e] contains the box (an empty child has e = -inf):
 //   n0 = (c0.c.x, c0.c.y, c0.c.z, c0.e.x)

@@ -1,26 +1,45 @@
 // Nearest-triangle distance per cell with the sign fused in (replaces the 160-ray estimate of
 // src/render/kernels/sdf_bake.cu:39-51 with the exact Euclidean distance).
 //
-// Work unit: a warp owns a tile of TX x TY x TZ cells (32 lanes, VPL cells per lane stacked in
-// z) taken from its block's chunk of neighbouring tiles, so long and short tiles balance across the
-// persistent grid. The warp walks the BVH together: at each node every lane measures its cells
-// against both child boxes, __any_sync decides whether any cell still needs a child, and the child
-// whose box centre is nearer the tile's centre goes first. Leaves are tested right away by
-// all lanes on the same triangle record (a broadcast 80-byte load), so lanes never diverge. The
-// deferred child is pushed as (node, child) and its box is re-tested against the tightened
-// bounds when popped. The stack lives in registers, one entry per lane, read with __shfl_sync.
+// Work unit: a warp owns a tile of TX x TY x TZ cells (32 lanes, VPL cells per lane stacked in z),
+// taken from its block's chunk of neighbouring tiles. It walks the packed 32-ary tree (ptree.cu)
+// and changes what its lanes stand for on the way down:
 //
-// Two passes keep one expensive tile from holding the whole GPU. Cells far inside a closed surface
-// are nearly equidistant to much of it, so their tiles walk a large part of the tree; a single
-// such tile, taken late by one warp, used to run alone for a quarter of the kernel. In pass A a
-// walk looks at the chunk counter every `step_budget` steps; once every chunk has been handed out
-// (the tail, where a long walk would keep one SM busy while the rest idle) it stops, stores its
-// cells' current bounds (squared distances, upper bounds of the answer) in the output and appends
-// the tile to a deferred list. Pass B gives each deferred tile a whole block: the tree is cut into
-// 2^kSplitBits subtrees below the root, the block's warps take subtrees from a shared counter,
-// each walks its subtree for all the tile's cells starting from the stored bounds, and the warps
-// publish their bounds to shared memory (atomicMin on the float bits, valid for non-negative
-// values) after every subtree.
+//   lanes = children   a node's 32 children (boxes; at the last level the blocks' oriented boxes)
+//                      are tested at once, each lane deciding for the whole tile whether its child
+//                      can hold a triangle nearer than the bounds found so far;
+//   lanes = cells      a block that survives is measured against every cell of the tile by the
+//                      distance to its oriented box; the cells that it could improve become
+//                      (block, cell) pairs in shared memory;
+//   lanes = triangles  pairs are taken 32 / n at a time, n lanes computing the exact distances to a
+//                      block's n triangles; the minimum goes to the cell's bound in shared memory.
+//
+// Before, all lanes were cells throughout: every node and triangle was tested by 128 cells although
+// most die on the first one's answer, 50-70 instructions a triangle. Testing children by lanes costs
+// about 4 instructions a child, and the exact test runs only for pairs that need it.
+//
+// Whole-tile test. Let c be the tile's centre and delta = q - c for a cell q. For a convex child
+// (box) with nearest point p to c, e = c - p, d = |e|, n = e / d, the child lies behind the plane
+// through p with normal n, so its distance to q is at least d + n . delta; and if its farthest
+// point from p is at D, its squared distance is at least d^2 + 2 e . delta + |delta|^2 - K with
+// K = D (2 rho - D) for D < rho, else rho^2, rho = max |delta| (|x - p|^2 + 2 delta . (p - x)
+// minimised over |x - p| <= D, and |c - x|^2 >= d^2 + |x - p|^2 by the projection onto a convex
+// set). On the other side the cells' current bounds u are majorised by planes, u <= a + g . delta
+// and u^2 - |delta|^2 <= A + G . delta (g, G fitted, a and A the largest residuals). A child is
+// dropped when either lower bound is above its plane over the whole box |delta_k| <= H_k, which is
+// one sum of three absolute values each. The first is tight near the surface, the second, where the
+// curvature of the distance cancels, for children small against their distance.
+//
+// Every test keeps a child by a margin above the rounding of both sides and of the exact test, so a
+// triangle is dropped only when its computed distance cannot be the minimum: the result is the
+// minimum over all triangles of the computed distance, whatever the order of the walk.
+//
+// Two passes keep one expensive tile from holding the whole GPU. In pass A a walk looks at the
+// chunk counter every few steps; once every chunk has been handed out (the tail) it stops, stores
+// its cells' bounds (squared distances, upper bounds of the answer) in the output and appends the
+// tile to a deferred list. Pass B gives each deferred tile a whole block: its warps take the nodes
+// of one level from a shared counter and walk below them for the same cells, whose bounds they
+// share in shared memory (atomicMin on the float bits, valid for non-negative values).
 //
 // Sign: parity counts the column's crossing heights above each cell (the crossing list is
 // built by parity.cu). Winding-number signs are applied afterwards by gwn.cu, which needs the
@@ -35,15 +54,9 @@
 namespace sdfb {
 namespace {
 
-// Pass A: a block takes chunks of consecutive tiles (a brick of neighbouring tiles) and its warps
-// take tiles from the block's chunk, so the warps sharing an SM's L1 walk overlapping parts of the
-// tree. Two blocks of 16 warps per SM: the walk waits on dependent node and record loads, and 32
-// resident warps hide more of that latency than 20 warps without spills did (64-mesh batch
-// 281 -> 259 ms; 24 warps at 80 registers: 267 ms). Pass B's block shares one tile: 16 warps over
-// 64 subtrees, which also keeps a small grid (fewer tiles than the GPU holds warps) busy once its
-// tiles are deferred.
-constexpr int kThreadsA = 512;
-constexpr int kMinBlocksA = 2;  // 32 warps per SM: 64 registers a thread, some of them spilled to L1
+// Two blocks of 16 warps per SM: the walk waits on dependent loads and shared-memory round trips.
+constexpr int kThreadsA = 128;
+constexpr int kMinBlocksA = 6;
 constexpr int kWarpsPerBlockA = kThreadsA / kWarp;
 // Tile order within a mesh: bricks of kBrickX x kBrickY x kBrickZ tiles, x fastest inside a brick
 // and across bricks. Tiles of a partial brick beyond the grid have no active cell.
@@ -52,7 +65,18 @@ constexpr int kChunkMax = 32;  // tiles per chunk when there are plenty
 constexpr unsigned long long kNoTile = ~0ull;
 constexpr int kDispatchSpin = 1 << 22;  // bound on a warp's wait for its block's next chunk
 constexpr int kThreads = 512;
-constexpr int kSplitBits = 6;  // pass B: 64 subtrees per deferred tile
+constexpr int kWarpsPerBlockB = kThreads / kWarp;
+constexpr uint32_t kMaxItems = 512;  // pass B: at most this many subtrees per deferred tile
+constexpr int kMaxLevels = 8;        // 2^31 triangles in blocks of 2 make 6 levels of 32-ary nodes
+constexpr int kStackSize = 32 * kMaxLevels;  // a node leaves at most 31 siblings behind on its level
+constexpr int kFlushAt = 16;                 // surviving blocks measured against the cells together
+constexpr int kSurvivors = kFlushAt + kWarp;
+constexpr int kDrainAt = 64;                 // pairs that start a round of exact tests
+// Steps of work as sdfb_opts.step_budget counts them, about 8 instructions each.
+constexpr int kStepsPerVisit = 16, kStepsPerBlock = 10, kStepsPerRound = 12;
+constexpr int kSearchVisits = 48;    // a search for a seed gives up after as many nodes
+constexpr float kCloseTile = 5.0f;           // squared distance of tile centres, in squared half diagonals
+constexpr uint32_t kNoSeed = ~0u;
 constexpr float kInf = __builtin_huge_valf();
 
 struct Shape {
@@ -66,7 +90,8 @@ struct WalkStats {
   bool overflow = false, corrupt = false;
 };
 
-// A tile's cells as one lane sees them.
+// A tile's cells as one lane sees them. A cell beyond the grid stands in for the nearest cell inside
+// it, so that every lane holds valid points; only active cells are written.
 template <int TX, int TY, int TZ>
 struct TileCells {
   static constexpr int kLayer = TX * TY;
@@ -75,12 +100,10 @@ struct TileCells {
   static_assert(kLayer * kLanesZ == kWarp && VPL * kLanesZ == TZ, "tile must cover whole warps");
   const MeshRec *M;
   GridDev g;
-  int vx, vy, vz0;  // this lane's column and first z; cell v is at z = vz0 + v * kLanesZ
-  float px, py, pz[VPL];
-  bool active[VPL];
-  float cx, cy, cz;  // tile centre
+  int x0, y0, z0;  // the tile's first cell
 
-  __device__ __forceinline__ void locate(const BatchDev &B, unsigned long long tile, int lane) {
+  // Returns false for a tile without a cell inside the grid.
+  __device__ __forceinline__ bool locate(const BatchDev &B, unsigned long long tile) {
     const int mesh = find_mesh(B.tile_starts, B.num_meshes, tile);
     M = &B.recs[mesh];
     g = M->g;
@@ -90,83 +113,29 @@ struct TileCells {
     const unsigned long long brick = local / kBrickTiles;
     const int w = static_cast<int>(local % kBrickTiles);
     const unsigned long long rest = brick / bricks_x;
-    const int tx = static_cast<int>(brick % bricks_x) * kBrickX + w % kBrickX;
-    const int ty = static_cast<int>(rest % bricks_y) * kBrickY + (w / kBrickX) % kBrickY;
-    const int tz = static_cast<int>(rest / bricks_y) * kBrickZ + w / (kBrickX * kBrickY);
-    cx = g.ox + (float(tx * TX) + 0.5f * TX) * g.voxel;
-    cy = g.oy + (float(ty * TY) + 0.5f * TY) * g.voxel;
-    cz = g.oz + (float(tz * TZ) + 0.5f * TZ) * g.voxel;
-    vx = tx * TX + lane % TX;
-    vy = ty * TY + (lane / TX) % TY;
-    vz0 = tz * TZ + lane / kLayer;
-    px = cell_center(g.ox, vx, g.voxel);
-    py = cell_center(g.oy, vy, g.voxel);
-#pragma unroll
-    for (int v = 0; v < VPL; ++v) {
-      const int vz = vz0 + v * kLanesZ;
-      active[v] = vx < g.nx && vy < g.ny && vz < g.nz;
-      pz[v] = cell_center(g.oz, vz, g.voxel);
-    }
+    x0 = (static_cast<int>(brick % bricks_x) * kBrickX + w % kBrickX) * TX;
+    y0 = (static_cast<int>(rest % bricks_y) * kBrickY + (w / kBrickX) % kBrickY) * TY;
+    z0 = (static_cast<int>(rest / bricks_y) * kBrickZ + w / (kBrickX * kBrickY)) * TZ;
+    return x0 < g.nx && y0 < g.ny && z0 < g.nz;
   }
-
-  __device__ __forceinline__ uint64_t cell(int v) const {
-    return (uint64_t(vz0 + v * kLanesZ) * g.ny + vy) * g.nx + vx;
+  __device__ __forceinline__ int vx(int lane) const { return x0 + lane % TX; }
+  __device__ __forceinline__ int vy(int lane) const { return y0 + (lane / TX) % TY; }
+  __device__ __forceinline__ int vz(int lane, int v) const { return z0 + lane / kLayer + v * kLanesZ; }
+  __device__ __forceinline__ float px(int lane) const { return cell_center(g.ox, min(vx(lane), g.nx - 1), g.voxel); }
+  __device__ __forceinline__ float py(int lane) const { return cell_center(g.oy, min(vy(lane), g.ny - 1), g.voxel); }
+  __device__ __forceinline__ float pz(int lane, int v) const {
+    return cell_center(g.oz, min(vz(lane, v), g.nz - 1), g.voxel);
+  }
+  __device__ __forceinline__ bool active(int lane, int v) const {
+    return vx(lane) < g.nx && vy(lane) < g.ny && vz(lane, v) < g.nz;
+  }
+  // Output index of the lane's cell v, or of the cell it stands in for.
+  __device__ __forceinline__ uint64_t cell(int lane, int v) const {
+    return (uint64_t(min(vz(lane, v), g.nz - 1)) * g.ny + min(vy(lane), g.ny - 1)) * g.nx + min(vx(lane), g.nx - 1);
   }
 };
 
-template <int VPL, bool COUNT>
-__device__ __forceinline__ void test_leaf(const DistTri *__restrict__ tris, int num_tris, int first, int count,
-                                          float px, float py, const float (&pz)[VPL], float (&best)[VPL],
-                                          WalkStats &ws) {
-  if (first < 0 || count > num_tris - first) {
-    ws.corrupt = true;
-    return;
-  }
-  for (int k = 0; k < count; ++k) {
-    const DistTri *tr = tris + first + k;
-    const float4 q0 = __ldg(&tr->q0), q3 = __ldg(&tr->q3), q1 = __ldg(&tr->q1), q2 = __ldg(&tr->q2),
-                 q4 = __ldg(&tr->q4);
-    // The x and y parts of the frame coordinates are shared by the lane's cells.
-    const float ax = px - q0.x, ay = py - q0.y;
-    const float sh = fmaf(ay, q3.y, ax * q3.x);
-    // The squared distance to the triangle's plane, h^2, bounds the squared distance to the
-    // triangle from below: skip the triangle when no cell could improve.
-    float az[VPL], h2[VPL];
-    bool need = false;
-#pragma unroll
-    for (int v = 0; v < VPL; ++v) {
-      az[v] = pz[v] - q0.z;
-      const float h = fmaf(az[v], q3.z, sh);
-      h2[v] = h * h;
-      need |= h2[v] < best[v];
-    }
-    if (COUNT) ws.plane_tests += kWarp * VPL;
-    if (!__any_sync(kFull, need)) continue;
-    // Then the distance to the triangle's bounding rectangle in its own plane, [0, b] x [0, c2],
-    // with h^2: much tighter where a cell is near the triangle's plane but beside the triangle
-    // (most cells that pass the plane bound). Its u part is edge AB's clamp in the full test.
-    const float su = fmaf(ay, q1.y, ax * q1.x), sv = fmaf(ay, q2.y, ax * q2.x);
-    // The in-plane coordinates are formed again by the full test (about one screen in eight
-    // passes), so they need not stay live across the vote.
-    need = false;
-#pragma unroll
-    for (int v = 0; v < VPL; ++v) {
-      const float du = dist_to_range(fmaf(az[v], q1.z, su), q0.w);
-      const float dw = dist_to_range(fmaf(az[v], q2.z, sv), q2.w);
-      need |= fmaf(du, du, fmaf(dw, dw, h2[v])) < best[v];
-    }
-    if (COUNT) ws.rect_tests += kWarp * VPL;
-    if (!__any_sync(kFull, need)) continue;
-#pragma unroll
-    for (int v = 0; v < VPL; ++v) {
-      const float u = fmaf(az[v], q1.z, su), w = fmaf(az[v], q2.z, sv);
-      best[v] = fminf(best[v], h2[v] + inplane_dist2(u, w, dist_to_range(u, q0.w), q0.w, q1.w, q2.w, q3.w, q4));
-    }
-    if (COUNT) ws.tri_tests += kWarp * VPL;
-  }
-}
-
-// When a walk may stop early: every `every` steps it reads the pass's tile counter, and it stops
+// When a walk may stop early: every `every` steps of work it reads the pass's tile counter, and it stops
 // once every tile has been handed out (the pass is in its tail, where a long walk would run
 // alone). every = 0: never.
 struct TailCheck {
@@ -175,164 +144,470 @@ struct TailCheck {
   int every;
 };
 
-// Walks the subtree below inner node `start` for this lane's cells, tightening best[] (squared
-// distances; inactive cells hold -1 and never ask for work). Returns false when the walk stopped
-// early by the tail check with work left (best[] then holds upper bounds); a walk past the limit a
-// correct tree allows stops with the corrupt flag.
-// Bounds of one walk: the step limit (a correct tree expands each inner node at most once per walk
-// and pops at most once per push) and the usable stack entries. The fault-injection bits shrink
-// them so that the error paths behind them can be tested.
+// Bounds of one walk: the most node visits (a walk visits each node at most once) and the usable stack
+// entries. The fault-injection bits shrink them so that the error paths behind them can be tested.
 struct WalkLimits {
-  int steps, stack;
+  int visits, stack;
 };
-template <int STACK>
-__device__ __forceinline__ WalkLimits walk_limits(int num_nodes, int fault) {
+__device__ __forceinline__ WalkLimits walk_limits(const DistTree &t, int stack_depth, int fault) {
   WalkLimits l;
-  l.steps = num_nodes > (INT_MAX - 64) / 2 ? INT_MAX - 1 : 2 * num_nodes + 64;
-  l.stack = STACK;
+  l.visits = static_cast<int>(min(t.num_tris, 0x7ffffff0u - 64u)) + 64;
+  l.stack = kStackSize;
   if (fault) {
-    if (fault & kFaultStepLimit) l.steps = 8;
-    if ((fault & kFaultStackAll) || (STACK == 32 && (fault & kFaultShallowStack))) l.stack = 2;
+    if (fault & kFaultStepLimit) l.visits = 0;
+    if ((fault & kFaultStackAll) || (stack_depth <= 32 && (fault & kFaultShallowStack))) l.stack = 2;
   }
   return l;
 }
 
-template <int VPL, int STACK, bool COUNT>
-__device__ __forceinline__ bool walk(const Node *__restrict__ nodes, const DistTri *__restrict__ tris, int num_nodes,
-                                     int num_tris, int start, TailCheck tail, WalkLimits lim, int lane, float tcx,
-                                     float tcy, float tcz, float px, float py, const float (&pz)[VPL],
-                                     float (&best)[VPL], WalkStats &ws) {
-  static_assert(STACK == 32 || STACK == 64, "stack depth is one or two registers per lane");
-  const int step_limit = lim.steps;
-  int next_check = tail.every > 0 ? tail.every : INT_MAX;
-  int cur = start, sp = 0, stk0 = 0, stk1 = 0;
-  for (int steps = 0;; ++steps) {
-    if (steps > step_limit || cur >= num_nodes) {
-      ws.corrupt = true;
-      return true;
+// Shared memory of one warp's walk. What is the same for all lanes lives here rather than in
+// registers (one broadcast load where it is needed): 80 instead of 120 registers a thread.
+struct WarpMem {
+  float4 centre;                // the tile's centre; w: rho
+  float4 half;                  // half extents of the cell centres about it; w: a
+  float4 lin, sq;               // (g, -) and (G, A): the planes above the bounds
+  DistTree t;
+  float z[8];                   // z of the tile's layers
+  uint32_t level_n[kMaxLevels], level_off[kMaxLevels];  // nodes of each level, first node in t.box
+  uint32_t stack[kStackSize];   // (level << 28) | node
+  uint32_t blocks[kSurvivors];  // surviving blocks; blocks[0] is the nearest of its node
+  uint32_t mesh;                // the mesh that t is of
+  uint32_t seed;                // the block that last improved the middle cell of the tile at seed_at
+  float seed_at[3];
+  uint16_t pairs[kDrainAt + kWarp * 4];  // (index into blocks << 7) | (v << 5) | lane
+};
+static_assert(kSurvivors <= 512, "a pair packs into 16 bits");
+
+// Exact squared distance from q to a triangle record.
+__device__ __forceinline__ float tri_dist2(const float4 &q0, const float4 &q1, const float4 &q2, const float4 &q3,
+                                           const float4 &q4, float qx, float qy, float qz) {
+  const float ax = qx - q0.x, ay = qy - q0.y, az = qz - q0.z;
+  const float h = fmaf(az, q3.z, fmaf(ay, q3.y, ax * q3.x));
+  const float u = fmaf(az, q1.z, fmaf(ay, q1.y, ax * q1.x)), w = fmaf(az, q2.z, fmaf(ay, q2.y, ax * q2.x));
+  return fmaf(h, h, inplane_dist2(u, w, dist_to_range(u, q0.w), q0.w, q1.w, q2.w, q3.w, q4));
+}
+
+template <int TX, int TY, int TZ, bool COUNT>
+struct Walker {
+  using Cells = TileCells<TX, TY, TZ>;
+  static constexpr int VPL = Cells::VPL;
+  static constexpr int kMiddle = (VPL / 2) * kWarp + 13;  // a cell about the middle of the tile
+  // Relative margin of the cells' bounds in the oriented box test (2e-6 in the distance, several
+  // times the rounding of the box distance and of the exact test; the boxes' half extents carry the
+  // part that scales with the block's size).
+  static constexpr float kKeep = 1.0f + 4e-6f;
+
+  WarpMem &m;
+  uint32_t *best;  // squared distance bounds (float bits) of the tile's cells: this warp's, or its block's
+  int lane;
+  float px, py, pz[VPL], keep[VPL];  // keep: best * kKeep
+  int steps = 0;                     // work of the current walk
+  WalkStats ws;
+
+  __device__ __forceinline__ Walker(WarpMem &mem, uint32_t *b, int l) : m(mem), best(b), lane(l) {}
+
+  __device__ __forceinline__ void set_tile(const Cells &c) {
+    const GridDev &g = c.g;
+    px = c.px(lane);
+    py = c.py(lane);
+#pragma unroll
+    for (int v = 0; v < VPL; ++v) pz[v] = c.pz(lane, v);
+    if (lane < TZ) m.z[lane] = cell_center(g.oz, min(c.z0 + lane, g.nz - 1), g.voxel);
+    const float cx = g.ox + (float(c.x0) + 0.5f * TX) * g.voxel, cy = g.oy + (float(c.y0) + 0.5f * TY) * g.voxel,
+                cz = g.oz + (float(c.z0) + 0.5f * TZ) * g.voxel;
+    // Half extents of the cell centres about (cx, cy, cz), with room for both sides' rounding.
+    const float hx = 0.50001f * (TX - 1) * g.voxel + 3e-7f * (fabsf(g.ox) + fabsf(cx)),
+                hy = 0.50001f * (TY - 1) * g.voxel + 3e-7f * (fabsf(g.oy) + fabsf(cy)),
+                hz = 0.50001f * (TZ - 1) * g.voxel + 3e-7f * (fabsf(g.oz) + fabsf(cz));
+    if (lane == 0) {
+      m.centre = make_float4(cx, cy, cz, sqrtf(hx * hx + hy * hy + hz * hz));
+      m.half = make_float4(hx, hy, hz, kInf);
+      m.lin.w = 12.0f / (float(VPL * kWarp) * g.voxel * g.voxel);  // for fit()
     }
-    if (steps >= next_check) {
-      unsigned long long handed = 0;
-      if (lane == 0) handed = *reinterpret_cast<const volatile unsigned long long *>(tail.counter);
-      handed = __shfl_sync(kFull, handed, 0);
-      if (handed >= tail.total) return false;
-      next_check = steps + tail.every;
+    __syncwarp();
+  }
+
+  // Nodes per level of the mesh's tree and where each level starts in t.box.
+  __device__ __forceinline__ void set_tree(const DistTree &tree, uint32_t mesh) {
+    if (lane < kMaxLevels) {
+      m.level_n[lane] = tree_level_count(tree.num_tris, tree.block_log2, lane);
+      uint32_t off = 0;
+      for (int l = 1; l < lane; ++l) off += tree_level_count(tree.num_tris, tree.block_log2, l);
+      m.level_off[lane] = off;
     }
-    if (cur < 0) {
-      if (sp == 0) return true;
-      --sp;
-      const int e = __shfl_sync(kFull, (STACK == 32 || sp < 32) ? stk0 : stk1, sp & 31);
-      if ((e >> 1) >= num_nodes) {
+    if (lane == 0) {
+      m.t = tree;
+      m.seed = kNoSeed;
+      *const_cast<volatile uint32_t *>(&m.mesh) = mesh;
+    }
+    __syncwarp();
+  }
+  __device__ __forceinline__ uint32_t root() const {
+    int l = 1;
+    while (l < kMaxLevels - 1 && m.level_n[l] > 1) ++l;
+    return static_cast<uint32_t>(l) << 28;
+  }
+
+  // Sum and maximum over the warp.
+  static __device__ __forceinline__ float wsum(float v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
+    return v;
+  }
+  static __device__ __forceinline__ float wmax(float v) {
+    return ordered_to_float(__reduce_max_sync(kFull, float_to_ordered(v)));
+  }
+
+  // Reads the bounds and fits the planes above them: g and G are the least squares slopes over the
+  // tile (the cells' offsets from the centre sum to about zero), taken about a middle cell's value.
+  __device__ __forceinline__ void fit() {
+    float su = 0.0f, sw = 0.0f, sz = 0.0f, swz = 0.0f, u[VPL], w[VPL];
+    const float4 c = m.centre;
+    const float dx = px - c.x, dy = py - c.y, dxy = dx * dx + dy * dy;
+#pragma unroll
+    for (int v = 0; v < VPL; ++v) {
+      const float b = __uint_as_float(best[v * kWarp + lane]);
+      const float dz = pz[v] - c.z;
+      keep[v] = b * kKeep;
+      u[v] = sqrtf(b);
+      w[v] = b - fmaf(dz, dz, dxy);
+    }
+    const float u0 = __shfl_sync(kFull, u[kMiddle / kWarp], kMiddle % kWarp),
+                w0 = __shfl_sync(kFull, w[kMiddle / kWarp], kMiddle % kWarp);
+#pragma unroll
+    for (int v = 0; v < VPL; ++v) {
+      const float dz = pz[v] - c.z, du = u[v] - u0, dw = w[v] - w0;
+      su += du;
+      sw += dw;
+      sz = fmaf(du, dz, sz);
+      swz = fmaf(dw, dz, swz);
+    }
+    const float n = m.lin.w;  // 1 / sum of squared offsets, but for the axes' cell counts
+    const float ix = n * (1.0f / (TX * TX - 1)), iy = n * (1.0f / (TY * TY - 1)),
+                iz = TZ > 1 ? n * (1.0f / (TZ > 1 ? TZ * TZ - 1 : 1)) : 0.0f;
+    const float gx = wsum(su * dx) * ix, gy = wsum(su * dy) * iy, gz = wsum(sz) * iz;
+    const float Gx = wsum(sw * dx) * ix, Gy = wsum(sw * dy) * iy, Gz = wsum(swz) * iz;
+    float ra = -kInf, rA = -kInf;
+#pragma unroll
+    for (int v = 0; v < VPL; ++v) {
+      const float dz = pz[v] - c.z;
+      ra = fmaxf(ra, u[v] - (gx * dx + gy * dy + gz * dz));
+      rA = fmaxf(rA, w[v] - (Gx * dx + Gy * dy + Gz * dz));
+    }
+    ra = wmax(ra);
+    rA = wmax(rA);
+    const float4 h = m.half;
+    __syncwarp();
+    if (lane == 0) {
+      m.half.w = ra + 2e-6f * (fabsf(ra) + h.x * fabsf(gx) + h.y * fabsf(gy) + h.z * fabsf(gz));
+      m.lin = make_float4(gx, gy, gz, n);
+      m.sq = make_float4(Gx, Gy, Gz,
+                         rA + 4e-6f * (fabsf(rA) + h.x * fabsf(Gx) + h.y * fabsf(Gy) + h.z * fabsf(Gz)));
+    }
+    __syncwarp();
+  }
+
+  // Whether a convex child with nearest point c - (ex, ey, ez) to the tile's centre, whose farthest
+  // point from there is at sqrt(D2), may hold a triangle nearer than the bounds of some cell. S is
+  // the size of the coordinates that e was formed from; a few 1e-7 of it is the error of e. A NaN
+  // anywhere (a mesh with non-finite vertices, reported elsewhere) drops the child.
+  __device__ __forceinline__ bool near(float rho, float ex, float ey, float ez, float d2, float D2, float S) const {
+    const float4 h = m.half, g = m.lin, G = m.sq;
+    const float inv = d2 > 0.0f ? rsqrtf(d2) : 0.0f;
+    const float d = d2 * inv;
+    const float lin = d - h.w - (h.x * fabsf(fmaf(ex, inv, -g.x)) + h.y * fabsf(fmaf(ey, inv, -g.y)) +
+                                 h.z * fabsf(fmaf(ez, inv, -g.z)));
+    const float D = sqrtf(D2);
+    const float K = D < rho ? D * (2.0f * rho - D) : rho * rho;
+    const float sq = d2 - K - G.w - (h.x * fabsf(fmaf(2.0f, ex, -G.x)) + h.y * fabsf(fmaf(2.0f, ey, -G.y)) +
+                                     h.z * fabsf(fmaf(2.0f, ez, -G.z)));
+    return lin <= 2e-6f * S * fmaf(rho, inv, 1.0f) && sq <= 4e-6f * S * (d + rho);
+  }
+
+  // Exact distances of the queued pairs, n = 2^block_log2 lanes to a pair.
+  __device__ __forceinline__ void drain(int &np) {
+    __syncwarp();
+    const int lb = m.t.block_log2, sub = lane & ((1 << lb) - 1);
+    const float4 *tris = m.t.tri;
+    for (int base = 0; base < np; base += kWarp >> lb) {
+      const int i = base + (lane >> lb);
+      const uint32_t e = m.pairs[min(i, np - 1)];
+      const int cl = e & 31, v = (e >> 5) & 3;
+      const uint32_t blk = m.blocks[e >> 7];
+      const float4 *tri = tree_tri(tris, (size_t(blk) << lb) + sub);
+      const float4 q0 = __ldg(tri), q1 = __ldg(tri + kTriPlane), q2 = __ldg(tri + 2 * kTriPlane),
+                   q3 = __ldg(tri + 3 * kTriPlane), q4 = __ldg(tri + 4 * kTriPlane);
+      float d2 = tri_dist2(q0, q1, q2, q3, q4, __shfl_sync(kFull, px, cl), __shfl_sync(kFull, py, cl),
+                           m.z[cl / Cells::kLayer + v * Cells::kLanesZ]);
+      for (int o = 1; o < (1 << lb); o <<= 1) d2 = fminf(d2, __shfl_xor_sync(kFull, d2, o));
+      if (sub == 0 && i < np) {
+        const uint32_t was = atomicMin(best + (e & 127), __float_as_uint(d2));
+        if ((e & 127) == kMiddle && __float_as_uint(d2) < was) m.seed = blk;
+      }
+      if (COUNT) ws.tri_tests += kWarp;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int v = 0; v < VPL; ++v) keep[v] = __uint_as_float(best[v * kWarp + lane]) * kKeep;
+    steps += ((np << lb) >> 5) * kStepsPerRound;
+    np = 0;
+  }
+
+  // Measures the surviving blocks against every cell, runs the pairs, refits the planes.
+  __device__ __forceinline__ void flush(int &nb) {
+    int np = 0;
+    bool any_pair = false;
+    const float4 *obb = m.t.obb;
+    for (int i = 0; i < nb; ++i) {
+      const float4 *o = tree_obb(obb, m.blocks[i]);
+      const float4 o0 = __ldg(o), o1 = __ldg(o + kObbPlane), o2 = __ldg(o + 2 * kObbPlane), o3 = __ldg(o + 3 * kObbPlane);
+      const float dx = px - o0.x, dy = py - o0.y;
+      const float s0 = fmaf(dy, o1.y, dx * o1.x), s1 = fmaf(dy, o2.y, dx * o2.x), s2 = fmaf(dy, o3.y, dx * o3.x);
+      bool want[VPL], some = false;
+#pragma unroll
+      for (int v = 0; v < VPL; ++v) {
+        const float dz = pz[v] - o0.z;
+        const float e0 = fmaxf(fabsf(fmaf(dz, o1.z, s0)) - o0.w, 0.0f);
+        const float e1 = fmaxf(fabsf(fmaf(dz, o2.z, s1)) - o1.w, 0.0f);
+        const float e2 = fmaxf(fabsf(fmaf(dz, o3.z, s2)) - o2.w, 0.0f);
+        want[v] = fmaf(e0, e0, fmaf(e1, e1, e2 * e2)) < keep[v];
+        some |= want[v];
+      }
+      if (COUNT) ws.rect_tests += kWarp * VPL;
+      if (!__any_sync(kFull, some)) continue;
+      any_pair = true;
+#pragma unroll
+      for (int v = 0; v < VPL; ++v) {
+        const uint32_t mask = __ballot_sync(kFull, want[v]);
+        if (want[v])
+          m.pairs[np + __popc(mask & ((1u << lane) - 1u))] = static_cast<uint16_t>((i << 7) | (v << 5) | lane);
+        np += __popc(mask);
+      }
+      if (np >= kDrainAt) drain(np);
+    }
+    if (np > 0) drain(np);
+    __syncwarp();
+    steps += nb * kStepsPerBlock;
+    nb = 0;
+    if (any_pair) fit();
+  }
+
+  // Finds the block to start from: of the blocks nearest to the middle of the last tiles of the
+  // block's warps, the one nearest to this tile's centre, if one of those tiles was close by; else a
+  // search from the root. (A warp that moves to another mesh meanwhile may leave a block number of
+  // that mesh behind: any block of the tree is a valid seed.)
+  __device__ __forceinline__ void pick_seed(const WarpMem *mem, int warps) {
+    const float4 c = m.centre;
+    uint32_t s = 0;
+    bool have = false;
+    if (lane < warps) {
+      const volatile WarpMem *o = mem + lane;
+      s = o->seed;
+      const float dx = o->seed_at[0] - c.x, dy = o->seed_at[1] - c.y, dz = o->seed_at[2] - c.z;
+      have = o->mesh == m.mesh && s < m.level_n[0] && dx * dx + dy * dy + dz * dz < kCloseTile * c.w * c.w;
+    }
+    if (!__any_sync(kFull, have)) {
+      search();
+      return;
+    }
+    const float d2 = have ? obb_dist2(s) : kInf;
+    const uint32_t near_key = __reduce_min_sync(kFull, have ? (__float_as_uint(d2) & ~31u) | lane : ~0u);
+    s = __shfl_sync(kFull, s, near_key & 31);
+    __syncwarp();
+    if (lane == 0) m.seed = s;
+    __syncwarp();
+  }
+
+  // Squared distance of the tile's centre to a block's oriented box.
+  __device__ __forceinline__ float obb_dist2(uint32_t blk) const {
+    const float4 c = m.centre;
+    const float4 *o = tree_obb(m.t.obb, blk);
+    const float4 o0 = __ldg(o), o1 = __ldg(o + kObbPlane), o2 = __ldg(o + 2 * kObbPlane), o3 = __ldg(o + 3 * kObbPlane);
+    const float dx = c.x - o0.x, dy = c.y - o0.y, dz = c.z - o0.z;
+    const float e0 = fmaxf(fabsf(fmaf(dz, o1.z, fmaf(dy, o1.y, dx * o1.x))) - o0.w, 0.0f);
+    const float e1 = fmaxf(fabsf(fmaf(dz, o2.z, fmaf(dy, o2.y, dx * o2.x))) - o1.w, 0.0f);
+    const float e2 = fmaxf(fabsf(fmaf(dz, o3.z, fmaf(dy, o3.y, dx * o3.x))) - o2.w, 0.0f);
+    return e0 * e0 + e1 * e1 + e2 * e2;
+  }
+
+  // Nearest block to the tile's centre, or near enough to it: a depth-first search, nearest child
+  // first, that gives up after kSearchVisits nodes.
+  __device__ __forceinline__ void search() {
+    const float4 c = m.centre;
+    const int lb = m.t.block_log2, sub = lane & ((1 << lb) - 1);
+    uint32_t cur = root(), seed = 0, bound = ~0u;  // bound: float bits of the squared distance found
+    int sp = 0;
+    for (int visits = 0; visits < kSearchVisits; ++visits) {
+      const int level = static_cast<int>(cur >> 28) - 1;
+      const uint32_t first = (cur & 0x0fffffffu) * 32, child = first + lane;
+      const bool valid = child < m.level_n[level];
+      float d2 = kInf;
+      if (valid) {
+        if (level == 0) {
+          d2 = obb_dist2(child);
+        } else {
+          const float4 *b = m.t.box + 2 * size_t(m.level_off[level] + child);
+          const float4 bc = __ldg(b), be = __ldg(b + 1);
+          d2 = box_dist2(c.x, c.y, c.z, bc.x, bc.y, bc.z, be.x, be.y, be.z);
+        }
+      }
+      const bool kept = valid && __float_as_uint(d2) < bound;
+      const uint32_t mask = __ballot_sync(kFull, kept);
+      if (mask) {
+        const int nl = __reduce_min_sync(kFull, kept ? (__float_as_uint(d2) & ~31u) | lane : ~0u) & 31;
+        const int cnt = __popc(mask), rank = __popc(mask & ((1u << lane) - 1u)) - (lane > nl ? 1 : 0);
+        if (level > 0) {
+          if (kept && lane != nl && sp + rank < kStackSize) m.stack[sp + rank] = static_cast<uint32_t>(level) << 28 | child;
+          sp = min(sp + cnt - 1, kStackSize);
+          cur = static_cast<uint32_t>(level) << 28 | (first + nl);
+          __syncwarp();
+          continue;
+        }
+        if (kept) m.blocks[lane == nl ? 0 : rank + 1] = child;
+        __syncwarp();
+        for (int base = 0; base < cnt; base += kWarp >> lb) {
+          const uint32_t blk = m.blocks[min(base + (lane >> lb), cnt - 1)];
+          const float4 *tri = tree_tri(m.t.tri, (size_t(blk) << lb) + sub);
+          const float e = tri_dist2(__ldg(tri), __ldg(tri + kTriPlane), __ldg(tri + 2 * kTriPlane),
+                                    __ldg(tri + 3 * kTriPlane), __ldg(tri + 4 * kTriPlane), c.x, c.y, c.z);
+          const uint32_t key = __reduce_min_sync(kFull, (__float_as_uint(fminf(e, 1e38f)) & ~31u) | lane);
+          if ((key | 31u) < bound) {
+            bound = key | 31u;
+            seed = __shfl_sync(kFull, blk, key & 31);
+          }
+        }
+        __syncwarp();
+      }
+      if (sp == 0) break;
+      cur = m.stack[--sp];
+    }
+    __syncwarp();
+    if (lane == 0) m.seed = seed;
+    __syncwarp();
+  }
+
+  // Starts the bounds from one triangle of the seed block.
+  __device__ __forceinline__ void start() {
+    const float4 *tri = tree_tri(m.t.tri, size_t(m.seed) << m.t.block_log2);
+    const float4 q0 = __ldg(tri), q1 = __ldg(tri + kTriPlane), q2 = __ldg(tri + 2 * kTriPlane),
+                 q3 = __ldg(tri + 3 * kTriPlane), q4 = __ldg(tri + 4 * kTriPlane);
+#pragma unroll
+    for (int v = 0; v < VPL; ++v)
+      best[v * kWarp + lane] = __float_as_uint(fminf(tri_dist2(q0, q1, q2, q3, q4, px, py, pz[v]), 1e38f));
+    if (lane < 3) m.seed_at[lane] = lane == 0 ? m.centre.x : (lane == 1 ? m.centre.y : m.centre.z);
+    if (COUNT) ws.tri_tests += kWarp * VPL;
+    __syncwarp();
+  }
+
+  // Walks below node `cur` ((level << 28) | node). Returns false when the tail check stopped it with
+  // work left (the bounds are then upper bounds); a walk past its step limit raises the corrupt flag.
+  __device__ __forceinline__ bool walk(uint32_t cur, TailCheck tail, WalkLimits lim) {
+    int sp = 0, nb = 0;
+    int next_check = tail.every > 0 ? tail.every : INT_MAX;
+    steps = 0;
+    for (int visits = 0;; ++visits, steps += kStepsPerVisit) {
+      if (visits > lim.visits) {
         ws.corrupt = true;
         return true;
       }
-      const Node *np = nodes + (e >> 1);
-      const float4 n0 = __ldg(&np->n0), n1 = __ldg(&np->n1), n2 = __ldg(&np->n2);
-      const int4 n3 = __ldg(&np->n3);
-      float cx, cy, cz, ex, ey, ez;  // the popped child's box: centre and half extent
-      int ref, cnt;
-      if (e & 1) {
-        cx = n1.z; cy = n1.w; cz = n2.x; ex = n2.y; ey = n2.z; ez = n2.w;
-        ref = n3.y; cnt = n3.w;
+      if (steps >= next_check) {
+        unsigned long long handed = 0;
+        if (lane == 0) handed = *reinterpret_cast<const volatile unsigned long long *>(tail.counter);
+        handed = __shfl_sync(kFull, handed, 0);
+        if (handed >= tail.total) return false;
+        next_check = steps + tail.every;
+      }
+      const int level = static_cast<int>(cur >> 28) - 1;  // the children's level
+      const uint32_t child = (cur & 0x0fffffffu) * 32 + lane;
+      const bool valid = child < m.level_n[level];
+      bool kept;
+      float d2;
+      const float4 c = m.centre;
+      if (level > 0) {
+        const float4 *b = m.t.box + 2 * size_t(m.level_off[level] + (valid ? child : 0));
+        const float4 bc = __ldg(b), be = __ldg(b + 1);
+        const float tx = c.x - bc.x, ty = c.y - bc.y, tz = c.z - bc.z;
+        const float ax = fabsf(tx), ay = fabsf(ty), az = fabsf(tz);
+        const float ex = fmaxf(ax - be.x, 0.0f), ey = fmaxf(ay - be.y, 0.0f), ez = fmaxf(az - be.z, 0.0f);
+        const float fx = fminf(ax, be.x) + be.x, fy = fminf(ay, be.y) + be.y, fz = fminf(az, be.z) + be.z;
+        d2 = ex * ex + ey * ey + ez * ez;
+        kept = near(c.w, copysignf(ex, tx), copysignf(ey, ty), copysignf(ez, tz), d2, fx * fx + fy * fy + fz * fz,
+                    ax + ay + az + be.x + be.y + be.z);
+        if (COUNT) ws.box_tests += kWarp;
       } else {
-        cx = n0.x; cy = n0.y; cz = n0.z; ex = n0.w; ey = n1.x; ez = n1.y;
-        ref = n3.x; cnt = n3.z;
+        const float4 *o = tree_obb(m.t.obb, valid ? child : 0);
+        const float4 o0 = __ldg(o), o1 = __ldg(o + kObbPlane), o2 = __ldg(o + 2 * kObbPlane),
+                     o3 = __ldg(o + 3 * kObbPlane);
+        const float dx = c.x - o0.x, dy = c.y - o0.y, dz = c.z - o0.z;
+        const float t0 = fmaf(dz, o1.z, fmaf(dy, o1.y, dx * o1.x)), t1 = fmaf(dz, o2.z, fmaf(dy, o2.y, dx * o2.x)),
+                    t2 = fmaf(dz, o3.z, fmaf(dy, o3.y, dx * o3.x));
+        const float a0 = fabsf(t0), a1 = fabsf(t1), a2 = fabsf(t2);
+        const float e0 = copysignf(fmaxf(a0 - o0.w, 0.0f), t0), e1 = copysignf(fmaxf(a1 - o1.w, 0.0f), t1),
+                    e2 = copysignf(fmaxf(a2 - o2.w, 0.0f), t2);
+        const float f0 = fminf(a0, o0.w) + o0.w, f1 = fminf(a1, o1.w) + o1.w, f2 = fminf(a2, o2.w) + o2.w;
+        d2 = e0 * e0 + e1 * e1 + e2 * e2;
+        kept = near(c.w, fmaf(e2, o3.x, fmaf(e1, o2.x, e0 * o1.x)), fmaf(e2, o3.y, fmaf(e1, o2.y, e0 * o1.y)),
+                    fmaf(e2, o3.z, fmaf(e1, o2.z, e0 * o1.z)), d2, f0 * f0 + f1 * f1 + f2 * f2,
+                    a0 + a1 + a2 + o0.w + o1.w + o2.w);
+        if (COUNT) ws.plane_tests += kWarp;
       }
-      bool want = false;
-#pragma unroll
-      for (int v = 0; v < VPL; ++v) want |= box_dist2(px, py, pz[v], cx, cy, cz, ex, ey, ez) < best[v];
-      if (COUNT) ws.box_tests += kWarp * VPL;
-      if (!__any_sync(kFull, want)) continue;
-      if (cnt > 0) test_leaf<VPL, COUNT>(tris, num_tris, ref, cnt, px, py, pz, best, ws);
-      else cur = ref;
-      continue;
-    }
-    const int node = cur;
-    const Node *np = nodes + node;
-    const float4 n0 = __ldg(&np->n0), n1 = __ldg(&np->n1), n2 = __ldg(&np->n2);
-    const int4 n3 = __ldg(&np->n3);
-    // Only the votes stay live: when the near child is a leaf, the far child's box is read again
-    // (an L1 hit) and re-tested after it, which keeps the per-cell distances out of the registers
-    // across the leaf test (fewer spills: 64-mesh batch 249 -> 244 ms).
-    bool w0 = false, w1 = false;
-#pragma unroll
-    for (int v = 0; v < VPL; ++v) {
-      w0 |= box_dist2(px, py, pz[v], n0.x, n0.y, n0.z, n0.w, n1.x, n1.y) < best[v];
-      w1 |= box_dist2(px, py, pz[v], n1.z, n1.w, n2.x, n2.y, n2.z, n2.w) < best[v];
-    }
-    if (COUNT) ws.box_tests += 2 * kWarp * VPL;
-    w0 = __any_sync(kFull, w0) && n3.z >= 0;
-    w1 = __any_sync(kFull, w1) && n3.w >= 0;
-    // Near child first: the one whose box centre is nearer the tile's centre (the same on every
-    // lane). The centres order the children where the tile lies inside both boxes, as near the
-    // top of the tree; the box distances tie there (3-7% fewer tests than ordering by them).
-    const float q0x = tcx - n0.x, q0y = tcy - n0.y, q0z = tcz - n0.z;
-    const float q1x = tcx - n1.z, q1y = tcy - n1.w, q1z = tcz - n2.x;
-    const bool second_first = q1x * q1x + q1y * q1y + q1z * q1z < q0x * q0x + q0y * q0y + q0z * q0z;
-    const int near_ref = second_first ? n3.y : n3.x, near_cnt = second_first ? n3.w : n3.z;
-    const int far_ref = second_first ? n3.x : n3.y, far_cnt = second_first ? n3.z : n3.w;
-    bool near_w = second_first ? w1 : w0, far_w = second_first ? w0 : w1;
-    cur = -1;
-    if (near_w && near_cnt == 0) {
-      cur = near_ref;
-      if (far_w) {
-        if (sp < lim.stack) {
-          const int e = (node << 1) | (second_first ? 0 : 1);
-          if (STACK == 32 || sp < 32) {
-            if (lane == sp) stk0 = e;
-          } else if (lane == sp - 32) {
-            stk1 = e;
+      kept = kept && valid;
+      const uint32_t mask = __ballot_sync(kFull, kept);
+      if (mask) {
+        // The nearest child goes first: it is walked next, or leads the list of blocks.
+        const uint32_t near_key = __reduce_min_sync(kFull, kept ? (__float_as_uint(d2) & ~31u) | lane : ~0u);
+        const int nl = near_key & 31;
+        const int cnt = __popc(mask);
+        const int rank = __popc(mask & ((1u << lane) - 1u)) - (lane > nl ? 1 : 0);  // among the others
+        if (level > 0) {
+          if (kept && lane != nl && sp + rank < lim.stack)
+            m.stack[sp + rank] = (static_cast<uint32_t>(level) << 28) | child;
+          sp += cnt - 1;
+          if (sp > lim.stack) {
+            ws.overflow = true;
+            sp = lim.stack;
           }
-          ++sp;
-        } else {
-          ws.overflow = true;
+          cur = (static_cast<uint32_t>(level) << 28) | ((cur & 0x0fffffffu) * 32 + nl);
+          __syncwarp();
+          continue;
         }
+        if (kept) m.blocks[nb + (lane == nl ? 0 : rank + 1)] = child;
+        nb += cnt;
+        __syncwarp();
+        if (nb >= kFlushAt) flush(nb);
       }
-      continue;
+      if (sp == 0) break;
+      cur = m.stack[--sp];
     }
-    if (near_w) {
-      test_leaf<VPL, COUNT>(tris, num_tris, near_ref, near_cnt, px, py, pz, best, ws);
-      if (far_w) {
-        bool w = false;
-        const Node *fp = nodes + node;
-        const float4 f0 = __ldg(&fp->n0), f1 = __ldg(&fp->n1), f2 = __ldg(&fp->n2);
-#pragma unroll
-        for (int v = 0; v < VPL; ++v)
-          w |= (second_first ? box_dist2(px, py, pz[v], f0.x, f0.y, f0.z, f0.w, f1.x, f1.y)
-                             : box_dist2(px, py, pz[v], f1.z, f1.w, f2.x, f2.y, f2.z, f2.w)) < best[v];
-        far_w = __any_sync(kFull, w);
-      }
-    }
-    if (far_w) {
-      if (far_cnt > 0) test_leaf<VPL, COUNT>(tris, num_tris, far_ref, far_cnt, px, py, pz, best, ws);
-      else cur = far_ref;
-    }
+    if (nb > 0) flush(nb);
+    return true;
   }
-}
+};
 
 // Signs (parity) and writes a tile's distances.
 template <int TX, int TY, int TZ>
-__device__ __forceinline__ void store_cells(const DistanceArgs &a, const TileCells<TX, TY, TZ> &c,
-                                            const float (&best)[TileCells<TX, TY, TZ>::VPL]) {
+__device__ __forceinline__ void store_cells(const DistanceArgs &a, const TileCells<TX, TY, TZ> &c, int lane,
+                                            const uint32_t *best) {
   constexpr int VPL = TileCells<TX, TY, TZ>::VPL;
   const MeshRec &M = *c.M;
   int inside[VPL];
 #pragma unroll
   for (int v = 0; v < VPL; ++v) inside[v] = 0;
-  if (M.sign == kSignParity && c.vx < c.g.nx && c.vy < c.g.ny) {
-    const uint64_t col = M.col_base + uint64_t(c.vy) * c.g.nx + c.vx;
+  const int vx = c.vx(lane), vy = c.vy(lane);
+  if (M.sign == kSignParity && vx < c.g.nx && vy < c.g.ny) {
+    const uint64_t col = M.col_base + uint64_t(vy) * c.g.nx + vx;
     const uint64_t s0 = __ldg(a.col_start + col), s1 = __ldg(a.col_start + col + 1);
     for (uint64_t k = s0; k < s1; ++k) {
       const float zc = __ldg(a.col_z + k);
 #pragma unroll
-      for (int v = 0; v < VPL; ++v) inside[v] ^= zc > c.pz[v] ? 1 : 0;
+      for (int v = 0; v < VPL; ++v) inside[v] ^= zc > c.pz(lane, v) ? 1 : 0;
     }
   }
 #pragma unroll
   for (int v = 0; v < VPL; ++v) {
-    if (!c.active[v]) continue;
-    const float d = sqrtf(best[v]);
-    M.dist[c.cell(v)] = inside[v] ? -d : d;
+    if (!c.active(lane, v)) continue;
+    const float d = sqrtf(__uint_as_float(best[v * kWarp + lane]));
+    M.dist[c.cell(lane, v)] = inside[v] ? -d : d;
   }
 }
 
@@ -384,18 +659,24 @@ __device__ unsigned long long next_tile(unsigned long long *state, unsigned long
 
 // Pass A: warps take tiles from their block's chunk, blocks take chunks from a global counter; a
 // tile still walking in the pass's tail (every chunk handed out) is deferred to pass B.
-template <int TX, int TY, int TZ, int STACK, bool COUNT>
+template <int TX, int TY, int TZ, bool COUNT>
 __global__ __launch_bounds__(kThreadsA, kMinBlocksA) void k_distance(DistanceArgs a) {
-  using Cells = TileCells<TX, TY, TZ>;
-  constexpr int VPL = Cells::VPL;
-  const int lane = threadIdx.x & 31;
+  using W = Walker<TX, TY, TZ, COUNT>;
+  constexpr int VPL = W::VPL;
+  __shared__ unsigned long long s_state;
+  __shared__ WarpMem s_mem[kWarpsPerBlockA];
+  __shared__ uint32_t s_best[kWarpsPerBlockA][VPL * kWarp];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const BatchDev &B = a.batch;
-  WalkStats ws;
   const unsigned long long total_chunks = (B.total_tiles + a.chunk_tiles - 1) / a.chunk_tiles;
   TailCheck tail{a.tile_counter, total_chunks,
-                 (a.defer_list && a.step_budget > 0) ? static_cast<int>(min(a.step_budget, 1ll << 30)) : 0};
+                 (a.defer_list && a.step_budget > 0)
+                     ? static_cast<int>(min(a.step_budget, 1ll << 30))
+                     : 0};
   const TailCheck never{nullptr, 0, 0};
-  __shared__ unsigned long long s_state;
+  W w(s_mem[warp], s_best[warp], lane);
+  uint32_t mesh = ~0u;
+  if (lane == 0) w.m.mesh = ~0u;
   if (threadIdx.x == 0) s_state = atomicAdd(a.tile_counter, 1ull) << 32;
   __syncthreads();
 
@@ -405,37 +686,26 @@ __global__ __launch_bounds__(kThreadsA, kMinBlocksA) void k_distance(DistanceArg
       tile = next_tile(&s_state, a.tile_counter, a.chunk_tiles, total_chunks, B.total_tiles, a.err, a.fault);
     tile = __shfl_sync(kFull, tile, 0);
     if (tile == kNoTile) break;
-    // Only what the walk reads stays live across it; the tile's cell indices, activity and output
-    // pointer are located again afterwards.
-    float best[VPL], px, py, pz[VPL], tcx, tcy, tcz;
-    const Node *nodes;
-    const DistTri *tris;
-    int bvh_nodes, bvh_tris, root;
+    WalkLimits lim;
     {
-      Cells c0;
-      c0.locate(B, tile, lane);
-#pragma unroll
-      for (int v = 0; v < VPL; ++v) {
-        best[v] = c0.active[v] ? kInf : -1.0f;
-        pz[v] = c0.pz[v];
+      typename W::Cells c;
+      if (!c.locate(B, tile)) continue;
+      const uint32_t index = static_cast<uint32_t>(c.M - B.recs);
+      const bool first = index != mesh;
+      if (first) {
+        mesh = index;
+        w.set_tree(c.M->tree, mesh);
       }
-      px = c0.px;
-      py = c0.py;
-      tcx = c0.cx;
-      tcy = c0.cy;
-      tcz = c0.cz;
-      nodes = c0.M->nodes;
-      tris = c0.M->tris;
-      bvh_nodes = c0.M->bvh_nodes;
-      bvh_tris = c0.M->bvh_tris;
-      root = c0.M->root;
+      lim = walk_limits(c.M->tree, a.stack_depth, a.fault);
+      w.set_tile(c);
+      w.pick_seed(s_mem, kWarpsPerBlockA);
     }
-    const WalkLimits lim = walk_limits<STACK>(bvh_nodes, a.fault);
-    bool done = walk<VPL, STACK, COUNT>(nodes, tris, bvh_nodes, bvh_tris, root, tail, lim, lane, tcx, tcy, tcz, px, py,
-                                        pz, best, ws);
-    Cells c;
-    c.locate(B, tile, lane);
-    const MeshRec &M = *c.M;
+    w.start();
+    w.fit();
+    bool done = w.walk(w.root(), tail, lim);
+    // The tile's indices are located again rather than kept in registers across the walk.
+    typename W::Cells c;
+    c.locate(B, tile);
     if (!done) {
       unsigned long long slot = 0;
       if (lane == 0) slot = atomicAdd(a.defer_counters, 1ull);
@@ -444,32 +714,36 @@ __global__ __launch_bounds__(kThreadsA, kMinBlocksA) void k_distance(DistanceArg
         if (lane == 0) a.defer_list[slot] = tile;
 #pragma unroll
         for (int v = 0; v < VPL; ++v)
-          if (c.active[v]) M.dist[c.cell(v)] = best[v];  // the bounds pass B starts from
+          if (c.active(lane, v))
+            c.M->dist[c.cell(lane, v)] = __uint_as_float(w.best[v * kWarp + lane]);  // pass B starts from these
         continue;
       }
       // The list is full: finish the tile here, from the bounds found so far.
-      walk<VPL, STACK, COUNT>(M.nodes, M.tris, M.bvh_nodes, M.bvh_tris, M.root, never, lim, lane, c.cx, c.cy, c.cz,
-                              c.px, c.py, c.pz, best, ws);
+      w.fit();
+      w.walk(w.root(), never, lim);
     }
-    store_cells<TX, TY, TZ>(a, c, best);
+    __syncwarp();
+    store_cells<TX, TY, TZ>(a, c, lane, w.best);
+    __syncwarp();
   }
-  flush_stats<COUNT>(a, ws, lane);
+  flush_stats<COUNT>(a, w.ws, lane);
 }
 
 // Pass B: one block per deferred tile; its warps share the tile's subtrees and bounds.
-template <int TX, int TY, int TZ, int STACK, bool COUNT>
+template <int TX, int TY, int TZ, bool COUNT>
 __global__ __launch_bounds__(kThreads) void k_distance_deferred(DistanceArgs a) {
-  using Cells = TileCells<TX, TY, TZ>;
-  constexpr int VPL = Cells::VPL;
-  constexpr int kItems = 1 << kSplitBits;
+  using W = Walker<TX, TY, TZ, COUNT>;
+  constexpr int VPL = W::VPL;
   __shared__ unsigned long long s_tile;
-  __shared__ int s_item;
+  __shared__ uint32_t s_item;
+  __shared__ WarpMem s_mem[kWarpsPerBlockB];
   __shared__ uint32_t s_best[VPL * kWarp];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const BatchDev &B = a.batch;
-  WalkStats ws;
   const unsigned long long count = a.defer_counters[0];
   const unsigned long long total = count < a.defer_capacity ? count : a.defer_capacity;
+  W w(s_mem[warp], s_best, lane);
+  uint32_t mesh = ~0u;
 
   for (;;) {
     if (threadIdx.x == 0) {
@@ -480,84 +754,36 @@ __global__ __launch_bounds__(kThreads) void k_distance_deferred(DistanceArgs a) 
     __syncthreads();
     const unsigned long long tile = s_tile;
     if (tile == ~0ull) break;
-    Cells c;
-    c.locate(B, tile, lane);
-    const MeshRec &M = *c.M;
-    float best[VPL];
-#pragma unroll
-    for (int v = 0; v < VPL; ++v) {
-      best[v] = c.active[v] ? M.dist[c.cell(v)] : -1.0f;
-      if (warp == 0) s_best[v * kWarp + lane] = __float_as_uint(c.active[v] ? best[v] : 0.0f);
+    typename W::Cells c;
+    c.locate(B, tile);
+    if (static_cast<uint32_t>(c.M - B.recs) != mesh) {
+      mesh = static_cast<uint32_t>(c.M - B.recs);
+      w.set_tree(c.M->tree, mesh);
     }
-    __syncthreads();
-    for (;;) {
-      int item = 0;
-      if (lane == 0) item = atomicAdd(&s_item, 1);
-      item = __shfl_sync(kFull, item, 0);
-      if (item >= kItems) break;
-#pragma unroll
-      for (int v = 0; v < VPL; ++v)
-        if (c.active[v]) best[v] = fminf(best[v], __uint_as_float(s_best[v * kWarp + lane]));
-      // Descend to this item's subtree: each node with two children consumes one bit of the item
-      // (most significant first); a leaf reached early is tested by the item whose remaining bits
-      // are all zero.
-      int cur = M.root, bits = kSplitBits;
-      bool walk_it = false;
-      for (int guard = 0; guard < 64; ++guard) {
-        if (bits == 0) {
-          walk_it = true;
-          break;
-        }
-        if (cur < 0 || cur >= M.bvh_nodes) {
-          ws.corrupt = true;
-          break;
-        }
-        const Node *np = M.nodes + cur;
-        const float4 n0 = __ldg(&np->n0), n1 = __ldg(&np->n1), n2 = __ldg(&np->n2);
-        const int4 n3 = __ldg(&np->n3);
-        const bool e0 = n3.z < 0, e1 = n3.w < 0;
-        if (e0 && e1) break;
-        int which;
-        if (!e0 && !e1) {
-          --bits;
-          which = (item >> bits) & 1;
-        } else {
-          which = e0 ? 1 : 0;
-        }
-        bool want = false;
-#pragma unroll
-        for (int v = 0; v < VPL; ++v) {
-          const float d = which ? box_dist2(c.px, c.py, c.pz[v], n1.z, n1.w, n2.x, n2.y, n2.z, n2.w)
-                                : box_dist2(c.px, c.py, c.pz[v], n0.x, n0.y, n0.z, n0.w, n1.x, n1.y);
-          want |= d < best[v];
-        }
-        if (COUNT) ws.box_tests += kWarp * VPL;
-        if (!__any_sync(kFull, want)) break;
-        const int ref = which ? n3.y : n3.x, cnt = which ? n3.w : n3.z;
-        if (cnt > 0) {
-          if ((item & ((1 << bits) - 1)) == 0)
-            test_leaf<VPL, COUNT>(M.tris, M.bvh_tris, ref, cnt, c.px, c.py, c.pz, best, ws);
-          break;
-        }
-        cur = ref;
-      }
-      if (walk_it)
-        walk<VPL, STACK, COUNT>(M.nodes, M.tris, M.bvh_nodes, M.bvh_tris, cur, TailCheck{nullptr, 0, 0},
-                                walk_limits<STACK>(M.bvh_nodes, a.fault), lane, c.cx, c.cy, c.cz, c.px, c.py, c.pz,
-                                best, ws);
-#pragma unroll
-      for (int v = 0; v < VPL; ++v)
-        if (c.active[v]) atomicMin(&s_best[v * kWarp + lane], __float_as_uint(best[v]));
-    }
-    __syncthreads();
+    w.set_tile(c);
     if (warp == 0) {
 #pragma unroll
-      for (int v = 0; v < VPL; ++v) best[v] = c.active[v] ? __uint_as_float(s_best[v * kWarp + lane]) : -1.0f;
-      store_cells<TX, TY, TZ>(a, c, best);
+      for (int v = 0; v < VPL; ++v) s_best[v * kWarp + lane] = __float_as_uint(c.M->dist[c.cell(lane, v)]);
     }
     __syncthreads();
+    // The lowest level with few enough nodes: one subtree per node.
+    int level = 1;
+    while (w.m.level_n[level] > kMaxItems) ++level;
+    const uint32_t items = w.m.level_n[level];
+    const WalkLimits lim = walk_limits(c.M->tree, a.stack_depth, a.fault);
+    w.fit();
+    for (;;) {
+      uint32_t item = 0;
+      if (lane == 0) item = atomicAdd(&s_item, 1u);
+      item = __shfl_sync(kFull, item, 0);
+      if (item >= items) break;
+      w.walk((static_cast<uint32_t>(level) << 28) | item, TailCheck{nullptr, 0, 0}, lim);
+    }
+    __syncthreads();
+    if (warp == 0) store_cells<TX, TY, TZ>(a, c, lane, s_best);
+    __syncthreads();
   }
-  flush_stats<COUNT>(a, ws, lane);
+  flush_stats<COUNT>(a, w.ws, lane);
 }
 
 template <typename K>
@@ -567,49 +793,45 @@ int blocks_per_sm(K kernel, int threads) {
   return per_sm > 0 ? per_sm : 1;
 }
 
-template <int I, int STACK, bool COUNT>
+template <int I, bool COUNT>
 cudaError_t launch_shape(const DistanceArgs &a, int num_sms, cudaStream_t st) {
   constexpr Shape s = kShapes[I];
-  static const int per_sm = blocks_per_sm(k_distance<s.tx, s.ty, s.tz, STACK, COUNT>, kThreadsA);
-  static const int per_sm_b = blocks_per_sm(k_distance_deferred<s.tx, s.ty, s.tz, STACK, COUNT>, kThreads);
+  static const int per_sm = blocks_per_sm(k_distance<s.tx, s.ty, s.tz, COUNT>, kThreadsA);
+  static const int per_sm_b = blocks_per_sm(k_distance_deferred<s.tx, s.ty, s.tz, COUNT>, kThreads);
   const unsigned long long warps_needed = a.batch.total_tiles;
   unsigned long long blocks = static_cast<unsigned long long>(num_sms) * per_sm;
   blocks = std::min<unsigned long long>(blocks, (warps_needed + kWarpsPerBlockA - 1) / kWarpsPerBlockA);
   if (blocks < 1) blocks = 1;
   // kChunkMax tiles per chunk when there are plenty, fewer when the tiles would not reach every
-  // warp several times over. Pass A uses no shared memory to speak of: all of it goes to L1.
-  static const bool carveout = cudaFuncSetAttribute(k_distance<s.tx, s.ty, s.tz, STACK, COUNT>,
-                                                    cudaFuncAttributePreferredSharedMemoryCarveout,
-                                                    cudaSharedmemCarveoutMaxL1) == cudaSuccess;
-  (void)carveout;
+  // warp several times over.
   DistanceArgs ca = a;
   ca.chunk_tiles = std::max<unsigned long long>(
       1, std::min<unsigned long long>(kChunkMax, a.batch.total_tiles / (blocks * kWarpsPerBlockA * 4)));
   cudaError_t e = cudaMemsetAsync(a.tile_counter, 0, sizeof(unsigned long long), st);
   if (e == cudaSuccess && a.defer_list) e = cudaMemsetAsync(a.defer_counters, 0, 2 * sizeof(unsigned long long), st);
   if (e != cudaSuccess) return e;
-  k_distance<s.tx, s.ty, s.tz, STACK, COUNT><<<static_cast<unsigned>(blocks), kThreadsA, 0, st>>>(ca);
+  k_distance<s.tx, s.ty, s.tz, COUNT><<<static_cast<unsigned>(blocks), kThreadsA, 0, st>>>(ca);
   note_launch();
   e = cudaGetLastError();
   if (e != cudaSuccess || !a.defer_list || a.step_budget <= 0) return e;
   // Pass B: a persistent grid; the number of deferred tiles is read on the device.
   const unsigned long long blocks_b =
       std::min<unsigned long long>(static_cast<unsigned long long>(num_sms) * per_sm_b, a.defer_capacity);
-  k_distance_deferred<s.tx, s.ty, s.tz, STACK, COUNT>
+  k_distance_deferred<s.tx, s.ty, s.tz, COUNT>
       <<<static_cast<unsigned>(std::max<unsigned long long>(blocks_b, 1)), kThreads, 0, st>>>(a);
   note_launch();
   return cudaGetLastError();
 }
 
-template <int STACK, bool COUNT>
+template <bool COUNT>
 cudaError_t launch_any(const DistanceArgs &a, int id, int num_sms, cudaStream_t st) {
   switch (id) {
-    case 0: return launch_shape<0, STACK, COUNT>(a, num_sms, st);
-    case 1: return launch_shape<1, STACK, COUNT>(a, num_sms, st);
-    case 2: return launch_shape<2, STACK, COUNT>(a, num_sms, st);
-    case 3: return launch_shape<3, STACK, COUNT>(a, num_sms, st);
-    case 4: return launch_shape<4, STACK, COUNT>(a, num_sms, st);
-    default: return launch_shape<5, STACK, COUNT>(a, num_sms, st);
+    case 0: return launch_shape<0, COUNT>(a, num_sms, st);
+    case 1: return launch_shape<1, COUNT>(a, num_sms, st);
+    case 2: return launch_shape<2, COUNT>(a, num_sms, st);
+    case 3: return launch_shape<3, COUNT>(a, num_sms, st);
+    case 4: return launch_shape<4, COUNT>(a, num_sms, st);
+    default: return launch_shape<5, COUNT>(a, num_sms, st);
   }
 }
 
@@ -644,14 +866,10 @@ uint64_t defer_capacity_for(uint64_t total_tiles) {
   return std::min<uint64_t>(total_tiles, std::max<uint64_t>(4096, total_tiles / 8));
 }
 
-cudaError_t distance_launch(const DistanceArgs &a, int tile_id, int stack_depth, int num_sms, cudaStream_t st) {
+cudaError_t distance_launch(const DistanceArgs &a, int tile_id, int num_sms, cudaStream_t st) {
   if (a.batch.total_tiles == 0) return cudaSuccess;
-  if (stack_depth <= 32) {
-    if (a.work_counters) return launch_any<32, true>(a, tile_id, num_sms, st);
-    return launch_any<32, false>(a, tile_id, num_sms, st);
-  }
-  if (a.work_counters) return launch_any<64, true>(a, tile_id, num_sms, st);
-  return launch_any<64, false>(a, tile_id, num_sms, st);
+  if (a.work_counters) return launch_any<true>(a, tile_id, num_sms, st);
+  return launch_any<false>(a, tile_id, num_sms, st);
 }
 
 }  // namespace sdfb

@@ -13,7 +13,6 @@
 namespace sdfb {
 
 struct TriRec;
-struct DistTri;
 struct Node;
 
 // Count of kernel launches issued by this library (every launcher calls note_launch once per
@@ -47,6 +46,42 @@ struct GridDev {
   int nx, ny, nz;
 };
 
+// One mesh's packed tree as the distance walk reads it (ptree.cu).
+struct DistTree {
+  const float4 *tri;    // DistTri records: groups of kTriPlane triangles, five planes of float4s each
+  const float4 *obb;    // oriented boxes of the blocks: groups of kObbPlane boxes, four planes each
+  const float4 *box;    // boxes of the nodes above (centre, half extent), level 1 first
+  uint32_t num_tris;
+  int block_log2;       // a block is 2^block_log2 triangles
+};
+
+// First plane of a triangle record or of a block's box; plane p is p * kTriPlane (kObbPlane) float4s
+// on, so consecutive records coalesce and one address serves all planes.
+constexpr int kTriPlane = 8, kObbPlane = 32;
+template <typename F4> __host__ __device__ __forceinline__ F4 *tree_tri(F4 *tri, size_t k) {
+  return tri + (k / kTriPlane) * (5 * kTriPlane) + k % kTriPlane;
+}
+template <typename F4> __host__ __device__ __forceinline__ F4 *tree_obb(F4 *obb, size_t b) {
+  return obb + (b / kObbPlane) * (4 * kObbPlane) + b % kObbPlane;
+}
+
+constexpr int kTreePad = 256;   // triangle slots of a mesh are padded to this
+constexpr int kTreeSizes = 3;   // block sizes that can be built: 2, 4, 8 (index k: 2 << k)
+
+// Nodes of a level of a packed tree: level 0 are the blocks.
+__host__ __device__ __forceinline__ uint32_t tree_level_count(uint32_t tris, int block_log2, int level) {
+  uint64_t n = (uint64_t(tris) + (1u << block_log2) - 1) >> block_log2;
+  for (int l = 0; l < level; ++l) n = (n + 31) >> 5;
+  return static_cast<uint32_t>(n);
+}
+
+// One mesh's packed tree as the build writes it: obb[k] / box[k] are null for block sizes not built.
+struct PTreeRec {
+  float4 *tri;
+  float4 *obb[kTreeSizes], *box[kTreeSizes];
+  uint32_t slots, num_tris;  // triangle slots: num_tris padded to kTreePad
+};
+
 enum SignKind : int { kSignNone = 0, kSignParity = 1, kSignGwn = 2 };
 
 // Device-side record of one mesh of a batch.
@@ -64,16 +99,12 @@ struct MeshRec {
   GridDev g;
   int sign;               // SignKind
   int leaf_size;          // 1..16
-  int root;               // virtual root node of this mesh (see lbvh.cu)
+  int pad;
   int cap_root;           // GWN: virtual root of this mesh's caps in the caps hierarchy, -1 if none
   const float *cverts;    // GWN: vertices of the caps (the parity mesh's vertices + loop centres)
   const uint32_t *cidx;   // GWN: cap triangles
   uint32_t cap_tris;      // GWN: number of cap triangles
-  int bvh_nodes;          // node count of the hierarchy holding this mesh (root < bvh_nodes)
-  // The hierarchy holding this mesh: the batch's combined tree, or the mesh's resident tree.
-  const Node *nodes;
-  const DistTri *tris;
-  int bvh_tris;           // records in that hierarchy
+  DistTree tree;          // the mesh's packed tree
   // GWN: the hierarchy holding this mesh's caps
   int cap_nodes_n, cap_inner_n, cap_recs_n;
   const Node *cap_nodes;
@@ -105,27 +136,35 @@ __host__ __device__ __forceinline__ int find_mesh(const uint64_t *starts, int n,
   return lo;
 }
 
+// ---- ptree.cu ---------------------------------------------------------------------------------
+// The distance hierarchies of a batch: one packed tree per mesh, each in its own region of memory.
+size_t ptree_temp_bytes(uint64_t total_tris, int num_meshes);
+// Bytes of one mesh's tree with the block sizes of `mask` (bit k: 2 << k triangles); fills `out` with
+// its arrays when the region's base address is given.
+size_t ptree_layout(uint32_t tris, int mask, char *base, PTreeRec *out);
+// trees and group_starts (one entry per mesh and the total; a group is kTreePad slots) are device
+// tables beside the batch's.
+cudaError_t ptree_build(const BatchDev &batch, const PTreeRec *trees, const uint64_t *group_starts, uint64_t groups,
+                        void *temp, size_t temp_bytes, uint32_t *err, cudaStream_t st);
+
 // ---- lbvh.cu ----------------------------------------------------------------------------------
-// The batch's acceleration structure: every mesh's triangles, sorted by (mesh, Morton code), under
-// one binary radix tree; each mesh's subtree is entered through its virtual root node, stored
-// after the inner nodes.
+// The winding number's hierarchy over the caps of a batch: every mesh's cap triangles, sorted by
+// (mesh, Morton code), under one binary radix tree; each mesh's subtree is entered through its
+// virtual root node, stored after the inner nodes.
 struct BvhDev {
-  DistTri *dtris = nullptr;        // distance hierarchy: T_total records in leaf order
-  TriRec *tris = nullptr;          // winding-number hierarchy: T_total records in leaf order
+  TriRec *tris = nullptr;          // T_total records in leaf order
   Node *nodes = nullptr;           // (T_total - 1) inner nodes + M virtual roots
   uint32_t *leaf_order = nullptr;  // local (per-mesh) triangle index of each record
   uint32_t *bounds = nullptr;      // 6 ordered-uint words per mesh: centroid min xyz, max xyz
-  float4 *node_moment = nullptr;   // winding-number hierarchy, per inner node: (sum of area x unit
-                                   // normal over its triangles, their total area)
+  float4 *node_moment = nullptr;   // per inner node: (sum of area x unit normal over its triangles,
+                                   // their total area)
   int num_inner = 0;               // max(T_total - 1, 0)
   int num_nodes = 0;               // num_inner + M
 };
 
 size_t lbvh_temp_bytes(uint64_t total_tris, int num_meshes);
-// winding = false: the distance hierarchy (DistTri records); true: the winding-number hierarchy
-// (TriRec records and per-node triangle areas).
-size_t lbvh_bytes(uint64_t total_tris, int num_meshes, bool winding);
-void lbvh_bind(BvhDev &b, void *mem, uint64_t total_tris, int num_meshes, bool winding);
+size_t lbvh_bytes(uint64_t total_tris, int num_meshes);
+void lbvh_bind(BvhDev &b, void *mem, uint64_t total_tris, int num_meshes);
 cudaError_t lbvh_build(const BatchDev &batch, BvhDev &b, void *temp, size_t temp_bytes, uint32_t *err,
                        cudaStream_t st);
 
@@ -154,7 +193,7 @@ struct DistanceArgs {
   unsigned long long chunk_tiles;     // tiles per chunk (set by the launcher)
   unsigned long long *work_counters;  // optional: [0] box, [1] triangle, [3] plane, [4] rectangle tests (lanes)
   // Deferral of long tiles (none when defer_list is null or step_budget <= 0): every step_budget
-  // traversal steps a walk checks whether all tiles have been handed out and, if so, defers its
+  // pairs of children measured a walk checks whether all tiles have been handed out and, if so, defers its
   // tile. The list holds defer_capacity tile indices; defer_counters[0] counts deferred tiles (it
   // may pass the capacity), [1] is the second pass's tile counter. Both counters are zeroed by the
   // launcher.
@@ -162,6 +201,7 @@ struct DistanceArgs {
   unsigned long long defer_capacity;
   unsigned long long *defer_counters;
   long long step_budget;
+  int stack_depth;  // sdfb_opts.stack_depth as used: only fault injection looks at it
   int fault;  // sdfb_opts.fault_inject bits (testing only; 0 in normal use)
 };
 
@@ -171,10 +211,9 @@ double distance_work_flops(int tile_id, const unsigned long long *counters);
 // tile shape id -> (tx, ty, tz)
 void tile_shape(int id, int &tx, int &ty, int &tz);
 uint64_t tiles_for(const GridDev &g, int tile_id);
-// stack_depth: 32 or 64 entries (32 keeps the stack in one register per lane).
 // Deferred-list capacity for a launch of total_tiles tiles.
 uint64_t defer_capacity_for(uint64_t total_tiles);
-cudaError_t distance_launch(const DistanceArgs &a, int tile_id, int stack_depth, int num_sms, cudaStream_t st);
+cudaError_t distance_launch(const DistanceArgs &a, int tile_id, int num_sms, cudaStream_t st);
 
 // Every (cell, triangle) pair of a ONE-mesh batch that passes the occupancy rule, as keys
 // (cell << tri_bits) | local triangle, appended in no particular order (the mesh's occupancy grid

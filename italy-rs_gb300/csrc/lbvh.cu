@@ -1,9 +1,8 @@
-// Device-built linear BVH over the triangles of a batch of meshes (replaces the OptiX GAS build
-// of src/convert/sdf_baker.cpp:170-193, which builds one acceleration structure per call).
+// Device-built linear BVH over the caps of a batch of meshes, for the winding number (gwn.cu); the
+// distance walk has its own tree (ptree.cu).
 //
 //   1. k_prep      gathers each indexed triangle of each mesh, checks indices and finiteness,
-//                  writes its box (and, for the winding-number hierarchy, its 64-byte record), and
-//                  reduces per-mesh centroid bounds.
+//                  writes its box and its 64-byte record, and reduces per-mesh centroid bounds.
 //   2. k_morton    key = (mesh << 30) | 30-bit Morton code of the box centre in its mesh's bounds.
 //   3. radix sort  (key, triangle) pairs, stable: meshes end up contiguous, each in Morton order.
 //   4. k_hierarchy binary radix tree over all keys (Karras 2012, "Maximizing Parallelism in the
@@ -15,10 +14,9 @@
 //   7. k_roots     one virtual root node per mesh, after the inner nodes, whose first child is
 //                  the mesh's subtree (or leaf) and whose second child is empty; traversal of a
 //                  mesh starts there.
-//   8. k_gather    triangle records in leaf order: 80-byte frame records (DistTri) for the
-//                  distance hierarchy, the k_prep records for the winding-number hierarchy.
-//   9. k_moments   (optional) per inner node the sum of area x unit normal of its triangles and
-//                  their total area (the winding number's far field, gwn.cu).
+//   8. k_gather    the k_prep records in leaf order.
+//   9. k_moments   per inner node the sum of area x unit normal of its triangles and their total
+//                  area (the winding number's far field).
 #include <algorithm>
 #include <cstdint>
 
@@ -113,7 +111,7 @@ __global__ __launch_bounds__(kThreads) void k_prep(BatchDev B, TriRec *__restric
     const bool finite = isfinite(a.x) && isfinite(a.y) && isfinite(a.z) && isfinite(b.x) && isfinite(b.y) &&
                         isfinite(b.z) && isfinite(c.x) && isfinite(c.y) && isfinite(c.z);
     if (!finite) atomic_or_err(err, kErrNonFinite);
-    if (rec) {
+    {
       const float e1x = b.x - a.x, e1y = b.y - a.y, e1z = b.z - a.z;
       const float e2x = c.x - a.x, e2y = c.y - a.y, e2z = c.z - a.z;
       const float e3x = c.x - b.x, e3y = c.y - b.y, e3z = c.z - b.z;
@@ -386,24 +384,12 @@ __global__ void k_roots(BatchDev B, int num_inner, const uint32_t *__restrict__ 
 
 __global__ __launch_bounds__(kThreads) void k_gather(BatchDev B, const uint32_t *__restrict__ vals,
                                                      const TriRec *__restrict__ rec, TriRec *__restrict__ out,
-                                                     DistTri *__restrict__ dout, uint32_t *__restrict__ order) {
+                                                     uint32_t *__restrict__ order) {
   const uint64_t k = uint64_t(blockIdx.x) * kThreads + threadIdx.x;
   if (k >= B.total_tris) return;
-  const uint32_t t = vals ? vals[k] : static_cast<uint32_t>(k);
-  const int mesh = find_mesh(B.tri_starts, B.num_meshes, t);
-  const uint64_t lt = t - B.tri_starts[mesh];
-  if (out) out[k] = rec[t];
-  if (dout) {
-    // The frame is built from the input vertices (k_prep has flagged bad indices already).
-    const MeshRec &M = B.recs[mesh];
-    const uint32_t V = M.num_verts;
-    uint32_t i0 = __ldg(M.idx + 3 * lt), i1 = __ldg(M.idx + 3 * lt + 1), i2 = __ldg(M.idx + 3 * lt + 2);
-    i0 = i0 < V ? i0 : 0;
-    i1 = i1 < V ? i1 : 0;
-    i2 = i2 < V ? i2 : 0;
-    dout[k] = make_dist_tri(load3(M.verts, i0), load3(M.verts, i1), load3(M.verts, i2));
-  }
-  order[k] = static_cast<uint32_t>(lt);
+  const uint32_t t = vals[k];
+  out[k] = rec[t];
+  order[k] = static_cast<uint32_t>(t - B.tri_starts[find_mesh(B.tri_starts, B.num_meshes, t)]);
 }
 
 // Far-field moments of every inner node, bottom-up like k_refit: (sum of a_i n_i, sum of a_i)
@@ -437,25 +423,24 @@ inline unsigned blocks_for(size_t n) { return static_cast<unsigned>((n + kThread
 
 size_t lbvh_temp_bytes(uint64_t total_tris, int num_meshes) { return temp_layout(total_tris, num_meshes, nullptr, nullptr); }
 
-size_t lbvh_bytes(uint64_t T, int M, bool winding) {
+size_t lbvh_bytes(uint64_t T, int M) {
   const size_t n = std::max<uint64_t>(T, 1), m = std::max<uint64_t>(T, 2) - 1;
-  return align256(n * (winding ? sizeof(TriRec) : sizeof(DistTri))) + align256((m + M) * sizeof(Node)) +
-         align256(n * 4) + align256(size_t(M) * 6 * 4) + (winding ? align256(m * sizeof(float4)) : 0);
+  return align256(n * sizeof(TriRec)) + align256((m + M) * sizeof(Node)) + align256(n * 4) +
+         align256(size_t(M) * 6 * 4) + align256(m * sizeof(float4));
 }
 
-void lbvh_bind(BvhDev &b, void *mem, uint64_t T, int M, bool winding) {
+void lbvh_bind(BvhDev &b, void *mem, uint64_t T, int M) {
   const size_t n = std::max<uint64_t>(T, 1), m = std::max<uint64_t>(T, 2) - 1;
   char *p = static_cast<char *>(mem);
-  b.tris = winding ? reinterpret_cast<TriRec *>(p) : nullptr;
-  b.dtris = winding ? nullptr : reinterpret_cast<DistTri *>(p);
-  p += align256(n * (winding ? sizeof(TriRec) : sizeof(DistTri)));
+  b.tris = reinterpret_cast<TriRec *>(p);
+  p += align256(n * sizeof(TriRec));
   b.nodes = reinterpret_cast<Node *>(p);
   p += align256((m + M) * sizeof(Node));
   b.leaf_order = reinterpret_cast<uint32_t *>(p);
   p += align256(n * 4);
   b.bounds = reinterpret_cast<uint32_t *>(p);
   p += align256(size_t(M) * 6 * 4);
-  b.node_moment = winding ? reinterpret_cast<float4 *>(p) : nullptr;
+  b.node_moment = reinterpret_cast<float4 *>(p);
   b.num_inner = T >= 2 ? static_cast<int>(T - 1) : 0;
   b.num_nodes = b.num_inner + M;
 }
@@ -471,7 +456,7 @@ cudaError_t lbvh_build(const BatchDev &B, BvhDev &b, void *temp, size_t temp_byt
   cudaError_t e;
   k_init_bounds<<<(6 * M + 255) / 256, 256, 0, st>>>(b.bounds, M);
   note_launch();
-  k_prep<<<blocks_for(T), kThreads, 0, st>>>(B, b.tris ? t.rec : nullptr, t.lo, t.hi, b.bounds, err);
+  k_prep<<<blocks_for(T), kThreads, 0, st>>>(B, t.rec, t.lo, t.hi, b.bounds, err);
   note_launch();
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
   const int n = static_cast<int>(T);
@@ -504,9 +489,9 @@ cudaError_t lbvh_build(const BatchDev &B, BvhDev &b, void *temp, size_t temp_byt
   }
   k_roots<<<(M + 127) / 128, 128, 0, st>>>(B, b.num_inner, vals, t.lo, t.hi, t.ilo, t.ihi, t.subtree, b.nodes, err);
   note_launch();
-  k_gather<<<blocks_for(T), kThreads, 0, st>>>(B, vals, t.rec, b.tris, b.dtris, b.leaf_order);
+  k_gather<<<blocks_for(T), kThreads, 0, st>>>(B, vals, t.rec, b.tris, b.leaf_order);
   note_launch();
-  if (b.node_moment && T >= 2) {
+  if (T >= 2) {
     if ((e = cudaMemsetAsync(t.visits, 0, sizeof(int) * (T - 1), st)) != cudaSuccess) return e;
     k_moments<<<blocks_for(T), kThreads, 0, st>>>(n, b.tris, t.child, t.iparent, t.lparent, t.visits, b.node_moment);
     note_launch();

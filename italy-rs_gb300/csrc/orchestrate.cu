@@ -1,8 +1,8 @@
 // The batch orchestrator behind every bake entry point.
 //
-//   upload mesh records + prefix tables -> BVH over all meshes (lbvh.cu) -> occupancy
+//   upload mesh records + prefix tables -> a packed tree per mesh (ptree.cu) -> occupancy
 //   (occupancy.cu) -> +z crossing lists of the parity and winding-number meshes (parity.cu) ->
-//   caps hierarchy for the winding number -> distance with fused parity sign, one persistent
+//   caps hierarchy for the winding number (lbvh.cu) -> distance with fused parity sign, one persistent
 //   launch over every mesh's tiles (distance.cu) -> winding-number signs (gwn.cu)
 //
 // CUDA events bracket each stage for the per-stage times in sdfb_stats. After the stream drains,
@@ -70,7 +70,7 @@ int bucket_grid(const sdfb_grid_desc &g) {
 void load_tuning(sdfb_ctx *ctx) {
   for (int i = 0; i < 32; ++i)
     for (int j = 0; j < 8; ++j) {
-      ctx->tuned_leaf[i][j] = 4;
+      ctx->tuned_leaf[i][j] = 2;
       ctx->tuned_tile[i][j] = 2;
       ctx->tuned_stack[i][j] = 64;
       ctx->tuned_budget[i][j] = kDefaultStepBudget;
@@ -154,14 +154,25 @@ inline size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
 struct Layout {
   std::vector<MeshRec> recs, cap_recs;
-  std::vector<uint64_t> tri, ptri, tile, gtile, cell, cap_tri, cap_zero;
+  std::vector<PTreeRec> trees;
+  std::vector<uint64_t> tri, ptri, tile, gtile, cell, group, cap_tri, cap_zero;
   uint64_t total_cols = 0, gwn_cells = 0, cap_total = 0;
   int tile_id = 2, stack = 64;
   long long step_budget = 0;
   bool resident = false;
   size_t o_recs = 0, o_tri = 0, o_ptri = 0, o_tile = 0, o_gtile = 0, o_cell = 0, o_caprecs = 0, o_captri = 0,
-         o_capzero = 0, bytes = 0;
+         o_capzero = 0, o_trees = 0, o_group = 0, tree_bytes = 0, bytes = 0;
 };
+
+// The block size of a mesh's tree (index k: 2 << k triangles) from its leaf size, 1..16: the largest
+// block not above it, at least 2 and at most 8 triangles.
+int block_index(int leaf) { return leaf >= 8 ? 2 : (leaf >= 4 ? 1 : 0); }
+
+// A tree's view for the walk, at block size index k or the nearest one built.
+DistTree tree_view(const PTreeRec &r, int k) {
+  for (int d = 0; d < kTreeSizes && !r.obb[k]; ++d) k = (k + 1) % kTreeSizes;
+  return DistTree{r.tri, r.obb[k], r.box[k], r.num_tris, k + 1};
+}
 
 void make_layout(sdfb_ctx *ctx, const std::vector<PlanMesh> &ms, const sdfb_opts &o, Layout &L) {
   const int M = static_cast<int>(ms.size());
@@ -180,10 +191,9 @@ void make_layout(sdfb_ctx *ctx, const std::vector<PlanMesh> &ms, const sdfb_opts
   L.step_budget = o.step_budget > 0 ? o.step_budget
                                     : (o.step_budget < 0 ? 0 : (batch ? ctx->batch_budget : ctx->tuned_budget[tb][nb]));
   L.resident = ms[0].bvh != nullptr;
-  uint64_t T_total = 0;
-  for (const auto &p : ms) T_total += p.T;
-  const int num_inner = T_total >= 2 ? static_cast<int>(T_total - 1) : 0;
   L.recs.resize(M);
+  L.trees.resize(M);
+  L.group.assign(M + 1, 0);
   L.tri.assign(M + 1, 0);
   L.ptri.assign(M + 1, 0);
   L.tile.assign(M + 1, 0);
@@ -211,14 +221,12 @@ void make_layout(sdfb_ctx *ctx, const std::vector<PlanMesh> &ms, const sdfb_opts
                                 : (o.leaf_size > 0 ? o.leaf_size
                                                    : ctx->tuned_leaf[bucket_tris(p.T)][bucket_grid(p.grid)]);
     r.leaf_size = std::max(1, std::min(leaf, 16));
-    r.root = num_inner + m;
     r.cap_root = -1;
     if (p.bvh) {
-      r.nodes = p.bvh->nodes;
-      r.tris = p.bvh->dtris;
-      r.bvh_nodes = p.bvh->num_nodes;
-      r.bvh_tris = p.bvh->num_tris;
-      r.root = p.bvh->root;
+      r.tree = tree_view(p.bvh->tree, block_index(r.leaf_size));
+    } else {
+      L.tree_bytes += ptree_layout(p.T, 1 << block_index(r.leaf_size), nullptr, &L.trees[m]);
+      L.group[m + 1] = L.group[m] + L.trees[m].slots / kTreePad;
     }
     const uint64_t cells = uint64_t(p.grid.nx) * p.grid.ny * p.grid.nz;
     r.tri_base = L.tri[m];
@@ -269,7 +277,6 @@ void make_layout(sdfb_ctx *ctx, const std::vector<PlanMesh> &ms, const sdfb_opts
   const int cap_inner = L.cap_total >= 2 ? static_cast<int>(L.cap_total - 1) : 0;
   for (int m = 0; m < M; ++m)
     if (L.recs[m].cap_root >= 0 && !ms[m].caps) L.recs[m].cap_root += cap_inner;
-  for (int k = 0; k < K; ++k) L.cap_recs[k].root = cap_inner + k;
   L.cap_zero.assign(K + 1, 0);
   size_t off = 0;
   auto put = [&](size_t bytes) {
@@ -286,17 +293,20 @@ void make_layout(sdfb_ctx *ctx, const std::vector<PlanMesh> &ms, const sdfb_opts
   L.o_caprecs = put(std::max(K, 1) * sizeof(MeshRec));
   L.o_captri = put((K + 1) * 8);
   L.o_capzero = put((K + 1) * 8);
+  L.o_trees = put(M * sizeof(PTreeRec));
+  L.o_group = put((M + 1) * 8);
   L.bytes = off;
 }
 
-// Points the records at the combined hierarchies built for this batch.
-void bind_built(Layout &L, const BvhDev &bvh, const BvhDev *caps) {
-  for (auto &r : L.recs) {
-    if (bvh.nodes) {
-      r.nodes = bvh.nodes;
-      r.tris = bvh.dtris;
-      r.bvh_nodes = bvh.num_nodes;
-      r.bvh_tris = static_cast<int>(L.tri.back());
+// Points the records at the hierarchies built for this batch: the trees in one buffer, one after the
+// other, and the combined hierarchy of the caps.
+void bind_built(Layout &L, char *trees, const BvhDev *caps) {
+  for (size_t m = 0; m < L.recs.size(); ++m) {
+    MeshRec &r = L.recs[m];
+    if (trees) {
+      const int k = block_index(r.leaf_size);
+      trees += ptree_layout(r.num_tris, 1 << k, trees, &L.trees[m]);
+      r.tree = tree_view(L.trees[m], k);
     }
     if (caps && r.cap_root >= 0 && !r.cap_nodes) {
       r.cap_nodes = caps->nodes;
@@ -321,6 +331,8 @@ void fill_staging(const Layout &L, char *s) {
   if (!L.cap_recs.empty()) std::memcpy(s + L.o_caprecs, L.cap_recs.data(), L.cap_recs.size() * sizeof(MeshRec));
   std::memcpy(s + L.o_captri, L.cap_tri.data(), L.cap_tri.size() * 8);
   std::memcpy(s + L.o_capzero, L.cap_zero.data(), L.cap_zero.size() * 8);
+  std::memcpy(s + L.o_trees, L.trees.data(), L.trees.size() * sizeof(PTreeRec));
+  std::memcpy(s + L.o_group, L.group.data(), L.group.size() * 8);
 }
 
 BatchDev batch_dev(const Layout &L, char *d) {
@@ -386,8 +398,8 @@ sdfb_status enqueue_batch(sdfb_ctx *ctx, Workspace &ws, cudaStream_t st, std::ve
   // Workspace.
   ENSURE(ws.batch_buf, L.bytes);
   if (!ws.staging.ensure(L.bytes)) return ctx_fail(ctx, SDFB_ERR_OUT_OF_MEMORY, "pinned staging");
-  if (build) ENSURE(ws.bvh, lbvh_bytes(T, M, false));
-  ENSURE(ws.build_tmp, std::max(build ? lbvh_temp_bytes(T, M) : size_t(0), occupancy_temp_bytes(T)));
+  if (build) ENSURE(ws.bvh, L.tree_bytes);
+  ENSURE(ws.build_tmp, std::max(build ? ptree_temp_bytes(T, M) : size_t(0), occupancy_temp_bytes(T)));
   ENSURE(ws.misc, 256);
   if (S.any_cross) {
     ENSURE(ws.par_tmp, parity_temp_bytes(L.ptri.back(), L.total_cols));
@@ -398,16 +410,15 @@ sdfb_status enqueue_batch(sdfb_ctx *ctx, Workspace &ws, cudaStream_t st, std::ve
     S.capacity = std::min<uint64_t>(ws.col_z.cap / 4, ws.col_s.cap);
   }
   if (K > 0) {
-    ENSURE(ws.caps_bvh, lbvh_bytes(L.cap_total, K, true));
+    ENSURE(ws.caps_bvh, lbvh_bytes(L.cap_total, K));
     ENSURE(ws.caps_tmp, lbvh_temp_bytes(L.cap_total, K));
   }
   if (S.any_gwn) ENSURE(ws.gwn_tmp, gwn_temp_bytes(L.gwn_cells));
   const uint64_t defer_cap = L.step_budget > 0 ? defer_capacity_for(L.tile.back()) : 0;
   if (defer_cap > 0) ENSURE(ws.defer, defer_cap * 8);
-  BvhDev bvh, caps;
-  if (build) lbvh_bind(bvh, ws.bvh.p, T, M, false);
-  if (K > 0) lbvh_bind(caps, ws.caps_bvh.p, L.cap_total, K, true);
-  bind_built(L, build ? bvh : BvhDev(), K > 0 ? &caps : nullptr);
+  BvhDev caps;
+  if (K > 0) lbvh_bind(caps, ws.caps_bvh.p, L.cap_total, K);
+  bind_built(L, build ? static_cast<char *>(ws.bvh.p) : nullptr, K > 0 ? &caps : nullptr);
   fill_staging(L, static_cast<char *>(ws.staging.p));
   const BatchDev B = batch_dev(L, static_cast<char *>(ws.batch_buf.p));
   const BatchDev CB = K > 0 ? caps_dev(L, static_cast<char *>(ws.batch_buf.p)) : BatchDev();
@@ -426,6 +437,7 @@ sdfb_status enqueue_batch(sdfb_ctx *ctx, Workspace &ws, cudaStream_t st, std::ve
   da.defer_capacity = defer_cap;
   da.defer_counters = reinterpret_cast<unsigned long long *>(static_cast<char *>(ws.misc.p) + kMiscDeferOffset);
   da.step_budget = L.step_budget;
+  da.stack_depth = L.stack;
   da.fault = o.fault_inject;
   GwnInput gi;
   gi.batch = B;
@@ -451,7 +463,10 @@ sdfb_status enqueue_batch(sdfb_ctx *ctx, Workspace &ws, cudaStream_t st, std::ve
     CK(rec(ws.ev[0]));
     if (build) {
       NvtxRange r("sdfb build");
-      CK(lbvh_build(B, bvh, ws.build_tmp.p, ws.build_tmp.cap, d_err, st));
+      const char *tab = static_cast<const char *>(ws.batch_buf.p);
+      CK(ptree_build(B, reinterpret_cast<const PTreeRec *>(tab + L.o_trees),
+                     reinterpret_cast<const uint64_t *>(tab + L.o_group), L.group.back(), ws.build_tmp.p,
+                     ws.build_tmp.cap, d_err, st));
     }
     CK(rec(ws.ev[1]));
     if (any_occ) {
@@ -472,7 +487,7 @@ sdfb_status enqueue_batch(sdfb_ctx *ctx, Workspace &ws, cudaStream_t st, std::ve
     CK(rec(ws.ev[3]));
     {
       NvtxRange r("sdfb distance");
-      CK(distance_launch(da, L.tile_id, L.stack, ctx->num_sms, st));
+      CK(distance_launch(da, L.tile_id, ctx->num_sms, st));
     }
     CK(rec(ws.ev[4]));
     if (S.any_gwn) {
@@ -627,65 +642,69 @@ sdfb_status run_batch(sdfb_ctx *ctx, cudaStream_t st, std::vector<PlanMesh> &ms,
 // ---------------------------------------------------------------------------------------------
 // Resident hierarchies (serving).
 
-size_t resident_bytes(uint64_t tris, bool winding) { return lbvh_bytes(tris, 1, winding); }
+size_t resident_bytes(uint32_t tris, bool winding) {
+  return winding ? lbvh_bytes(tris, 1) : ptree_layout(tris, (1 << kTreeSizes) - 1, nullptr, nullptr);
+}
 
 sdfb_status build_resident(sdfb_ctx *ctx, Workspace &ws, cudaStream_t st, const PlanMesh &p, void *mem,
                            ResidentBvh &out, void *cap_mem, ResidentBvh &cap_out) {
   if (!ws.init()) return ctx_fail(ctx, SDFB_ERR_CUDA, "cannot create events");
   const bool with_caps = p.cT > 0 && cap_mem;
-  MeshRec r[2];
-  std::memset(r, 0, sizeof r);
-  r[0].verts = p.verts;
-  r[0].idx = p.idx;
-  r[0].num_verts = p.V;
-  r[0].num_tris = p.T;
-  r[0].leaf_size = std::max(1, std::min(p.leaf > 0 ? p.leaf : ctx->tuned_leaf[bucket_tris(p.T)][bucket_grid(p.grid)], 16));
-  r[1].verts = p.cverts;
-  r[1].idx = p.cidx;
-  r[1].num_verts = p.pV;
-  r[1].num_tris = p.cT;
-  r[1].leaf_size = 4;
-  const uint64_t tables[2][2] = {{0, p.T}, {0, p.cT}};
-  const uint64_t zero[2] = {0, 0};
-  const size_t bytes = 256 * 6;
-  ENSURE(ws.batch_buf, bytes);
-  if (!ws.staging.ensure(bytes)) return ctx_fail(ctx, SDFB_ERR_OUT_OF_MEMORY, "pinned staging");
-  ENSURE(ws.build_tmp, std::max(lbvh_temp_bytes(p.T, 1), with_caps ? lbvh_temp_bytes(p.cT, 1) : size_t(0)));
+  // Every block size: the requests' grids, which decide the one used, are not known yet.
+  ptree_layout(p.T, (1 << kTreeSizes) - 1, static_cast<char *>(mem), &out.tree);
+  out.num_tris = static_cast<int>(p.T);
+  struct Tables {
+    alignas(256) MeshRec mesh, caps;
+    alignas(256) PTreeRec tree;
+    alignas(256) uint64_t tris[2], cap_tris[2], zero[2], groups[2];
+  };
+  ENSURE(ws.batch_buf, sizeof(Tables));
+  if (!ws.staging.ensure(sizeof(Tables))) return ctx_fail(ctx, SDFB_ERR_OUT_OF_MEMORY, "pinned staging");
+  ENSURE(ws.build_tmp, std::max(ptree_temp_bytes(p.T, 1), with_caps ? lbvh_temp_bytes(p.cT, 1) : size_t(0)));
   ENSURE(ws.misc, 256);
-  char *hs = static_cast<char *>(ws.staging.p);
-  std::memset(hs, 0, bytes);
-  std::memcpy(hs, &r[0], sizeof(MeshRec));
-  std::memcpy(hs + 256, tables[0], 16);
-  std::memcpy(hs + 512, zero, 16);
-  std::memcpy(hs + 768, &r[1], sizeof(MeshRec));
-  std::memcpy(hs + 1024, tables[1], 16);
-  CK(cudaMemcpyAsync(ws.batch_buf.p, hs, bytes, cudaMemcpyHostToDevice, st));
+  Tables &h = *static_cast<Tables *>(ws.staging.p);
+  std::memset(static_cast<void *>(&h), 0, sizeof h);
+  h.mesh.verts = p.verts;
+  h.mesh.idx = p.idx;
+  h.mesh.num_verts = p.V;
+  h.mesh.num_tris = p.T;
+  h.caps.verts = p.cverts;
+  h.caps.idx = p.cidx;
+  h.caps.num_verts = p.pV;
+  h.caps.num_tris = p.cT;
+  h.caps.leaf_size = 4;
+  h.tree = out.tree;
+  h.tris[1] = p.T;
+  h.cap_tris[1] = p.cT;
+  h.groups[1] = out.tree.slots / kTreePad;
+  CK(cudaMemcpyAsync(ws.batch_buf.p, &h, sizeof h, cudaMemcpyHostToDevice, st));
   CK(cudaMemsetAsync(ws.misc.p, 0, 256, st));
-  char *d = static_cast<char *>(ws.batch_buf.p);
-  auto one = [&](int off_rec, int off_tab, uint64_t T, void *m, bool areas, ResidentBvh &o) -> sdfb_status {
+  const Tables *d = static_cast<const Tables *>(ws.batch_buf.p);
+  uint32_t *d_err = static_cast<uint32_t *>(ws.misc.p);
+  auto batch = [&](const MeshRec *rec, const uint64_t *starts, uint64_t T) {
     BatchDev B;
     B.num_meshes = 1;
-    B.recs = reinterpret_cast<const MeshRec *>(d + off_rec);
-    B.tri_starts = reinterpret_cast<const uint64_t *>(d + off_tab);
-    B.ptri_starts = B.tile_starts = B.gwn_tile_starts = B.cell_starts = reinterpret_cast<const uint64_t *>(d + 512);
+    B.recs = rec;
+    B.tri_starts = starts;
+    B.ptri_starts = B.tile_starts = B.gwn_tile_starts = B.cell_starts = d->zero;
     B.total_tris = T;
-    BvhDev b;
-    lbvh_bind(b, m, T, 1, areas);
-    CK(lbvh_build(B, b, ws.build_tmp.p, ws.build_tmp.cap, static_cast<uint32_t *>(ws.misc.p), st));
-    o.nodes = b.nodes;
-    o.dtris = b.dtris;
-    o.tris = b.tris;
-    o.leaf_order = b.leaf_order;
-    o.node_moment = b.node_moment;
-    o.num_nodes = b.num_nodes;
-    o.num_inner = b.num_inner;
-    o.num_tris = static_cast<int>(T);
-    o.root = b.num_inner;  // the single virtual root
-    return SDFB_OK;
+    return B;
   };
-  sdfb_status s = one(0, 256, p.T, mem, false, out);
-  if (s != SDFB_OK) return s;
-  if (with_caps && (s = one(768, 1024, p.cT, cap_mem, true, cap_out)) != SDFB_OK) return s;
+  CK(ptree_build(batch(&d->mesh, d->tris, p.T), &d->tree, d->groups, h.groups[1], ws.build_tmp.p, ws.build_tmp.cap,
+                 d_err, st));
+  if (with_caps) {
+    BvhDev b;
+    lbvh_bind(b, cap_mem, p.cT, 1);
+    CK(lbvh_build(batch(&d->caps, d->cap_tris, p.cT), b, ws.build_tmp.p, ws.build_tmp.cap, d_err, st));
+    cap_out.nodes = b.nodes;
+    cap_out.tris = b.tris;
+    cap_out.leaf_order = b.leaf_order;
+    cap_out.node_moment = b.node_moment;
+    cap_out.num_nodes = b.num_nodes;
+    cap_out.num_inner = b.num_inner;
+    cap_out.num_tris = static_cast<int>(p.cT);
+    cap_out.root = b.num_inner;  // the single virtual root
+  }
   uint32_t h_err = 0;
   CK(cudaMemcpyAsync(&h_err, ws.misc.p, 4, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));

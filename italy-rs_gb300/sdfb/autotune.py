@@ -1,16 +1,15 @@
 """Autotuner for the bake's launch parameters on the GPU it runs on.
 
 Three parameters of the distance pass trade against each other with the mesh and the grid:
-  * leaf size (triangles per BVH leaf, 1..16): small leaves test fewer triangles per visit but add
-    node tests and stack traffic;
-  * tile shape (the cells one warp walks the BVH for, ids 1..6 = 4x4x2, 8x4x1, 4x4x4, 8x4x2,
-    4x4x8, 8x4x4 cells with 1, 1, 2, 2, 4, 4 cells per lane): bigger tiles share one traversal
+  * leaf size (triangles per block of the packed tree, 2, 4 or 8): small blocks need fewer exact
+    distances, large ones fewer boxes; where triangles are much smaller than voxels large blocks win;
+  * tile shape (the cells one warp walks the tree for, ids 1..6 = 4x4x2, 8x4x1, 4x4x4, 8x4x2,
+    4x4x8, 8x4x4 cells with 1, 1, 2, 2, 4, 4 cells per lane): bigger tiles share one walk
     among more cells but visit the union of their candidates;
-  * traversal stack depth (32 or 64 entries): the shallow stack needs fewer registers but a deep
-    tree overflows it (the bake then reruns that launch with 64);
-  * step budget (traversal steps before a tile is handed to the block-per-tile second pass, or
-    never): a small budget moves more tiles into the pass that splits a tile's walk over a block,
-    which pays on small grids (fewer tiles than the GPU holds warps).
+  * step budget (work steps between a tile's looks at whether it should be handed to the
+    block-per-tile second pass, or never): a small budget moves more tiles into the pass that splits
+    a tile's walk over a block, which pays on small grids (fewer tiles than the GPU holds warps).
+The table also holds a traversal stack depth; every tree fits either, so it stays at 64.
 
 For each (log2 triangles, log2 grid edge) bucket of a sweep of displaced spheres and grids, the tuner
 times whole device-buffer bakes (CUDA events on the bake's stream, median of `reps`) under a
@@ -40,10 +39,10 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 DEFAULT_OUT = os.path.join(os.path.dirname(HERE), "tuning", "gb300.tsv")
 
 TILES = (1, 2, 3, 4, 5, 6)
-LEAVES = (1, 2, 3, 4, 6, 8, 12, 16)
-STACKS = (32, 64)
-BUDGETS = (-1, 32, 128, 512, 1024, 2048, 4096)
-START = (4, 3, 64, 1024)  # leaf, tile id (1-based), stack, step budget: the built-in defaults
+LEAVES = (2, 4, 8)
+STACKS = (64,)
+BUDGETS = (-1, 64, 256, 512, 1024, 2048, 4096, 8192, 32768)
+START = (2, 3, 64, 2048)  # leaf, tile id (1-based), stack, step budget: the built-in defaults
 
 # (mesh, grid edge): displaced icospheres of levels 3..7 (1,280 .. 327,680 triangles) on 32^3 .. 512^3
 # grids, and displaced tori of 131,072 and 1,048,576 triangles (thin tubes; the largest meshes a
