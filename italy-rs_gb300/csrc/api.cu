@@ -85,6 +85,7 @@ void sdfb_ctx::release_all() {
   for (int i = 0; DevBuf *b = all_bufs(i); ++i) b->release();
   ws.release();
   staging_small.release();
+  gate_pin.release();
 }
 
 uint64_t sdfb_ctx::device_bytes() const {
@@ -149,23 +150,6 @@ sdfb_opts opts_or_default(const sdfb_opts *o) {
 // Host-side preparation.
 
 namespace {
-
-// Sign of one mesh from the options and, for AUTO, the watertight gate on the host copy.
-// Returns -1 when an index is out of range (AUTO only).
-int resolve_sign(const sdfb_opts &o, const float *hv, uint32_t V, const uint32_t *hi, uint32_t T, int *watertight) {
-  *watertight = -1;
-  switch (o.sign_mode) {
-    case SDFB_SIGN_PARITY: return kSignParity;
-    case SDFB_SIGN_GWN: return kSignGwn;
-    case SDFB_SIGN_NONE: return kSignNone;
-    default: break;
-  }
-  const int w = indexed_mesh_watertight(hv, V, hi, T);
-  if (w == -2) return -1;
-  *watertight = w == 1 ? 1 : 0;
-  return w == 1 ? kSignParity : kSignGwn;
-}
-
 
 // The device address of a page-locked host buffer (cudaHostAlloc, cudaHostRegister, a pinned
 // tensor), or null for pageable memory. The distance kernel writes such a distance output
@@ -252,19 +236,23 @@ sdfb_status device_caps(sdfb_ctx *ctx, cudaStream_t st, std::vector<PlanMesh> &m
   return SDFB_OK;
 }
 
-sdfb_status device_sign(sdfb_ctx *ctx, const sdfb_opts &o, const float *d_verts, uint32_t V, const uint32_t *d_idx,
-                        uint32_t T, cudaStream_t st, int *sign, int *watertight) {
-  *watertight = -1;
-  if (o.sign_mode != SDFB_SIGN_AUTO) {
-    *sign = resolve_sign(o, nullptr, 0, nullptr, 0, watertight);
-    return SDFB_OK;
+sdfb_status device_signs(sdfb_ctx *ctx, const sdfb_opts &o, PlanMesh *ms, size_t count, cudaStream_t st,
+                         size_t *bad) {
+  size_t at = 0;
+  if (o.sign_mode != SDFB_SIGN_PARITY && o.sign_mode != SDFB_SIGN_GWN && o.sign_mode != SDFB_SIGN_NONE) {
+    std::vector<PlanMesh *> v(count);
+    for (size_t m = 0; m < count; ++m) v[m] = ms + m;
+    const sdfb_status s = device_gate(ctx, v, st, bad ? bad : &at);
+    if (s != SDFB_OK) return s;
   }
-  ENSURE(ctx->weld_tmp, indexed_gate_temp_bytes(V, T));
-  int w = 0;
-  CK(indexed_watertight_device(d_verts, V, d_idx, T, ctx->weld_tmp.p, ctx->weld_tmp.cap, &w, ctx->num_sms, st));
-  if (w == -2) return ctx_fail(ctx, SDFB_ERR_BAD_MESH, "triangle index out of range");
-  *watertight = w == 1 ? 1 : 0;
-  *sign = w == 1 ? kSignParity : kSignGwn;
+  for (size_t m = 0; m < count; ++m) {
+    switch (o.sign_mode) {
+      case SDFB_SIGN_PARITY: ms[m].sign = kSignParity; break;
+      case SDFB_SIGN_GWN: ms[m].sign = kSignGwn; break;
+      case SDFB_SIGN_NONE: ms[m].sign = kSignNone; break;
+      default: ms[m].sign = ms[m].watertight == 1 ? kSignParity : kSignGwn;
+    }
+  }
   return SDFB_OK;
 }
 
@@ -371,7 +359,7 @@ sdfb_status sdfb_bake_device(sdfb_ctx *ctx, const float *d_verts, uint32_t num_v
   p.grid = *grid;
   p.dist = o.no_distance ? nullptr : d_dist_out;
   p.occ = o.no_occupancy ? nullptr : d_occ_out;
-  sdfb_status s = device_sign(ctx, o, d_verts, num_verts, d_idx, num_tris, st, &p.sign, &p.watertight);
+  sdfb_status s = device_signs(ctx, o, &p, 1, st);
   if (s != SDFB_OK) return s;
   if ((s = device_caps(ctx, st, ms)) != SDFB_OK) return s;
   return run_batch(ctx, st, ms, o, false, stats);
@@ -398,21 +386,19 @@ sdfb_status sdfb_bake(sdfb_ctx *ctx, const float *verts, uint32_t num_verts, con
   if (want_occ) ENSURE(ctx->out_occ, cells);
   CK(cudaMemcpyAsync(ctx->in_verts.p, verts, size_t(num_verts) * 12, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(ctx->in_idx.p, idx, size_t(num_tris) * 12, cudaMemcpyHostToDevice, st));
-  sdfb_status sg = device_sign(ctx, o, static_cast<const float *>(ctx->in_verts.p), num_verts,
-                               static_cast<const uint32_t *>(ctx->in_idx.p), num_tris, st, &p.sign, &p.watertight);
-  if (sg != SDFB_OK) return sg;
   p.verts = static_cast<const float *>(ctx->in_verts.p);
   p.idx = static_cast<const uint32_t *>(ctx->in_idx.p);
   p.V = num_verts;
   p.T = num_tris;
   p.grid = *grid;
+  sdfb_status s = device_signs(ctx, o, &p, 1, st);
+  if (s != SDFB_OK) return s;
   float *const direct_dist =
       (want_dist && p.sign != kSignGwn) ? static_cast<float *>(mapped_host(dist_out)) : nullptr;
   uint8_t *const direct_occ = nullptr;
   p.dist = want_dist ? (direct_dist ? direct_dist : static_cast<float *>(ctx->out_dist.p)) : nullptr;
   p.occ = want_occ ? (direct_occ ? direct_occ : static_cast<uint8_t *>(ctx->out_occ.p)) : nullptr;
-  sdfb_status s = device_caps(ctx, st, ms);
-  if (s != SDFB_OK) return s;
+  if ((s = device_caps(ctx, st, ms)) != SDFB_OK) return s;
   s = run_batch(ctx, st, ms, o, false, stats);
   if (s != SDFB_OK) return s;
   if (want_dist && !direct_dist)
@@ -450,25 +436,33 @@ sdfb_status sdfb_bake_soup(sdfb_ctx *ctx, const float *positions, uint32_t num_t
   CK(cudaMemcpyAsync(ctx->in_idx.p, ident.data(), size_t(V) * 4, cudaMemcpyHostToDevice, st));
   // Weld on the device (first occurrence kept) for the watertight gate and for a crack-free
   // crossing mesh: welded indices in in_idx2, unique positions in in_verts2.
+  const size_t weld_bytes = (weld_temp_bytes(V) + 255) & ~size_t(255);
   ENSURE(ctx->in_idx2, size_t(V) * 4);
   ENSURE(ctx->in_verts2, size_t(V) * 12);
-  ENSURE(ctx->weld_tmp, std::max(weld_temp_bytes(V) + size_t(V) * 4 + 256, watertight_temp_bytes(num_tris)));
+  ENSURE(ctx->weld_tmp, weld_bytes + watertight_temp_bytes(num_tris));
+  if (!ctx->gate_pin.ensure(32)) return ctx_fail(ctx, SDFB_ERR_OUT_OF_MEMORY, "pinned staging");
   uint32_t *d_welded = static_cast<uint32_t *>(ctx->in_idx2.p);
-  uint32_t *d_first = reinterpret_cast<uint32_t *>(static_cast<char *>(ctx->weld_tmp.p) + weld_temp_bytes(V));
-  uint32_t U = 0;
-  CK(weld_device(static_cast<const float *>(ctx->in_verts.p), V, weld_cell(bounds_min, bounds_max), d_welded, d_first,
-                 ctx->weld_tmp.p, weld_temp_bytes(V), &U, ctx->num_sms, st));
-  CK(gather_unique(static_cast<const float *>(ctx->in_verts.p), d_first, U, static_cast<float *>(ctx->in_verts2.p),
-                   ctx->num_sms, st));
+  char *d_tmp = static_cast<char *>(ctx->weld_tmp.p);
+  const uint64_t *d_unique = nullptr;
+  CK(weld_enqueue(static_cast<const float *>(ctx->in_verts.p), V, weld_cell(bounds_min, bounds_max), d_welded,
+                  static_cast<float *>(ctx->in_verts2.p), d_tmp, weld_bytes, &d_unique, ctx->num_sms, st));
+  uint64_t *h = static_cast<uint64_t *>(ctx->gate_pin.p);  // unique positions, boundary - 1, non-manifold - 1
+  CK(cudaMemcpyAsync(h, d_unique, 8, cudaMemcpyDeviceToHost, st));
   std::vector<PlanMesh> ms(1);
   PlanMesh &p = ms[0];
   if (o.sign_mode == SDFB_SIGN_AUTO) {
-    uint64_t b = 0, m = 0;
-    CK(watertight_device(d_welded, num_tris, U, ctx->weld_tmp.p, ctx->weld_tmp.cap, &b, &m, ctx->num_sms, st));
-    p.watertight = (b == 0 && m == 0) ? 1 : 0;
+    const unsigned long long *d_counts = nullptr;
+    CK(watertight_enqueue(d_welded, num_tris, d_tmp + weld_bytes, watertight_temp_bytes(num_tris), &d_counts,
+                          ctx->num_sms, st));
+    CK(cudaMemcpyAsync(h + 1, d_counts, 16, cudaMemcpyDeviceToHost, st));
+  }
+  CK(cudaStreamSynchronize(st));
+  const uint32_t U = static_cast<uint32_t>(h[0]);
+  if (o.sign_mode == SDFB_SIGN_AUTO) {
+    p.watertight = (h[1] + 1 == 0 && h[2] + 1 == 0) ? 1 : 0;
     p.sign = p.watertight ? kSignParity : kSignGwn;
   } else {
-    p.sign = resolve_sign(o, nullptr, 0, nullptr, 0, &p.watertight);
+    p.sign = o.sign_mode == SDFB_SIGN_PARITY ? kSignParity : (o.sign_mode == SDFB_SIGN_NONE ? kSignNone : kSignGwn);
   }
   p.verts = static_cast<const float *>(ctx->in_verts.p);
   p.idx = static_cast<const uint32_t *>(ctx->in_idx.p);
@@ -511,7 +505,7 @@ sdfb_status sdfb_weld_device(sdfb_ctx *ctx, const float *d_positions, uint32_t n
   cudaSetDevice(ctx->device);
   const cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
   ENSURE(ctx->weld_tmp, weld_temp_bytes(num_positions));
-  CK(weld_device(d_positions, num_positions, weld_cell(bounds_min, bounds_max), d_welded_out, nullptr, ctx->weld_tmp.p,
+  CK(weld_device(d_positions, num_positions, weld_cell(bounds_min, bounds_max), d_welded_out, ctx->weld_tmp.p,
                  ctx->weld_tmp.cap, num_unique, ctx->num_sms, st));
   return SDFB_OK;
 }
@@ -527,8 +521,7 @@ sdfb_status sdfb_is_watertight_device(sdfb_ctx *ctx, const uint32_t *d_welded_id
   uint64_t b = 0, m = 0;
   if (num_tris) {
     ENSURE(ctx->weld_tmp, watertight_temp_bytes(num_tris));
-    CK(watertight_device(d_welded_idx, num_tris, 0, ctx->weld_tmp.p, ctx->weld_tmp.cap, &b, &m,
-                         ctx->num_sms, st));
+    CK(watertight_device(d_welded_idx, num_tris, ctx->weld_tmp.p, ctx->weld_tmp.cap, &b, &m, ctx->num_sms, st));
   }
   *watertight_out = (num_tris && b == 0 && m == 0) ? 1 : 0;  // no triangles: not watertight
   if (boundary_edges) *boundary_edges = b;
@@ -691,14 +684,14 @@ sdfb_status sdfb_bake_batch_device(sdfb_ctx *ctx, uint32_t count, const sdfb_mes
     p.grid = grids[m];
     p.dist = (o.no_distance || !dist_outs) ? nullptr : dist_outs[m];
     p.occ = (o.no_occupancy || !occ_outs) ? nullptr : occ_outs[m];
-    const sdfb_status sg = device_sign(ctx, o, d.verts, d.num_verts, d.idx, d.num_tris, st, &p.sign, &p.watertight);
-    if (sg != SDFB_OK) {
-      const std::string e = ctx->err;
-      return ctx_fail(ctx, sg, "mesh %u: %s", m, e.c_str());
-    }
   }
-  const sdfb_status s = device_caps(ctx, st, ms);
-  if (s != SDFB_OK) return s;
+  size_t bad = 0;
+  sdfb_status s = device_signs(ctx, o, ms.data(), count, st, &bad);
+  if (s == SDFB_ERR_BAD_MESH) {
+    const std::string e = ctx->err;
+    return ctx_fail(ctx, s, "mesh %zu: %s", bad, e.c_str());
+  }
+  if (s != SDFB_OK || (s = device_caps(ctx, st, ms)) != SDFB_OK) return s;
   return run_batch(ctx, st, ms, o, true, stats);
 }
 
@@ -735,21 +728,24 @@ sdfb_status sdfb_bake_batch(sdfb_ctx *ctx, uint32_t count, const sdfb_mesh_desc 
     uint32_t *di = static_cast<uint32_t *>(ctx->in_idx.p) + oi;
     CK(cudaMemcpyAsync(dv, d.verts, size_t(d.num_verts) * 12, cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(di, d.idx, size_t(d.num_tris) * 12, cudaMemcpyHostToDevice, st));
-    const sdfb_status sg = device_sign(ctx, o, dv, d.num_verts, di, d.num_tris, st, &p.sign, &p.watertight);
-    if (sg != SDFB_OK) {
-      const std::string e = ctx->err;
-      return ctx_fail(ctx, sg, "mesh %u: %s", m, e.c_str());
-    }
     p.verts = dv;
     p.idx = di;
     p.V = d.num_verts;
     p.T = d.num_tris;
     p.grid = grids[m];
-    if (want_dist && dist_outs[m] && p.sign != kSignGwn)
-      direct_dist[m] = static_cast<float *>(mapped_host(dist_outs[m]));
     ov += size_t(d.num_verts) * 3;
     oi += size_t(d.num_tris) * 3;
   }
+  size_t bad = 0;
+  sdfb_status s = device_signs(ctx, o, ms.data(), count, st, &bad);
+  if (s == SDFB_ERR_BAD_MESH) {
+    const std::string e = ctx->err;
+    return ctx_fail(ctx, s, "mesh %zu: %s", bad, e.c_str());
+  }
+  if (s != SDFB_OK) return s;
+  for (uint32_t m = 0; m < count; ++m)
+    if (want_dist && dist_outs[m] && ms[m].sign != kSignGwn)
+      direct_dist[m] = static_cast<float *>(mapped_host(dist_outs[m]));
   // Outputs: pinned caller buffers directly, the rest through device buffers copied out afterwards.
   uint64_t staged = 0;
   for (uint32_t m = 0; m < count; ++m) {
@@ -769,8 +765,7 @@ sdfb_status sdfb_bake_batch(sdfb_ctx *ctx, uint32_t count, const sdfb_mesh_desc 
       p.occ = direct_occ[m] ? direct_occ[m] : static_cast<uint8_t *>(ctx->out_occ.p) + occ_off;
     if (stage) occ_off += cells;
   }
-  sdfb_status s = device_caps(ctx, st, ms);
-  if (s != SDFB_OK) return s;
+  if ((s = device_caps(ctx, st, ms)) != SDFB_OK) return s;
   s = run_batch(ctx, st, ms, o, true, stats);
   if (s != SDFB_OK) return s;
   for (uint32_t m = 0; m < count; ++m) {

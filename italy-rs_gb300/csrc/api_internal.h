@@ -142,7 +142,7 @@ struct sdfb_ctx {
   DevBuf cons_grid, cons_io;  // consumer check: a grid and its queries / results
   DevBuf weld_tmp;            // device weld / watertight census
   DevBuf caps_tmp, caps_misc; // device-built winding-number caps: temporaries, totals and error word
-  PinBuf staging_small;
+  PinBuf staging_small, gate_pin;
   Workspace ws;
   int tuned_leaf[32][8];  // [log2 T][log2 n - 4]
   int tuned_tile[32][8];
@@ -166,11 +166,15 @@ void load_tuning(sdfb_ctx *ctx);
 
 sdfb_status ctx_fail(sdfb_ctx *ctx, sdfb_status st, const char *fmt, ...);
 sdfb_status ctx_cuda(sdfb_ctx *ctx, cudaError_t e, const char *what);
-// Sign mode of a mesh in device memory: forced modes pass through; AUTO runs the weld + watertight
-// gate on the device (parity when watertight, else the winding number). Fails with BAD_MESH on an
-// index out of range.
-sdfb_status device_sign(sdfb_ctx *ctx, const sdfb_opts &o, const float *d_verts, uint32_t V, const uint32_t *d_idx,
-                        uint32_t T, cudaStream_t st, int *sign, int *watertight);
+// Sign modes of meshes in device memory: forced modes pass through; AUTO runs the weld + watertight
+// gate on the device, for all of them together (parity when watertight, else the winding number).
+// Fails with BAD_MESH on an index out of range (*bad, optional: the mesh).
+sdfb_status device_signs(sdfb_ctx *ctx, const sdfb_opts &o, PlanMesh *ms, size_t count, cudaStream_t st,
+                         size_t *bad = nullptr);
+// weld.cu: sets the watertight verdict of indexed meshes in device memory (the weld of their vertices
+// over their bounds, then the edge census of the welded triangles; equivalent to the reference's test
+// on the de-indexed soup). Synchronises the stream. BAD_MESH: mesh *bad has an index >= V.
+sdfb_status device_gate(sdfb_ctx *ctx, const std::vector<PlanMesh *> &ms, cudaStream_t st, size_t *bad);
 // sdfb_voxelize_sparse; also returns the device list of the count occupied cells' linear indices
 // (valid until the context's next call) and the grid it used.
 sdfb_status voxelize_sparse_run(sdfb_ctx *ctx, const float *positions, uint32_t num_tris, const float bounds_min[3],

@@ -223,27 +223,25 @@ cudaError_t occupancy_hits(const BatchDev &B, void *temp, size_t temp_bytes, uin
                            unsigned long long *hit_count, int tri_bits, int num_sms, cudaStream_t st);
 
 // ---- weld.cu ----------------------------------------------------------------------------------
+// v[i] = i for i < n.
+cudaError_t iota_device(uint32_t *v, uint64_t n, int num_sms, cudaStream_t st);
 // weldPositions on the device: welded[i] = the first-occurrence number of position i's lattice key
-// (cell: the weld lattice, weld_cell in host_mesh.h); first_of (optional, num_unique entries) gets
-// each number's first position. Synchronises the stream (*num_unique is host memory).
+// (cell: the weld lattice, weld_cell in host_mesh.h); unique (optional) gets each number's first
+// position. *num_unique points at the count in device memory (valid until temp is reused).
 size_t weld_temp_bytes(uint64_t n);
-cudaError_t weld_device(const float *pos, uint64_t n, float cell, uint32_t *welded, uint32_t *first_of, void *temp,
-                        size_t temp_bytes, uint32_t *num_unique, int num_sms, cudaStream_t st);
-// out[u] = pos[first_of[u]] (3 floats) for u < U.
-cudaError_t gather_unique(const float *pos, const uint32_t *first_of, uint64_t U, float *out, int num_sms,
-                          cudaStream_t st);
-// Edge census of a welded triangle list (degenerate triangles skipped); every index must be below
-// num_unique (0: unknown). Synchronises the stream.
+cudaError_t weld_enqueue(const float *pos, uint64_t n, float cell, uint32_t *welded, float *unique, void *temp,
+                         size_t temp_bytes, const uint64_t **num_unique, int num_sms, cudaStream_t st);
+// The same, waiting for the count.
+cudaError_t weld_device(const float *pos, uint64_t n, float cell, uint32_t *welded, void *temp, size_t temp_bytes,
+                        uint32_t *num_unique, int num_sms, cudaStream_t st);
+// Edge census of a welded triangle list (degenerate triangles skipped). *counts points at two device
+// values: boundary edges - 1 and non-manifold edges - 1.
 size_t watertight_temp_bytes(uint64_t T);
-cudaError_t watertight_device(const uint32_t *welded, uint64_t T, uint32_t num_unique, void *temp, size_t temp_bytes,
-                              uint64_t *boundary, uint64_t *nonmanifold, int num_sms, cudaStream_t st);
-
-// The watertight gate of an indexed mesh on the device (the weld of its vertices over their
-// bounds, then the edge census of the welded triangles; equivalent to the reference's test on the
-// de-indexed soup). *result: 1 watertight, 0 not, -2 an index >= V. Synchronises the stream.
-size_t indexed_gate_temp_bytes(uint64_t V, uint64_t T);
-cudaError_t indexed_watertight_device(const float *verts, uint32_t V, const uint32_t *idx, uint32_t T, void *temp,
-                                      size_t temp_bytes, int *result, int num_sms, cudaStream_t st);
+cudaError_t watertight_enqueue(const uint32_t *welded, uint64_t T, void *temp, size_t temp_bytes,
+                               const unsigned long long **counts, int num_sms, cudaStream_t st);
+// The same, waiting for the counts.
+cudaError_t watertight_device(const uint32_t *welded, uint64_t T, void *temp, size_t temp_bytes, uint64_t *boundary,
+                              uint64_t *nonmanifold, int num_sms, cudaStream_t st);
 
 // ---- sparse.cu --------------------------------------------------------------------------------
 size_t sparse_temp_bytes(size_t cells, size_t max_out);

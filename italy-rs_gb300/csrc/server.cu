@@ -649,12 +649,15 @@ sdfb_status sdfb_mesh_register(sdfb_server *srv, const float *verts, uint32_t nu
   sdfb_opts auto_opts;
   std::memset(&auto_opts, 0, sizeof auto_opts);
   auto_opts.sign_mode = SDFB_SIGN_AUTO;
-  int sign = kSignParity, watertight = -1;
-  const sdfb_status gs = device_sign(rc, auto_opts, static_cast<const float *>(r->verts.p), num_verts,
-                                     static_cast<const uint32_t *>(r->idx.p), num_tris, st, &sign, &watertight);
+  PlanMesh gate;
+  gate.verts = static_cast<const float *>(r->verts.p);
+  gate.idx = static_cast<const uint32_t *>(r->idx.p);
+  gate.V = num_verts;
+  gate.T = num_tris;
+  const sdfb_status gs = device_signs(rc, auto_opts, &gate, 1, st);
   if (gs != SDFB_OK) return undo(gs, rc->err);
-  r->sign = sign;
-  r->watertight = watertight;
+  r->sign = gate.sign;
+  r->watertight = gate.watertight;
   size_t cap_bytes = 0;
   if (r->sign == kSignGwn) {
     // caps built on the device in the registration slot's buffers, then copied to exact-size
