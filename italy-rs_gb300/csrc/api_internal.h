@@ -221,7 +221,7 @@ sdfb_status device_caps(sdfb_ctx *ctx, cudaStream_t st, std::vector<PlanMesh> &m
 constexpr int kGwnCellsPerLane = 4;
 constexpr int kGwnTileZ = 2 * kGwnCellsPerLane;
 // gwn.cu: flips the sign of cells whose generalized winding number says inside (enqueued only).
-size_t gwn_temp_bytes(uint64_t gwn_cells);
+size_t gwn_temp_bytes(uint64_t gwn_cells, uint64_t gwn_tiles);
 cudaError_t gwn_enqueue(const GwnInput &in, void *temp, int num_sms, cudaStream_t st);
 uint64_t *gwn_refine_counter(void *temp);
 // Cells whose sign needed the direct FP64 sum over every cap triangle (the last pass).

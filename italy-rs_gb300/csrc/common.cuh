@@ -197,15 +197,11 @@ __device__ __forceinline__ bool column_crossing(f3 a, f3 b, f3 c, float px, floa
 
 // ---------------------------------------------------------------------------------------------
 // Triangle record of the winding-number hierarchy: 64 bytes, four float4s, in BVH leaf order.
-//   r0 = (v0, 1/|e1|^2)    e1 = v1 - v0
-//   r1 = (e1, 1/|e2|^2)    e2 = v2 - v0
-//   r2 = (e2, 1/|e3|^2)    e3 = v2 - v1
-//   r3 = (n,  |n|)         n = e1 x e2 (|n| is twice the area)
+//   r0 = (v0, -)   r1 = (v1, -)   r2 = (v2, -)
+//   r3 = (n,  |n|)         n = (v1 - v0) x (v2 - v0) (|n| is twice the area)
 struct TriRec {
   float4 r0, r1, r2, r3;
 };
-
-__device__ __forceinline__ float inv_or_zero(float x) { return x > 0.0f ? 1.0f / x : 0.0f; }
 
 // ---------------------------------------------------------------------------------------------
 // Triangle record for distance queries: 80 bytes, five float4s (kept in planes by ptree.cu). Each triangle

@@ -114,12 +114,11 @@ __global__ __launch_bounds__(kThreads) void k_prep(BatchDev B, TriRec *__restric
     {
       const float e1x = b.x - a.x, e1y = b.y - a.y, e1z = b.z - a.z;
       const float e2x = c.x - a.x, e2y = c.y - a.y, e2z = c.z - a.z;
-      const float e3x = c.x - b.x, e3y = c.y - b.y, e3z = c.z - b.z;
       const float nx = e1y * e2z - e1z * e2y, ny = e1z * e2x - e1x * e2z, nz = e1x * e2y - e1y * e2x;
       TriRec r;
-      r.r0 = make_float4(a.x, a.y, a.z, inv_or_zero(e1x * e1x + e1y * e1y + e1z * e1z));
-      r.r1 = make_float4(e1x, e1y, e1z, inv_or_zero(e2x * e2x + e2y * e2y + e2z * e2z));
-      r.r2 = make_float4(e2x, e2y, e2z, inv_or_zero(e3x * e3x + e3y * e3y + e3z * e3z));
+      r.r0 = make_float4(a.x, a.y, a.z, 0.0f);
+      r.r1 = make_float4(b.x, b.y, b.z, 0.0f);
+      r.r2 = make_float4(c.x, c.y, c.z, 0.0f);
       r.r3 = make_float4(nx, ny, nz, sqrtf(nx * nx + ny * ny + nz * nz));
       rec[t] = r;
     }

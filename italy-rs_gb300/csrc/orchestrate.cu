@@ -413,7 +413,7 @@ sdfb_status enqueue_batch(sdfb_ctx *ctx, Workspace &ws, cudaStream_t st, std::ve
     ENSURE(ws.caps_bvh, lbvh_bytes(L.cap_total, K));
     ENSURE(ws.caps_tmp, lbvh_temp_bytes(L.cap_total, K));
   }
-  if (S.any_gwn) ENSURE(ws.gwn_tmp, gwn_temp_bytes(L.gwn_cells));
+  if (S.any_gwn) ENSURE(ws.gwn_tmp, gwn_temp_bytes(L.gwn_cells, L.gtile.back()));
   const uint64_t defer_cap = L.step_budget > 0 ? defer_capacity_for(L.tile.back()) : 0;
   if (defer_cap > 0) ENSURE(ws.defer, defer_cap * 8);
   BvhDev caps;

@@ -1,0 +1,37 @@
+"""Winding-number signs where the grouped walk can go wrong: grids smaller than a tile and just past
+one, single triangles, one wide opening (large caps beside the cells) and overlapping shells, against
+the FP64 sum over every triangle."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _mesh(kind):
+    from sdfb import meshgen as mg
+    if kind == "triangle":
+        return np.array([[-0.3, -0.2, 0.1], [0.35, -0.1, -0.2], [0.0, 0.4, 0.15]], np.float32), np.array([[0, 1, 2]], np.uint32)
+    v, f = mg.displaced_icosphere(3, 0.33, 3)
+    if kind == "bowl":  # a wide opening: its fan of caps crosses the whole mesh
+        return v, np.ascontiguousarray(f[v[f].mean(axis=1)[:, 2] < 0.12])
+    w, g = mg.displaced_icosphere(3, 0.25, 4, center=(0.12, 0.05, -0.1))
+    return mg.delete_faces(*mg.concat([(v, f), (w, g[:, ::-1])]), 0.03, 5)  # opposite orientations
+
+
+@pytest.mark.parametrize("kind", ["triangle", "bowl", "shells"])
+@pytest.mark.parametrize("dims", [(1, 1, 1), (3, 5, 2), (4, 4, 8), (5, 9, 17), (33, 31, 30)])
+def test_group_walk_signs(ctx, oracle, kind, dims):
+    """Every cell whose FP64 winding number is not on the level set, in and out of the band; a cell
+    within 1e-6 of the surface or a cap has no robust side."""
+    import sdfb
+    v, f = _mesh(kind)
+    voxel = 0.9 / max(dims)
+    origin = tuple(-0.5 * voxel * d + 0.003 for d in dims)
+    g = sdfb.make_grid(origin, voxel, dims)
+    d, _ = ctx.bake(v, f, g, sdfb.make_opts(sign_mode=sdfb.SIGN_GWN))
+    w = oracle.gwn(v, f, origin, voxel, dims)
+    d64 = oracle.distance(v, f, origin, voxel, dims)
+    sure = (np.abs(np.abs(w) - 0.5) > 1e-6) & (d64 > 1e-6)
+    assert np.array_equal(d.reshape(-1)[sure] < 0, np.abs(w[sure]) > 0.5)
