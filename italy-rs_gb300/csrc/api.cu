@@ -236,9 +236,10 @@ sdfb_status device_caps(sdfb_ctx *ctx, cudaStream_t st, std::vector<PlanMesh> &m
   return SDFB_OK;
 }
 
-sdfb_status device_signs(sdfb_ctx *ctx, const sdfb_opts &o, PlanMesh *ms, size_t count, cudaStream_t st,
+sdfb_status device_signs(sdfb_ctx *ctx, const sdfb_opts &o, PlanMesh *ms, size_t count, bool needed, cudaStream_t st,
                          size_t *bad) {
   size_t at = 0;
+  if (!needed) return SDFB_OK;
   if (o.sign_mode != SDFB_SIGN_PARITY && o.sign_mode != SDFB_SIGN_GWN && o.sign_mode != SDFB_SIGN_NONE) {
     std::vector<PlanMesh *> v(count);
     for (size_t m = 0; m < count; ++m) v[m] = ms + m;
@@ -359,7 +360,7 @@ sdfb_status sdfb_bake_device(sdfb_ctx *ctx, const float *d_verts, uint32_t num_v
   p.grid = *grid;
   p.dist = o.no_distance ? nullptr : d_dist_out;
   p.occ = o.no_occupancy ? nullptr : d_occ_out;
-  sdfb_status s = device_signs(ctx, o, &p, 1, st);
+  sdfb_status s = device_signs(ctx, o, &p, 1, p.dist || !p.occ || stats, st);
   if (s != SDFB_OK) return s;
   if ((s = device_caps(ctx, st, ms)) != SDFB_OK) return s;
   return run_batch(ctx, st, ms, o, false, stats);
@@ -391,7 +392,7 @@ sdfb_status sdfb_bake(sdfb_ctx *ctx, const float *verts, uint32_t num_verts, con
   p.V = num_verts;
   p.T = num_tris;
   p.grid = *grid;
-  sdfb_status s = device_signs(ctx, o, &p, 1, st);
+  sdfb_status s = device_signs(ctx, o, &p, 1, want_dist || !want_occ || stats, st);
   if (s != SDFB_OK) return s;
   float *const direct_dist =
       (want_dist && p.sign != kSignGwn) ? static_cast<float *>(mapped_host(dist_out)) : nullptr;
@@ -434,35 +435,40 @@ sdfb_status sdfb_bake_soup(sdfb_ctx *ctx, const float *positions, uint32_t num_t
   if (want_occ) ENSURE(ctx->out_occ, cells);
   CK(cudaMemcpyAsync(ctx->in_verts.p, positions, size_t(V) * 12, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(ctx->in_idx.p, ident.data(), size_t(V) * 4, cudaMemcpyHostToDevice, st));
-  // Weld on the device (first occurrence kept) for the watertight gate and for a crack-free
-  // crossing mesh: welded indices in in_idx2, unique positions in in_verts2.
-  const size_t weld_bytes = (weld_temp_bytes(V) + 255) & ~size_t(255);
-  ENSURE(ctx->in_idx2, size_t(V) * 4);
-  ENSURE(ctx->in_verts2, size_t(V) * 12);
-  ENSURE(ctx->weld_tmp, weld_bytes + watertight_temp_bytes(num_tris));
-  if (!ctx->gate_pin.ensure(32)) return ctx_fail(ctx, SDFB_ERR_OUT_OF_MEMORY, "pinned staging");
-  uint32_t *d_welded = static_cast<uint32_t *>(ctx->in_idx2.p);
-  char *d_tmp = static_cast<char *>(ctx->weld_tmp.p);
-  const uint64_t *d_unique = nullptr;
-  CK(weld_enqueue(static_cast<const float *>(ctx->in_verts.p), V, weld_cell(bounds_min, bounds_max), d_welded,
-                  static_cast<float *>(ctx->in_verts2.p), d_tmp, weld_bytes, &d_unique, ctx->num_sms, st));
-  uint64_t *h = static_cast<uint64_t *>(ctx->gate_pin.p);  // unique positions, boundary - 1, non-manifold - 1
-  CK(cudaMemcpyAsync(h, d_unique, 8, cudaMemcpyDeviceToHost, st));
   std::vector<PlanMesh> ms(1);
   PlanMesh &p = ms[0];
-  if (o.sign_mode == SDFB_SIGN_AUTO) {
-    const unsigned long long *d_counts = nullptr;
-    CK(watertight_enqueue(d_welded, num_tris, d_tmp + weld_bytes, watertight_temp_bytes(num_tris), &d_counts,
-                          ctx->num_sms, st));
-    CK(cudaMemcpyAsync(h + 1, d_counts, 16, cudaMemcpyDeviceToHost, st));
-  }
-  CK(cudaStreamSynchronize(st));
-  const uint32_t U = static_cast<uint32_t>(h[0]);
-  if (o.sign_mode == SDFB_SIGN_AUTO) {
-    p.watertight = (h[1] + 1 == 0 && h[2] + 1 == 0) ? 1 : 0;
-    p.sign = p.watertight ? kSignParity : kSignGwn;
-  } else {
-    p.sign = o.sign_mode == SDFB_SIGN_PARITY ? kSignParity : (o.sign_mode == SDFB_SIGN_NONE ? kSignNone : kSignGwn);
+  uint32_t U = 0;
+  uint32_t *d_welded = nullptr;
+  // Occupancy alone, without statistics, needs neither the sign nor the welded crossing mesh.
+  if (want_dist || !want_occ || stats) {
+    // Weld on the device (first occurrence kept) for the watertight gate and for a crack-free
+    // crossing mesh: welded indices in in_idx2, unique positions in in_verts2.
+    const size_t weld_bytes = (weld_temp_bytes(V) + 255) & ~size_t(255);
+    ENSURE(ctx->in_idx2, size_t(V) * 4);
+    ENSURE(ctx->in_verts2, size_t(V) * 12);
+    ENSURE(ctx->weld_tmp, weld_bytes + watertight_temp_bytes(num_tris));
+    if (!ctx->gate_pin.ensure(32)) return ctx_fail(ctx, SDFB_ERR_OUT_OF_MEMORY, "pinned staging");
+    d_welded = static_cast<uint32_t *>(ctx->in_idx2.p);
+    char *d_tmp = static_cast<char *>(ctx->weld_tmp.p);
+    const uint64_t *d_unique = nullptr;
+    CK(weld_enqueue(static_cast<const float *>(ctx->in_verts.p), V, weld_cell(bounds_min, bounds_max), d_welded,
+                    static_cast<float *>(ctx->in_verts2.p), d_tmp, weld_bytes, &d_unique, ctx->num_sms, st));
+    uint64_t *h = static_cast<uint64_t *>(ctx->gate_pin.p);  // unique positions, boundary - 1, non-manifold - 1
+    CK(cudaMemcpyAsync(h, d_unique, 8, cudaMemcpyDeviceToHost, st));
+    if (o.sign_mode == SDFB_SIGN_AUTO) {
+      const unsigned long long *d_counts = nullptr;
+      CK(watertight_enqueue(d_welded, num_tris, d_tmp + weld_bytes, watertight_temp_bytes(num_tris), &d_counts,
+                            ctx->num_sms, st));
+      CK(cudaMemcpyAsync(h + 1, d_counts, 16, cudaMemcpyDeviceToHost, st));
+    }
+    CK(cudaStreamSynchronize(st));
+    U = static_cast<uint32_t>(h[0]);
+    if (o.sign_mode == SDFB_SIGN_AUTO) {
+      p.watertight = (h[1] + 1 == 0 && h[2] + 1 == 0) ? 1 : 0;
+      p.sign = p.watertight ? kSignParity : kSignGwn;
+    } else {
+      p.sign = o.sign_mode == SDFB_SIGN_PARITY ? kSignParity : (o.sign_mode == SDFB_SIGN_NONE ? kSignNone : kSignGwn);
+    }
   }
   p.verts = static_cast<const float *>(ctx->in_verts.p);
   p.idx = static_cast<const uint32_t *>(ctx->in_idx.p);
@@ -630,7 +636,7 @@ sdfb_status voxelize_sparse_run(sdfb_ctx *ctx, const float *positions, uint32_t 
   B.total_tris = num_tris;
   B.total_cells = cells;
   CK(occupancy_batch(B, static_cast<uint32_t *>(ctx->first_tri.p), ctx->sparse_tmp.p, ctx->sparse_tmp.cap, nullptr,
-                     ctx->num_sms, st));
+                     nullptr, ctx->num_sms, st));
   uint64_t total = 0;
   CK(sparse_count(static_cast<const uint8_t *>(ctx->out_occ.p), cells, ctx->sparse_tmp.p, ctx->sparse_tmp.cap, &total,
                   st));
@@ -686,7 +692,7 @@ sdfb_status sdfb_bake_batch_device(sdfb_ctx *ctx, uint32_t count, const sdfb_mes
     p.occ = (o.no_occupancy || !occ_outs) ? nullptr : occ_outs[m];
   }
   size_t bad = 0;
-  sdfb_status s = device_signs(ctx, o, ms.data(), count, st, &bad);
+  sdfb_status s = device_signs(ctx, o, ms.data(), count, !occupancy_alone(ms) || stats, st, &bad);
   if (s == SDFB_ERR_BAD_MESH) {
     const std::string e = ctx->err;
     return ctx_fail(ctx, s, "mesh %zu: %s", bad, e.c_str());
@@ -737,7 +743,7 @@ sdfb_status sdfb_bake_batch(sdfb_ctx *ctx, uint32_t count, const sdfb_mesh_desc 
     oi += size_t(d.num_tris) * 3;
   }
   size_t bad = 0;
-  sdfb_status s = device_signs(ctx, o, ms.data(), count, st, &bad);
+  sdfb_status s = device_signs(ctx, o, ms.data(), count, want_dist || !want_occ || stats, st, &bad);
   if (s == SDFB_ERR_BAD_MESH) {
     const std::string e = ctx->err;
     return ctx_fail(ctx, s, "mesh %zu: %s", bad, e.c_str());

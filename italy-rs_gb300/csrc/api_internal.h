@@ -168,9 +168,13 @@ sdfb_status ctx_fail(sdfb_ctx *ctx, sdfb_status st, const char *fmt, ...);
 sdfb_status ctx_cuda(sdfb_ctx *ctx, cudaError_t e, const char *what);
 // Sign modes of meshes in device memory: forced modes pass through; AUTO runs the weld + watertight
 // gate on the device, for all of them together (parity when watertight, else the winding number).
-// Fails with BAD_MESH on an index out of range (*bad, optional: the mesh).
-sdfb_status device_signs(sdfb_ctx *ctx, const sdfb_opts &o, PlanMesh *ms, size_t count, cudaStream_t st,
+// Fails with BAD_MESH on an index out of range (*bad, optional: the mesh). `needed` false (a bake of
+// occupancy alone that reports no statistics): nothing asks for the sign, and it stays none; the
+// occupancy kernels check the mesh.
+sdfb_status device_signs(sdfb_ctx *ctx, const sdfb_opts &o, PlanMesh *ms, size_t count, bool needed, cudaStream_t st,
                          size_t *bad = nullptr);
+// Whether a batch asks for occupancy grids and nothing else: it needs no hierarchy.
+bool occupancy_alone(const std::vector<PlanMesh> &ms);
 // weld.cu: sets the watertight verdict of indexed meshes in device memory (the weld of their vertices
 // over their bounds, then the edge census of the welded triangles; equivalent to the reference's test
 // on the de-indexed soup). Synchronises the stream. BAD_MESH: mesh *bad has an index >= V.

@@ -171,9 +171,10 @@ cudaError_t lbvh_build(const BatchDev &batch, BvhDev &b, void *temp, size_t temp
 // ---- occupancy.cu -----------------------------------------------------------------------------
 size_t occupancy_temp_bytes(uint64_t total_tris);
 // Clears and fills every mesh's occ grid (meshes with occ == null are skipped). first_tri
-// (optional, for a batch of one) receives per cell the smallest triangle index that hits it.
+// (optional, for a batch of one) receives per cell the smallest triangle index that hits it; err
+// (optional) bad indices and non-finite vertices.
 cudaError_t occupancy_batch(const BatchDev &batch, uint32_t *first_tri, void *temp, size_t temp_bytes,
-                            unsigned long long *sat_tests, int num_sms, cudaStream_t st);
+                            unsigned long long *sat_tests, uint32_t *err, int num_sms, cudaStream_t st);
 
 // ---- parity.cu --------------------------------------------------------------------------------
 // Column crossing lists along +z over the parity and winding-number meshes (their pverts / pidx):

@@ -116,7 +116,7 @@ extern "C" sdfb_status sdfb_occupancy_noalloc(const float *d_verts, uint32_t num
   B.total_cells = cells;
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const cudaError_t e = occupancy_batch(B, nullptr, d + kRecordBytes, kScratchBytes - kRecordBytes, nullptr,
+  const cudaError_t e = occupancy_batch(B, nullptr, d + kRecordBytes, kScratchBytes - kRecordBytes, nullptr, nullptr,
                                         sms > 0 ? sms : 1, st);
   if (e != cudaSuccess) {
     cudaGetLastError();

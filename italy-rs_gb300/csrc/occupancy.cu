@@ -32,8 +32,8 @@ __device__ __forceinline__ f3 vload(const float *v, uint32_t i) {
 
 // Triangle t (global) with its mesh's clamped candidate box. Out-of-range indices read vertex 0
 // (the bake reports the mesh as bad; reads stay in bounds). A mesh without an occupancy output
-// gets an empty box.
-__device__ __forceinline__ TriCells tri_cells(const BatchDev &B, uint64_t t) {
+// gets an empty box. err (optional): bad indices and non-finite vertices are flagged there.
+__device__ __forceinline__ TriCells tri_cells(const BatchDev &B, uint64_t t, uint32_t *err = nullptr) {
   TriCells r;
   r.mesh = find_mesh(B.tri_starts, B.num_meshes, t);
   const MeshRec &M = B.recs[r.mesh];
@@ -43,6 +43,12 @@ __device__ __forceinline__ TriCells tri_cells(const BatchDev &B, uint64_t t) {
   r.a = vload(M.verts, i0 < V ? i0 : 0);
   r.b = vload(M.verts, i1 < V ? i1 : 0);
   r.c = vload(M.verts, i2 < V ? i2 : 0);
+  if (err) {
+    if (i0 >= V || i1 >= V || i2 >= V) atomic_or_err(err, kErrBadIndex);
+    if (!isfinite(r.a.x) || !isfinite(r.a.y) || !isfinite(r.a.z) || !isfinite(r.b.x) || !isfinite(r.b.y) ||
+        !isfinite(r.b.z) || !isfinite(r.c.x) || !isfinite(r.c.y) || !isfinite(r.c.z))
+      atomic_or_err(err, kErrNonFinite);
+  }
   const GridDev &g = M.g;
   const float mn[3] = {min_ref(min_ref(r.a.x, r.b.x), r.c.x), min_ref(min_ref(r.a.y, r.b.y), r.c.y),
                        min_ref(min_ref(r.a.z, r.b.z), r.c.z)};
@@ -64,10 +70,10 @@ __device__ __forceinline__ TriCells tri_cells(const BatchDev &B, uint64_t t) {
 
 // Candidate cells per triangle, as 64-bit counts: one triangle across a large grid can have more
 // than 2^32 candidate cells.
-__global__ __launch_bounds__(kThreads) void k_occ_items(BatchDev B, uint64_t *__restrict__ items) {
+__global__ __launch_bounds__(kThreads) void k_occ_items(BatchDev B, uint64_t *__restrict__ items, uint32_t *err) {
   const uint64_t t = uint64_t(blockIdx.x) * kThreads + threadIdx.x;
   if (t >= B.total_tris) return;
-  const TriCells tc = tri_cells(B, t);
+  const TriCells tc = tri_cells(B, t, err);
   if (tc.hi[0] < tc.lo[0]) {
     items[t] = 0;
     return;
@@ -196,7 +202,7 @@ size_t occ_layout(uint64_t T, char *base, OccTemp *o) {
 size_t occupancy_temp_bytes(uint64_t total_tris) { return occ_layout(total_tris, nullptr, nullptr); }
 
 cudaError_t occupancy_batch(const BatchDev &B, uint32_t *first_tri, void *temp, size_t temp_bytes,
-                            unsigned long long *sat_tests, int num_sms, cudaStream_t st) {
+                            unsigned long long *sat_tests, uint32_t *err, int num_sms, cudaStream_t st) {
   const uint64_t T = B.total_tris;
   cudaError_t e;
   if (B.total_cells) {
@@ -211,7 +217,7 @@ cudaError_t occupancy_batch(const BatchDev &B, uint32_t *first_tri, void *temp, 
   if (T == 0) return cudaGetLastError();
   OccTemp o;
   if (occ_layout(T, static_cast<char *>(temp), &o) > temp_bytes) return cudaErrorMemoryAllocation;
-  k_occ_items<<<static_cast<unsigned>((T + kThreads - 1) / kThreads), kThreads, 0, st>>>(B, o.items);
+  k_occ_items<<<static_cast<unsigned>((T + kThreads - 1) / kThreads), kThreads, 0, st>>>(B, o.items, err);
   note_launch();
   if ((e = exclusive_scan_u64(o.items, o.starts, T, Scratch{o.scratch, o.scratch_bytes}, st)) != cudaSuccess) return e;
   if (first_tri)
@@ -236,7 +242,7 @@ cudaError_t occupancy_hits(const BatchDev &B, void *temp, size_t temp_bytes, uin
   if (T == 0) return cudaGetLastError();
   OccTemp o;
   if (occ_layout(T, static_cast<char *>(temp), &o) > temp_bytes) return cudaErrorMemoryAllocation;
-  k_occ_items<<<static_cast<unsigned>((T + kThreads - 1) / kThreads), kThreads, 0, st>>>(B, o.items);
+  k_occ_items<<<static_cast<unsigned>((T + kThreads - 1) / kThreads), kThreads, 0, st>>>(B, o.items, nullptr);
   note_launch();
   if ((e = exclusive_scan_u64(o.items, o.starts, T, Scratch{o.scratch, o.scratch_bytes}, st)) != cudaSuccess) return e;
   HitSink sink;

@@ -366,6 +366,11 @@ BatchDev caps_dev(const Layout &L, char *d) {
 
 }  // namespace
 
+bool occupancy_alone(const std::vector<PlanMesh> &ms) {
+  return std::none_of(ms.begin(), ms.end(), [](const PlanMesh &p) { return p.dist != nullptr; }) &&
+         std::any_of(ms.begin(), ms.end(), [](const PlanMesh &p) { return p.occ != nullptr; });
+}
+
 sdfb_status enqueue_batch(sdfb_ctx *ctx, Workspace &ws, cudaStream_t st, std::vector<PlanMesh> &ms,
                           const sdfb_opts &o, bool use_graph, BatchState &S) {
   if (ms.empty()) return ctx_fail(ctx, SDFB_ERR_INVALID_ARGUMENT, "empty batch");
@@ -393,7 +398,7 @@ sdfb_status enqueue_batch(sdfb_ctx *ctx, Workspace &ws, cudaStream_t st, std::ve
   S.stack = L.stack;
   S.leaf0 = L.recs[0].leaf_size;
   const bool any_occ = std::any_of(ms.begin(), ms.end(), [](const PlanMesh &p) { return p.occ != nullptr; });
-  const bool build = !L.resident;
+  const bool build = !L.resident && !occupancy_alone(ms);
 
   // Workspace.
   ENSURE(ws.batch_buf, L.bytes);
@@ -471,7 +476,7 @@ sdfb_status enqueue_batch(sdfb_ctx *ctx, Workspace &ws, cudaStream_t st, std::ve
     CK(rec(ws.ev[1]));
     if (any_occ) {
       NvtxRange r("sdfb occupancy");
-      CK(occupancy_batch(B, nullptr, ws.build_tmp.p, ws.build_tmp.cap, d_sat, ctx->num_sms, st));
+      CK(occupancy_batch(B, nullptr, ws.build_tmp.p, ws.build_tmp.cap, d_sat, d_err, ctx->num_sms, st));
     }
     CK(rec(ws.ev[2]));
     if (S.any_cross) {

@@ -654,7 +654,7 @@ sdfb_status sdfb_mesh_register(sdfb_server *srv, const float *verts, uint32_t nu
   gate.idx = static_cast<const uint32_t *>(r->idx.p);
   gate.V = num_verts;
   gate.T = num_tris;
-  const sdfb_status gs = device_signs(rc, auto_opts, &gate, 1, st);
+  const sdfb_status gs = device_signs(rc, auto_opts, &gate, 1, true, st);
   if (gs != SDFB_OK) return undo(gs, rc->err);
   r->sign = gate.sign;
   r->watertight = gate.watertight;
