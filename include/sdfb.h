@@ -349,7 +349,7 @@ const char *sdfb_server_last_error(const sdfb_server *srv);
  * allocator and cudaFree's device-wide synchronisation. All buffers are device memory supplied by
  * the caller;
  * work is enqueued on `stream` (a cudaStream_t, NULL = the legacy default stream) and not waited
- * for. Working memory is one fixed device array inside the library (about 16 MiB, held on every
+ * for. Working memory is one fixed device array inside the library (about 8 MiB, held on every
  * device that loads the library until the process exits), so:
  *   - meshes above 1,048,576 triangles are rejected with SDFB_ERR_INVALID_ARGUMENT;
  *   - the first call on each device sets up the array's address and must come before any stream

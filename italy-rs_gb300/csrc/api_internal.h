@@ -100,15 +100,17 @@ struct GwnInput {
 
 // Workspace::misc (256 bytes, zeroed before every bake): error flags at 0, the distance tile
 // counter at 64, work counters at 128 (box, triangle, SAT, plane tests), the deferral counters at
-// 160.
+// 192, the crossings at 216.
 constexpr size_t kMiscDeferOffset = 192;
+constexpr size_t kMiscCrossOffset = 216;
 // Steps of work between a distance tile's looks at whether it should go to the block-per-tile pass.
 constexpr int kDefaultStepBudget = 2048;
 
 // Device workspace of one bake in flight. The context owns one; the serving loop owns one per
 // stream so consecutive waves overlap.
 struct Workspace {
-  DevBuf batch_buf, bvh, build_tmp, par_tmp, col_start, col_z, col_s, caps_bvh, caps_tmp, misc, gwn_tmp, defer;
+  DevBuf batch_buf, bvh, build_tmp, par_tmp, col_start, col_z, col_s, caps_bvh, caps_tmp, misc, gwn_tmp, defer,
+      col_bits;
   PinBuf staging;
   cudaEvent_t ev[8] = {};
   uint64_t col_capacity_hint = 0;

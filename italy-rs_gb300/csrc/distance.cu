@@ -41,9 +41,9 @@
 // of one level from a shared counter and walk below them for the same cells, whose bounds they
 // share in shared memory (atomicMin on the float bits, valid for non-negative values).
 //
-// Sign: parity counts the column's crossing heights above each cell (the crossing list is
-// built by parity.cu). Winding-number signs are applied afterwards by gwn.cu, which needs the
-// unsigned distance to find the near-surface band.
+// Sign: parity counts the column's crossing bits at and above each cell (parity.cu). Winding-number
+// signs are applied afterwards by gwn.cu, which needs the unsigned distance to find the near-surface
+// band.
 #include <algorithm>
 #include <climits>
 #include <cstdint>
@@ -590,24 +590,24 @@ __device__ __forceinline__ void store_cells(const DistanceArgs &a, const TileCel
                                             const uint32_t *best) {
   constexpr int VPL = TileCells<TX, TY, TZ>::VPL;
   const MeshRec &M = *c.M;
-  int inside[VPL];
-#pragma unroll
-  for (int v = 0; v < VPL; ++v) inside[v] = 0;
+  // A cell is inside when an odd number of its column's bits lie at or above its layer. The tile's
+  // layers share a word (their first is a multiple of their number, which divides 32).
+  static_assert(32 % TZ == 0, "a tile's layers lie in one word");
+  uint32_t word = 0, above = 0;
   const int vx = c.vx(lane), vy = c.vy(lane);
-  if (M.sign == kSignParity && vx < c.g.nx && vy < c.g.ny) {
-    const uint64_t col = M.col_base + uint64_t(vy) * c.g.nx + vx;
-    const uint64_t s0 = __ldg(a.col_start + col), s1 = __ldg(a.col_start + col + 1);
-    for (uint64_t k = s0; k < s1; ++k) {
-      const float zc = __ldg(a.col_z + k);
-#pragma unroll
-      for (int v = 0; v < VPL; ++v) inside[v] ^= zc > c.pz(lane, v) ? 1 : 0;
-    }
+  const bool parity = M.sign == kSignParity && vx < c.g.nx && vy < c.g.ny;
+  if (parity) {
+    const int words = (c.g.nz + 31) / 32;
+    const uint32_t *col = a.bits + M.bit_base + (uint64_t(vy) * c.g.nx + vx) * words;
+    word = __ldg(col + c.z0 / 32);
+    for (int k = c.z0 / 32 + 1; k < words; ++k) above ^= __ldg(col + k);
   }
 #pragma unroll
   for (int v = 0; v < VPL; ++v) {
     if (!c.active(lane, v)) continue;
     const float d = sqrtf(__uint_as_float(best[v * kWarp + lane]));
-    M.dist[c.cell(lane, v)] = inside[v] ? -d : d;
+    const bool inside = (__popc(word >> (c.vz(lane, v) & 31)) + __popc(above)) & 1;
+    M.dist[c.cell(lane, v)] = inside ? -d : d;
   }
 }
 

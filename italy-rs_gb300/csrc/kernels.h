@@ -95,7 +95,8 @@ struct MeshRec {
   uint32_t num_verts, num_tris, pnum_verts, pnum_tris;
   uint64_t tri_base;      // first global triangle = first sorted position of this mesh
   uint64_t cell_base;     // first global cell
-  uint64_t col_base;      // first global column (parity meshes only)
+  uint64_t col_base;      // first global column (winding-number meshes only)
+  uint64_t bit_base;      // first word of the crossing bits (parity meshes only)
   GridDev g;
   int sign;               // SignKind
   int leaf_size;          // 1..16
@@ -122,7 +123,8 @@ struct BatchDev {
   const uint64_t *tile_starts = nullptr;      // distance tiles
   const uint64_t *gwn_tile_starts = nullptr;  // winding-number tiles (only GWN meshes have any)
   const uint64_t *cell_starts = nullptr;      // cells
-  uint64_t total_tris = 0, total_ptris = 0, total_cells = 0, total_cols = 0, total_tiles = 0, total_gwn_tiles = 0;
+  uint64_t total_tris = 0, total_ptris = 0, total_cells = 0, total_cols = 0, total_tiles = 0, total_gwn_tiles = 0,
+           total_bit_words = 0;
 };
 
 // Largest m in [0, n) with starts[m] <= x (starts[0] = 0).
@@ -177,18 +179,19 @@ cudaError_t occupancy_batch(const BatchDev &batch, uint32_t *first_tri, void *te
                             unsigned long long *sat_tests, uint32_t *err, int num_sms, cudaStream_t st);
 
 // ---- parity.cu --------------------------------------------------------------------------------
-// Column crossing lists along +z over the parity and winding-number meshes (their pverts / pidx):
-// col_start[total_cols + 1] (uint64 starts), col_z[capacity] heights, col_s[capacity] orientations.
+// Crossings of the columns' +z lines with the meshes' pverts / pidx. Parity meshes: bits, per column
+// ceil(nz / 32) words (total_bit_words in all), toggled at the highest layer below each crossing.
+// Winding-number meshes: lists, col_start[total_cols + 1] (uint64 starts), col_z[capacity] heights,
+// col_s[capacity] orientations. *crossings (zeroed by the caller) counts them all.
 size_t parity_temp_bytes(uint64_t total_ptris, uint64_t total_cols);
-cudaError_t parity_columns(const BatchDev &batch, uint64_t *col_start, float *col_z, int8_t *col_s,
-                           uint64_t capacity, void *temp, size_t temp_bytes, uint32_t *err, int num_sms,
-                           cudaStream_t st);
+cudaError_t parity_columns(const BatchDev &batch, uint32_t *bits, uint64_t *col_start, float *col_z, int8_t *col_s,
+                           uint64_t capacity, void *temp, size_t temp_bytes, unsigned long long *crossings,
+                           uint32_t *err, int num_sms, cudaStream_t st);
 
 // ---- distance.cu ------------------------------------------------------------------------------
 struct DistanceArgs {
   BatchDev batch;             // each mesh record names its hierarchy and root
-  const uint64_t *col_start;  // parity
-  const float *col_z;
+  const uint32_t *bits;       // parity: crossing bits
   uint32_t *err;
   unsigned long long *tile_counter;   // pass A's chunk counter, zeroed by the launcher
   unsigned long long chunk_tiles;     // tiles per chunk (set by the launcher)

@@ -38,9 +38,8 @@ namespace {
 
 constexpr uint32_t kNoAllocMaxTris = 1u << 20;  // 1,048,576 triangles
 constexpr size_t kRecordBytes = 4096;           // one MeshRec and its prefix tables
-// Candidate counts (8 B per triangle), their exclusive scan (8 B per triangle + 1), the scan's
-// block sums, plus alignment slack: about 16 MiB in all.
-constexpr size_t kScratchBytes = kRecordBytes + size_t(kNoAllocMaxTris) * 16 + (size_t(1) << 16);
+// The list of triangles with many candidate cells (8 B per triangle) and its counts: about 8 MiB.
+constexpr size_t kScratchBytes = kRecordBytes + size_t(kNoAllocMaxTris) * 8 + (size_t(1) << 16);
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 

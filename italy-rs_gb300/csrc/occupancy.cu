@@ -1,9 +1,6 @@
-// Dense occupancy: the reference's candidate-cell loop (src/convert/sdf_baker.cpp:89-118) as a
-// load-balanced expansion over (triangle, candidate cell) items.
-//
-// k_occ_items counts each triangle's clamped candidate box with the reference's FP32 rounding;
-// an exclusive scan turns the counts into item starts; k_occ_test takes chunks of items, runs the
-// exact-rounding SAT test (common.cuh) and stores 1 for hits. Several triangles may store 1 into
+// Dense occupancy: the reference's candidate-cell loop (src/convert/sdf_baker.cpp:89-118), one item
+// per (triangle, candidate cell) of the triangle's clamped candidate box (expand.cuh), each running the
+// exact-rounding SAT test (common.cuh) and storing 1 for a hit. Several triangles may store 1 into
 // the same byte; the stores carry the same value, so no atomics are needed and the result does
 // not depend on their order.
 #include <algorithm>
@@ -18,12 +15,11 @@ namespace {
 
 constexpr int kThreads = 256;
 
-inline size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
-
 struct TriCells {
   f3 a, b, c;
   int lo[3], hi[3];
   int mesh;
+  uint32_t local;  // index within the mesh
 };
 
 __device__ __forceinline__ f3 vload(const float *v, uint32_t i) {
@@ -38,6 +34,7 @@ __device__ __forceinline__ TriCells tri_cells(const BatchDev &B, uint64_t t, uin
   r.mesh = find_mesh(B.tri_starts, B.num_meshes, t);
   const MeshRec &M = B.recs[r.mesh];
   const uint64_t lt = t - B.tri_starts[r.mesh];
+  r.local = static_cast<uint32_t>(lt);
   const uint32_t V = M.num_verts;
   const uint32_t i0 = __ldg(M.idx + 3 * lt), i1 = __ldg(M.idx + 3 * lt + 1), i2 = __ldg(M.idx + 3 * lt + 2);
   r.a = vload(M.verts, i0 < V ? i0 : 0);
@@ -68,23 +65,11 @@ __device__ __forceinline__ TriCells tri_cells(const BatchDev &B, uint64_t t, uin
   return r;
 }
 
-// Candidate cells per triangle, as 64-bit counts: one triangle across a large grid can have more
-// than 2^32 candidate cells.
-__global__ __launch_bounds__(kThreads) void k_occ_items(BatchDev B, uint64_t *__restrict__ items, uint32_t *err) {
-  const uint64_t t = uint64_t(blockIdx.x) * kThreads + threadIdx.x;
-  if (t >= B.total_tris) return;
-  const TriCells tc = tri_cells(B, t, err);
-  if (tc.hi[0] < tc.lo[0]) {
-    items[t] = 0;
-    return;
-  }
-  items[t] = uint64_t(tc.hi[0] - tc.lo[0] + 1) * uint64_t(tc.hi[1] - tc.lo[1] + 1) * uint64_t(tc.hi[2] - tc.lo[2] + 1);
-}
-
 // Clears the occupancy grids of the batch (one pass over the global cells). A thread clears 16
 // consecutive cells, with one 16-byte store where they lie in one mesh's grid at an aligned
-// address (so a warp writes 512 contiguous bytes), else byte by byte.
-__global__ __launch_bounds__(kThreads) void k_occ_clear(BatchDev B) {
+// address (so a warp writes 512 contiguous bytes), else byte by byte. Clears the list's counts too.
+__global__ __launch_bounds__(kThreads) void k_occ_clear(BatchDev B, BigList big) {
+  if (blockIdx.x == 0 && threadIdx.x < 2) big.counts[threadIdx.x] = 0;
   const uint64_t stride = uint64_t(gridDim.x) * kThreads * 16;
   for (uint64_t c0 = (uint64_t(blockIdx.x) * kThreads + threadIdx.x) * 16; c0 < B.total_cells; c0 += stride) {
     int m = find_mesh(B.cell_starts, B.num_meshes, c0);
@@ -129,130 +114,93 @@ __device__ __forceinline__ void append_hit(const HitSink &h, bool hit, uint64_t 
   }
 }
 
-template <bool FIRST, bool HITS>
-__global__ __launch_bounds__(kThreads) void k_occ_test(BatchDev B, const uint64_t *__restrict__ starts,
-                                                       uint32_t *__restrict__ first_tri,
-                                                       unsigned long long *__restrict__ sat_tests, HitSink sink) {
-  const uint64_t T = B.total_tris;
-  const uint64_t total = starts[T];
-  const uint64_t stride = uint64_t(gridDim.x) * kThreads * kExpandChunk;
-  unsigned long long tests = 0;
-  for (uint64_t w0 = (uint64_t(blockIdx.x) * kThreads + threadIdx.x) * kExpandChunk; w0 < total; w0 += stride) {
-    uint64_t t = item_owner(starts, static_cast<uint32_t>(T), w0);
-    TriCells tc = tri_cells(B, t);
-    uint64_t tstart = starts[t], tend = starts[t + 1];
-    const uint64_t wend = min(w0 + kExpandChunk, total);
-    for (uint64_t w = w0; w < wend; ++w) {
-      while (w >= tend) {
-        ++t;
-        tstart = tend;
-        tend = starts[t + 1];
-        if (tend > tstart) tc = tri_cells(B, t);
-      }
-      const MeshRec &M = B.recs[tc.mesh];
-      const GridDev &g = M.g;
-      const uint64_t k = w - tstart;
-      const uint32_t sx = tc.hi[0] - tc.lo[0] + 1, sy = tc.hi[1] - tc.lo[1] + 1;
-      const int x = tc.lo[0] + static_cast<int>(k % sx);
-      const int y = tc.lo[1] + static_cast<int>((k / sx) % sy);
-      const int z = tc.lo[2] + static_cast<int>(k / (uint64_t(sx) * sy));
-      const f3 c = {cell_center(g.ox, x, g.voxel), cell_center(g.oy, y, g.voxel), cell_center(g.oz, z, g.voxel)};
-      ++tests;
-      const bool hit = sat_overlap(c, __fmul_rn(g.voxel, 0.5f), tc.a, tc.b, tc.c);
-      const uint64_t cell = (uint64_t(z) * g.ny + y) * g.nx + x;
-      if (hit) {
-        M.occ[cell] = 1;
-        if (FIRST) atomicMin(first_tri + cell, static_cast<uint32_t>(t - B.tri_starts[tc.mesh]));
-      }
-      if (HITS) append_hit(sink, hit, (cell << sink.tri_bits) | (t - B.tri_starts[tc.mesh]));
-    }
-  }
-  if (sat_tests) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) tests += __shfl_xor_sync(kFull, tests, o);
-    if ((threadIdx.x & 31) == 0 && tests) atomicAdd(sat_tests, tests);
-  }
-}
+template <bool FIRST, bool HITS> struct OccOp {
+  using Tri = TriCells;
+  uint32_t *first_tri;
+  unsigned long long *sat_tests;
+  uint32_t *err;
+  HitSink sink;
 
-struct OccTemp {
-  uint64_t *items;
-  uint64_t *starts;
-  void *scratch;
-  size_t scratch_bytes;
+  // Candidate cells, as a 64-bit count: a triangle across a large grid can have more than 2^32.
+  __device__ __forceinline__ uint64_t setup(const BatchDev &B, uint64_t t, Tri &tri) const {
+    tri = tri_cells(B, t, err);
+    if (tri.hi[0] < tri.lo[0]) return 0;
+    return uint64_t(tri.hi[0] - tri.lo[0] + 1) * uint64_t(tri.hi[1] - tri.lo[1] + 1) *
+           uint64_t(tri.hi[2] - tri.lo[2] + 1);
+  }
+  __device__ __forceinline__ void item(const BatchDev &B, const Tri &tri, uint64_t k) const {
+    const MeshRec &M = B.recs[tri.mesh];
+    const GridDev &g = M.g;
+    const uint32_t sx = tri.hi[0] - tri.lo[0] + 1, sy = tri.hi[1] - tri.lo[1] + 1;
+    int dx, dy, dz;
+    if ((k >> 32) == 0) {  // 32-bit divisions where they do
+      const uint32_t k32 = static_cast<uint32_t>(k), row = k32 / sx;
+      dx = static_cast<int>(k32 - row * sx);
+      dz = static_cast<int>(row / sy);
+      dy = static_cast<int>(row - dz * sy);
+    } else {
+      dx = static_cast<int>(k % sx);
+      dy = static_cast<int>((k / sx) % sy);
+      dz = static_cast<int>(k / (uint64_t(sx) * sy));
+    }
+    const int x = tri.lo[0] + dx, y = tri.lo[1] + dy, z = tri.lo[2] + dz;
+    const f3 c = {cell_center(g.ox, x, g.voxel), cell_center(g.oy, y, g.voxel), cell_center(g.oz, z, g.voxel)};
+    const bool hit = sat_overlap(c, __fmul_rn(g.voxel, 0.5f), tri.a, tri.b, tri.c);
+    const uint64_t cell = (uint64_t(z) * g.ny + y) * g.nx + x;
+    if (hit) {
+      M.occ[cell] = 1;
+      if (FIRST) atomicMin(first_tri + cell, tri.local);
+    }
+    if (HITS) append_hit(sink, hit, (cell << sink.tri_bits) | tri.local);
+  }
+  __device__ __forceinline__ void finish(const BatchDev &, unsigned long long items) const {
+    if (sat_tests && items && threadIdx.x == 0) atomicAdd(sat_tests, items);
+  }
 };
 
-size_t occ_layout(uint64_t T, char *base, OccTemp *o) {
-  size_t off = 0;
-  auto take = [&](size_t bytes) {
-    char *p = base ? base + off : nullptr;
-    off += align256(bytes);
-    return p;
-  };
-  OccTemp x;
-  x.items = reinterpret_cast<uint64_t *>(take(size_t(T) * 8 + 8));
-  x.starts = reinterpret_cast<uint64_t *>(take((size_t(T) + 1) * 8));
-  x.scratch_bytes = scan_scratch_bytes(T);
-  x.scratch = take(x.scratch_bytes);
-  if (o) *o = x;
-  return off;
+cudaError_t clear(const BatchDev &B, const BigList &big, int num_sms, cudaStream_t st) {
+  const uint64_t blocks = std::max<uint64_t>(
+      1, std::min<uint64_t>((B.total_cells + kThreads * 16 - 1) / (kThreads * 16), uint64_t(num_sms) * 16));
+  k_occ_clear<<<static_cast<unsigned>(blocks), kThreads, 0, st>>>(B, big);
+  note_launch();
+  return cudaGetLastError();
 }
 
 }  // namespace
 
-size_t occupancy_temp_bytes(uint64_t total_tris) { return occ_layout(total_tris, nullptr, nullptr); }
+size_t occupancy_temp_bytes(uint64_t total_tris) { return big_list_bytes(total_tris); }
 
 cudaError_t occupancy_batch(const BatchDev &B, uint32_t *first_tri, void *temp, size_t temp_bytes,
                             unsigned long long *sat_tests, uint32_t *err, int num_sms, cudaStream_t st) {
   const uint64_t T = B.total_tris;
-  cudaError_t e;
-  if (B.total_cells) {
-    const uint64_t blocks = std::min<uint64_t>((B.total_cells + kThreads * 16 - 1) / (kThreads * 16), uint64_t(num_sms) * 16);
-    k_occ_clear<<<static_cast<unsigned>(blocks), kThreads, 0, st>>>(B);
-    note_launch();
-  }
+  if (big_list_bytes(T) > temp_bytes) return cudaErrorMemoryAllocation;
+  const BigList big = big_list(temp, T);
+  cudaError_t e = clear(B, big, num_sms, st);
+  if (e != cudaSuccess) return e;
   if (first_tri) {
     if (B.num_meshes != 1) return cudaErrorInvalidValue;
     if ((e = cudaMemsetAsync(first_tri, 0xff, B.total_cells * 4, st)) != cudaSuccess) return e;
   }
-  if (T == 0) return cudaGetLastError();
-  OccTemp o;
-  if (occ_layout(T, static_cast<char *>(temp), &o) > temp_bytes) return cudaErrorMemoryAllocation;
-  k_occ_items<<<static_cast<unsigned>((T + kThreads - 1) / kThreads), kThreads, 0, st>>>(B, o.items, err);
-  note_launch();
-  if ((e = exclusive_scan_u64(o.items, o.starts, T, Scratch{o.scratch, o.scratch_bytes}, st)) != cudaSuccess) return e;
-  if (first_tri)
-    k_occ_test<true, false><<<num_sms * 8, kThreads, 0, st>>>(B, o.starts, first_tri, sat_tests, HitSink());
-  else
-    k_occ_test<false, false><<<num_sms * 8, kThreads, 0, st>>>(B, o.starts, nullptr, sat_tests, HitSink());
-  note_launch();
-  return cudaGetLastError();
+  if (T == 0) return cudaSuccess;
+  if (first_tri) return expand(B, T, big, OccOp<true, false>{first_tri, sat_tests, err, HitSink()}, num_sms, st);
+  return expand(B, T, big, OccOp<false, false>{nullptr, sat_tests, err, HitSink()}, num_sms, st);
 }
 
 cudaError_t occupancy_hits(const BatchDev &B, void *temp, size_t temp_bytes, uint64_t *keys, uint64_t capacity,
                            unsigned long long *hit_count, int tri_bits, int num_sms, cudaStream_t st) {
   if (B.num_meshes != 1) return cudaErrorInvalidValue;
   const uint64_t T = B.total_tris;
+  if (big_list_bytes(T) > temp_bytes) return cudaErrorMemoryAllocation;
+  const BigList big = big_list(temp, T);
   cudaError_t e = cudaMemsetAsync(hit_count, 0, sizeof(unsigned long long), st);
-  if (e != cudaSuccess) return e;
-  if (B.total_cells) {
-    const uint64_t blocks = std::min<uint64_t>((B.total_cells + kThreads * 16 - 1) / (kThreads * 16), uint64_t(num_sms) * 16);
-    k_occ_clear<<<static_cast<unsigned>(blocks), kThreads, 0, st>>>(B);
-    note_launch();
-  }
-  if (T == 0) return cudaGetLastError();
-  OccTemp o;
-  if (occ_layout(T, static_cast<char *>(temp), &o) > temp_bytes) return cudaErrorMemoryAllocation;
-  k_occ_items<<<static_cast<unsigned>((T + kThreads - 1) / kThreads), kThreads, 0, st>>>(B, o.items, nullptr);
-  note_launch();
-  if ((e = exclusive_scan_u64(o.items, o.starts, T, Scratch{o.scratch, o.scratch_bytes}, st)) != cudaSuccess) return e;
+  if (e != cudaSuccess || (e = clear(B, big, num_sms, st)) != cudaSuccess) return e;
+  if (T == 0) return cudaSuccess;
   HitSink sink;
   sink.keys = keys;
   sink.capacity = capacity;
   sink.count = hit_count;
   sink.tri_bits = tri_bits;
-  k_occ_test<false, true><<<num_sms * 8, kThreads, 0, st>>>(B, o.starts, nullptr, nullptr, sink);
-  note_launch();
-  return cudaGetLastError();
+  return expand(B, T, big, OccOp<false, true>{nullptr, nullptr, nullptr, sink}, num_sms, st);
 }
 
 }  // namespace sdfb

@@ -1,7 +1,7 @@
 // The batch orchestrator behind every bake entry point.
 //
 //   upload mesh records + prefix tables -> a packed tree per mesh (ptree.cu) -> occupancy
-//   (occupancy.cu) -> +z crossing lists of the parity and winding-number meshes (parity.cu) ->
+//   (occupancy.cu) -> +z crossings of the parity and winding-number meshes (parity.cu) ->
 //   caps hierarchy for the winding number (lbvh.cu) -> distance with fused parity sign, one persistent
 //   launch over every mesh's tiles (distance.cu) -> winding-number signs (gwn.cu)
 //
@@ -132,14 +132,14 @@ void Workspace::release() {
     graph_key.clear();
   }
   DevBuf *b[] = {&batch_buf, &bvh, &build_tmp, &par_tmp, &col_start, &col_z, &col_s, &caps_bvh, &caps_tmp, &misc,
-                 &gwn_tmp, &defer};
+                 &gwn_tmp, &defer, &col_bits};
   for (DevBuf *x : b) x->release();
   staging.release();
 }
 
 uint64_t Workspace::bytes() const {
   const DevBuf *b[] = {&batch_buf, &bvh, &build_tmp, &par_tmp, &col_start, &col_z, &col_s, &caps_bvh, &caps_tmp,
-                       &misc, &gwn_tmp, &defer};
+                       &misc, &gwn_tmp, &defer, &col_bits};
   uint64_t s = 0;
   for (const DevBuf *x : b) s += x->cap;
   return s;
@@ -156,7 +156,7 @@ struct Layout {
   std::vector<MeshRec> recs, cap_recs;
   std::vector<PTreeRec> trees;
   std::vector<uint64_t> tri, ptri, tile, gtile, cell, group, cap_tri, cap_zero;
-  uint64_t total_cols = 0, gwn_cells = 0, cap_total = 0;
+  uint64_t total_cols = 0, bit_words = 0, gwn_cells = 0, cap_total = 0;
   int tile_id = 2, stack = 64;
   long long step_budget = 0;
   bool resident = false;
@@ -236,7 +236,10 @@ void make_layout(sdfb_ctx *ctx, const std::vector<PlanMesh> &ms, const sdfb_opts
     const bool crossings = r.sign == kSignParity || r.sign == kSignGwn;
     L.ptri[m + 1] = L.ptri[m] + (crossings ? r.pnum_tris : 0);
     r.col_base = cols;
-    if (crossings) cols += uint64_t(p.grid.nx) * p.grid.ny;
+    r.bit_base = L.bit_words;
+    const uint64_t mesh_cols = uint64_t(p.grid.nx) * p.grid.ny;
+    if (r.sign == kSignGwn) cols += mesh_cols;
+    if (r.sign == kSignParity) L.bit_words += mesh_cols * ((uint64_t(p.grid.nz) + 31) / 32);
     L.tile[m + 1] = L.tile[m] + (p.dist ? tiles_for(r.g, L.tile_id) : 0);
     const bool gwn = p.dist && r.sign == kSignGwn;
     L.gtile[m + 1] = L.gtile[m] + (gwn ? uint64_t((p.grid.nx + 3) / 4) * uint64_t((p.grid.ny + 3) / 4) *
@@ -348,6 +351,7 @@ BatchDev batch_dev(const Layout &L, char *d) {
   B.total_ptris = L.ptri.back();
   B.total_cells = L.cell.back();
   B.total_cols = L.total_cols;
+  B.total_bit_words = L.bit_words;
   B.total_tiles = L.tile.back();
   B.total_gwn_tiles = L.gtile.back();
   return B;
@@ -408,8 +412,10 @@ sdfb_status enqueue_batch(sdfb_ctx *ctx, Workspace &ws, cudaStream_t st, std::ve
   ENSURE(ws.misc, 256);
   if (S.any_cross) {
     ENSURE(ws.par_tmp, parity_temp_bytes(L.ptri.back(), L.total_cols));
+    if (L.bit_words) ENSURE(ws.col_bits, L.bit_words * 4);
     ENSURE(ws.col_start, (L.total_cols + 1) * 8);
-    const uint64_t want = std::max<uint64_t>(ws.col_capacity_hint, 4 * L.total_cols + 2 * L.ptri.back());
+    const uint64_t lists = L.total_cols ? 4 * L.total_cols + 2 * L.ptri.back() : 0;
+    const uint64_t want = std::max<uint64_t>(ws.col_capacity_hint, lists);
     ENSURE(ws.col_z, want * 4);
     ENSURE(ws.col_s, want);
     S.capacity = std::min<uint64_t>(ws.col_z.cap / 4, ws.col_s.cap);
@@ -433,8 +439,7 @@ sdfb_status enqueue_batch(sdfb_ctx *ctx, Workspace &ws, cudaStream_t st, std::ve
   unsigned long long *d_sat = d_work + 2;
   DistanceArgs da{};
   da.batch = B;
-  da.col_start = static_cast<const uint64_t *>(ws.col_start.p);
-  da.col_z = static_cast<const float *>(ws.col_z.p);
+  da.bits = static_cast<const uint32_t *>(ws.col_bits.p);
   da.err = d_err;
   da.tile_counter = d_tile;
   da.work_counters = o.count_work ? d_work : nullptr;
@@ -481,9 +486,11 @@ sdfb_status enqueue_batch(sdfb_ctx *ctx, Workspace &ws, cudaStream_t st, std::ve
     CK(rec(ws.ev[2]));
     if (S.any_cross) {
       NvtxRange r("sdfb crossings");
-      CK(parity_columns(B, static_cast<uint64_t *>(ws.col_start.p), static_cast<float *>(ws.col_z.p),
-                        static_cast<int8_t *>(ws.col_s.p), S.capacity, ws.par_tmp.p, ws.par_tmp.cap, d_err,
-                        ctx->num_sms, st));
+      unsigned long long *d_cross =
+          reinterpret_cast<unsigned long long *>(static_cast<char *>(ws.misc.p) + kMiscCrossOffset);
+      CK(parity_columns(B, static_cast<uint32_t *>(ws.col_bits.p), static_cast<uint64_t *>(ws.col_start.p),
+                        static_cast<float *>(ws.col_z.p), static_cast<int8_t *>(ws.col_s.p), S.capacity, ws.par_tmp.p,
+                        ws.par_tmp.cap, d_cross, d_err, ctx->num_sms, st));
     }
     if (K > 0) {
       NvtxRange r("sdfb caps build");
@@ -510,7 +517,7 @@ sdfb_status enqueue_batch(sdfb_ctx *ctx, Workspace &ws, cudaStream_t st, std::ve
                              static_cast<const uint8_t *>(ws.staging.p) + L.bytes);
     const void *ptrs[] = {ws.batch_buf.p, ws.bvh.p,  ws.build_tmp.p, ws.par_tmp.p,  ws.col_start.p,
                           ws.col_z.p,     ws.col_s.p, ws.misc.p,      ws.staging.p,  ws.caps_bvh.p,
-                          ws.caps_tmp.p,  ws.gwn_tmp.p, ws.defer.p, static_cast<void *>(st)};
+                          ws.caps_tmp.p,  ws.gwn_tmp.p, ws.defer.p, ws.col_bits.p, static_cast<void *>(st)};
     const uint64_t extra[] = {uint64_t(L.tile_id), uint64_t(L.stack), S.capacity, L.bytes, ws.build_tmp.cap,
                               ws.par_tmp.cap, ws.caps_tmp.cap, uint64_t(o.band_voxels * 1e6f),
                               uint64_t(L.step_budget), defer_cap, uint64_t(uint32_t(o.fault_inject))};
@@ -611,7 +618,7 @@ sdfb_status finish_batch(sdfb_ctx *ctx, Workspace &ws, cudaStream_t st, const Ba
     sv.rect_tests = w[4];
     sv.flops_distance = distance_work_flops(S.tile_id, w);
     if (S.any_cross)
-      cudaMemcpy(&sv.crossings, static_cast<uint64_t *>(ws.col_start.p) + S.total_cols, 8, cudaMemcpyDeviceToHost);
+      cudaMemcpy(&sv.crossings, static_cast<char *>(ws.misc.p) + kMiscCrossOffset, 8, cudaMemcpyDeviceToHost);
     if (S.any_gwn) {
       cudaMemcpy(&sv.gwn_fp64_cells, gwn_refine_counter(ws.gwn_tmp.p), 8, cudaMemcpyDeviceToHost);
       cudaMemcpy(&sv.gwn_direct_cells, gwn_direct_counter(ws.gwn_tmp.p), 8, cudaMemcpyDeviceToHost);

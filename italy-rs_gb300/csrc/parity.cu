@@ -8,13 +8,15 @@
 // with exact orientation predicates and simulation of simplicity (common.cuh), so a line through
 // a shared edge or vertex is counted exactly once and the parity is exact for every column.
 //
-//   k_col_items   candidate columns per triangle (centres inside its xy bounds, with slack)
-//   scan          item starts
-//   k_col_hits<0> exact test per (triangle, column) item; counts crossings per column (atomics)
-//   scan          column starts
-//   k_col_hits<1> same test; writes each crossing height into its column's slot range
-// The order of heights inside a column is irrelevant: the distance kernel only counts those
-// above each cell.
+// Parity meshes keep a bit a cell, layers along a word: a crossing at height z flips the inside bit of
+// every cell below it, so it toggles one bit, that of the highest such layer, and a cell is inside when
+// an odd number of toggles lie at or above it (the distance kernel counts them). One pass over the
+// (triangle, column) items (expand.cuh), one XOR a crossing, 1/32 of the distance grid's size.
+//
+// Winding-number meshes need every crossing's height and orientation: a first pass counts them per
+// column, a scan gives the columns their slots and a second pass fills them, in any order. (Parity
+// meshes took these three steps too, and the distance kernel compared every cell with every height of
+// its column.)
 #include <algorithm>
 #include <cstdint>
 
@@ -24,8 +26,6 @@
 
 namespace sdfb {
 namespace {
-
-constexpr int kThreads = 256;
 
 inline size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
@@ -71,64 +71,75 @@ __device__ __forceinline__ TriCols tri_cols(const BatchDev &B, uint64_t t) {
   return r;
 }
 
-// Candidate columns per triangle, as 64-bit counts (a triangle across a wide, flat grid can cover
-// more than 2^32 columns).
-__global__ __launch_bounds__(kThreads) void k_col_items(BatchDev B, uint64_t *__restrict__ items) {
-  const uint64_t t = uint64_t(blockIdx.x) * kThreads + threadIdx.x;
-  if (t >= B.total_ptris) return;
-  const TriCols tc = tri_cols(B, t);
-  items[t] = tc.x1 < tc.x0 ? 0ull : uint64_t(tc.x1 - tc.x0 + 1) * uint64_t(tc.y1 - tc.y0 + 1);
+// Layers whose cell centres are below z, of nz. The estimate is corrected against the centres
+// themselves, which do not decrease with the layer.
+__device__ __forceinline__ int layers_below(const GridDev &g, float z) {
+  const float f = (z - g.oz) / g.voxel + 0.5f;
+  int k = f > 0.0f ? (f < float(g.nz) ? static_cast<int>(f) : g.nz) : 0;
+  while (k > 0 && !(cell_center(g.oz, k - 1, g.voxel) < z)) --k;
+  while (k < g.nz && cell_center(g.oz, k, g.voxel) < z) ++k;
+  return k;
 }
 
-template <bool FILL>
-__global__ __launch_bounds__(kThreads) void k_col_hits(BatchDev B, const uint64_t *__restrict__ starts,
-                                                       uint32_t *__restrict__ col_count,
-                                                       const uint64_t *__restrict__ col_start,
-                                                       float *__restrict__ col_z, int8_t *__restrict__ col_s,
-                                                       uint64_t capacity, uint32_t *__restrict__ err) {
-  const uint64_t T = B.total_ptris;
-  const uint64_t total = starts[T];
-  const uint64_t stride = uint64_t(gridDim.x) * kThreads * kExpandChunk;
-  for (uint64_t w0 = (uint64_t(blockIdx.x) * kThreads + threadIdx.x) * kExpandChunk; w0 < total; w0 += stride) {
-    uint64_t t = item_owner(starts, static_cast<uint32_t>(T), w0);
-    TriCols tc = tri_cols(B, t);
-    uint64_t tstart = starts[t], tend = starts[t + 1];
-    const uint64_t wend = min(w0 + kExpandChunk, total);
-    for (uint64_t w = w0; w < wend; ++w) {
-      while (w >= tend) {
-        ++t;
-        tstart = tend;
-        tend = starts[t + 1];
-        if (tend > tstart) tc = tri_cols(B, t);
+// FILL: the winding-number meshes' second pass; else their count, and the parity meshes' bits.
+template <bool FILL> struct ColumnOp {
+  using Tri = TriCols;
+  uint32_t *col_count, *bits;
+  const uint64_t *col_start;
+  float *col_z;
+  int8_t *col_s;
+  uint64_t capacity;
+  unsigned long long *crossings;
+  uint32_t *err;
+  uint32_t found = 0;
+
+  // Candidate columns, as a 64-bit count (a triangle across a wide, flat grid can cover more than 2^32).
+  __device__ __forceinline__ uint64_t setup(const BatchDev &B, uint64_t t, Tri &tri) const {
+    tri = tri_cols(B, t);
+    if (tri.x1 < tri.x0 || (FILL && B.recs[tri.mesh].sign != kSignGwn)) return 0;
+    return uint64_t(tri.x1 - tri.x0 + 1) * uint64_t(tri.y1 - tri.y0 + 1);
+  }
+  __device__ __forceinline__ void item(const BatchDev &B, const Tri &tri, uint64_t k) {
+    const MeshRec &M = B.recs[tri.mesh];
+    const GridDev &g = M.g;
+    const uint32_t sx = tri.x1 - tri.x0 + 1;
+    const uint64_t row = (k >> 32) == 0 ? static_cast<uint32_t>(k) / sx : k / sx;
+    const int x = tri.x0 + static_cast<int>(k - row * sx), y = tri.y0 + static_cast<int>(row);
+    const float px = cell_center(g.ox, x, g.voxel), py = cell_center(g.oy, y, g.voxel);
+    float z;
+    int sgn;
+    const bool hit = column_crossing(tri.a, tri.b, tri.c, px, py, z, sgn);
+    if (!hit) return;
+    ++found;
+    if (!FILL && M.sign == kSignParity) {
+      const int below = layers_below(g, z);
+      if (below > 0) {
+        const uint64_t words = (uint64_t(g.nz) + 31) / 32;
+        atomicXor(bits + M.bit_base + (uint64_t(y) * g.nx + x) * words + (below - 1) / 32, 1u << ((below - 1) & 31));
       }
-      const MeshRec &M = B.recs[tc.mesh];
-      const GridDev &g = M.g;
-      const uint64_t k = w - tstart;
-      const uint32_t sx = tc.x1 - tc.x0 + 1;
-      const int x = tc.x0 + static_cast<int>(k % sx);
-      const int y = tc.y0 + static_cast<int>(k / sx);
-      const float px = cell_center(g.ox, x, g.voxel), py = cell_center(g.oy, y, g.voxel);
-      float z;
-      int sgn;
-      if (!column_crossing(tc.a, tc.b, tc.c, px, py, z, sgn)) continue;
-      const uint64_t col = M.col_base + uint64_t(y) * g.nx + x;
-      const uint32_t slot = atomicAdd(col_count + col, 1u);
-      if (FILL) {
-        const uint64_t at = col_start[col] + slot;
-        if (at < capacity) {
-          col_z[at] = z;
-          col_s[at] = static_cast<int8_t>(sgn);
-        } else {
-          atomic_or_err(err, kErrCrossingOverflow);
-        }
+      return;
+    }
+    const uint64_t col = M.col_base + uint64_t(y) * g.nx + x;
+    const uint32_t slot = atomicAdd(col_count + col, 1u);
+    if (FILL) {
+      const uint64_t at = col_start[col] + slot;
+      if (at < capacity) {
+        col_z[at] = z;
+        col_s[at] = static_cast<int8_t>(sgn);
+      } else {
+        atomic_or_err(err, kErrCrossingOverflow);
       }
     }
   }
-}
+  __device__ __forceinline__ void finish(const BatchDev &, unsigned long long) const {
+    if (FILL) return;
+    const uint32_t sum = __reduce_add_sync(kFull, found);
+    if (sum && (threadIdx.x & 31) == 0) atomicAdd(crossings, static_cast<unsigned long long>(sum));
+  }
+};
 
 struct ParTemp {
-  uint64_t *items;
-  uint64_t *starts;
+  void *big;
   uint32_t *col_count;
   void *scratch;
   size_t scratch_bytes;
@@ -142,10 +153,9 @@ size_t par_layout(uint64_t T, uint64_t ncols, char *base, ParTemp *o) {
     return p;
   };
   ParTemp x;
-  x.items = reinterpret_cast<uint64_t *>(take(size_t(T) * 8 + 8));
-  x.starts = reinterpret_cast<uint64_t *>(take((size_t(T) + 1) * 8));
+  x.big = take(big_list_bytes(T));
   x.col_count = reinterpret_cast<uint32_t *>(take(ncols * 4 + 4));
-  x.scratch_bytes = std::max(scan_scratch_bytes(T), scan_scratch_bytes(ncols));
+  x.scratch_bytes = scan_scratch_bytes(ncols);
   x.scratch = take(x.scratch_bytes);
   if (o) *o = x;
   return off;
@@ -157,26 +167,26 @@ size_t parity_temp_bytes(uint64_t total_ptris, uint64_t total_cols) {
   return par_layout(total_ptris, total_cols, nullptr, nullptr);
 }
 
-cudaError_t parity_columns(const BatchDev &B, uint64_t *col_start, float *col_z, int8_t *col_s, uint64_t capacity,
-                           void *temp, size_t temp_bytes, uint32_t *err, int num_sms, cudaStream_t st) {
+cudaError_t parity_columns(const BatchDev &B, uint32_t *bits, uint64_t *col_start, float *col_z, int8_t *col_s,
+                           uint64_t capacity, void *temp, size_t temp_bytes, unsigned long long *crossings,
+                           uint32_t *err, int num_sms, cudaStream_t st) {
   const uint64_t T = B.total_ptris, ncols = B.total_cols;
   ParTemp o;
   if (par_layout(T, ncols, static_cast<char *>(temp), &o) > temp_bytes) return cudaErrorMemoryAllocation;
-  cudaError_t e;
-  if ((e = cudaMemsetAsync(o.col_count, 0, ncols * 4, st)) != cudaSuccess) return e;
-  if (T == 0) return cudaMemsetAsync(col_start, 0, (ncols + 1) * 8, st);
-  const Scratch sc{o.scratch, o.scratch_bytes};
-  k_col_items<<<static_cast<unsigned>((T + kThreads - 1) / kThreads), kThreads, 0, st>>>(B, o.items);
-  note_launch();
-  if ((e = exclusive_scan_u64(o.items, o.starts, T, sc, st)) != cudaSuccess) return e;
-  const unsigned grid = num_sms * 8;
-  k_col_hits<false><<<grid, kThreads, 0, st>>>(B, o.starts, o.col_count, nullptr, nullptr, nullptr, 0, err);
-  note_launch();
-  if ((e = exclusive_scan_u32(o.col_count, col_start, ncols, sc, st)) != cudaSuccess) return e;
-  if ((e = cudaMemsetAsync(o.col_count, 0, ncols * 4, st)) != cudaSuccess) return e;
-  k_col_hits<true><<<grid, kThreads, 0, st>>>(B, o.starts, o.col_count, col_start, col_z, col_s, capacity, err);
-  note_launch();
-  return cudaGetLastError();
+  if (T == 0) return cudaErrorInvalidValue;
+  const BigList big = big_list(o.big, T);
+  cudaError_t e = cudaMemsetAsync(big.counts, 0, 16, st);
+  if (e == cudaSuccess && B.total_bit_words) e = cudaMemsetAsync(bits, 0, B.total_bit_words * 4, st);
+  if (e == cudaSuccess && ncols) e = cudaMemsetAsync(o.col_count, 0, ncols * 4, st);
+  if (e != cudaSuccess) return e;
+  e = expand(B, T, big, ColumnOp<false>{o.col_count, bits, nullptr, nullptr, nullptr, 0, crossings, err, 0}, num_sms, st);
+  if (e != cudaSuccess || ncols == 0) return e;
+  if ((e = exclusive_scan_u32(o.col_count, col_start, ncols, Scratch{o.scratch, o.scratch_bytes}, st)) != cudaSuccess ||
+      (e = cudaMemsetAsync(o.col_count, 0, ncols * 4, st)) != cudaSuccess ||
+      (e = cudaMemsetAsync(big.counts, 0, 16, st)) != cudaSuccess)
+    return e;
+  return expand(B, T, big, ColumnOp<true>{o.col_count, nullptr, col_start, col_z, col_s, capacity, nullptr, err, 0}, num_sms,
+                st);
 }
 
 }  // namespace sdfb
