@@ -31,10 +31,8 @@ struct Scratch {
 // hold n + 1 values. Scratch need: scan_scratch_bytes(n).
 size_t scan_scratch_bytes(size_t n);
 cudaError_t exclusive_scan_u32(const uint32_t *in, uint64_t *out, size_t n, Scratch s, cudaStream_t st);
-// The same for uint64 counts (per-triangle candidate counts, which can pass 2^32 on large grids).
-cudaError_t exclusive_scan_u64(const uint64_t *in, uint64_t *out, size_t n, Scratch s, cudaStream_t st);
 
-// Stable LSD radix sort of (key, value) pairs on bits [0, bits) of the keys, 8 bits per pass.
+// Stable LSD radix sort of (key, value) pairs on bits [0, bits) of the keys; higher bits are zero.
 // keys/vals hold the input and receive the result; keys_alt/vals_alt are same-size temporaries.
 size_t sort_scratch_bytes(size_t n);
 cudaError_t radix_sort_pairs(uint64_t *keys, uint32_t *vals, uint64_t *keys_alt, uint32_t *vals_alt, size_t n,
