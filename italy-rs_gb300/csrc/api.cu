@@ -6,6 +6,8 @@
 //
 // Replaces italy::bakeSdf (src/convert/sdf_baker.cpp:137-310) and italy::voxelizeMesh
 // (src/convert/voxelize.cpp:52-107).
+#include <unistd.h>
+
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -75,7 +77,7 @@ sdfb_ctx::~sdfb_ctx() {
 
 DevBuf *sdfb_ctx::all_bufs(int i) {
   DevBuf *b[] = {&in_verts, &in_idx,   &in_verts2, &in_idx2,    &in_caps,   &in_capidx, &out_dist,
-                 &out_occ,  &first_tri, &sparse_tmp, &sparse_out, &mat_rec,  &mat_in,    &mat_tri,
+                 &out_occ,  &first_tri, &sparse_tmp, &sparse_out, &sparse_xyz, &mat_rec,  &mat_in,    &mat_tri,
                  &hit_keys, &hit_vals,  &hit_alt,   &mat_cells, &cons_grid, &cons_io,    &weld_tmp,
                  &caps_tmp, &caps_misc};
   return i < int(sizeof b / sizeof b[0]) ? b[i] : nullptr;
@@ -85,6 +87,7 @@ void sdfb_ctx::release_all() {
   for (int i = 0; DevBuf *b = all_bufs(i); ++i) b->release();
   ws.release();
   staging_small.release();
+  mat_pin.release();
   gate_pin.release();
 }
 
@@ -427,14 +430,12 @@ sdfb_status sdfb_bake_soup(sdfb_ctx *ctx, const float *positions, uint32_t num_t
   const cudaStream_t st = ctx->stream;
   const uint64_t cells = uint64_t(grid_out->nx) * grid_out->ny * grid_out->nz;
   const bool want_dist = dist_out && !o.no_distance, want_occ = occ_out && !o.no_occupancy;
-  std::vector<uint32_t> ident(V);
-  for (uint32_t i = 0; i < V; ++i) ident[i] = i;
   ENSURE(ctx->in_verts, size_t(V) * 12);
   ENSURE(ctx->in_idx, size_t(V) * 4);
   if (want_dist) ENSURE(ctx->out_dist, cells * 4);
   if (want_occ) ENSURE(ctx->out_occ, cells);
   CK(cudaMemcpyAsync(ctx->in_verts.p, positions, size_t(V) * 12, cudaMemcpyHostToDevice, st));
-  CK(cudaMemcpyAsync(ctx->in_idx.p, ident.data(), size_t(V) * 4, cudaMemcpyHostToDevice, st));
+  CK(iota_device(static_cast<uint32_t *>(ctx->in_idx.p), V, ctx->num_sms, st));
   std::vector<PlanMesh> ms(1);
   PlanMesh &p = ms[0];
   uint32_t U = 0;
@@ -596,15 +597,13 @@ sdfb_status voxelize_sparse_run(sdfb_ctx *ctx, const float *positions, uint32_t 
   const uint32_t V = 3 * num_tris;
   const size_t cells = size_t(resolution) * resolution * resolution;
   const cudaStream_t st = ctx->stream;
-  std::vector<uint32_t> ident(V);
-  for (uint32_t i = 0; i < V; ++i) ident[i] = i;
   ENSURE(ctx->in_verts, size_t(V) * 12);
   ENSURE(ctx->in_idx, size_t(V) * 4);
   ENSURE(ctx->out_occ, cells);
   ENSURE(ctx->first_tri, cells * 4);
   ENSURE(ctx->sparse_tmp, std::max(occupancy_temp_bytes(num_tris), sparse_temp_bytes(cells, 0)));
   CK(cudaMemcpyAsync(ctx->in_verts.p, positions, size_t(V) * 12, cudaMemcpyHostToDevice, st));
-  CK(cudaMemcpyAsync(ctx->in_idx.p, ident.data(), size_t(V) * 4, cudaMemcpyHostToDevice, st));
+  CK(iota_device(static_cast<uint32_t *>(ctx->in_idx.p), V, ctx->num_sms, st));
   // a batch of one mesh with an occupancy output only
   MeshRec r;
   std::memset(&r, 0, sizeof r);
@@ -642,24 +641,29 @@ sdfb_status voxelize_sparse_run(sdfb_ctx *ctx, const float *positions, uint32_t 
                   st));
   *count = total;
   if (total == 0) return SDFB_OK;
+  const size_t counted = ctx->sparse_tmp.cap;
   ENSURE(ctx->sparse_tmp, sparse_temp_bytes(cells, total));
   ENSURE(ctx->out_dist, total * 4);
   int bits = 1;
   while (bits < 32 && (uint64_t(1) << bits) < num_tris) ++bits;
   CK(sparse_emit(static_cast<const uint8_t *>(ctx->out_occ.p), static_cast<const uint32_t *>(ctx->first_tri.p), cells,
-                 total, bits, ctx->sparse_tmp.p, ctx->sparse_tmp.cap, static_cast<uint32_t *>(ctx->out_dist.p), st));
+                 total, bits, ctx->sparse_tmp.cap == counted, ctx->sparse_tmp.p, ctx->sparse_tmp.cap,
+                 static_cast<uint32_t *>(ctx->out_dist.p), st));
   if (d_list) *d_list = static_cast<const uint32_t *>(ctx->out_dist.p);
   const uint64_t n = std::min<uint64_t>(total, cap);
-  std::vector<uint32_t> lin(n);
-  if (n) CK(cudaMemcpyAsync(lin.data(), ctx->out_dist.p, n * 4, cudaMemcpyDeviceToHost, st));
-  CK(cudaStreamSynchronize(st));
-  const uint64_t rr = uint64_t(resolution);
-  for (uint64_t i = 0; i < n; ++i) {
-    const uint64_t c = lin[i];
-    cells_out[3 * i] = static_cast<int32_t>(c % rr);
-    cells_out[3 * i + 1] = static_cast<int32_t>((c / rr) % rr);
-    cells_out[3 * i + 2] = static_cast<int32_t>(c / (rr * rr));
+  if (n) {
+    ENSURE(ctx->sparse_xyz, n * 12);
+    CK(sparse_coords(static_cast<const uint32_t *>(ctx->out_dist.p), n, static_cast<uint32_t>(resolution),
+                     static_cast<int32_t *>(ctx->sparse_xyz.p), st));
+    // Meanwhile the caller's pages are faulted in from here: a copy into pages that were never written
+    // faults them from the device (a million triangles at 512, into fresh memory: 6.2 ms for 0.83).
+    volatile char *out = reinterpret_cast<volatile char *>(cells_out);
+    const size_t page = static_cast<size_t>(sysconf(_SC_PAGESIZE));
+    for (size_t b = 0; b < n * 12; b += page) out[b] = 0;
+    out[n * 12 - 1] = 0;
+    CK(cudaMemcpyAsync(cells_out, ctx->sparse_xyz.p, n * 12, cudaMemcpyDeviceToHost, st));
   }
+  CK(cudaStreamSynchronize(st));
   return SDFB_OK;
 }
 

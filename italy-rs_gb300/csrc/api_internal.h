@@ -137,14 +137,14 @@ struct sdfb_ctx {
   std::string err;
   // inputs / outputs of host-buffer calls
   DevBuf in_verts, in_idx, in_verts2, in_idx2, in_caps, in_capidx, out_dist, out_occ, first_tri, sparse_tmp,
-      sparse_out;
+      sparse_out, sparse_xyz;
   // materials: the batch record, material tables and texels, per-triangle materials, sorted hits,
   // per-cell outputs
   DevBuf mat_rec, mat_in, mat_tri, hit_keys, hit_vals, hit_alt, mat_cells;
   DevBuf cons_grid, cons_io;  // consumer check: a grid and its queries / results
   DevBuf weld_tmp;            // device weld / watertight census
   DevBuf caps_tmp, caps_misc; // device-built winding-number caps: temporaries, totals and error word
-  PinBuf staging_small, gate_pin;
+  PinBuf staging_small, gate_pin, mat_pin;
   Workspace ws;
   int tuned_leaf[32][8];  // [log2 T][log2 n - 4]
   int tuned_tile[32][8];

@@ -250,8 +250,12 @@ size_t sparse_temp_bytes(size_t cells, size_t max_out);
 // Counts occupied cells (synchronises the stream; *h_total is host memory).
 cudaError_t sparse_count(const uint8_t *occ, size_t cells, void *temp, size_t temp_bytes, uint64_t *h_total,
                          cudaStream_t st);
-// Writes the occupied cell indices ordered by (first triangle, cell index) into cells_out.
+// Writes the occupied cell indices ordered by (first triangle, cell index) into cells_out. counted:
+// temp still holds what sparse_count left there.
 cudaError_t sparse_emit(const uint8_t *occ, const uint32_t *first_tri, size_t cells, uint64_t total, int tri_bits,
-                        void *temp, size_t temp_bytes, uint32_t *cells_out, cudaStream_t st);
+                        bool counted, void *temp, size_t temp_bytes, uint32_t *cells_out, cudaStream_t st);
+
+// x, y and z of n listed cells of a res^3 grid.
+cudaError_t sparse_coords(const uint32_t *list, uint64_t n, uint32_t res, int32_t *xyz, cudaStream_t st);
 
 }  // namespace sdfb

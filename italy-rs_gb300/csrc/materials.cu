@@ -211,13 +211,11 @@ sdfb_status soup_batch(sdfb_ctx *ctx, const float *positions, uint32_t T, const 
                        BatchDev &B) {
   const uint64_t V = uint64_t(3) * T;
   const uint64_t cells = uint64_t(g.nx) * g.ny * g.nz;
-  std::vector<uint32_t> ident(V);
-  for (uint64_t i = 0; i < V; ++i) ident[i] = static_cast<uint32_t>(i);
   ENSURE(ctx->in_verts, V * 12);
   ENSURE(ctx->in_idx, V * 4);
   ENSURE(ctx->out_occ, cells);
   CK(cudaMemcpyAsync(ctx->in_verts.p, positions, V * 12, cudaMemcpyHostToDevice, st));
-  CK(cudaMemcpyAsync(ctx->in_idx.p, ident.data(), V * 4, cudaMemcpyHostToDevice, st));
+  CK(iota_device(static_cast<uint32_t *>(ctx->in_idx.p), V, ctx->num_sms, st));
   MeshRec r;
   std::memset(&r, 0, sizeof r);
   r.verts = static_cast<const float *>(ctx->in_verts.p);
@@ -232,13 +230,13 @@ sdfb_status soup_batch(sdfb_ctx *ctx, const float *positions, uint32_t T, const 
   static_assert(sizeof(MeshRec) <= 256, "the mesh record fits its slot");
   const size_t bytes = 256 * 4;
   ENSURE(ctx->mat_rec, bytes + 64);  // + the hit counter at byte 1024
-  std::vector<char> hs(bytes, 0);
-  std::memcpy(hs.data(), &r, sizeof r);
-  std::memcpy(hs.data() + 256, tables[0], 16);
-  std::memcpy(hs.data() + 512, tables[1], 16);
-  std::memcpy(hs.data() + 768, zero, 16);
-  CK(cudaMemcpyAsync(ctx->mat_rec.p, hs.data(), bytes, cudaMemcpyHostToDevice, st));
-  CK(cudaStreamSynchronize(st));  // hs and ident are host locals
+  if (!ctx->staging_small.ensure(bytes)) return ctx_fail(ctx, SDFB_ERR_OUT_OF_MEMORY, "pinned staging");
+  char *hs = static_cast<char *>(ctx->staging_small.p);
+  std::memcpy(hs, &r, sizeof r);
+  std::memcpy(hs + 256, tables[0], 16);
+  std::memcpy(hs + 512, tables[1], 16);
+  std::memcpy(hs + 768, zero, 16);
+  CK(cudaMemcpyAsync(ctx->mat_rec.p, hs, bytes, cudaMemcpyHostToDevice, st));
   char *d = static_cast<char *>(ctx->mat_rec.p);
   B = BatchDev();
   B.num_meshes = 1;
@@ -253,33 +251,39 @@ sdfb_status soup_batch(sdfb_ctx *ctx, const float *positions, uint32_t T, const 
 
 // Per-triangle materials into ctx->mat_tri: T float4 (r, g, b, metallic) then T roughness floats.
 sdfb_status triangle_materials(sdfb_ctx *ctx, const sdfb_materials &m, uint32_t T, cudaStream_t st) {
-  // One device block: materials | textures | sRGB table | per-triangle indices | uvs | texels.
-  std::vector<MatRec> mats(m.num_materials);
+  // One device block: materials | textures | sRGB table | per-triangle indices | uvs | texels. The
+  // first three are put together in pinned memory; the rest goes from the caller's.
+  const size_t o_mat = 0, o_tex = align256(m.num_materials * sizeof(MatRec));
+  const size_t o_lut = o_tex + align256(std::max<size_t>(m.num_textures, 1) * sizeof(TexRec));
+  constexpr size_t kLutBytes = 256 * sizeof(float);
+  if (!ctx->mat_pin.ensure(o_lut + kLutBytes)) return ctx_fail(ctx, SDFB_ERR_OUT_OF_MEMORY, "pinned staging");
+  char *h = static_cast<char *>(ctx->mat_pin.p);
+  MatRec *mats = reinterpret_cast<MatRec *>(h + o_mat);
   for (uint32_t i = 0; i < m.num_materials; ++i) {
     const sdfb_material &s = m.materials[i];
     mats[i] = MatRec{{s.base_color[0], s.base_color[1], s.base_color[2], s.metallic, s.roughness},
                      s.base_color_texture};
   }
-  std::vector<TexRec> tex(m.num_textures);
+  TexRec *tex = reinterpret_cast<TexRec *>(h + o_tex);
   uint64_t pix = 0;
   for (uint32_t k = 0; k < m.num_textures; ++k) {
     const sdfb_texture &t = m.textures[k];
     tex[k] = TexRec{pix, t.width, t.height, t.srgb ? 1 : 0, 0};
     if (t.width > 0 && t.height > 0) pix += uint64_t(t.width) * uint64_t(t.height) * 4;
   }
-  float lut[256];
-  srgb_to_linear_table(lut);
-  const size_t o_mat = 0, o_tex = align256(mats.size() * sizeof(MatRec));
-  const size_t o_lut = o_tex + align256(std::max<size_t>(tex.size(), 1) * sizeof(TexRec));
-  const size_t o_tri = o_lut + align256(sizeof lut);
+  struct Lut {
+    float f[256];
+    Lut() { srgb_to_linear_table(f); }
+  };
+  static const Lut lut;
+  std::memcpy(h + o_lut, lut.f, kLutBytes);
+  const size_t o_tri = o_lut + align256(kLutBytes);
   const size_t o_uv = o_tri + align256(m.num_triangle_material * 4 + 4);
   const size_t o_pix = o_uv + align256(m.num_uvs * 8 + 8);
   const size_t total = o_pix + align256(pix + 4);
   ENSURE(ctx->mat_in, total);
   char *d = static_cast<char *>(ctx->mat_in.p);
-  CK(cudaMemcpyAsync(d + o_mat, mats.data(), mats.size() * sizeof(MatRec), cudaMemcpyHostToDevice, st));
-  if (!tex.empty()) CK(cudaMemcpyAsync(d + o_tex, tex.data(), tex.size() * sizeof(TexRec), cudaMemcpyHostToDevice, st));
-  CK(cudaMemcpyAsync(d + o_lut, lut, sizeof lut, cudaMemcpyHostToDevice, st));
+  CK(cudaMemcpyAsync(d, h, o_lut + kLutBytes, cudaMemcpyHostToDevice, st));
   if (m.num_triangle_material)
     CK(cudaMemcpyAsync(d + o_tri, m.triangle_material, m.num_triangle_material * 4, cudaMemcpyHostToDevice, st));
   if (m.num_uvs) CK(cudaMemcpyAsync(d + o_uv, m.uvs, m.num_uvs * 8, cudaMemcpyHostToDevice, st));
@@ -306,7 +310,6 @@ sdfb_status triangle_materials(sdfb_ctx *ctx, const sdfb_materials &m, uint32_t 
   k_tri_material<<<(T + kThreads - 1) / kThreads, kThreads, 0, st>>>(a, T, cm, rough);
   note_launch();
   CK(cudaGetLastError());
-  CK(cudaStreamSynchronize(st));  // the host tables above are locals
   return SDFB_OK;
 }
 

@@ -3,8 +3,8 @@
 //
 // Atomics-free per-tile compaction: k_tile_count counts occupied cells per 4096-cell tile (16 cells
 // per thread, one 16-byte load each); a scan gives each tile its output offset; k_tile_write scans
-// its tile inside the block and writes (first triangle, cell) pairs in cell order. A stable radix sort by first triangle then yields the
-// reference's insertion order: a cell is inserted by the first triangle that hits it, and one
+// its tile inside the block and writes (first triangle, cell) pairs in cell order. A stable radix sort
+// by first triangle then yields the reference's insertion order: a cell is inserted by the first triangle that hits it, and one
 // triangle inserts its cells in z, y, x loop order, which is increasing cell index.
 #include <algorithm>
 #include <cstdint>
@@ -104,6 +104,16 @@ __global__ __launch_bounds__(kThreads) void k_tile_write(const uint8_t *__restri
   }
 }
 
+__global__ __launch_bounds__(kThreads) void k_coords(const uint32_t *__restrict__ list, uint64_t n, uint32_t res,
+                                                     int32_t *__restrict__ xyz) {
+  for (uint64_t i = uint64_t(blockIdx.x) * kThreads + threadIdx.x; i < n; i += uint64_t(gridDim.x) * kThreads) {
+    const uint32_t c = list[i], row = c / res;
+    xyz[3 * i] = static_cast<int32_t>(c - row * res);
+    xyz[3 * i + 1] = static_cast<int32_t>(row % res);
+    xyz[3 * i + 2] = static_cast<int32_t>(row / res);
+  }
+}
+
 struct SparseTemp {
   uint32_t *counts;
   uint64_t *starts;
@@ -122,7 +132,7 @@ size_t sparse_layout(size_t cells, size_t max_out, char *base, SparseTemp *o) {
     return p;
   };
   SparseTemp x;
-  x.counts = reinterpret_cast<uint32_t *>(take(tiles * 4 + 4));
+  x.counts = reinterpret_cast<uint32_t *>(take(tiles * 4 + 4));  // counts and starts lie first, whatever max_out
   x.starts = reinterpret_cast<uint64_t *>(take((tiles + 1) * 8));
   x.keys = reinterpret_cast<uint64_t *>(take(max_out * 8 + 8));
   x.keys_alt = reinterpret_cast<uint64_t *>(take(max_out * 8 + 8));
@@ -150,24 +160,32 @@ cudaError_t sparse_count(const uint8_t *occ, size_t cells, void *temp, size_t te
   return cudaStreamSynchronize(st);
 }
 
-// After sparse_count: writes the `total` occupied cell indices, ordered by (first triangle, cell),
+// After sparse_count (counted: its tile counts are still in temp): writes the `total` occupied cell indices, ordered by (first triangle, cell),
 // into cells_out (device, total uint32). tri_bits = bits needed for a triangle index.
 cudaError_t sparse_emit(const uint8_t *occ, const uint32_t *first_tri, size_t cells, uint64_t total, int tri_bits,
-                        void *temp, size_t temp_bytes, uint32_t *cells_out, cudaStream_t st) {
+                        bool counted, void *temp, size_t temp_bytes, uint32_t *cells_out, cudaStream_t st) {
   SparseTemp o;
   if (sparse_layout(cells, total, static_cast<char *>(temp), &o) > temp_bytes) return cudaErrorMemoryAllocation;
   const size_t tiles = (cells + kTile - 1) / kTile;
-  // recount: the workspace may have been reallocated since sparse_count
-  k_tile_count<<<static_cast<unsigned>(tiles), kThreads, 0, st>>>(occ, cells, o.counts);
-  note_launch();
-  cudaError_t e0 = exclusive_scan_u32(o.counts, o.starts, tiles, Scratch{o.scratch, o.scratch_bytes}, st);
-  if (e0 != cudaSuccess) return e0;
+  if (!counted) {
+    k_tile_count<<<static_cast<unsigned>(tiles), kThreads, 0, st>>>(occ, cells, o.counts);
+    note_launch();
+    const cudaError_t e = exclusive_scan_u32(o.counts, o.starts, tiles, Scratch{o.scratch, o.scratch_bytes}, st);
+    if (e != cudaSuccess) return e;
+  }
   k_tile_write<<<static_cast<unsigned>(tiles), kThreads, 0, st>>>(occ, first_tri, cells, o.starts, o.keys, cells_out);
   note_launch();
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   return radix_sort_pairs(o.keys, cells_out, o.keys_alt, o.vals_alt, total, tri_bits,
                           Scratch{o.scratch, o.scratch_bytes}, st);
+}
+
+cudaError_t sparse_coords(const uint32_t *list, uint64_t n, uint32_t res, int32_t *xyz, cudaStream_t st) {
+  k_coords<<<static_cast<unsigned>(std::min<uint64_t>((n + kThreads - 1) / kThreads, 1u << 16)), kThreads, 0, st>>>(
+      list, n, res, xyz);
+  note_launch();
+  return cudaGetLastError();
 }
 
 }  // namespace sdfb
