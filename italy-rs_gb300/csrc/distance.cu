@@ -37,9 +37,16 @@
 // Two passes keep one expensive tile from holding the whole GPU. In pass A a walk looks at the
 // chunk counter every few steps; once every chunk has been handed out (the tail) it stops, stores
 // its cells' bounds (squared distances, upper bounds of the answer) in the output and appends the
-// tile to a deferred list. Pass B gives each deferred tile a whole block: its warps take the nodes
-// of one level from a shared counter and walk below them for the same cells, whose bounds they
-// share in shared memory (atomicMin on the float bits, valid for non-negative values).
+// tile to a deferred list. Pass B gives each deferred tile a whole block, which goes down the tree a
+// level at a time: its warps take the level's surviving nodes from a shared list, test their children
+// and list those that survive for the next level; at the last they measure the blocks against the
+// cells, whose bounds they share in shared memory (atomicMin on the float bits, valid for
+// non-negative values). A pass starts from bounds that are nearly final, so what it takes is set by
+// how evenly the warps share the rest. Before, its 16 warps took the subtrees of one fixed level: bakes
+// of 82k triangles at 256^3 went from 5.25 to 5.12 ms, of 1M at 128^3 from 6.90 to 6.30 ms. Handing
+// over the first pass's stack instead, few nodes with uneven subtrees, made the passes 4.8 -> 5.2 ms
+// and 6.3 -> 7.1 ms. 12 warps, two blocks an SM: against 16 warps and one, both passes over 97 x 61 x
+// 43 cells take 201-281 us for 178-240 (8 warps and three: 178-233, but 168 for 160 us at 64^3).
 //
 // Sign: parity counts the column's crossing bits at and above each cell (parity.cu). Winding-number
 // signs are applied afterwards by gwn.cu, which needs the unsigned distance to find the near-surface
@@ -54,9 +61,9 @@
 namespace sdfb {
 namespace {
 
-// Two blocks of 16 warps per SM: the walk waits on dependent loads and shared-memory round trips.
+// 7 blocks an SM at 72 registers a thread: against 6 blocks at 80, 1 to 3% less time from 64^3 up.
 constexpr int kThreadsA = 128;
-constexpr int kMinBlocksA = 6;
+constexpr int kMinBlocksA = 7;
 constexpr int kWarpsPerBlockA = kThreadsA / kWarp;
 // Tile order within a mesh: bricks of kBrickX x kBrickY x kBrickZ tiles, x fastest inside a brick
 // and across bricks. Tiles of a partial brick beyond the grid have no active cell.
@@ -64,9 +71,10 @@ constexpr int kBrickX = 4, kBrickY = 4, kBrickZ = 2, kBrickTiles = kBrickX * kBr
 constexpr int kChunkMax = 32;  // tiles per chunk when there are plenty
 constexpr unsigned long long kNoTile = ~0ull;
 constexpr int kDispatchSpin = 1 << 22;  // bound on a warp's wait for its block's next chunk
-constexpr int kThreads = 512;
+constexpr int kThreads = 384;
+constexpr int kMinBlocksB = 2;
 constexpr int kWarpsPerBlockB = kThreads / kWarp;
-constexpr uint32_t kMaxItems = 512;  // pass B: at most this many subtrees per deferred tile
+constexpr uint32_t kFrontier = 2048;  // pass B: nodes of a level that the block keeps
 constexpr int kMaxLevels = 8;        // 2^31 triangles in blocks of 2 make 6 levels of 32-ary nodes
 constexpr int kStackSize = 32 * kMaxLevels;  // a node leaves at most 31 siblings behind on its level
 constexpr int kFlushAt = 16;                 // surviving blocks measured against the cells together
@@ -499,6 +507,52 @@ struct Walker {
     __syncwarp();
   }
 
+  // Whether the lane's child on `level` may matter, and its squared distance to the tile's centre.
+  __device__ __forceinline__ bool test(int level, uint32_t child, float &d2) {
+    const bool valid = child < m.level_n[level];
+    bool kept;
+    const float4 c = m.centre;
+    if (level > 0) {
+      const float4 *b = m.t.box + 2 * size_t(m.level_off[level] + (valid ? child : 0));
+      const float4 bc = __ldg(b), be = __ldg(b + 1);
+      const float tx = c.x - bc.x, ty = c.y - bc.y, tz = c.z - bc.z;
+      const float ax = fabsf(tx), ay = fabsf(ty), az = fabsf(tz);
+      const float ex = fmaxf(ax - be.x, 0.0f), ey = fmaxf(ay - be.y, 0.0f), ez = fmaxf(az - be.z, 0.0f);
+      const float fx = fminf(ax, be.x) + be.x, fy = fminf(ay, be.y) + be.y, fz = fminf(az, be.z) + be.z;
+      d2 = ex * ex + ey * ey + ez * ez;
+      kept = near(c.w, copysignf(ex, tx), copysignf(ey, ty), copysignf(ez, tz), d2, fx * fx + fy * fy + fz * fz,
+                  ax + ay + az + be.x + be.y + be.z);
+      if (COUNT) ws.box_tests += kWarp;
+    } else {
+      const float4 *o = tree_obb(m.t.obb, valid ? child : 0);
+      const float4 o0 = __ldg(o), o1 = __ldg(o + kObbPlane), o2 = __ldg(o + 2 * kObbPlane),
+                   o3 = __ldg(o + 3 * kObbPlane);
+      const float dx = c.x - o0.x, dy = c.y - o0.y, dz = c.z - o0.z;
+      const float t0 = fmaf(dz, o1.z, fmaf(dy, o1.y, dx * o1.x)), t1 = fmaf(dz, o2.z, fmaf(dy, o2.y, dx * o2.x)),
+                  t2 = fmaf(dz, o3.z, fmaf(dy, o3.y, dx * o3.x));
+      const float a0 = fabsf(t0), a1 = fabsf(t1), a2 = fabsf(t2);
+      const float e0 = copysignf(fmaxf(a0 - o0.w, 0.0f), t0), e1 = copysignf(fmaxf(a1 - o1.w, 0.0f), t1),
+                  e2 = copysignf(fmaxf(a2 - o2.w, 0.0f), t2);
+      const float f0 = fminf(a0, o0.w) + o0.w, f1 = fminf(a1, o1.w) + o1.w, f2 = fminf(a2, o2.w) + o2.w;
+      d2 = e0 * e0 + e1 * e1 + e2 * e2;
+      kept = near(c.w, fmaf(e2, o3.x, fmaf(e1, o2.x, e0 * o1.x)), fmaf(e2, o3.y, fmaf(e1, o2.y, e0 * o1.y)),
+                  fmaf(e2, o3.z, fmaf(e1, o2.z, e0 * o1.z)), d2, f0 * f0 + f1 * f1 + f2 * f2,
+                  a0 + a1 + a2 + o0.w + o1.w + o2.w);
+      if (COUNT) ws.plane_tests += kWarp;
+    }
+    return kept && valid;
+  }
+
+  // Takes the kept blocks into the list, the nearest first.
+  __device__ __forceinline__ void take_blocks(bool kept, uint32_t child, uint32_t mask, float d2, int &nb) {
+    const int nl = __reduce_min_sync(kFull, kept ? (__float_as_uint(d2) & ~31u) | lane : ~0u) & 31;
+    const int rank = __popc(mask & ((1u << lane) - 1u)) - (lane > nl ? 1 : 0);
+    if (kept) m.blocks[nb + (lane == nl ? 0 : rank + 1)] = child;
+    nb += __popc(mask);
+    __syncwarp();
+    if (nb >= kFlushAt) flush(nb);
+  }
+
   // Walks below node `cur` ((level << 28) | node). Returns false when the tail check stopped it with
   // work left (the bounds are then upper bounds); a walk past its step limit raises the corrupt flag.
   __device__ __forceinline__ bool walk(uint32_t cur, TailCheck tail, WalkLimits lim) {
@@ -519,47 +573,14 @@ struct Walker {
       }
       const int level = static_cast<int>(cur >> 28) - 1;  // the children's level
       const uint32_t child = (cur & 0x0fffffffu) * 32 + lane;
-      const bool valid = child < m.level_n[level];
-      bool kept;
       float d2;
-      const float4 c = m.centre;
-      if (level > 0) {
-        const float4 *b = m.t.box + 2 * size_t(m.level_off[level] + (valid ? child : 0));
-        const float4 bc = __ldg(b), be = __ldg(b + 1);
-        const float tx = c.x - bc.x, ty = c.y - bc.y, tz = c.z - bc.z;
-        const float ax = fabsf(tx), ay = fabsf(ty), az = fabsf(tz);
-        const float ex = fmaxf(ax - be.x, 0.0f), ey = fmaxf(ay - be.y, 0.0f), ez = fmaxf(az - be.z, 0.0f);
-        const float fx = fminf(ax, be.x) + be.x, fy = fminf(ay, be.y) + be.y, fz = fminf(az, be.z) + be.z;
-        d2 = ex * ex + ey * ey + ez * ez;
-        kept = near(c.w, copysignf(ex, tx), copysignf(ey, ty), copysignf(ez, tz), d2, fx * fx + fy * fy + fz * fz,
-                    ax + ay + az + be.x + be.y + be.z);
-        if (COUNT) ws.box_tests += kWarp;
-      } else {
-        const float4 *o = tree_obb(m.t.obb, valid ? child : 0);
-        const float4 o0 = __ldg(o), o1 = __ldg(o + kObbPlane), o2 = __ldg(o + 2 * kObbPlane),
-                     o3 = __ldg(o + 3 * kObbPlane);
-        const float dx = c.x - o0.x, dy = c.y - o0.y, dz = c.z - o0.z;
-        const float t0 = fmaf(dz, o1.z, fmaf(dy, o1.y, dx * o1.x)), t1 = fmaf(dz, o2.z, fmaf(dy, o2.y, dx * o2.x)),
-                    t2 = fmaf(dz, o3.z, fmaf(dy, o3.y, dx * o3.x));
-        const float a0 = fabsf(t0), a1 = fabsf(t1), a2 = fabsf(t2);
-        const float e0 = copysignf(fmaxf(a0 - o0.w, 0.0f), t0), e1 = copysignf(fmaxf(a1 - o1.w, 0.0f), t1),
-                    e2 = copysignf(fmaxf(a2 - o2.w, 0.0f), t2);
-        const float f0 = fminf(a0, o0.w) + o0.w, f1 = fminf(a1, o1.w) + o1.w, f2 = fminf(a2, o2.w) + o2.w;
-        d2 = e0 * e0 + e1 * e1 + e2 * e2;
-        kept = near(c.w, fmaf(e2, o3.x, fmaf(e1, o2.x, e0 * o1.x)), fmaf(e2, o3.y, fmaf(e1, o2.y, e0 * o1.y)),
-                    fmaf(e2, o3.z, fmaf(e1, o2.z, e0 * o1.z)), d2, f0 * f0 + f1 * f1 + f2 * f2,
-                    a0 + a1 + a2 + o0.w + o1.w + o2.w);
-        if (COUNT) ws.plane_tests += kWarp;
-      }
-      kept = kept && valid;
+      const bool kept = test(level, child, d2);
       const uint32_t mask = __ballot_sync(kFull, kept);
       if (mask) {
-        // The nearest child goes first: it is walked next, or leads the list of blocks.
-        const uint32_t near_key = __reduce_min_sync(kFull, kept ? (__float_as_uint(d2) & ~31u) | lane : ~0u);
-        const int nl = near_key & 31;
-        const int cnt = __popc(mask);
-        const int rank = __popc(mask & ((1u << lane) - 1u)) - (lane > nl ? 1 : 0);  // among the others
-        if (level > 0) {
+        if (level > 0) {  // the nearest child is walked next
+          const int nl = __reduce_min_sync(kFull, kept ? (__float_as_uint(d2) & ~31u) | lane : ~0u) & 31;
+          const int cnt = __popc(mask);
+          const int rank = __popc(mask & ((1u << lane) - 1u)) - (lane > nl ? 1 : 0);  // among the others
           if (kept && lane != nl && sp + rank < lim.stack)
             m.stack[sp + rank] = (static_cast<uint32_t>(level) << 28) | child;
           sp += cnt - 1;
@@ -571,10 +592,7 @@ struct Walker {
           __syncwarp();
           continue;
         }
-        if (kept) m.blocks[nb + (lane == nl ? 0 : rank + 1)] = child;
-        nb += cnt;
-        __syncwarp();
-        if (nb >= kFlushAt) flush(nb);
+        take_blocks(kept, child, mask, d2, nb);
       }
       if (sp == 0) break;
       cur = m.stack[--sp];
@@ -731,11 +749,11 @@ __global__ __launch_bounds__(kThreadsA, kMinBlocksA) void k_distance(DistanceArg
 
 // Pass B: one block per deferred tile; its warps share the tile's subtrees and bounds.
 template <int TX, int TY, int TZ, bool COUNT>
-__global__ __launch_bounds__(kThreads) void k_distance_deferred(DistanceArgs a) {
+__global__ __launch_bounds__(kThreads, kMinBlocksB) void k_distance_deferred(DistanceArgs a) {
   using W = Walker<TX, TY, TZ, COUNT>;
   constexpr int VPL = W::VPL;
   __shared__ unsigned long long s_tile;
-  __shared__ uint32_t s_item;
+  __shared__ uint32_t s_item, s_count[2], s_nodes[2][kFrontier];
   __shared__ WarpMem s_mem[kWarpsPerBlockB];
   __shared__ uint32_t s_best[VPL * kWarp];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -750,6 +768,9 @@ __global__ __launch_bounds__(kThreads) void k_distance_deferred(DistanceArgs a) 
       const unsigned long long k = atomicAdd(a.defer_counters + 1, 1ull);
       s_tile = k < total ? a.defer_list[k] : ~0ull;
       s_item = 0;
+      s_nodes[0][0] = 0;  // the root
+      s_count[0] = 1;
+      s_count[1] = 0;
     }
     __syncthreads();
     const unsigned long long tile = s_tile;
@@ -766,19 +787,43 @@ __global__ __launch_bounds__(kThreads) void k_distance_deferred(DistanceArgs a) 
       for (int v = 0; v < VPL; ++v) s_best[v * kWarp + lane] = __float_as_uint(c.M->dist[c.cell(lane, v)]);
     }
     __syncthreads();
-    // The lowest level with few enough nodes: one subtree per node.
-    int level = 1;
-    while (w.m.level_n[level] > kMaxItems) ++level;
-    const uint32_t items = w.m.level_n[level];
     const WalkLimits lim = walk_limits(c.M->tree, a.stack_depth, a.fault);
     w.fit();
-    for (;;) {
-      uint32_t item = 0;
-      if (lane == 0) item = atomicAdd(&s_item, 1u);
-      item = __shfl_sync(kFull, item, 0);
-      if (item >= items) break;
-      w.walk((static_cast<uint32_t>(level) << 28) | item, TailCheck{nullptr, 0, 0}, lim);
+    const uint32_t root = w.root();
+    int cur = 0, nb = 0;
+    for (int level = static_cast<int>(root >> 28); level > 0; --level, cur ^= 1) {
+      const uint32_t items = min(s_count[cur], kFrontier);
+      for (;;) {
+        uint32_t item = 0;
+        if (lane == 0) item = atomicAdd(&s_item, 1u);
+        item = __shfl_sync(kFull, item, 0);
+        if (item >= items) break;
+        const uint32_t child = s_nodes[cur][item] * 32 + lane;
+        float d2;
+        const bool kept = w.test(level - 1, child, d2);
+        const uint32_t mask = __ballot_sync(kFull, kept);
+        if (!mask) continue;
+        if (level == 1) {
+          w.take_blocks(kept, child, mask, d2, nb);
+          continue;
+        }
+        uint32_t at = 0;
+        if (lane == 0) at = atomicAdd(&s_count[cur ^ 1], static_cast<uint32_t>(__popc(mask)));
+        at = __shfl_sync(kFull, at, 0) + __popc(mask & ((1u << lane) - 1u));
+        if (kept && at < kFrontier) s_nodes[cur ^ 1][at] = child;
+        // No room: the subtree is walked here.
+        for (uint32_t over = __ballot_sync(kFull, kept && at >= kFrontier); over; over &= over - 1)
+          w.walk((static_cast<uint32_t>(level - 1) << 28) | __shfl_sync(kFull, child, __ffs(over) - 1),
+                 TailCheck{nullptr, 0, 0}, lim);
+      }
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        s_item = 0;
+        s_count[cur] = 0;
+      }
+      __syncthreads();
     }
+    if (nb > 0) w.flush(nb);
     __syncthreads();
     if (warp == 0) store_cells<TX, TY, TZ>(a, c, lane, s_best);
     __syncthreads();
