@@ -195,6 +195,7 @@ sdfb_status device_caps(sdfb_ctx *ctx, cudaStream_t st, std::vector<PlanMesh> &m
   ENSURE(ctx->in_capidx, np * 4);
   ENSURE(ctx->caps_tmp, caps_temp_bytes(tmax));
   ENSURE(ctx->caps_misc, 256 + ng * 16);
+  if (!ctx->gate_pin.ensure(32)) return ctx_fail(ctx, SDFB_ERR_OUT_OF_MEMORY, "pinned staging");
   uint32_t *d_err = static_cast<uint32_t *>(ctx->caps_misc.p);
   uint64_t *d_tot = reinterpret_cast<uint64_t *>(static_cast<char *>(ctx->caps_misc.p) + 256);
   CK(cudaMemsetAsync(d_err, 0, 4, st));
@@ -211,7 +212,7 @@ sdfb_status device_caps(sdfb_ctx *ctx, cudaStream_t st, std::vector<PlanMesh> &m
     CK(cudaMemcpyAsync(dv, bv, size_t(V) * 12, cudaMemcpyDeviceToDevice, st));
     CK(cudaMemcpyAsync(dp, bi, size_t(T) * 12, cudaMemcpyDeviceToDevice, st));
     CK(caps_device(bv, V, bi, T, ctx->caps_tmp.p, ctx->caps_tmp.cap, dv + 3 * size_t(V), dp + 3 * size_t(T),
-                   d_tot + 2 * k, d_err, ctx->num_sms, st));
+                   d_tot + 2 * k, static_cast<uint64_t *>(ctx->gate_pin.p), d_err, ctx->num_sms, st));
     p.pverts = p.cverts = dv;
     p.pidx = dp;
     p.cidx = dp + 3 * size_t(T);

@@ -211,15 +211,16 @@ sdfb_status build_resident(sdfb_ctx *ctx, Workspace &ws, cudaStream_t st, const 
 
 // caps.cu: boundary caps of an indexed mesh on the device. centres receives up to 3T loop centres
 // (3 floats each), cap_tris up to 3T cap triangles (indices; centre c is vertex V + c); totals[0] =
-// cap triangles (boundary half-edges), totals[1] = loops. Enqueued only.
+// cap triangles (boundary half-edges), totals[1] = loops. Synchronises the stream once, for the number
+// of boundary half-edges (pinned: 8 bytes of pinned host memory); the rest is enqueued only.
 size_t caps_temp_bytes(uint64_t T);
 cudaError_t caps_device(const float *verts, uint32_t V, const uint32_t *idx, uint32_t T, void *temp,
-                        size_t temp_bytes, float *centres, uint32_t *cap_tris, uint64_t *totals, uint32_t *err,
-                        int num_sms, cudaStream_t st);
+                        size_t temp_bytes, float *centres, uint32_t *cap_tris, uint64_t *totals, uint64_t *pinned,
+                        uint32_t *err, int num_sms, cudaStream_t st);
 // The crossing mesh (mesh + caps) and the caps of every winding-number mesh of ms that has a
 // distance output, built on the device into the context's buffers; sets their pverts / pidx /
 // cverts / cidx and counts. The caps close the crossing mesh already set (pverts / pidx, as the
-// soup bake's welded mesh), else the mesh itself. One read of the totals synchronises the stream.
+// soup bake's welded mesh), else the mesh itself. Reading counts and totals synchronises the stream.
 // every_gwn: also the winding-number meshes without a distance output (resident meshes).
 sdfb_status device_caps(sdfb_ctx *ctx, cudaStream_t st, std::vector<PlanMesh> &ms, bool every_gwn = false);
 

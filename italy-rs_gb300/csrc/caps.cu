@@ -20,8 +20,8 @@
 //                   order, and one fan triangle (head, tail, centre) per half-edge
 //
 // Any closing caps give the same winding number of the mesh itself, so the pairing at vertices
-// where several loops meet does not change a sign. Every size is bounded by 3T; kernels read the
-// data-dependent counts from device memory, and the caller reads the two totals once.
+// where several loops meet does not change a sign. Memory is sized for 3T half-edges; once they are
+// known the host reads their number, and the caller reads the two totals at the end.
 #include <algorithm>
 #include <cstdint>
 
@@ -140,15 +140,17 @@ __global__ __launch_bounds__(kThreads) void k_cap_emit(const uint64_t *__restric
   }
 }
 
-// Sort keys of the half-edges by tail (which = 0) or head (1); slots past the count sort last.
-__global__ __launch_bounds__(kThreads) void k_cap_end_keys(const uint2 *__restrict__ half,
-                                                           const uint64_t *__restrict__ total, uint64_t n, int which,
-                                                           uint64_t sentinel, uint64_t *__restrict__ keys,
-                                                           uint32_t *__restrict__ vals) {
-  const uint64_t nb = *total;
-  for (uint64_t h = uint64_t(blockIdx.x) * kThreads + threadIdx.x; h < n; h += uint64_t(gridDim.x) * kThreads) {
-    keys[h] = h < nb ? uint64_t(which ? half[h].y : half[h].x) : sentinel;
-    vals[h] = static_cast<uint32_t>(h);
+// Sort keys of the nb half-edges: their tails and their heads.
+__global__ __launch_bounds__(kThreads) void k_cap_end_keys(const uint2 *__restrict__ half, uint64_t nb,
+                                                           uint64_t *__restrict__ out_keys,
+                                                           uint32_t *__restrict__ out_vals,
+                                                           uint64_t *__restrict__ in_keys,
+                                                           uint32_t *__restrict__ in_vals) {
+  for (uint64_t h = uint64_t(blockIdx.x) * kThreads + threadIdx.x; h < nb; h += uint64_t(gridDim.x) * kThreads) {
+    const uint2 e = half[h];
+    out_keys[h] = e.x;
+    in_keys[h] = e.y;
+    out_vals[h] = in_vals[h] = static_cast<uint32_t>(h);
   }
 }
 
@@ -168,10 +170,9 @@ __device__ __forceinline__ uint64_t lower_bound64(const uint64_t *__restrict__ a
 __global__ __launch_bounds__(kThreads) void k_cap_pair(const uint64_t *__restrict__ in_keys,
                                                        const uint32_t *__restrict__ in_order,
                                                        const uint64_t *__restrict__ out_keys,
-                                                       const uint32_t *__restrict__ out_order,
-                                                       const uint64_t *__restrict__ total, uint32_t *__restrict__ succ,
-                                                       uint32_t *__restrict__ lab, uint32_t *__restrict__ err) {
-  const uint64_t nb = *total;
+                                                       const uint32_t *__restrict__ out_order, uint64_t nb,
+                                                       uint32_t *__restrict__ succ, uint32_t *__restrict__ lab,
+                                                       uint32_t *__restrict__ err) {
   for (uint64_t j = uint64_t(blockIdx.x) * kThreads + threadIdx.x; j < nb; j += uint64_t(gridDim.x) * kThreads) {
     const uint64_t x = in_keys[j];
     const uint64_t rank = j - lower_bound64(in_keys, nb, x);
@@ -189,10 +190,8 @@ __global__ __launch_bounds__(kThreads) void k_cap_pair(const uint64_t *__restric
 
 // One doubling step: lab2 = min(lab, lab[nxt]), nxt2 = nxt[nxt].
 __global__ __launch_bounds__(kThreads) void k_cap_jump(const uint32_t *__restrict__ nxt,
-                                                       const uint32_t *__restrict__ lab,
-                                                       const uint64_t *__restrict__ total, uint32_t *__restrict__ nxt2,
-                                                       uint32_t *__restrict__ lab2) {
-  const uint64_t nb = *total;
+                                                       const uint32_t *__restrict__ lab, uint64_t nb,
+                                                       uint32_t *__restrict__ nxt2, uint32_t *__restrict__ lab2) {
   for (uint64_t h = uint64_t(blockIdx.x) * kThreads + threadIdx.x; h < nb; h += uint64_t(gridDim.x) * kThreads) {
     const uint32_t m = nxt[h];
     lab2[h] = min(lab[h], lab[m]);
@@ -200,23 +199,18 @@ __global__ __launch_bounds__(kThreads) void k_cap_jump(const uint32_t *__restric
   }
 }
 
-__global__ __launch_bounds__(kThreads) void k_cap_cycle_keys(const uint32_t *__restrict__ lab,
-                                                             const uint64_t *__restrict__ total, uint64_t n,
-                                                             uint64_t sentinel, uint64_t *__restrict__ keys,
-                                                             uint32_t *__restrict__ vals) {
-  const uint64_t nb = *total;
-  for (uint64_t h = uint64_t(blockIdx.x) * kThreads + threadIdx.x; h < n; h += uint64_t(gridDim.x) * kThreads) {
-    keys[h] = h < nb ? uint64_t(lab[h]) : sentinel;
+__global__ __launch_bounds__(kThreads) void k_cap_cycle_keys(const uint32_t *__restrict__ lab, uint64_t nb,
+                                                             uint64_t *__restrict__ keys, uint32_t *__restrict__ vals) {
+  for (uint64_t h = uint64_t(blockIdx.x) * kThreads + threadIdx.x; h < nb; h += uint64_t(gridDim.x) * kThreads) {
+    keys[h] = lab[h];
     vals[h] = static_cast<uint32_t>(h);
   }
 }
 
-__global__ __launch_bounds__(kThreads) void k_cap_loop_flags(const uint64_t *__restrict__ keys,
-                                                             const uint64_t *__restrict__ total, uint64_t n,
+__global__ __launch_bounds__(kThreads) void k_cap_loop_flags(const uint64_t *__restrict__ keys, uint64_t nb,
                                                              uint32_t *__restrict__ flag) {
-  const uint64_t nb = *total;
-  for (uint64_t j = uint64_t(blockIdx.x) * kThreads + threadIdx.x; j < n; j += uint64_t(gridDim.x) * kThreads)
-    flag[j] = (j < nb && (j == 0 || keys[j] != keys[j - 1])) ? 1u : 0u;
+  for (uint64_t j = uint64_t(blockIdx.x) * kThreads + threadIdx.x; j < nb; j += uint64_t(gridDim.x) * kThreads)
+    flag[j] = (j == 0 || keys[j] != keys[j - 1]) ? 1u : 0u;
 }
 
 // Loop c starts at sorted position j (flag set): its centre, the mean of its half-edges' tails
@@ -227,10 +221,8 @@ __global__ __launch_bounds__(kThreads) void k_cap_loops(const float *__restrict_
                                                         const uint64_t *__restrict__ keys,
                                                         const uint32_t *__restrict__ order,
                                                         const uint32_t *__restrict__ flag,
-                                                        const uint64_t *__restrict__ loop_start,
-                                                        const uint64_t *__restrict__ total, float *__restrict__ centres,
-                                                        uint32_t *__restrict__ cap_tris) {
-  const uint64_t nb = *total;
+                                                        const uint64_t *__restrict__ loop_start, uint64_t nb,
+                                                        float *__restrict__ centres, uint32_t *__restrict__ cap_tris) {
   for (uint64_t j = uint64_t(blockIdx.x) * kThreads + threadIdx.x; j < nb; j += uint64_t(gridDim.x) * kThreads) {
     if (!flag[j]) continue;
     const uint64_t c = loop_start[j];
@@ -256,12 +248,6 @@ __global__ __launch_bounds__(kThreads) void k_cap_loops(const float *__restrict_
   }
 }
 
-__global__ void k_cap_totals(const uint64_t *__restrict__ starts, uint64_t n, const uint64_t *__restrict__ loop_start,
-                             uint64_t *__restrict__ totals) {
-  totals[0] = starts[n];
-  totals[1] = loop_start[n];
-}
-
 int bits_for_index(uint64_t V) {
   int b = 1;
   while (b < 32 && (uint64_t(1) << b) < V) ++b;
@@ -276,8 +262,8 @@ using namespace sdfb;
 size_t caps_temp_bytes(uint64_t T) { return cap_layout(T, nullptr, nullptr) + 256; }
 
 cudaError_t caps_device(const float *verts, uint32_t V, const uint32_t *idx, uint32_t T, void *temp,
-                        size_t temp_bytes, float *centres, uint32_t *cap_tris, uint64_t *totals, uint32_t *err,
-                        int num_sms, cudaStream_t st) {
+                        size_t temp_bytes, float *centres, uint32_t *cap_tris, uint64_t *totals, uint64_t *pinned,
+                        uint32_t *err, int num_sms, cudaStream_t st) {
   if (T == 0) return cudaMemsetAsync(totals, 0, 16, st);
   CapTemp t;
   if (cap_layout(T, static_cast<char *>(temp), &t) > temp_bytes) return cudaErrorMemoryAllocation;
@@ -287,7 +273,6 @@ cudaError_t caps_device(const float *verts, uint32_t V, const uint32_t *idx, uin
   // every (lo << bits | hi) is below 2^(2 bits): the sentinel sorts last
   const int edge_bits = bits < 32 ? 2 * bits + 1 : 64;
   const uint64_t edge_sentinel = bits < 32 ? (uint64_t(1) << (2 * bits)) : ~0ull;
-  const uint64_t end_sentinel = uint64_t(1) << 32;  // above every vertex index and half-edge label
   cudaError_t e;
   uint32_t *sign = t.vals_alt;  // free once the edge sort is done
   k_cap_edges<<<grid_for(n, num_sms), kThreads, 0, st>>>(idx, T, V, bits, edge_sentinel, t.keys, t.vals, err);
@@ -298,41 +283,46 @@ cudaError_t caps_device(const float *verts, uint32_t V, const uint32_t *idx, uin
   if ((e = exclusive_scan_u32(t.cnt, t.starts, n, sc, st)) != cudaSuccess) return e;
   k_cap_emit<<<grid_for(n, num_sms), kThreads, 0, st>>>(t.keys, t.cnt, sign, t.starts, n, bits, t.half);
   note_launch();
-  const uint64_t *nb = t.starts + n;  // boundary half-edges
-  // by tail
-  k_cap_end_keys<<<grid_for(n, num_sms), kThreads, 0, st>>>(t.half, nb, n, 0, end_sentinel, t.out_keys, t.out_order);
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  // The number of boundary half-edges sizes everything below: a fiftieth of the edges where 2% of the
+  // faces are missing, so that three sorts of all the edges' slots (50 us each at 30k) become small ones.
+  if ((e = cudaMemcpyAsync(pinned, t.starts + n, 8, cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
+      (e = cudaMemcpyAsync(totals, t.starts + n, 8, cudaMemcpyDeviceToDevice, st)) != cudaSuccess ||
+      (e = cudaStreamSynchronize(st)) != cudaSuccess)
+    return e;
+  const uint64_t nb = *pinned;
+  if (nb == 0) return cudaMemsetAsync(totals + 1, 0, 8, st);
+  const unsigned blocks = grid_for(nb, num_sms);
+  k_cap_end_keys<<<blocks, kThreads, 0, st>>>(t.half, nb, t.out_keys, t.out_order, t.in_keys, t.in_order);
   note_launch();
-  if ((e = radix_sort_pairs(t.out_keys, t.out_order, t.keys_alt, t.vals_alt, n, 33, sc, st)) != cudaSuccess) return e;
-  // by head
-  k_cap_end_keys<<<grid_for(n, num_sms), kThreads, 0, st>>>(t.half, nb, n, 1, end_sentinel, t.in_keys, t.in_order);
-  note_launch();
-  if ((e = radix_sort_pairs(t.in_keys, t.in_order, t.keys_alt, t.vals_alt, n, 33, sc, st)) != cudaSuccess) return e;
-  k_cap_pair<<<grid_for(n, num_sms), kThreads, 0, st>>>(t.in_keys, t.in_order, t.out_keys, t.out_order, nb, t.succ,
-                                                        t.lab, err);
+  if ((e = radix_sort_pairs(t.out_keys, t.out_order, t.keys_alt, t.vals_alt, nb, bits, sc, st)) != cudaSuccess ||
+      (e = radix_sort_pairs(t.in_keys, t.in_order, t.keys_alt, t.vals_alt, nb, bits, sc, st)) != cudaSuccess)
+    return e;
+  k_cap_pair<<<blocks, kThreads, 0, st>>>(t.in_keys, t.in_order, t.out_keys, t.out_order, nb, t.succ, t.lab, err);
   note_launch();
   // pointer jumping: after r rounds every half-edge knows the smallest index among its next 2^r
   const uint32_t *nx = t.succ;
   uint32_t *lab = t.lab, *lab2 = t.lab2, *nxa = t.nxt, *nxb = t.nxt2;
   int rounds = 1;
-  while (rounds < 40 && (uint64_t(1) << rounds) < n) ++rounds;
+  while (rounds < 40 && (uint64_t(1) << rounds) < nb) ++rounds;
   for (int r = 0; r < rounds; ++r) {
-    k_cap_jump<<<grid_for(n, num_sms), kThreads, 0, st>>>(nx, lab, nb, nxa, lab2);
+    k_cap_jump<<<blocks, kThreads, 0, st>>>(nx, lab, nb, nxa, lab2);
     note_launch();
     std::swap(lab, lab2);
     nx = nxa;
     std::swap(nxa, nxb);
   }
   // group by cycle
-  k_cap_cycle_keys<<<grid_for(n, num_sms), kThreads, 0, st>>>(lab, nb, n, end_sentinel, t.keys, t.vals);
+  k_cap_cycle_keys<<<blocks, kThreads, 0, st>>>(lab, nb, t.keys, t.vals);
   note_launch();
-  if ((e = radix_sort_pairs(t.keys, t.vals, t.keys_alt, t.vals_alt, n, 33, sc, st)) != cudaSuccess) return e;
-  k_cap_loop_flags<<<grid_for(n, num_sms), kThreads, 0, st>>>(t.keys, nb, n, t.loop_flag);
+  if ((e = radix_sort_pairs(t.keys, t.vals, t.keys_alt, t.vals_alt, nb, bits_for_index(nb), sc, st)) != cudaSuccess)
+    return e;
+  k_cap_loop_flags<<<blocks, kThreads, 0, st>>>(t.keys, nb, t.loop_flag);
   note_launch();
-  if ((e = exclusive_scan_u32(t.loop_flag, t.loop_start, n, sc, st)) != cudaSuccess) return e;
-  k_cap_loops<<<grid_for(n, num_sms), kThreads, 0, st>>>(verts, V, t.half, t.keys, t.vals, t.loop_flag, t.loop_start,
-                                                         nb, centres, cap_tris);
+  if ((e = exclusive_scan_u32(t.loop_flag, t.loop_start, nb, sc, st)) != cudaSuccess) return e;
+  k_cap_loops<<<blocks, kThreads, 0, st>>>(verts, V, t.half, t.keys, t.vals, t.loop_flag, t.loop_start, nb, centres,
+                                           cap_tris);
   note_launch();
-  k_cap_totals<<<1, 1, 0, st>>>(t.starts, n, t.loop_start, totals);
-  note_launch();
-  return cudaGetLastError();
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  return cudaMemcpyAsync(totals + 1, t.loop_start + nb, 8, cudaMemcpyDeviceToDevice, st);
 }

@@ -55,3 +55,24 @@ def test_tree_batch_of_unequal_meshes(ctx):
     dists, _ = ctx.bake_batch(meshes, grids, opts)
     for (v, i), g, d in zip(meshes, grids, dists):
         assert np.array_equal(d, ctx.bake(v, i, g, opts)[0])
+
+
+@pytest.mark.parametrize("leaf", [2, 8])
+def test_block_pass_with_more_nodes_than_it_keeps(ctx, oracle, leaf):
+    """Cells about the centre of a sphere: every node of every level may hold the nearest triangle, at
+    blocks of two 5120 nodes on the last level (the pass keeps 2048 and walks the others' subtrees)."""
+    import sdfb
+    from sdfb import meshgen as mg
+    v, f = mg.icosphere(7)
+    v, n, voxel = (v * 0.4).astype(np.float32), (3, 4, 5), 1e-3
+    origin = tuple(-0.5 * voxel * k for k in n)
+    g = sdfb.make_grid(origin, voxel, n)
+    d64 = oracle.distance(v, f, origin, voxel, n)
+    ref = None
+    for tile, budget in ((1, -1), (1, 64), (4, 64), (5, 64), (6, 64)):
+        d, _ = ctx.bake(v, f, g, sdfb.make_opts(sign_mode=sdfb.SIGN_NONE, leaf_size=leaf, tile=tile, step_budget=budget,
+                                                no_occupancy=True), want_occ=False)
+        if ref is None:
+            ref = d
+            assert np.abs(d.reshape(-1) - d64).max() <= TOL * 0.8  # the sphere's diameter, not the grid's
+        assert np.array_equal(d, ref), (tile, budget)
