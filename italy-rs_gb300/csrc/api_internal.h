@@ -96,6 +96,7 @@ struct GwnInput {
   float band_voxels;
   uint32_t *err;
   uint64_t gwn_cells;  // cells of the winding-number meshes (refine list capacity)
+  uint32_t most_caps;  // cap triangles of the mesh that has most
 };
 
 // Workspace::misc (256 bytes, zeroed before every bake): error flags at 0, the distance tile

@@ -35,7 +35,8 @@
 //     near caps' solid angles in FP32 with a bound on their rounding error (solid_angle_bounded),
 //     then the cells that stay undecided twice more with fine subtrees (kTau64Fine, kTau64Finest), a
 //     warp to a cell and solid angles in FP64; a cell still undecided goes to
-//   pass 3 (FP64 sum over every cap triangle of its mesh, one block per cell).
+//   pass 3 (FP64 sum over every cap triangle of its mesh, one block per cell), which takes the coarse
+//     pass's cells at once when they and the caps are few.
 // A sign is only given where the summed bounds prove it, so the FP32 solid angles of pass 2 change
 // none: they filter the cells that need FP64 ones (FP64 runs at 1/64 of the FP32 rate here).
 #include <algorithm>
@@ -49,6 +50,7 @@ using namespace sdfb;
 namespace {
 
 constexpr int kThreads = 256;
+constexpr int kMinBlocks = 3;  // 80 registers: sign stage of the 512^3 scene 11.6 ms at 2, 10.1 at 3, 11.5 at 4
 constexpr int kWarps = kThreads / kWarp;
 constexpr double kInv4Pi = 0.07957747154594767;
 // Largest far-field error bound (sr) taken for one cap subtree. A cell is decided once the summed
@@ -102,11 +104,14 @@ __device__ __forceinline__ float solid_angle_bounded(V3<float> a, V3<float> b, V
   return 2.0f * atan2f(det, den);
 }
 
-// Cells of a tile left to pass 2: bit l of cells[v] is lane l's cell v.
+// Up to 32 of a tile's cells left to pass 2, from the (32 part)-th on: bit l of cells[v] is lane l's
+// cell v. A part is a warp's work there: whole tiles leave the last warps with four walks each (10k
+// triangles at res 100: k_gwn64 199 us for 96).
 struct TileCells {
-  uint64_t tile;
+  uint64_t tile_part;  // tile | part << kPartShift
   uint32_t cells[kGwnCellsPerLane];
 };
+constexpr int kPartShift = 56;
 
 struct GwnArgs {
   BatchDev batch;  // each GWN mesh record names its caps hierarchy
@@ -114,13 +119,22 @@ struct GwnArgs {
   const float *col_z;
   const int8_t *col_s;
   float band_voxels;
-  TileCells *tiles;  // pass 1 -> pass 2 (coarse): tiles with cells to refine
+  TileCells *tiles;  // pass 1 -> pass 2 (coarse): tiles' parts with cells to refine
   unsigned long long *listed_tiles, *refine_count;  // their number, and their cells'
   uint64_t *cells;  // pass 2 (coarse) -> pass 2 (fine): global cells
   unsigned long long *cell_count;
   unsigned long long *tile_counter;
+  uint32_t most_caps;  // of a mesh
   uint32_t *err;
 };
+
+// Whether the cells that the coarse pass left are summed directly. The two fine passes take at least
+// the latency of one cell's walk each, 100 and 190 us at 600 caps and 0.35 ms at 3600, however few the
+// cells; the direct sum takes about 75 cycles of an SM a cap and cell, 0.5 ms at the bound. Sign stage
+// with the fine passes and without: 50 cells, 600 caps 0.60-0.77 -> 0.37-0.44 ms; 200 cells, 3600 caps
+// 1.66-1.80 -> 0.92-0.97 ms.
+constexpr unsigned long long kDirectWork = 1 << 21;  // caps times cells
+__device__ __forceinline__ bool few(const GwnArgs &a) { return *a.cell_count * a.most_caps <= kDirectWork; }
 
 // Signed crossings of the column above height pz (the integer winding number of mesh + caps).
 __device__ __forceinline__ int column_winding(const GwnArgs &a, const MeshRec &M, int vx, int vy, float pz) {
@@ -380,7 +394,7 @@ struct GwnTile {
 };
 
 // Pass 1: FP32 over the tiles of the winding-number meshes.
-__global__ __launch_bounds__(kThreads) void k_gwn32(GwnArgs a) {
+__global__ __launch_bounds__(kThreads, kMinBlocks) void k_gwn32(GwnArgs a) {
   constexpr int V = kGwnCellsPerLane;
   const int lane = threadIdx.x & 31;
   const BatchDev &B = a.batch;
@@ -432,12 +446,20 @@ __global__ __launch_bounds__(kThreads) void k_gwn32(GwnArgs a) {
       left[v] = __ballot_sync(kFull, refine);
       count += __popc(left[v]);
     }
-    if (count && lane == 0) {
-      TileCells &o = a.tiles[atomicAdd(a.listed_tiles, 1ull)];
-      o.tile = tile;
+    if (count) {
+      const int parts = (count + kWarp - 1) / kWarp;
+      unsigned long long at = 0;
+      if (lane == 0) {
+        at = atomicAdd(a.listed_tiles, static_cast<unsigned long long>(parts));
+        atomicAdd(a.refine_count, static_cast<unsigned long long>(count));
+      }
+      at = __shfl_sync(kFull, at, 0);
+      if (lane < parts) {
+        TileCells &o = a.tiles[at + lane];
+        o.tile_part = tile | uint64_t(lane) << kPartShift;
 #pragma unroll
-      for (int v = 0; v < V; ++v) o.cells[v] = left[v];
-      atomicAdd(a.refine_count, static_cast<unsigned long long>(count));
+        for (int v = 0; v < V; ++v) o.cells[v] = left[v];
+      }
     }
   }
   if (corrupt) atomic_or_err(a.err, kErrCorruptTree);
@@ -454,9 +476,9 @@ __device__ __forceinline__ bool undecided64(const MeshRec &M, uint64_t cell, int
   return !(c + e < 0.5);
 }
 
-// Pass 2, coarse: a listed tile's cells, 32 at a time. The list lengths are read on the device, so no
+// Pass 2, coarse: a listed tile's cells, 32 a warp. The list lengths are read on the device, so no
 // pass needs a host round trip.
-__global__ __launch_bounds__(kThreads) void k_gwn64(GwnArgs a) {
+__global__ __launch_bounds__(kThreads, kMinBlocks) void k_gwn64(GwnArgs a) {
   const unsigned long long n = *a.listed_tiles;
   const int lane = threadIdx.x & 31;
   const BatchDev &B = a.batch;
@@ -466,7 +488,7 @@ __global__ __launch_bounds__(kThreads) void k_gwn64(GwnArgs a) {
   for (unsigned long long k = blockIdx.x * (unsigned long long)kWarps + (threadIdx.x >> 5); k < n;
        k += (unsigned long long)gridDim.x * kWarps) {
     const TileCells &in = a.tiles[k];
-    const GwnTile t(B, in.tile);
+    const GwnTile t(B, in.tile_part & ((1ull << kPartShift) - 1));
     const MeshRec &M = B.recs[t.mesh];
     const GridDev g = M.g;
     float gx, gy, gz;
@@ -474,35 +496,34 @@ __global__ __launch_bounds__(kThreads) void k_gwn64(GwnArgs a) {
     int total = 0;
 #pragma unroll
     for (int v = 0; v < kGwnCellsPerLane; ++v) total += __popc(in.cells[v]);
-    for (int base = 0; base < total; base += kWarp) {
-      // this lane's cell: the (base + lane)-th listed one of the tile
-      const bool active = base + lane < total;
-      int rank = active ? base + lane : base, v = 0;
+    // this lane's cell: the (base + lane)-th listed one of the tile
+    const int base = static_cast<int>(in.tile_part >> kPartShift) * kWarp;
+    const bool active = base + lane < total;
+    int rank = active ? base + lane : base, v = 0;
 #pragma unroll
-      for (int j = 0; j < kGwnCellsPerLane - 1; ++j) {
-        const int c = __popc(in.cells[j]);
-        if (v == j && rank >= c) {
-          rank -= c;
-          ++v;
-        }
+    for (int j = 0; j < kGwnCellsPerLane - 1; ++j) {
+      const int c = __popc(in.cells[j]);
+      if (v == j && rank >= c) {
+        rank -= c;
+        ++v;
       }
-      const int src = __fns(in.cells[v], 0, rank + 1);
-      const int vx = t.vx(src), vy = t.vy(src), vz = t.vz(src, v);
-      const float qz[1] = {cell_center(g.oz, vz, g.voxel)};
-      const bool act[1] = {active};
-      double wex[1] = {0.0}, eps[1] = {0.0};
-      if (M.cap_root >= 0)
-        caps_walk<double, false, false, 1>(M, mem, act, cell_center(g.ox, vx, g.voxel), cell_center(g.oy, vy, g.voxel),
-                                           qz, gx, gy, gz, rho_g, kTau64, wex, eps, corrupt);
-      const uint64_t cell = (uint64_t(vz) * g.ny + vy) * g.nx + vx;
-      const bool left = active && undecided64(M, cell, column_winding(a, M, vx, vy, qz[0]), wex[0], eps[0]);
-      const unsigned mask = __ballot_sync(kFull, left);
-      if (mask) {
-        unsigned long long at = 0;
-        if (lane == 0) at = atomicAdd(a.cell_count, static_cast<unsigned long long>(__popc(mask)));
-        at = __shfl_sync(kFull, at, 0) + __popc(mask & ((1u << lane) - 1u));
-        if (left) a.cells[at] = B.cell_starts[t.mesh] + cell;
-      }
+    }
+    const int src = __fns(in.cells[v], 0, rank + 1);
+    const int vx = t.vx(src), vy = t.vy(src), vz = t.vz(src, v);
+    const float qz[1] = {cell_center(g.oz, vz, g.voxel)};
+    const bool act[1] = {active};
+    double wex[1] = {0.0}, eps[1] = {0.0};
+    if (M.cap_root >= 0)
+      caps_walk<double, false, false, 1>(M, mem, act, cell_center(g.ox, vx, g.voxel), cell_center(g.oy, vy, g.voxel),
+                                         qz, gx, gy, gz, rho_g, kTau64, wex, eps, corrupt);
+    const uint64_t cell = (uint64_t(vz) * g.ny + vy) * g.nx + vx;
+    const bool left = active && undecided64(M, cell, column_winding(a, M, vx, vy, qz[0]), wex[0], eps[0]);
+    const unsigned mask = __ballot_sync(kFull, left);
+    if (mask) {
+      unsigned long long at = 0;
+      if (lane == 0) at = atomicAdd(a.cell_count, static_cast<unsigned long long>(__popc(mask)));
+      at = __shfl_sync(kFull, at, 0) + __popc(mask & ((1u << lane) - 1u));
+      if (left) a.cells[at] = B.cell_starts[t.mesh] + cell;
     }
   }
   if (corrupt) atomic_or_err(a.err, kErrCorruptTree);
@@ -523,6 +544,7 @@ __device__ __forceinline__ void cell_of(const BatchDev &B, uint64_t gcell, int &
 __global__ __launch_bounds__(kThreads) void k_gwn64_fine(GwnArgs a, float tau, const uint64_t *__restrict__ in,
                                                          const unsigned long long *in_count, uint64_t *out,
                                                          unsigned long long *out_count) {
+  if (few(a)) return;
   const unsigned long long n = *in_count;
   const int lane = threadIdx.x & 31;
   const BatchDev &B = a.batch;
@@ -549,11 +571,17 @@ __global__ __launch_bounds__(kThreads) void k_gwn64_fine(GwnArgs a, float tau, c
 }
 
 // Pass 3: one block per remaining cell, FP64 sum over every cap triangle of its mesh.
-__global__ __launch_bounds__(kThreads) void k_gwn_direct(GwnArgs a, const uint64_t *__restrict__ in,
-                                                         const unsigned long long *in_count) {
+__global__ __launch_bounds__(kThreads) void k_gwn_direct(GwnArgs a, unsigned long long *last_count) {
   __shared__ double part[kThreads / kWarp];
   const BatchDev &B = a.batch;
-  const unsigned long long n = *in_count;
+  const uint64_t *__restrict__ in = a.cells;
+  unsigned long long n;
+  if (few(a)) {
+    n = *a.cell_count;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *last_count = n;
+  } else {
+    n = *last_count;
+  }
   for (unsigned long long k = blockIdx.x; k < n; k += gridDim.x) {
     int mesh, vx, vy, vz;
     uint64_t cell;
@@ -591,9 +619,11 @@ __global__ __launch_bounds__(kThreads) void k_gwn_direct(GwnArgs a, const uint64
 
 namespace {
 // counters | cells of the coarse pass | cells of the fine pass, sharing their room with the tiles' list
-// (read by the coarse pass alone; a tile of kGwnCellsPerLane x 32 cells takes 24 bytes)
+// (read by the coarse pass alone; 24 bytes for 32 cells of a tile)
 size_t list_bytes(uint64_t gwn_cells) { return (gwn_cells * 8 + 255) & ~size_t(255); }
-size_t tile_list_bytes(uint64_t gwn_tiles) { return (gwn_tiles * sizeof(TileCells) + 255) & ~size_t(255); }
+size_t tile_list_bytes(uint64_t gwn_tiles) {
+  return (gwn_tiles * kGwnCellsPerLane * sizeof(TileCells) + 255) & ~size_t(255);
+}
 }  // namespace
 
 size_t gwn_temp_bytes(uint64_t gwn_cells, uint64_t gwn_tiles) {
@@ -619,6 +649,7 @@ cudaError_t gwn_enqueue(const GwnInput &in, void *temp, int num_sms, cudaStream_
   a.cells = reinterpret_cast<uint64_t *>(base + 256);
   a.tiles = reinterpret_cast<TileCells *>(base + 256 + list_bytes(in.gwn_cells));
   uint64_t *fine = reinterpret_cast<uint64_t *>(a.tiles);  // the coarse pass has read the tiles by then (stream order)
+  a.most_caps = in.most_caps;
   a.err = in.err;
   cudaError_t e = cudaMemsetAsync(counters, 0, 64, st);
   if (e != cudaSuccess) return e;
@@ -640,7 +671,7 @@ cudaError_t gwn_enqueue(const GwnInput &in, void *temp, int num_sms, cudaStream_
   k_gwn64_fine<<<static_cast<unsigned>(wave_fine), kThreads, 0, st>>>(a, kTau64Finest, fine, fine_count, a.cells,
                                                                       last_count);
   note_launch();
-  k_gwn_direct<<<static_cast<unsigned>(num_sms * 4), kThreads, 0, st>>>(a, a.cells, last_count);
+  k_gwn_direct<<<static_cast<unsigned>(num_sms * 4), kThreads, 0, st>>>(a, last_count);
   note_launch();
   return cudaGetLastError();
 }

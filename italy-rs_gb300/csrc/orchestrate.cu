@@ -449,7 +449,7 @@ sdfb_status enqueue_batch(sdfb_ctx *ctx, Workspace &ws, cudaStream_t st, std::ve
   da.step_budget = L.step_budget;
   da.stack_depth = L.stack;
   da.fault = o.fault_inject;
-  GwnInput gi;
+  GwnInput gi{};
   gi.batch = B;
   gi.col_start = static_cast<const uint64_t *>(ws.col_start.p);
   gi.col_z = static_cast<const float *>(ws.col_z.p);
@@ -457,6 +457,7 @@ sdfb_status enqueue_batch(sdfb_ctx *ctx, Workspace &ws, cudaStream_t st, std::ve
   gi.band_voxels = o.band_voxels;
   gi.err = d_err;
   gi.gwn_cells = L.gwn_cells;
+  for (const MeshRec &r : L.recs) gi.most_caps = std::max(gi.most_caps, r.cap_tris);
 
   bool capturing = false;
   // Inside a capture, an event record must be an external node to time the replay.

@@ -35,3 +35,23 @@ def test_group_walk_signs(ctx, oracle, kind, dims):
     d64 = oracle.distance(v, f, origin, voxel, dims)
     sure = (np.abs(np.abs(w) - 0.5) > 1e-6) & (d64 > 1e-6)
     assert np.array_equal(d.reshape(-1)[sure] < 0, np.abs(w[sure]) > 0.5)
+
+
+@pytest.mark.parametrize("level, direct", [(3, True), (7, False)])
+def test_cells_left_by_the_coarse_pass(ctx, oracle, level, direct):
+    """A bowl's opening, where many cells lie near the level set: with a short rim they are summed
+    directly, with a long one walked again, and both give the FP64 sum's sides."""
+    import sdfb
+    from sdfb import meshgen as mg
+    v, f = mg.displaced_icosphere(level, 0.33, 3)
+    f = np.ascontiguousarray(f[v[f].mean(axis=1)[:, 2] < 0.12])
+    dims = (130, 131, 40)
+    voxel, origin = 0.7 / 130, (-0.351, -0.352, 0.0)
+    st = sdfb.Stats()
+    d, _ = ctx.bake(v, f, sdfb.make_grid(origin, voxel, dims), sdfb.make_opts(sign_mode=sdfb.SIGN_GWN), stats=st)
+    assert st.gwn_fp64_cells > 0 and (st.gwn_direct_cells > 100) == direct
+    samples = np.sort(np.random.default_rng(level).choice(np.prod(dims), 3000, replace=False)).astype(np.int64)
+    w = oracle.gwn(v, f, origin, voxel, dims, samples=samples)
+    d64 = oracle.distance(v, f, origin, voxel, dims, samples=samples)
+    sure = (np.abs(np.abs(w) - 0.5) > 1e-6) & (d64 > 1e-6)
+    assert np.array_equal(d.reshape(-1)[samples][sure] < 0, np.abs(w[sure]) > 0.5)
