@@ -72,6 +72,8 @@ void PinBuf::release() {
 }
 
 sdfb_ctx::~sdfb_ctx() {
+  if (gate_fork) cudaEventDestroy(gate_fork);
+  if (gate_stream) cudaStreamDestroy(gate_stream);
   if (stream) cudaStreamDestroy(stream);
 }
 
@@ -241,13 +243,20 @@ sdfb_status device_caps(sdfb_ctx *ctx, cudaStream_t st, std::vector<PlanMesh> &m
 }
 
 sdfb_status device_signs(sdfb_ctx *ctx, const sdfb_opts &o, PlanMesh *ms, size_t count, bool needed, cudaStream_t st,
-                         size_t *bad) {
+                         size_t *bad, const std::function<sdfb_status()> &meanwhile) {
   size_t at = 0;
   if (!needed) return SDFB_OK;
   if (o.sign_mode != SDFB_SIGN_PARITY && o.sign_mode != SDFB_SIGN_GWN && o.sign_mode != SDFB_SIGN_NONE) {
     std::vector<PlanMesh *> v(count);
     for (size_t m = 0; m < count; ++m) v[m] = ms + m;
-    const sdfb_status s = device_gate(ctx, v, st, bad ? bad : &at);
+    sdfb_status s;
+    if (meanwhile) {
+      if ((s = fork_gate(ctx, st)) != SDFB_OK) return s;
+      s = device_gate(ctx, v, ctx->gate_stream, bad ? bad : &at, meanwhile);
+      if (s != SDFB_OK) cudaStreamSynchronize(st);  // what meanwhile enqueued reads the caller's mesh
+    } else {
+      s = device_gate(ctx, v, st, bad ? bad : &at);
+    }
     if (s != SDFB_OK) return s;
   }
   for (size_t m = 0; m < count; ++m) {
@@ -285,7 +294,9 @@ sdfb_status sdfb_ctx_create(int32_t device, sdfb_ctx **out) {
   sdfb_ctx *ctx = new sdfb_ctx();
   ctx->device = device;
   ctx->num_sms = prop.multiProcessorCount;
-  if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess) {
+  if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaStreamCreateWithFlags(&ctx->gate_stream, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreateWithFlags(&ctx->gate_fork, cudaEventDisableTiming) != cudaSuccess) {
     delete ctx;
     return SDFB_ERR_CUDA;
   }
@@ -364,10 +375,14 @@ sdfb_status sdfb_bake_device(sdfb_ctx *ctx, const float *d_verts, uint32_t num_v
   p.grid = *grid;
   p.dist = o.no_distance ? nullptr : d_dist_out;
   p.occ = o.no_occupancy ? nullptr : d_occ_out;
-  sdfb_status s = device_signs(ctx, o, &p, 1, p.dist || !p.occ || stats, st);
+  // With statistics the stages run one after another, so that each has its own time.
+  std::function<sdfb_status()> tree;
+  if (p.dist && !stats) tree = [&] { return early_tree(ctx, st, ms, o); };
+  sdfb_status s = device_signs(ctx, o, &p, 1, p.dist || !p.occ || stats, st, nullptr, tree);
   if (s != SDFB_OK) return s;
-  if ((s = device_caps(ctx, st, ms)) != SDFB_OK) return s;
-  return run_batch(ctx, st, ms, o, false, stats);
+  if ((s = device_caps(ctx, st, ms)) == SDFB_OK) s = run_batch(ctx, st, ms, o, false, stats, p.bvh != nullptr);
+  if (s != SDFB_OK && p.bvh) cudaStreamSynchronize(st);  // the early build reads the caller's mesh
+  return s;
 }
 
 sdfb_status sdfb_bake(sdfb_ctx *ctx, const float *verts, uint32_t num_verts, const uint32_t *idx, uint32_t num_tris,
@@ -396,7 +411,9 @@ sdfb_status sdfb_bake(sdfb_ctx *ctx, const float *verts, uint32_t num_verts, con
   p.V = num_verts;
   p.T = num_tris;
   p.grid = *grid;
-  sdfb_status s = device_signs(ctx, o, &p, 1, want_dist || !want_occ || stats, st);
+  std::function<sdfb_status()> tree;
+  if (want_dist && !stats) tree = [&] { return early_tree(ctx, st, ms, o); };
+  sdfb_status s = device_signs(ctx, o, &p, 1, want_dist || !want_occ || stats, st, nullptr, tree);
   if (s != SDFB_OK) return s;
   float *const direct_dist =
       (want_dist && p.sign != kSignGwn) ? static_cast<float *>(mapped_host(dist_out)) : nullptr;
@@ -404,7 +421,7 @@ sdfb_status sdfb_bake(sdfb_ctx *ctx, const float *verts, uint32_t num_verts, con
   p.dist = want_dist ? (direct_dist ? direct_dist : static_cast<float *>(ctx->out_dist.p)) : nullptr;
   p.occ = want_occ ? (direct_occ ? direct_occ : static_cast<uint8_t *>(ctx->out_occ.p)) : nullptr;
   if ((s = device_caps(ctx, st, ms)) != SDFB_OK) return s;
-  s = run_batch(ctx, st, ms, o, false, stats);
+  s = run_batch(ctx, st, ms, o, false, stats, p.bvh != nullptr);
   if (s != SDFB_OK) return s;
   if (want_dist && !direct_dist)
     CK(cudaMemcpyAsync(dist_out, ctx->out_dist.p, cells * 4, cudaMemcpyDeviceToHost, st));
@@ -439,6 +456,11 @@ sdfb_status sdfb_bake_soup(sdfb_ctx *ctx, const float *positions, uint32_t num_t
   CK(iota_device(static_cast<uint32_t *>(ctx->in_idx.p), V, ctx->num_sms, st));
   std::vector<PlanMesh> ms(1);
   PlanMesh &p = ms[0];
+  p.verts = static_cast<const float *>(ctx->in_verts.p);
+  p.idx = static_cast<const uint32_t *>(ctx->in_idx.p);
+  p.V = V;
+  p.T = num_tris;
+  p.grid = *grid_out;
   uint32_t U = 0;
   uint32_t *d_welded = nullptr;
   // Occupancy alone, without statistics, needs neither the sign nor the welded crossing mesh.
@@ -453,17 +475,28 @@ sdfb_status sdfb_bake_soup(sdfb_ctx *ctx, const float *positions, uint32_t num_t
     d_welded = static_cast<uint32_t *>(ctx->in_idx2.p);
     char *d_tmp = static_cast<char *>(ctx->weld_tmp.p);
     const uint64_t *d_unique = nullptr;
+    // Beside it, unless the stages are timed one by one, the tree of the soup.
+    const bool beside = want_dist && !stats;
+    if (beside && (s = fork_gate(ctx, st)) != SDFB_OK) return s;
+    const cudaStream_t gs = beside ? ctx->gate_stream : st;
     CK(weld_enqueue(static_cast<const float *>(ctx->in_verts.p), V, weld_cell(bounds_min, bounds_max), d_welded,
-                    static_cast<float *>(ctx->in_verts2.p), d_tmp, weld_bytes, &d_unique, ctx->num_sms, st));
+                    static_cast<float *>(ctx->in_verts2.p), d_tmp, weld_bytes, &d_unique, ctx->num_sms, gs));
     uint64_t *h = static_cast<uint64_t *>(ctx->gate_pin.p);  // unique positions, boundary - 1, non-manifold - 1
-    CK(cudaMemcpyAsync(h, d_unique, 8, cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(h, d_unique, 8, cudaMemcpyDeviceToHost, gs));
     if (o.sign_mode == SDFB_SIGN_AUTO) {
       const unsigned long long *d_counts = nullptr;
       CK(watertight_enqueue(d_welded, num_tris, d_tmp + weld_bytes, watertight_temp_bytes(num_tris), &d_counts,
-                            ctx->num_sms, st));
-      CK(cudaMemcpyAsync(h + 1, d_counts, 16, cudaMemcpyDeviceToHost, st));
+                            ctx->num_sms, gs));
+      CK(cudaMemcpyAsync(h + 1, d_counts, 16, cudaMemcpyDeviceToHost, gs));
     }
-    CK(cudaStreamSynchronize(st));
+    if (beside) {
+      p.dist = static_cast<float *>(ctx->out_dist.p);
+      if ((s = early_tree(ctx, st, ms, o)) != SDFB_OK) {
+        cudaStreamSynchronize(gs);
+        return s;
+      }
+    }
+    CK(cudaStreamSynchronize(gs));
     U = static_cast<uint32_t>(h[0]);
     if (o.sign_mode == SDFB_SIGN_AUTO) {
       p.watertight = (h[1] + 1 == 0 && h[2] + 1 == 0) ? 1 : 0;
@@ -472,11 +505,6 @@ sdfb_status sdfb_bake_soup(sdfb_ctx *ctx, const float *positions, uint32_t num_t
       p.sign = o.sign_mode == SDFB_SIGN_PARITY ? kSignParity : (o.sign_mode == SDFB_SIGN_NONE ? kSignNone : kSignGwn);
     }
   }
-  p.verts = static_cast<const float *>(ctx->in_verts.p);
-  p.idx = static_cast<const uint32_t *>(ctx->in_idx.p);
-  p.V = V;
-  p.T = num_tris;
-  p.grid = *grid_out;
   float *const direct_dist =
       (want_dist && p.sign != kSignGwn) ? static_cast<float *>(mapped_host(dist_out)) : nullptr;
   p.dist = want_dist ? (direct_dist ? direct_dist : static_cast<float *>(ctx->out_dist.p)) : nullptr;
@@ -494,7 +522,7 @@ sdfb_status sdfb_bake_soup(sdfb_ctx *ctx, const float *positions, uint32_t num_t
     p.pV = U;
     p.pT = num_tris;
   }
-  s = run_batch(ctx, st, ms, o, false, stats);
+  s = run_batch(ctx, st, ms, o, false, stats, p.bvh != nullptr);
   if (s != SDFB_OK) return s;
   if (want_dist && !direct_dist)
     CK(cudaMemcpyAsync(dist_out, ctx->out_dist.p, cells * 4, cudaMemcpyDeviceToHost, st));

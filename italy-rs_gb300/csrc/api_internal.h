@@ -2,6 +2,7 @@
 #pragma once
 
 #include <cstdint>
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -112,7 +113,7 @@ constexpr int kDefaultStepBudget = 2048;
 struct Workspace {
   DevBuf batch_buf, bvh, build_tmp, par_tmp, col_start, col_z, col_s, caps_bvh, caps_tmp, misc, gwn_tmp, defer,
       col_bits;
-  PinBuf staging;
+  PinBuf staging, early_staging;
   cudaEvent_t ev[8] = {};
   uint64_t col_capacity_hint = 0;
   cudaGraphExec_t graph = nullptr;  // the last batch's launch sequence, replayed while it repeats
@@ -135,6 +136,10 @@ struct BatchState {
 struct sdfb_ctx {
   int device = 0, num_sms = 0;
   cudaStream_t stream = nullptr;
+  // The gate's own stream, and where it forks from a call's stream (see early_tree).
+  cudaStream_t gate_stream = nullptr;
+  cudaEvent_t gate_fork = nullptr;
+  ResidentBvh early;
   std::string err;
   // inputs / outputs of host-buffer calls
   DevBuf in_verts, in_idx, in_verts2, in_idx2, in_caps, in_capidx, out_dist, out_occ, first_tri, sparse_tmp,
@@ -173,15 +178,22 @@ sdfb_status ctx_cuda(sdfb_ctx *ctx, cudaError_t e, const char *what);
 // gate on the device, for all of them together (parity when watertight, else the winding number).
 // Fails with BAD_MESH on an index out of range (*bad, optional: the mesh). `needed` false (a bake of
 // occupancy alone that reports no statistics): nothing asks for the sign, and it stays none; the
-// occupancy kernels check the mesh.
+// occupancy kernels check the mesh. meanwhile: work for the call's own stream that does not depend on
+// the sign, enqueued while the gate runs beside it on the context's gate stream.
 sdfb_status device_signs(sdfb_ctx *ctx, const sdfb_opts &o, PlanMesh *ms, size_t count, bool needed, cudaStream_t st,
-                         size_t *bad = nullptr);
+                         size_t *bad = nullptr, const std::function<sdfb_status()> &meanwhile = nullptr);
 // Whether a batch asks for occupancy grids and nothing else: it needs no hierarchy.
 bool occupancy_alone(const std::vector<PlanMesh> &ms);
 // weld.cu: sets the watertight verdict of indexed meshes in device memory (the weld of their vertices
 // over their bounds, then the edge census of the welded triangles; equivalent to the reference's test
 // on the de-indexed soup). Synchronises the stream. BAD_MESH: mesh *bad has an index >= V.
-sdfb_status device_gate(sdfb_ctx *ctx, const std::vector<PlanMesh *> &ms, cudaStream_t st, size_t *bad);
+sdfb_status device_gate(sdfb_ctx *ctx, const std::vector<PlanMesh *> &ms, cudaStream_t st, size_t *bad,
+                        const std::function<sdfb_status()> &meanwhile = nullptr);
+// Makes the gate stream wait for what is on st.
+sdfb_status fork_gate(sdfb_ctx *ctx, cudaStream_t st);
+// Enqueues the build of a single mesh's tree on st, before its sign is known, and points the mesh at
+// it. The following run_batch has to be told (prebuilt), so that it keeps the build's error flags.
+sdfb_status early_tree(sdfb_ctx *ctx, cudaStream_t st, std::vector<PlanMesh> &ms, const sdfb_opts &o);
 // sdfb_voxelize_sparse; also returns the device list of the count occupied cells' linear indices
 // (valid until the context's next call) and the grid it used.
 sdfb_status voxelize_sparse_run(sdfb_ctx *ctx, const float *positions, uint32_t num_tris, const float bounds_min[3],
@@ -196,14 +208,14 @@ sdfb_opts opts_or_default(const sdfb_opts *o);
 // resident hierarchy or none does (then one hierarchy over all of them is built). use_graph:
 // capture the launch sequence into a CUDA graph and replay it while the batch is unchanged.
 sdfb_status enqueue_batch(sdfb_ctx *ctx, Workspace &ws, cudaStream_t st, std::vector<PlanMesh> &meshes,
-                          const sdfb_opts &opts, bool use_graph, BatchState &state);
+                          const sdfb_opts &opts, bool use_graph, BatchState &state, bool prebuilt = false);
 // Waits for the stream, reads the device error word and fills stats. SDFB_ERR_BUSY means the
 // crossing list outgrew its buffer: enqueue the same batch again (the buffer has been resized).
 sdfb_status finish_batch(sdfb_ctx *ctx, Workspace &ws, cudaStream_t st, const BatchState &state,
                          const std::vector<PlanMesh> &meshes, sdfb_stats *stats);
 // enqueue + finish, retrying a crossing-list overflow and a shallow-stack overflow.
 sdfb_status run_batch(sdfb_ctx *ctx, cudaStream_t st, std::vector<PlanMesh> &meshes, const sdfb_opts &opts,
-                      bool use_graph, sdfb_stats *stats);
+                      bool use_graph, sdfb_stats *stats, bool prebuilt = false);
 // Builds the hierarchy of one mesh (and of its caps when cT > 0) into `mem` / `cap_mem`, which
 // must hold resident_bytes(T) / resident_bytes(cT, true). Enqueued on st with ws's temporaries.
 size_t resident_bytes(uint32_t tris, bool winding = false);

@@ -135,6 +135,7 @@ void Workspace::release() {
                  &gwn_tmp, &defer, &col_bits};
   for (DevBuf *x : b) x->release();
   staging.release();
+  early_staging.release();
 }
 
 uint64_t Workspace::bytes() const {
@@ -376,7 +377,7 @@ bool occupancy_alone(const std::vector<PlanMesh> &ms) {
 }
 
 sdfb_status enqueue_batch(sdfb_ctx *ctx, Workspace &ws, cudaStream_t st, std::vector<PlanMesh> &ms,
-                          const sdfb_opts &o, bool use_graph, BatchState &S) {
+                          const sdfb_opts &o, bool use_graph, BatchState &S, bool prebuilt) {
   if (ms.empty()) return ctx_fail(ctx, SDFB_ERR_INVALID_ARGUMENT, "empty batch");
   cudaGetLastError();  // start from a clean error state
   if (!ws.init()) return ctx_fail(ctx, SDFB_ERR_CUDA, "cannot create events");
@@ -469,7 +470,7 @@ sdfb_status enqueue_batch(sdfb_ctx *ctx, Workspace &ws, cudaStream_t st, std::ve
     {
       NvtxRange r("sdfb prepare");
       CK(cudaMemcpyAsync(ws.batch_buf.p, ws.staging.p, L.bytes, cudaMemcpyHostToDevice, st));
-      CK(cudaMemsetAsync(ws.misc.p, 0, 256, st));
+      if (!prebuilt) CK(cudaMemsetAsync(ws.misc.p, 0, 256, st));  // the early build's flags stand
     }
     CK(rec(ws.ev[0]));
     if (build) {
@@ -635,11 +636,11 @@ sdfb_status finish_batch(sdfb_ctx *ctx, Workspace &ws, cudaStream_t st, const Ba
 }
 
 sdfb_status run_batch(sdfb_ctx *ctx, cudaStream_t st, std::vector<PlanMesh> &ms, const sdfb_opts &o, bool use_graph,
-                      sdfb_stats *stats) {
+                      sdfb_stats *stats, bool prebuilt) {
   sdfb_opts oo = o;
   for (int attempt = 0; attempt < 4; ++attempt) {
     BatchState S;
-    sdfb_status s = enqueue_batch(ctx, ctx->ws, st, ms, oo, use_graph, S);
+    sdfb_status s = enqueue_batch(ctx, ctx->ws, st, ms, oo, use_graph, S, prebuilt && attempt == 0);
     if (s != SDFB_OK) return s;
     s = finish_batch(ctx, ctx->ws, st, S, ms, stats);
     if (s == SDFB_ERR_BUSY) continue;  // crossing list resized
@@ -650,6 +651,45 @@ sdfb_status run_batch(sdfb_ctx *ctx, cudaStream_t st, std::vector<PlanMesh> &ms,
     return s;
   }
   return ctx_fail(ctx, SDFB_ERR_INTERNAL, "bake did not settle after retries");
+}
+
+// ---------------------------------------------------------------------------------------------
+// The tree of a single mesh, while its gate runs. Both are short chains of small kernels that leave
+// most of the GPU idle and wait for nothing of each other, 45 us each at 1k triangles: bakes of 32^3,
+// 64^3 and 97 x 61 x 43 cells 239 -> 209, 398 -> 354 and 457 -> 404 us.
+
+sdfb_status fork_gate(sdfb_ctx *ctx, cudaStream_t st) {
+  CK(cudaEventRecord(ctx->gate_fork, st));
+  CK(cudaStreamWaitEvent(ctx->gate_stream, ctx->gate_fork, 0));
+  return SDFB_OK;
+}
+
+sdfb_status early_tree(sdfb_ctx *ctx, cudaStream_t st, std::vector<PlanMesh> &ms, const sdfb_opts &o) {
+  if (ms.size() != 1 || ms[0].bvh || ms[0].T >= (1u << 31)) return SDFB_OK;  // left to enqueue_batch
+  Workspace &ws = ctx->ws;
+  cudaGetLastError();
+  if (!ws.init()) return ctx_fail(ctx, SDFB_ERR_CUDA, "cannot create events");
+  t_alloc_cap = o.alloc_cap_kib > 0 ? uint64_t(o.alloc_cap_kib) << 10 : 0;
+  Layout L;
+  make_layout(ctx, ms, o, L);
+  ENSURE(ws.batch_buf, L.bytes);
+  if (!ws.early_staging.ensure(L.bytes)) return ctx_fail(ctx, SDFB_ERR_OUT_OF_MEMORY, "pinned staging");
+  ENSURE(ws.bvh, L.tree_bytes);
+  ENSURE(ws.build_tmp, std::max(ptree_temp_bytes(ms[0].T, 1), occupancy_temp_bytes(ms[0].T)));
+  ENSURE(ws.misc, 256);
+  bind_built(L, static_cast<char *>(ws.bvh.p), nullptr);
+  fill_staging(L, static_cast<char *>(ws.early_staging.p));
+  char *tab = static_cast<char *>(ws.batch_buf.p);
+  CK(cudaMemcpyAsync(tab, ws.early_staging.p, L.bytes, cudaMemcpyHostToDevice, st));
+  CK(cudaMemsetAsync(ws.misc.p, 0, 256, st));
+  CK(ptree_build(batch_dev(L, tab), reinterpret_cast<const PTreeRec *>(tab + L.o_trees),
+                 reinterpret_cast<const uint64_t *>(tab + L.o_group), L.group.back(), ws.build_tmp.p,
+                 ws.build_tmp.cap, static_cast<uint32_t *>(ws.misc.p), st));
+  ctx->early = ResidentBvh();
+  ctx->early.tree = L.trees[0];
+  ctx->early.num_tris = static_cast<int>(ms[0].T);
+  ms[0].bvh = &ctx->early;
+  return SDFB_OK;
 }
 
 // ---------------------------------------------------------------------------------------------

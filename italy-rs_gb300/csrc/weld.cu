@@ -370,7 +370,8 @@ cudaError_t watertight_device(const uint32_t *welded, uint64_t T, void *temp, si
 
 }  // namespace sdfb
 
-sdfb_status device_gate(sdfb_ctx *ctx, const std::vector<PlanMesh *> &ms, cudaStream_t st, size_t *bad) {
+sdfb_status device_gate(sdfb_ctx *ctx, const std::vector<PlanMesh *> &ms, cudaStream_t st, size_t *bad,
+                        const std::function<sdfb_status()> &meanwhile) {
   // Records first (uploaded), then everything that starts at ~0, then the slots of the vertices.
   const size_t n = ms.size();
   if (n == 0) return SDFB_OK;
@@ -437,7 +438,10 @@ sdfb_status device_gate(sdfb_ctx *ctx, const std::vector<PlanMesh *> &ms, cudaSt
   note_launch();
   e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaMemcpyAsync(h, d + o_result, n * 24, cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  const sdfb_status early = meanwhile && e == cudaSuccess ? meanwhile() : SDFB_OK;
+  const cudaError_t w = cudaStreamSynchronize(st);
+  if (e == cudaSuccess) e = w;
+  if (early != SDFB_OK) return early;
   if (e != cudaSuccess) return ctx_cuda(ctx, e, "watertight gate");
   for (size_t m = 0; m < n; ++m) {
     if (h[3 * m + 2] != ~0ull) {
