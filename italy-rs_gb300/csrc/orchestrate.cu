@@ -177,7 +177,8 @@ DistTree tree_view(const PTreeRec &r, int k) {
 
 void make_layout(sdfb_ctx *ctx, const std::vector<PlanMesh> &ms, const sdfb_opts &o, Layout &L) {
   const int M = static_cast<int>(ms.size());
-  // Batch-wide tile shape and stack depth: tuned for the mesh with the most cells, unless forced.
+  // Batch-wide tile shape and stack depth: tuned for the mesh with the most cells, unless forced. Not the
+  // step budget: the longest tiles are often those of another mesh, of more triangles a cell.
   size_t big = 0;
   for (int m = 1; m < M; ++m)
     if (uint64_t(ms[m].grid.nx) * ms[m].grid.ny * ms[m].grid.nz >
@@ -189,8 +190,8 @@ void make_layout(sdfb_ctx *ctx, const std::vector<PlanMesh> &ms, const sdfb_opts
                                                            : (batch ? ctx->batch_tile : ctx->tuned_tile[tb][nb]);
   L.stack = (o.stack_depth == 32 || o.stack_depth == 64) ? o.stack_depth
                                                          : (batch ? ctx->batch_stack : ctx->tuned_stack[tb][nb]);
-  L.step_budget = o.step_budget > 0 ? o.step_budget
-                                    : (o.step_budget < 0 ? 0 : (batch ? ctx->batch_budget : ctx->tuned_budget[tb][nb]));
+  const int tuned_budget = batch ? ctx->batch_budget : (M > 1 ? kBatchStepBudget : ctx->tuned_budget[tb][nb]);
+  L.step_budget = o.step_budget > 0 ? o.step_budget : (o.step_budget < 0 ? 0 : tuned_budget);
   L.resident = ms[0].bvh != nullptr;
   L.recs.resize(M);
   L.trees.resize(M);

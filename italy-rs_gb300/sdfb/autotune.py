@@ -12,14 +12,15 @@ Three parameters of the distance pass trade against each other with the mesh and
 The table also holds a traversal stack depth; every tree fits either, so it stays at 64.
 
 For each (log2 triangles, log2 grid edge) bucket of a sweep of displaced spheres and grids, the tuner
-times whole device-buffer bakes (CUDA events on the bake's stream, median of `reps`) under a
+times device-buffer bakes (the bake's own device time, median of `reps`; the geometric mean over a cubic
+and a ragged grid of the bucket, whose tiles the GPU holds in different numbers) under a
 coordinate descent over the four parameters, then fills every bucket of the table from the
 nearest measured one and writes "tri_bucket grid_bucket leaf tile stack budget" lines (tile
 0-based, budget 0 = never) that
 the library reads at context creation (tuning/gb300.tsv beside lib/, or the file SDFB_TUNING names).
 
-A batch takes its tile shape, stack depth and budget from the bucket of its mesh with the most
-cells. The batch mode (--batch) times a 64-mesh batch (1e3..1e6 triangles, 32^3..256^3 grids) with
+A batch takes its tile shape and stack depth from the bucket of its mesh with the most cells, and a
+step budget of its own (the longest tiles are often another mesh's). The batch mode (--batch) times a 64-mesh batch (1e3..1e6 triangles, 32^3..256^3 grids) with
 those choices and under a coordinate descent over batch-wide (tile, stack, budget) settings; when
 the best beats the table's choice by more than BATCH_GAIN it writes a "batch tile stack budget"
 line into the table, which the library then uses for every bake of more than one mesh, and
@@ -53,6 +54,11 @@ SWEEP = [(3, 32), (3, 64), (3, 128), (3, 256), (4, 64), (4, 128), (4, 256), (5, 
 QUICK = [(4, 128), (6, 256), (7, 256)]
 BATCH_GAIN = 0.02  # a batch-wide line is written only when it saves more than this fraction
 TORI = {"torus128k": (512, 128), "torus1m": (1024, 512)}  # nu x nv quads, 2 nu nv triangles
+
+
+def sweep_grids(n: int):
+    """The grids that stand for a bucket: both have their longest edge in [n, 2n)."""
+    return [(n, n, n), (round(1.5 * n), n, round(0.7 * n))]
 
 
 def sweep_mesh(meshgen, key):
@@ -168,32 +174,31 @@ def _time_batch(ctx, torch, sdfb, devm, grids, outs, params, reps: int) -> float
     return times[len(times) // 2]
 
 
-def _time_bake(ctx, torch, sdfb, dev, grid, params, reps: int) -> float:
+def _time_bake(ctx, sdfb, dev, grids, params, reps: int) -> float:
+    """Geometric mean over the grids of the median device time of a bake."""
     leaf, tile, stack, budget = params
     opts = sdfb.make_opts(sign_mode=sdfb.SIGN_PARITY, leaf_size=leaf, tile=tile, stack_depth=stack,
                           step_budget=budget)
-    stream = torch.cuda.current_stream()
     dv, nv, di, nt, dd, do = dev
-    ctx.bake_device(dv, nv, di, nt, grid, opts, dd, do, stream.cuda_stream)  # warm-up
-    times = []
-    for _ in range(reps):
-        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        e0.record(stream)
-        ctx.bake_device(dv, nv, di, nt, grid, opts, dd, do, stream.cuda_stream)
-        e1.record(stream)
-        e1.synchronize()
-        times.append(e0.elapsed_time(e1))
-    times.sort()
-    return times[len(times) // 2]
+    product = 1.0
+    for grid in grids:
+        times = []
+        for _ in range(reps + 1):  # the first is a warm-up
+            st = sdfb.Stats()
+            ctx.bake_device(dv, nv, di, nt, grid, opts, dd, do, stats=st)
+            times.append(st.ms_total)
+        times = sorted(times[1:])
+        product *= times[len(times) // 2]
+    return product ** (1.0 / len(grids))
 
 
-def tune_case(ctx, torch, sdfb, dev, grid, reps: int, log=print):
+def tune_case(ctx, sdfb, dev, grids, reps: int, log=print):
     """Coordinate descent: tile, leaf, stack, budget, then tile again. Returns (params, ms)."""
     cache = {}
 
     def t(p):
         if p not in cache:
-            cache[p] = _time_bake(ctx, torch, sdfb, dev, grid, p, reps)
+            cache[p] = _time_bake(ctx, sdfb, dev, grids, p, reps)
         return cache[p]
 
     best = START
@@ -214,7 +219,7 @@ def main(argv=None):
     ap = argparse.ArgumentParser(description=__doc__.splitlines()[0])
     ap.add_argument("--out", default=DEFAULT_OUT)
     ap.add_argument("--quick", action="store_true", help="three buckets only")
-    ap.add_argument("--reps", type=int, default=3)
+    ap.add_argument("--reps", type=int, default=9)
     ap.add_argument("--batch", action="store_true", help="tune batch-wide settings against the table at --out")
     args = ap.parse_args(argv)
 
@@ -257,15 +262,17 @@ def main(argv=None):
         if level not in meshes:
             meshes[level] = sweep_mesh(meshgen, level)
         v, f = meshes[level]
-        grid = sdfb.make_grid((-0.5, -0.5, -0.5), 1.0 / n, (n, n, n))
+        grids = [sdfb.make_grid(tuple(-0.5 * d / max(g) for d in g), 1.0 / max(g), g) for g in sweep_grids(n)]
+        cells = max(g.cells for g in grids)
         dv = torch.from_numpy(np.ascontiguousarray(v, np.float32)).cuda()
         di = torch.from_numpy(np.ascontiguousarray(f, np.int32)).cuda()
-        dd = torch.empty(grid.cells, dtype=torch.float32, device="cuda")
-        do = torch.empty(grid.cells, dtype=torch.uint8, device="cuda")
+        dd = torch.empty(cells, dtype=torch.float32, device="cuda")
+        do = torch.empty(cells, dtype=torch.uint8, device="cuda")
+        torch.cuda.synchronize()
         key = (bucket_tris(len(f)), bucket_grid(n))
-        print(f"  {len(f):>7} triangles, {n}^3 grid -> bucket {key}", flush=True)
-        params, ms = tune_case(ctx, torch, sdfb, (dv.data_ptr(), len(v), di.data_ptr(), len(f),
-                                                  dd.data_ptr(), do.data_ptr()), grid, args.reps)
+        print(f"  {len(f):>7} triangles, {n}^3 and ragged grids -> bucket {key}", flush=True)
+        params, ms = tune_case(ctx, sdfb, (dv.data_ptr(), len(v), di.data_ptr(), len(f),
+                                                  dd.data_ptr(), do.data_ptr()), grids, args.reps)
         if key not in measured or ms < times[key]:
             measured[key], times[key] = params, ms
         del dv, di, dd, do
