@@ -9,7 +9,7 @@ Three parameters of the distance pass trade against each other with the mesh and
   * step budget (work steps between a tile's looks at whether it should be handed to the
     block-per-tile second pass, or never): a small budget moves more tiles into the pass that splits
     a tile's walk over a block, which pays on small grids (fewer tiles than the GPU holds warps).
-The table also holds a traversal stack depth; every tree fits either, so it stays at 64.
+The table also holds a traversal stack depth, 32 or 64; every tree fits either.
 
 For each (log2 triangles, log2 grid edge) bucket of a sweep of displaced spheres and grids, the tuner
 times device-buffer bakes (the bake's own device time, median of `reps`; the geometric mean over a cubic
@@ -41,7 +41,7 @@ DEFAULT_OUT = os.path.join(os.path.dirname(HERE), "tuning", "gb300.tsv")
 
 TILES = (1, 2, 3, 4, 5, 6)
 LEAVES = (2, 4, 8)
-STACKS = (64,)
+STACKS = (32, 64)
 BUDGETS = (-1, 64, 256, 512, 1024, 2048, 4096, 8192, 32768)
 START = (2, 3, 64, 2048)  # leaf, tile id (1-based), stack, step budget: the built-in defaults
 
