@@ -1,23 +1,25 @@
 // Expansion of per-triangle work into items (candidate cells or columns) without a device-wide scan.
 //
-// A thread block takes 256 consecutive triangles: every thread sets up one triangle and counts its
-// items, the block scans the counts in shared memory, and its threads take the items in order, each
+// A thread block takes 256 consecutive triangles (32 of a small mesh): a thread sets up one triangle and
+// counts its items, the block scans the counts in shared memory, and its threads take the items in order, each
 // finding the owner by binary search in the shared starts and reading the triangle from shared
-// memory. A triangle with more than kBigItems items goes to a list instead; a second kernel gives
-// each of those a whole block, and one with more than kHugeItems the whole grid.
+// memory. A triangle with more than kWarpItems items goes to a list instead; a second kernel gives each
+// of those a warp, one with more than kBlockItems a block and one with more than kGridItems the grid.
+// (A block takes as long as its triangles have items: with the list from 4096 items on, the occupancy
+// stage of 1280 triangles at 128^3 and 256^3 took 179 and 891 us, now 27 and 45.)
 //
 // Before, a kernel counted, three launches scanned the counts of all triangles and threads walked the
 // device-wide starts from owner to owner: a walk over the empty triangles of a mesh much finer than
 // its grid is a serial chain of loads (1M triangles on 128^2 columns 241 us, 157k triangles of a
 // mixed batch 260 us, for the column test alone). Now the whole bake of the former takes 6.90 ms for
 // 7.10, a 32^3 bake of 960 triangles 291 us for 327 and a 256^3 occupancy grid of 4k triangles 76 us
-// for 97: what is left is launches, the clear and, for few large triangles, their items.
+// for 97.
 //
 // An Op describes the work:
 //   Op::Tri                       the triangle as its items need it, trivially copyable, whole words
 //   op.setup(B, t, tri) -> count  the triangle (global index t) and its number of items
 //   op.item(B, tri, k)            item k
-//   op.finish(B, items)           at the end, by every thread together, with the items its block ran
+//   op.finish(B, items)           at the end, by every thread; over the threads, items adds up to those run
 // Every thread has its own copy of the op, so item() may keep sums in it for finish().
 #pragma once
 
@@ -29,33 +31,43 @@
 namespace sdfb {
 
 constexpr int kExpandThreads = 256;
-constexpr uint64_t kBigItems = 4096, kHugeItems = 1 << 18;
+// A warp's worth of items and more go to a warp (16: 81,920 triangles at 256^3 37 -> 49 us, 64: eight mixed
+// meshes 43 -> 49 us), from 512 to a block (2048: 320 triangles at 128^3 31 -> 48 us).
+constexpr uint64_t kWarpItems = 48, kBlockItems = 512, kGridItems = 1 << 18;
+constexpr uint64_t kGridList = 1024;
 
-// Triangles left to the second kernel: big ones from the front of the list, huge ones from its end.
-// counts: two numbers, zero before the first kernel.
+// Triangles left to the second kernel: those for a warp from the front of `tris`, those for a block from
+// its end, those for the grid in a list of their own (as far as it holds them). counts: zero before the
+// first kernel.
 struct BigList {
-  unsigned long long *counts;
-  uint64_t *tris;  // n entries
+  unsigned long long *counts;  // warp, block, grid
+  uint64_t *grid;              // kGridList entries
+  uint64_t *tris;              // n entries
   uint64_t n;
 };
 
-template <class Op> __global__ __launch_bounds__(kExpandThreads) void k_expand(BatchDev B, uint64_t n, BigList big, Op op) {
+template <class Op, int OWN>
+__global__ __launch_bounds__(kExpandThreads) void k_expand(BatchDev B, uint64_t n, BigList big, Op op) {
   using Tri = typename Op::Tri;
   constexpr int kWords = sizeof(Tri) / 4;
   static_assert(sizeof(Tri) % 4 == 0, "a triangle is whole words");
-  __shared__ uint32_t s_tri[kWords][kExpandThreads];
-  __shared__ uint32_t s_start[kExpandThreads + 1];
+  __shared__ uint32_t s_tri[kWords][OWN];
+  __shared__ uint32_t s_start[OWN + 1];
   __shared__ uint32_t s_warp[kExpandThreads / kWarp];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint64_t t = uint64_t(blockIdx.x) * kExpandThreads + threadIdx.x;
+  const uint64_t t = uint64_t(blockIdx.x) * OWN + threadIdx.x;
   uint32_t count = 0;
-  if (t < n) {
+  if (threadIdx.x < OWN && t < n) {
     Tri tri;
     const uint64_t c = op.setup(B, t, tri);
-    if (c > kBigItems) {
-      const bool huge = c > kHugeItems;
-      const unsigned long long at = atomicAdd(big.counts + (huge ? 1 : 0), 1ull);
-      big.tris[huge ? n - 1 - at : at] = t;
+    if (c > kWarpItems) {
+      unsigned long long at = kGridList;
+      if (c > kGridItems && (at = atomicAdd(big.counts + 2, 1ull)) < kGridList) big.grid[at] = t;
+      if (at >= kGridList) {
+        const bool block = c > kBlockItems;
+        at = atomicAdd(big.counts + (block ? 1 : 0), 1ull);
+        big.tris[block ? n - 1 - at : at] = t;
+      }
     } else if (c) {
       count = static_cast<uint32_t>(c);
       const uint32_t *w = reinterpret_cast<const uint32_t *>(&tri);
@@ -73,14 +85,14 @@ template <class Op> __global__ __launch_bounds__(kExpandThreads) void k_expand(B
   __syncthreads();
   uint32_t before = 0;
   for (int w = 0; w < warp; ++w) before += s_warp[w];
-  s_start[threadIdx.x + 1] = before + incl;
+  if (threadIdx.x < OWN) s_start[threadIdx.x + 1] = before + incl;
   if (threadIdx.x == 0) s_start[0] = 0;
   __syncthreads();
-  const uint32_t total = s_start[kExpandThreads];
+  const uint32_t total = s_start[OWN];
   for (uint32_t w = threadIdx.x; w < total; w += kExpandThreads) {
     int j = 0;  // the last triangle that starts at or before w (an empty one starts where the next does)
 #pragma unroll
-    for (int step = kExpandThreads / 2; step; step >>= 1)
+    for (int step = OWN / 2; step; step >>= 1)
       if (s_start[j + step] <= w) j += step;
     Tri tri;
     uint32_t *x = reinterpret_cast<uint32_t *>(&tri);
@@ -89,39 +101,58 @@ template <class Op> __global__ __launch_bounds__(kExpandThreads) void k_expand(B
     op.item(B, tri, uint64_t(w - s_start[j]));
   }
   __syncwarp();
-  op.finish(B, total);
+  op.finish(B, threadIdx.x == 0 ? total : 0);
 }
 
 template <class Op>
 __global__ __launch_bounds__(kExpandThreads) void k_expand_big(BatchDev B, BigList big, Op op) {
-  const unsigned long long nbig = big.counts[0], nhuge = big.counts[1];
-  unsigned long long items = 0;
-  for (unsigned long long i = blockIdx.x; i < nbig; i += gridDim.x) {
+  constexpr int kWarps = kExpandThreads / kWarp;
+  const unsigned long long nwarp = big.counts[0], nblock = big.counts[1];
+  const unsigned long long ngrid = min(big.counts[2], static_cast<unsigned long long>(kGridList));
+  const int lane = threadIdx.x & 31;
+  const unsigned long long warp = blockIdx.x * (unsigned long long)kWarps + (threadIdx.x >> 5);
+  unsigned long long items = 0;  // of the first lane, or thread, that ran them
+  for (unsigned long long i = warp; i < nwarp; i += gridDim.x * (unsigned long long)kWarps) {
     typename Op::Tri tri;
     const uint64_t c = op.setup(B, big.tris[i], tri);
-    for (uint64_t k = threadIdx.x; k < c; k += kExpandThreads) op.item(B, tri, k);
-    items += c;
+    for (uint64_t k = lane; k < c; k += kWarp) op.item(B, tri, k);
+    if (lane == 0) items += c;
   }
-  for (unsigned long long i = 0; i < nhuge; ++i) {
+  for (unsigned long long i = blockIdx.x; i < nblock; i += gridDim.x) {
     typename Op::Tri tri;
     const uint64_t c = op.setup(B, big.tris[big.n - 1 - i], tri);
+    for (uint64_t k = threadIdx.x; k < c; k += kExpandThreads) op.item(B, tri, k);
+    if (threadIdx.x == 0) items += c;
+  }
+  for (unsigned long long i = 0; i < ngrid; ++i) {
+    typename Op::Tri tri;
+    const uint64_t c = op.setup(B, big.grid[i], tri);
     const uint64_t stride = uint64_t(gridDim.x) * kExpandThreads;
-    for (uint64_t k = uint64_t(blockIdx.x) * kExpandThreads + threadIdx.x; k < c; k += stride) op.item(B, tri, k);
-    if (blockIdx.x == 0) items += c;
+    const uint64_t first = uint64_t(blockIdx.x) * kExpandThreads + threadIdx.x;
+    for (uint64_t k = first; k < c; k += stride) op.item(B, tri, k);
+    if (first == 0) items += c;
   }
   __syncwarp();
   op.finish(B, items);
 }
 
 // Bytes of a list for n triangles, and the list in that memory (counts first; the caller clears them).
-inline size_t big_list_bytes(uint64_t n) { return 256 + ((n * 8 + 255) & ~size_t(255)); }
+inline size_t big_list_bytes(uint64_t n) { return 256 + kGridList * 8 + ((n * 8 + 255) & ~size_t(255)); }
 inline BigList big_list(void *mem, uint64_t n) {
-  return BigList{static_cast<unsigned long long *>(mem), reinterpret_cast<uint64_t *>(static_cast<char *>(mem) + 256), n};
+  char *p = static_cast<char *>(mem);
+  return BigList{reinterpret_cast<unsigned long long *>(p), reinterpret_cast<uint64_t *>(p + 256),
+                 reinterpret_cast<uint64_t *>(p + 256 + kGridList * 8), n};
 }
 
 template <class Op>
 cudaError_t expand(const BatchDev &B, uint64_t n, const BigList &big, const Op &op, int num_sms, cudaStream_t st) {
-  k_expand<Op><<<static_cast<unsigned>((n + kExpandThreads - 1) / kExpandThreads), kExpandThreads, 0, st>>>(B, n, big, op);
+  // 32 triangles a block where 256 would leave SMs with one block or none: the occupancy stage of 4,096
+  // triangles at 64^3 37 -> 20 us.
+  if (n < uint64_t(num_sms) * 2 * kExpandThreads)
+    k_expand<Op, 32><<<static_cast<unsigned>((n + 31) / 32), kExpandThreads, 0, st>>>(B, n, big, op);
+  else
+    k_expand<Op, kExpandThreads>
+        <<<static_cast<unsigned>((n + kExpandThreads - 1) / kExpandThreads), kExpandThreads, 0, st>>>(B, n, big, op);
   note_launch();
   k_expand_big<Op><<<static_cast<unsigned>(num_sms * 4), kExpandThreads, 0, st>>>(B, big, op);
   note_launch();

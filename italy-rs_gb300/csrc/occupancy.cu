@@ -69,7 +69,7 @@ __device__ __forceinline__ TriCells tri_cells(const BatchDev &B, uint64_t t, uin
 // consecutive cells, with one 16-byte store where they lie in one mesh's grid at an aligned
 // address (so a warp writes 512 contiguous bytes), else byte by byte. Clears the list's counts too.
 __global__ __launch_bounds__(kThreads) void k_occ_clear(BatchDev B, BigList big) {
-  if (blockIdx.x == 0 && threadIdx.x < 2) big.counts[threadIdx.x] = 0;
+  if (blockIdx.x == 0 && threadIdx.x < 3) big.counts[threadIdx.x] = 0;
   const uint64_t stride = uint64_t(gridDim.x) * kThreads * 16;
   for (uint64_t c0 = (uint64_t(blockIdx.x) * kThreads + threadIdx.x) * 16; c0 < B.total_cells; c0 += stride) {
     int m = find_mesh(B.cell_starts, B.num_meshes, c0);
@@ -154,7 +154,7 @@ template <bool FIRST, bool HITS> struct OccOp {
     if (HITS) append_hit(sink, hit, (cell << sink.tri_bits) | tri.local);
   }
   __device__ __forceinline__ void finish(const BatchDev &, unsigned long long items) const {
-    if (sat_tests && items && threadIdx.x == 0) atomicAdd(sat_tests, items);
+    if (sat_tests && items) atomicAdd(sat_tests, items);
   }
 };
 

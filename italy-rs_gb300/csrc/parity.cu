@@ -175,7 +175,7 @@ cudaError_t parity_columns(const BatchDev &B, uint32_t *bits, uint64_t *col_star
   if (par_layout(T, ncols, static_cast<char *>(temp), &o) > temp_bytes) return cudaErrorMemoryAllocation;
   if (T == 0) return cudaErrorInvalidValue;
   const BigList big = big_list(o.big, T);
-  cudaError_t e = cudaMemsetAsync(big.counts, 0, 16, st);
+  cudaError_t e = cudaMemsetAsync(big.counts, 0, 24, st);
   if (e == cudaSuccess && B.total_bit_words) e = cudaMemsetAsync(bits, 0, B.total_bit_words * 4, st);
   if (e == cudaSuccess && ncols) e = cudaMemsetAsync(o.col_count, 0, ncols * 4, st);
   if (e != cudaSuccess) return e;
@@ -183,7 +183,7 @@ cudaError_t parity_columns(const BatchDev &B, uint32_t *bits, uint64_t *col_star
   if (e != cudaSuccess || ncols == 0) return e;
   if ((e = exclusive_scan_u32(o.col_count, col_start, ncols, Scratch{o.scratch, o.scratch_bytes}, st)) != cudaSuccess ||
       (e = cudaMemsetAsync(o.col_count, 0, ncols * 4, st)) != cudaSuccess ||
-      (e = cudaMemsetAsync(big.counts, 0, 16, st)) != cudaSuccess)
+      (e = cudaMemsetAsync(big.counts, 0, 24, st)) != cudaSuccess)
     return e;
   return expand(B, T, big, ColumnOp<true>{o.col_count, nullptr, col_start, col_z, col_s, capacity, nullptr, err, 0}, num_sms,
                 st);

@@ -55,3 +55,18 @@ def test_candidates_of_a_batch(ctx):
         for (v, f), g, d, o in zip(meshes, grids, dists, occs):
             d1, o1 = ctx.bake(v, f, g, opts)
             assert np.array_equal(d, d1) and np.array_equal(o, o1)
+
+
+def test_more_grid_wide_triangles_than_listed(ctx):
+    """1100 copies of a triangle of 320k candidate columns and cells (1024 are kept for the whole grid):
+    the occupancy of one."""
+    import sdfb
+    dims, voxel = (601, 530, 9), 1.0 / 64
+    tri = np.array([[-1.0, -1.0, 0.03], [12.0, -2.0, 0.08], [-2.0, 11.0, 0.11]], np.float32)
+    g = sdfb.make_grid((0, 0, 0), voxel, dims)
+    occ = []
+    for n in (1, 1100):
+        v = np.tile(tri, (n, 1))
+        _, o = ctx.bake(v, np.arange(3 * n, dtype=np.uint32).reshape(-1, 3), g, sdfb.make_opts(), want_dist=False)
+        occ.append(o)
+    assert occ[0].any() and np.array_equal(*occ)
