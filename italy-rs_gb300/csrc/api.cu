@@ -72,9 +72,16 @@ void PinBuf::release() {
 }
 
 sdfb_ctx::~sdfb_ctx() {
-  if (gate_fork) cudaEventDestroy(gate_fork);
+  for (cudaEvent_t e : {gate_fork, gate_done, occ_fork, occ_done})
+    if (e) cudaEventDestroy(e);
   if (gate_stream) cudaStreamDestroy(gate_stream);
   if (stream) cudaStreamDestroy(stream);
+}
+
+bool sdfb_ctx::make_events() {
+  for (cudaEvent_t *e : {&gate_fork, &gate_done, &occ_fork, &occ_done})
+    if (!*e && cudaEventCreateWithFlags(e, cudaEventDisableTiming) != cudaSuccess) return false;
+  return true;
 }
 
 DevBuf *sdfb_ctx::all_bufs(int i) {
@@ -242,6 +249,12 @@ sdfb_status device_caps(sdfb_ctx *ctx, cudaStream_t st, std::vector<PlanMesh> &m
   return SDFB_OK;
 }
 
+// Waits for what a failed call has enqueued early: it reads and writes the caller's buffers.
+static void settle(sdfb_ctx *ctx, cudaStream_t st) {
+  cudaStreamSynchronize(ctx->gate_stream);
+  cudaStreamSynchronize(st);
+}
+
 sdfb_status device_signs(sdfb_ctx *ctx, const sdfb_opts &o, PlanMesh *ms, size_t count, bool needed, cudaStream_t st,
                          size_t *bad, const std::function<sdfb_status()> &meanwhile) {
   size_t at = 0;
@@ -253,7 +266,7 @@ sdfb_status device_signs(sdfb_ctx *ctx, const sdfb_opts &o, PlanMesh *ms, size_t
     if (meanwhile) {
       if ((s = fork_gate(ctx, st)) != SDFB_OK) return s;
       s = device_gate(ctx, v, ctx->gate_stream, bad ? bad : &at, meanwhile);
-      if (s != SDFB_OK) cudaStreamSynchronize(st);  // what meanwhile enqueued reads the caller's mesh
+      if (s != SDFB_OK) settle(ctx, st);
     } else {
       s = device_gate(ctx, v, st, bad ? bad : &at);
     }
@@ -295,8 +308,7 @@ sdfb_status sdfb_ctx_create(int32_t device, sdfb_ctx **out) {
   ctx->device = device;
   ctx->num_sms = prop.multiProcessorCount;
   if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaStreamCreateWithFlags(&ctx->gate_stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaEventCreateWithFlags(&ctx->gate_fork, cudaEventDisableTiming) != cudaSuccess) {
+      cudaStreamCreateWithFlags(&ctx->gate_stream, cudaStreamNonBlocking) != cudaSuccess || !ctx->make_events()) {
     delete ctx;
     return SDFB_ERR_CUDA;
   }
@@ -381,7 +393,7 @@ sdfb_status sdfb_bake_device(sdfb_ctx *ctx, const float *d_verts, uint32_t num_v
   sdfb_status s = device_signs(ctx, o, &p, 1, p.dist || !p.occ || stats, st, nullptr, tree);
   if (s != SDFB_OK) return s;
   if ((s = device_caps(ctx, st, ms)) == SDFB_OK) s = run_batch(ctx, st, ms, o, false, stats, p.bvh != nullptr);
-  if (s != SDFB_OK && p.bvh) cudaStreamSynchronize(st);  // the early build reads the caller's mesh
+  if (s != SDFB_OK && p.bvh) settle(ctx, st);
   return s;
 }
 
@@ -411,21 +423,22 @@ sdfb_status sdfb_bake(sdfb_ctx *ctx, const float *verts, uint32_t num_verts, con
   p.V = num_verts;
   p.T = num_tris;
   p.grid = *grid;
+  p.occ = want_occ ? static_cast<uint8_t *>(ctx->out_occ.p) : nullptr;
   std::function<sdfb_status()> tree;
   if (want_dist && !stats) tree = [&] { return early_tree(ctx, st, ms, o); };
   sdfb_status s = device_signs(ctx, o, &p, 1, want_dist || !want_occ || stats, st, nullptr, tree);
   if (s != SDFB_OK) return s;
   float *const direct_dist =
       (want_dist && p.sign != kSignGwn) ? static_cast<float *>(mapped_host(dist_out)) : nullptr;
-  uint8_t *const direct_occ = nullptr;
   p.dist = want_dist ? (direct_dist ? direct_dist : static_cast<float *>(ctx->out_dist.p)) : nullptr;
-  p.occ = want_occ ? (direct_occ ? direct_occ : static_cast<uint8_t *>(ctx->out_occ.p)) : nullptr;
-  if ((s = device_caps(ctx, st, ms)) != SDFB_OK) return s;
-  s = run_batch(ctx, st, ms, o, false, stats, p.bvh != nullptr);
-  if (s != SDFB_OK) return s;
+  if ((s = device_caps(ctx, st, ms)) == SDFB_OK) s = run_batch(ctx, st, ms, o, false, stats, p.bvh != nullptr);
+  if (s != SDFB_OK) {
+    if (p.bvh) settle(ctx, st);
+    return s;
+  }
   if (want_dist && !direct_dist)
     CK(cudaMemcpyAsync(dist_out, ctx->out_dist.p, cells * 4, cudaMemcpyDeviceToHost, st));
-  if (want_occ && !direct_occ) CK(cudaMemcpyAsync(occ_out, ctx->out_occ.p, cells, cudaMemcpyDeviceToHost, st));
+  if (want_occ) CK(cudaMemcpyAsync(occ_out, ctx->out_occ.p, cells, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
   return SDFB_OK;
 }
@@ -489,14 +502,16 @@ sdfb_status sdfb_bake_soup(sdfb_ctx *ctx, const float *positions, uint32_t num_t
                             ctx->num_sms, gs));
       CK(cudaMemcpyAsync(h + 1, d_counts, 16, cudaMemcpyDeviceToHost, gs));
     }
+    CK(cudaEventRecord(ctx->gate_done, gs));
     if (beside) {
       p.dist = static_cast<float *>(ctx->out_dist.p);
+      p.occ = want_occ ? static_cast<uint8_t *>(ctx->out_occ.p) : nullptr;
       if ((s = early_tree(ctx, st, ms, o)) != SDFB_OK) {
-        cudaStreamSynchronize(gs);
+        settle(ctx, st);
         return s;
       }
     }
-    CK(cudaStreamSynchronize(gs));
+    CK(cudaEventSynchronize(ctx->gate_done));
     U = static_cast<uint32_t>(h[0]);
     if (o.sign_mode == SDFB_SIGN_AUTO) {
       p.watertight = (h[1] + 1 == 0 && h[2] + 1 == 0) ? 1 : 0;
@@ -515,7 +530,10 @@ sdfb_status sdfb_bake_soup(sdfb_ctx *ctx, const float *positions, uint32_t num_t
     p.pidx = d_welded;
     p.pV = U;
     p.pT = num_tris;
-    if ((s = device_caps(ctx, st, ms)) != SDFB_OK) return s;
+    if ((s = device_caps(ctx, st, ms)) != SDFB_OK) {
+      if (p.bvh) settle(ctx, st);
+      return s;
+    }
   } else if (p.sign == kSignParity && want_dist) {
     p.pverts = static_cast<const float *>(ctx->in_verts2.p);
     p.pidx = static_cast<const uint32_t *>(ctx->in_idx2.p);
@@ -523,7 +541,10 @@ sdfb_status sdfb_bake_soup(sdfb_ctx *ctx, const float *positions, uint32_t num_t
     p.pT = num_tris;
   }
   s = run_batch(ctx, st, ms, o, false, stats, p.bvh != nullptr);
-  if (s != SDFB_OK) return s;
+  if (s != SDFB_OK) {
+    if (p.bvh) settle(ctx, st);
+    return s;
+  }
   if (want_dist && !direct_dist)
     CK(cudaMemcpyAsync(dist_out, ctx->out_dist.p, cells * 4, cudaMemcpyDeviceToHost, st));
   if (want_occ) CK(cudaMemcpyAsync(occ_out, ctx->out_occ.p, cells, cudaMemcpyDeviceToHost, st));

@@ -116,7 +116,7 @@ constexpr int kBatchStepBudget = 4096;
 // stream so consecutive waves overlap.
 struct Workspace {
   DevBuf batch_buf, bvh, build_tmp, par_tmp, col_start, col_z, col_s, caps_bvh, caps_tmp, misc, gwn_tmp, defer,
-      col_bits;
+      col_bits, early_buf, occ_tmp;
   PinBuf staging, early_staging;
   cudaEvent_t ev[8] = {};
   uint64_t col_capacity_hint = 0;
@@ -142,7 +142,7 @@ struct sdfb_ctx {
   cudaStream_t stream = nullptr;
   // The gate's own stream, and where it forks from a call's stream (see early_tree).
   cudaStream_t gate_stream = nullptr;
-  cudaEvent_t gate_fork = nullptr;
+  cudaEvent_t gate_fork = nullptr, gate_done = nullptr, occ_fork = nullptr, occ_done = nullptr;
   ResidentBvh early;
   std::string err;
   // inputs / outputs of host-buffer calls
@@ -165,6 +165,7 @@ struct sdfb_ctx {
   int batch_tile = -1, batch_stack = 64, batch_budget = 0;
 
   ~sdfb_ctx();
+  bool make_events();
   DevBuf *all_bufs(int i);
   void release_all();
   uint64_t device_bytes() const;
@@ -196,7 +197,8 @@ sdfb_status device_gate(sdfb_ctx *ctx, const std::vector<PlanMesh *> &ms, cudaSt
 // Makes the gate stream wait for what is on st.
 sdfb_status fork_gate(sdfb_ctx *ctx, cudaStream_t st);
 // Enqueues the build of a single mesh's tree on st, before its sign is known, and points the mesh at
-// it. The following run_batch has to be told (prebuilt), so that it keeps the build's error flags.
+// it, and its occupancy on the gate stream. The following run_batch has to be told (prebuilt), so that it
+// keeps the error flags, leaves the occupancy out and waits for it.
 sdfb_status early_tree(sdfb_ctx *ctx, cudaStream_t st, std::vector<PlanMesh> &ms, const sdfb_opts &o);
 // sdfb_voxelize_sparse; also returns the device list of the count occupied cells' linear indices
 // (valid until the context's next call) and the grid it used.

@@ -132,7 +132,7 @@ void Workspace::release() {
     graph_key.clear();
   }
   DevBuf *b[] = {&batch_buf, &bvh, &build_tmp, &par_tmp, &col_start, &col_z, &col_s, &caps_bvh, &caps_tmp, &misc,
-                 &gwn_tmp, &defer, &col_bits};
+                 &gwn_tmp, &defer, &col_bits, &early_buf, &occ_tmp};
   for (DevBuf *x : b) x->release();
   staging.release();
   early_staging.release();
@@ -140,7 +140,7 @@ void Workspace::release() {
 
 uint64_t Workspace::bytes() const {
   const DevBuf *b[] = {&batch_buf, &bvh, &build_tmp, &par_tmp, &col_start, &col_z, &col_s, &caps_bvh, &caps_tmp,
-                       &misc, &gwn_tmp, &defer, &col_bits};
+                       &misc, &gwn_tmp, &defer, &col_bits, &early_buf, &occ_tmp};
   uint64_t s = 0;
   for (const DevBuf *x : b) s += x->cap;
   return s;
@@ -482,7 +482,7 @@ sdfb_status enqueue_batch(sdfb_ctx *ctx, Workspace &ws, cudaStream_t st, std::ve
                      ws.build_tmp.cap, d_err, st));
     }
     CK(rec(ws.ev[1]));
-    if (any_occ) {
+    if (any_occ && !prebuilt) {
       NvtxRange r("sdfb occupancy");
       CK(occupancy_batch(B, nullptr, ws.build_tmp.p, ws.build_tmp.cap, d_sat, d_err, ctx->num_sms, st));
     }
@@ -509,6 +509,7 @@ sdfb_status enqueue_batch(sdfb_ctx *ctx, Workspace &ws, cudaStream_t st, std::ve
       NvtxRange r("sdfb winding number");
       CK(gwn_enqueue(gi, ws.gwn_tmp.p, ctx->num_sms, st));
     }
+    if (any_occ && prebuilt) CK(cudaStreamWaitEvent(st, ctx->occ_done, 0));
     CK(rec(ws.ev[5]));
     return SDFB_OK;
   };
@@ -673,19 +674,28 @@ sdfb_status early_tree(sdfb_ctx *ctx, cudaStream_t st, std::vector<PlanMesh> &ms
   t_alloc_cap = o.alloc_cap_kib > 0 ? uint64_t(o.alloc_cap_kib) << 10 : 0;
   Layout L;
   make_layout(ctx, ms, o, L);
-  ENSURE(ws.batch_buf, L.bytes);
+  ENSURE(ws.early_buf, L.bytes);
   if (!ws.early_staging.ensure(L.bytes)) return ctx_fail(ctx, SDFB_ERR_OUT_OF_MEMORY, "pinned staging");
   ENSURE(ws.bvh, L.tree_bytes);
   ENSURE(ws.build_tmp, std::max(ptree_temp_bytes(ms[0].T, 1), occupancy_temp_bytes(ms[0].T)));
   ENSURE(ws.misc, 256);
+  if (ms[0].occ) ENSURE(ws.occ_tmp, occupancy_temp_bytes(ms[0].T));
   bind_built(L, static_cast<char *>(ws.bvh.p), nullptr);
   fill_staging(L, static_cast<char *>(ws.early_staging.p));
-  char *tab = static_cast<char *>(ws.batch_buf.p);
+  char *tab = static_cast<char *>(ws.early_buf.p);
   CK(cudaMemcpyAsync(tab, ws.early_staging.p, L.bytes, cudaMemcpyHostToDevice, st));
   CK(cudaMemsetAsync(ws.misc.p, 0, 256, st));
-  CK(ptree_build(batch_dev(L, tab), reinterpret_cast<const PTreeRec *>(tab + L.o_trees),
+  const BatchDev B = batch_dev(L, tab);
+  uint32_t *d_err = static_cast<uint32_t *>(ws.misc.p);
+  if (ms[0].occ) {
+    CK(cudaEventRecord(ctx->occ_fork, st));
+    CK(cudaStreamWaitEvent(ctx->gate_stream, ctx->occ_fork, 0));
+    CK(occupancy_batch(B, nullptr, ws.occ_tmp.p, ws.occ_tmp.cap, nullptr, d_err, ctx->num_sms, ctx->gate_stream));
+    CK(cudaEventRecord(ctx->occ_done, ctx->gate_stream));
+  }
+  CK(ptree_build(B, reinterpret_cast<const PTreeRec *>(tab + L.o_trees),
                  reinterpret_cast<const uint64_t *>(tab + L.o_group), L.group.back(), ws.build_tmp.p,
-                 ws.build_tmp.cap, static_cast<uint32_t *>(ws.misc.p), st));
+                 ws.build_tmp.cap, d_err, st));
   ctx->early = ResidentBvh();
   ctx->early.tree = L.trees[0];
   ctx->early.num_tris = static_cast<int>(ms[0].T);

@@ -220,7 +220,7 @@ std::unique_ptr<sdfb_ctx> make_private_ctx(int device, int num_sms, const sdfb_c
   }
   if (cudaStreamCreateWithPriority(&c->stream, cudaStreamNonBlocking, high_priority ? greatest : least) != cudaSuccess)
     return nullptr;
-  if (!c->ws.init()) return nullptr;
+  if (!c->ws.init() || !c->make_events()) return nullptr;
   std::memcpy(c->tuned_leaf, tuned->tuned_leaf, sizeof c->tuned_leaf);
   std::memcpy(c->tuned_tile, tuned->tuned_tile, sizeof c->tuned_tile);
   std::memcpy(c->tuned_stack, tuned->tuned_stack, sizeof c->tuned_stack);

@@ -438,9 +438,9 @@ sdfb_status device_gate(sdfb_ctx *ctx, const std::vector<PlanMesh *> &ms, cudaSt
   note_launch();
   e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaMemcpyAsync(h, d + o_result, n * 24, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaEventRecord(ctx->gate_done, st);
   const sdfb_status early = meanwhile && e == cudaSuccess ? meanwhile() : SDFB_OK;
-  const cudaError_t w = cudaStreamSynchronize(st);
-  if (e == cudaSuccess) e = w;
+  if (e == cudaSuccess) e = cudaEventSynchronize(ctx->gate_done);
   if (early != SDFB_OK) return early;
   if (e != cudaSuccess) return ctx_cuda(ctx, e, "watertight gate");
   for (size_t m = 0; m < n; ++m) {
