@@ -102,7 +102,7 @@ struct GwnInput {
 
 // Workspace::misc (256 bytes, zeroed before every bake): error flags at 0, the distance tile
 // counter at 64, work counters at 128 (box, triangle, SAT, plane tests), the deferral counters at
-// 192, the crossings at 216.
+// 192, the crossings and their pass's three counters at 216.
 constexpr size_t kMiscDeferOffset = 192;
 constexpr size_t kMiscCrossOffset = 216;
 // Steps of work between a distance tile's looks at whether it should go to the block-per-tile pass.

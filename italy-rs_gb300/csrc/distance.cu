@@ -852,12 +852,9 @@ cudaError_t launch_shape(const DistanceArgs &a, int num_sms, cudaStream_t st) {
   DistanceArgs ca = a;
   ca.chunk_tiles = std::max<unsigned long long>(
       1, std::min<unsigned long long>(kChunkMax, a.batch.total_tiles / (blocks * kWarpsPerBlockA * 4)));
-  cudaError_t e = cudaMemsetAsync(a.tile_counter, 0, sizeof(unsigned long long), st);
-  if (e == cudaSuccess && a.defer_list) e = cudaMemsetAsync(a.defer_counters, 0, 2 * sizeof(unsigned long long), st);
-  if (e != cudaSuccess) return e;
   k_distance<s.tx, s.ty, s.tz, COUNT><<<static_cast<unsigned>(blocks), kThreadsA, 0, st>>>(ca);
   note_launch();
-  e = cudaGetLastError();
+  const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || !a.defer_list || a.step_budget <= 0) return e;
   // Pass B: a persistent grid; the number of deferred tiles is read on the device.
   const unsigned long long blocks_b =

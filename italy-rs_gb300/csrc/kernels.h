@@ -180,10 +180,11 @@ cudaError_t occupancy_batch(const BatchDev &batch, uint32_t *first_tri, void *te
 // Crossings of the columns' +z lines with the meshes' pverts / pidx. Parity meshes: bits, per column
 // ceil(nz / 32) words (total_bit_words in all), toggled at the highest layer below each crossing.
 // Winding-number meshes: lists, col_start[total_cols + 1] (uint64 starts), col_z[capacity] heights,
-// col_s[capacity] orientations. *crossings (zeroed by the caller) counts them all.
+// col_s[capacity] orientations. counters: the number of all crossings, then three of the pass itself;
+// all zero before.
 size_t parity_temp_bytes(uint64_t total_ptris, uint64_t total_cols);
 cudaError_t parity_columns(const BatchDev &batch, uint32_t *bits, uint64_t *col_start, float *col_z, int8_t *col_s,
-                           uint64_t capacity, void *temp, size_t temp_bytes, unsigned long long *crossings,
+                           uint64_t capacity, void *temp, size_t temp_bytes, unsigned long long *counters,
                            uint32_t *err, int num_sms, cudaStream_t st);
 
 // ---- distance.cu ------------------------------------------------------------------------------
@@ -191,14 +192,13 @@ struct DistanceArgs {
   BatchDev batch;             // each mesh record names its hierarchy and root
   const uint32_t *bits;       // parity: crossing bits
   uint32_t *err;
-  unsigned long long *tile_counter;   // pass A's chunk counter, zeroed by the launcher
+  unsigned long long *tile_counter;   // pass A's chunk counter, zero before the launch
   unsigned long long chunk_tiles;     // tiles per chunk (set by the launcher)
   unsigned long long *work_counters;  // optional: [0] box, [1] triangle, [3] plane, [4] rectangle tests (lanes)
   // Deferral of long tiles (none when defer_list is null or step_budget <= 0): every step_budget
   // pairs of children measured a walk checks whether all tiles have been handed out and, if so, defers its
   // tile. The list holds defer_capacity tile indices; defer_counters[0] counts deferred tiles (it
-  // may pass the capacity), [1] is the second pass's tile counter. Both counters are zeroed by the
-  // launcher.
+  // may pass the capacity), [1] is the second pass's tile counter. Both are zero before the launch.
   unsigned long long *defer_list;
   unsigned long long defer_capacity;
   unsigned long long *defer_counters;

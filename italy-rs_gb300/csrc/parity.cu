@@ -168,23 +168,26 @@ size_t parity_temp_bytes(uint64_t total_ptris, uint64_t total_cols) {
 }
 
 cudaError_t parity_columns(const BatchDev &B, uint32_t *bits, uint64_t *col_start, float *col_z, int8_t *col_s,
-                           uint64_t capacity, void *temp, size_t temp_bytes, unsigned long long *crossings,
+                           uint64_t capacity, void *temp, size_t temp_bytes, unsigned long long *counters,
                            uint32_t *err, int num_sms, cudaStream_t st) {
   const uint64_t T = B.total_ptris, ncols = B.total_cols;
   ParTemp o;
   if (par_layout(T, ncols, static_cast<char *>(temp), &o) > temp_bytes) return cudaErrorMemoryAllocation;
   if (T == 0) return cudaErrorInvalidValue;
-  const BigList big = big_list(o.big, T);
-  cudaError_t e = cudaMemsetAsync(big.counts, 0, 24, st);
-  if (e == cudaSuccess && B.total_bit_words) e = cudaMemsetAsync(bits, 0, B.total_bit_words * 4, st);
+  BigList big = big_list(o.big, T);
+  unsigned long long *const second = big.counts;
+  big.counts = counters + 1;
+  cudaError_t e = cudaSuccess;
+  if (B.total_bit_words) e = cudaMemsetAsync(bits, 0, B.total_bit_words * 4, st);
   if (e == cudaSuccess && ncols) e = cudaMemsetAsync(o.col_count, 0, ncols * 4, st);
   if (e != cudaSuccess) return e;
-  e = expand(B, T, big, ColumnOp<false>{o.col_count, bits, nullptr, nullptr, nullptr, 0, crossings, err, 0}, num_sms, st);
+  e = expand(B, T, big, ColumnOp<false>{o.col_count, bits, nullptr, nullptr, nullptr, 0, counters, err, 0}, num_sms, st);
   if (e != cudaSuccess || ncols == 0) return e;
   if ((e = exclusive_scan_u32(o.col_count, col_start, ncols, Scratch{o.scratch, o.scratch_bytes}, st)) != cudaSuccess ||
       (e = cudaMemsetAsync(o.col_count, 0, ncols * 4, st)) != cudaSuccess ||
-      (e = cudaMemsetAsync(big.counts, 0, 24, st)) != cudaSuccess)
+      (e = cudaMemsetAsync(second, 0, 24, st)) != cudaSuccess)
     return e;
+  big.counts = second;
   return expand(B, T, big, ColumnOp<true>{o.col_count, nullptr, col_start, col_z, col_s, capacity, nullptr, err, 0}, num_sms,
                 st);
 }
