@@ -113,7 +113,7 @@ typedef struct sdfb_stats {
   int32_t stack_used;
   double ms_total;         /* first to last event on the device */
   double ms_prepare;       /* upload of the batch tables and counter reset */
-  double ms_build;         /* triangle records, Morton codes, sort, hierarchy, refit, layout */
+  double ms_build;         /* triangle bounds, Hilbert keys, sort, blocks and the nodes above them */
   double ms_occupancy;
   double ms_sign;          /* parity crossings or winding-number band */
   double ms_distance;      /* nearest-triangle traversal (+ fused sign) */

@@ -99,27 +99,6 @@ int watertight_flag(const uint32_t *tri, size_t ntris, uint64_t *boundary, uint6
   return (*boundary == 0 && *nonmanifold == 0) ? 1 : 0;
 }
 
-int indexed_mesh_watertight(const float *verts, uint32_t V, const uint32_t *idx, uint32_t T) {
-  if (T == 0 || V == 0) return -1;
-  float bmin[3] = {verts[0], verts[1], verts[2]}, bmax[3] = {verts[0], verts[1], verts[2]};
-  for (uint32_t i = 1; i < V; ++i)
-    for (int a = 0; a < 3; ++a) {
-      const float v = verts[3 * size_t(i) + a];
-      bmin[a] = v < bmin[a] ? v : bmin[a];
-      bmax[a] = v > bmax[a] ? v : bmax[a];
-    }
-  std::vector<uint32_t> w(V);
-  weld_positions(verts, V, bmin, bmax, w.data());
-  std::vector<uint32_t> tri(3 * size_t(T));
-  for (size_t k = 0; k < 3 * size_t(T); ++k) {
-    const uint32_t i = idx[k];
-    if (i >= V) return -2;
-    tri[k] = w[i];
-  }
-  uint64_t b, m;
-  return watertight_flag(tri.data(), T, &b, &m);
-}
-
 void srgb_to_linear_table(float out[256]) {
   for (int b = 0; b < 256; ++b) {
     const float c = static_cast<float>(b) / 255.0f;

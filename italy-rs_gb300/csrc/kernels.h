@@ -98,7 +98,6 @@ struct MeshRec {
   GridDev g;
   int sign;               // SignKind
   int leaf_size;          // 1..16
-  int pad;
   int cap_root;           // GWN: virtual root of this mesh's caps in the caps hierarchy, -1 if none
   const float *cverts;    // GWN: vertices of the caps (the parity mesh's vertices + loop centres)
   const uint32_t *cidx;   // GWN: cap triangles
