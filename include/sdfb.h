@@ -103,7 +103,8 @@ typedef struct sdfb_opts {
 #define SDFB_FAULT_STACK_ALL 8     /* every traversal stack holds 2 entries -> OVERFLOW */
 
 /* Per-call statistics, filled when the pointer is non-null. Times are CUDA-event times on the
- * bake stream (ms); counts are exact. */
+ * bake stream (ms); counts are exact. A single-mesh call that asks for them runs its stages one after
+ * another; one that does not builds the tree and tests occupancy while the sign is being found. */
 typedef struct sdfb_stats {
   uint32_t struct_size;
   int32_t sign_mode_used;
