@@ -235,7 +235,7 @@ struct Walker {
     if (lane == 0) {
       m.centre = make_float4(cx, cy, cz, sqrtf(hx * hx + hy * hy + hz * hz));
       m.half = make_float4(hx, hy, hz, kInf);
-      m.lin.w = 12.0f / (float(VPL * kWarp) * g.voxel * g.voxel);  // for fit()
+      m.lin.w = 1.0f / g.voxel;  // for fit()
     }
     __syncwarp();
   }
@@ -272,10 +272,13 @@ struct Walker {
   }
 
   // Reads the bounds and fits the planes above them: g and G are the least squares slopes over the
-  // tile (the cells' offsets from the centre sum to about zero), taken about a middle cell's value.
+  // tile (the cells' offsets from the centre sum to about zero), taken about a middle cell's value. The
+  // sums take the offsets in voxels, so that they hold nothing larger than a squared length, as the bounds
+  // themselves. Where one passes FP32's range all the same its plane becomes +inf, which drops nothing.
   __device__ __forceinline__ void fit() {
     float su = 0.0f, sw = 0.0f, sz = 0.0f, swz = 0.0f, u[VPL], w[VPL];
     const float4 c = m.centre;
+    const float n = m.lin.w;  // 1 / voxel
     const float dx = px - c.x, dy = py - c.y, dxy = dx * dx + dy * dy;
 #pragma unroll
     for (int v = 0; v < VPL; ++v) {
@@ -289,17 +292,18 @@ struct Walker {
                 w0 = __shfl_sync(kFull, w[kMiddle / kWarp], kMiddle % kWarp);
 #pragma unroll
     for (int v = 0; v < VPL; ++v) {
-      const float dz = pz[v] - c.z, du = u[v] - u0, dw = w[v] - w0;
+      const float kz = (pz[v] - c.z) * n, du = u[v] - u0, dw = w[v] - w0;
       su += du;
       sw += dw;
-      sz = fmaf(du, dz, sz);
-      swz = fmaf(dw, dz, swz);
+      sz = fmaf(du, kz, sz);
+      swz = fmaf(dw, kz, swz);
     }
-    const float n = m.lin.w;  // 1 / sum of squared offsets, but for the axes' cell counts
-    const float ix = n * (1.0f / (TX * TX - 1)), iy = n * (1.0f / (TY * TY - 1)),
-                iz = TZ > 1 ? n * (1.0f / (TZ > 1 ? TZ * TZ - 1 : 1)) : 0.0f;
-    const float gx = wsum(su * dx) * ix, gy = wsum(su * dy) * iy, gz = wsum(sz) * iz;
-    const float Gx = wsum(sw * dx) * ix, Gy = wsum(sw * dy) * iy, Gz = wsum(swz) * iz;
+    const float kx = dx * n, ky = dy * n;
+    constexpr float kCells = 12.0f / (VPL * kWarp);  // over the sum of squared offsets, but for the axes' cell counts
+    const float ix = n * (kCells / (TX * TX - 1)), iy = n * (kCells / (TY * TY - 1)),
+                iz = TZ > 1 ? n * (kCells / (TZ > 1 ? TZ * TZ - 1 : 1)) : 0.0f;
+    float gx = wsum(su * kx) * ix, gy = wsum(su * ky) * iy, gz = wsum(sz) * iz;
+    float Gx = wsum(sw * kx) * ix, Gy = wsum(sw * ky) * iy, Gz = wsum(swz) * iz;
     float ra = -kInf, rA = -kInf;
 #pragma unroll
     for (int v = 0; v < VPL; ++v) {
@@ -312,6 +316,14 @@ struct Walker {
     const float4 h = m.half;
     __syncwarp();
     if (lane == 0) {
+      if (!(fabsf(gx) + fabsf(gy) + fabsf(gz) + fabsf(ra) < kInf)) {
+        gx = gy = gz = 0.0f;
+        ra = kInf;
+      }
+      if (!(fabsf(Gx) + fabsf(Gy) + fabsf(Gz) + fabsf(rA) < kInf)) {
+        Gx = Gy = Gz = 0.0f;
+        rA = kInf;
+      }
       m.half.w = ra + 2e-6f * (fabsf(ra) + h.x * fabsf(gx) + h.y * fabsf(gy) + h.z * fabsf(gz));
       m.lin = make_float4(gx, gy, gz, n);
       m.sq = make_float4(Gx, Gy, Gz,
@@ -322,8 +334,9 @@ struct Walker {
 
   // Whether a convex child with nearest point c - (ex, ey, ez) to the tile's centre, whose farthest
   // point from there is at sqrt(D2), may hold a triangle nearer than the bounds of some cell. S is
-  // the size of the coordinates that e was formed from; a few 1e-7 of it is the error of e. A NaN
-  // anywhere (a mesh with non-finite vertices, reported elsewhere) drops the child.
+  // the size of the coordinates that e was formed from; a few 1e-7 of it is the error of e. A child
+  // that makes a NaN (non-finite vertices, reported elsewhere, or a d2 past FP32) is dropped; a plane never
+  // makes one (see fit).
   __device__ __forceinline__ bool near(float rho, float ex, float ey, float ez, float d2, float D2, float S) const {
     const float4 h = m.half, g = m.lin, G = m.sq;
     const float inv = d2 > 0.0f ? rsqrtf(d2) : 0.0f;
@@ -503,7 +516,7 @@ struct Walker {
   __device__ __forceinline__ void start() {
     float b[VPL];
 #pragma unroll
-    for (int v = 0; v < VPL; ++v) b[v] = 1e38f;
+    for (int v = 0; v < VPL; ++v) b[v] = kInf;
     const int lb = m.t.block_log2;
     for (int k = 0; k < (1 << lb); ++k) {
       const float4 *tri = tree_tri(m.t.tri, (size_t(m.seed) << lb) + k);
