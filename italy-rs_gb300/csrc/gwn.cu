@@ -186,7 +186,8 @@ __device__ __forceinline__ float4 leaf_moment(const TriRec *tr, int count) {
 // false when they are too close (r <= 2 (|e| + rho_g)) or the error bound exceeds tau; else
 // val = D . (c - q) / r^3 and err bounds |Omega - val|. One reciprocal square root per distance and
 // one approximate reciprocal for the bound (each within 2 ulp, far inside the 1e-5 margin that the
-// bound carries); the acceptance test err <= tau is taken as A 2 rho <= tau g^3 with a 1e-6 margin.
+// bound carries); the acceptance test err <= tau is taken as A 2 rho <= tau g^3 with a 1e-6 margin. g^3 has
+// to lie where both stay normal: __fdividef gives 0 for divisors above 2^126.
 __device__ __forceinline__ bool far_field(float qx, float qy, float qz, float rho_g, const float4 &n0,
                                           const float4 &n1, const float4 &n2, int which, const float4 &m, float tau,
                                           float &val, float &err) {
@@ -201,7 +202,7 @@ __device__ __forceinline__ bool far_field(float qx, float qy, float qz, float rh
   const float g = r2 * ir - rho;
   const float g3 = g * g * g;
   const float lim = m.w * 2.0f * rho;
-  if (!(g3 > 1e-30f) || !(lim <= tau * (1.0f - 1e-6f) * g3)) return false;
+  if (!(g3 > 1e-30f && g3 < 8e37f) || !(lim <= tau * (1.0f - 1e-6f) * g3)) return false;
   val = (m.x * dx + m.y * dy + m.z * dz) * (ir * ir * ir);
   constexpr float kRel = 1e-5f;
   err = __fdividef(lim, g3) * (1.0f + kRel) + kRel * fabsf(val);

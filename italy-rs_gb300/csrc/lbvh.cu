@@ -119,7 +119,7 @@ __global__ __launch_bounds__(kThreads) void k_prep(BatchDev B, TriRec *__restric
       r.r0 = make_float4(a.x, a.y, a.z, 0.0f);
       r.r1 = make_float4(b.x, b.y, b.z, 0.0f);
       r.r2 = make_float4(c.x, c.y, c.z, 0.0f);
-      r.r3 = make_float4(nx, ny, nz, sqrtf(nx * nx + ny * ny + nz * nz));
+      r.r3 = make_float4(nx, ny, nz, norm3df(nx, ny, nz));  // its squares, powers of four, would leave FP32 early
       rec[t] = r;
     }
     const float4 l = make_float4(fminf(fminf(a.x, b.x), c.x), fminf(fminf(a.y, b.y), c.y),

@@ -31,7 +31,7 @@ def test_distance_at_scale(ctx, exponent):
             assert np.abs(d / s - ref).max() <= 16 * 2.0 ** -24 * 2.0, opts
 
 
-@pytest.mark.parametrize("exponent", [-20, 24])
+@pytest.mark.parametrize("exponent", [-20, 24, 40])
 @pytest.mark.parametrize("kind", ["bowl", "shells"])
 @pytest.mark.parametrize("band", [1.0, 1000.0])
 def test_signs_at_scale(ctx, kind, band, exponent):
