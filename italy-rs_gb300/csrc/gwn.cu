@@ -89,10 +89,12 @@ __device__ __forceinline__ T solid_angle(V3<T> a, V3<T> b, V3<T> c) {
 // denominator 50 u L (11 u in the product of lengths, 9 u in each of the other three terms, 3 u of
 // the partial sums), so the vector (den, det) of length R moves by at most 53 u L and the angle 2 atan2
 // by at most 2.2 * 53 u L / R while that is below a quarter, plus the rounding of atan2f and of the
-// sum. Otherwise, and for a NaN, nothing is known: |Omega| <= 2 pi on both sides. L / R is taken from det
-// and den over L, whose squares stay in range where those of the cubes det and den do not (from lengths of
-// 2.6e6 on). Lengths whose own squares or products come near the ends of FP32's range are not known either:
-// den is at most 4 L, and what underflows is below 1e-12 of L.
+// sum, unless the move takes the vector across the cut of atan2 (den < 0, det = 0: the point lies in the
+// triangle, to rounding), where the angle jumps by 4 pi. There, otherwise, and for a NaN, nothing is known:
+// |Omega| <= 2 pi on both sides. L / R is taken from det and den over L, whose squares stay in range where
+// those of the cubes det and den do not (from lengths of 2.6e6 on). Lengths whose own squares or products come
+// near the ends of FP32's range are not known either: den is at most 4 L, and what underflows is below 1e-12
+// of L.
 __device__ __forceinline__ float solid_angle_bounded(V3<float> a, V3<float> b, V3<float> c, float &err) {
   const float aa = a.x * a.x + a.y * a.y + a.z * a.z, bb = b.x * b.x + b.y * b.y + b.z * b.z,
               cc = c.x * c.x + c.y * c.y + c.z * c.z;
@@ -105,7 +107,8 @@ __device__ __forceinline__ float solid_angle_bounded(V3<float> a, V3<float> b, V
   const float s = 1.0f / L, x = den * s, y = det * s;
   const float rel = rsqrtf(x * x + y * y);
   const bool in_range = L < 8e37f && fminf(L, fminf(aa, fminf(bb, cc))) > 1e-32f;
-  err = in_range && rel < 7e4f ? fmaf(8e-6f, rel, 2e-6f) : 13.0f;
+  const bool cut = x < 4e-6f && fabsf(y) < 2e-6f;  // 50 u and 16 u are 3e-6 and 1e-6
+  err = in_range && !cut && rel < 7e4f ? fmaf(8e-6f, rel, 2e-6f) : 13.0f;
   return 2.0f * atan2f(det, den);
 }
 
