@@ -14,7 +14,7 @@
 // with a use count beside each; the running numbers of edges used once (boundary) and more than
 // twice (non-manifold) follow from the count each use finds.
 //
-// The gate of a whole batch is three launches and one read back. As three radix sorts over the
+// The gate of a batch is three launches and one read back. As three radix sorts over the
 // lattice keys and one over the edges it was 40-80 launches and four read backs a mesh: a bake of
 // 1,280 triangles at 32^3 531 -> 322 us, occupancy of 81,920 triangles at 256^3 790 -> 375 us, a
 // 64-mesh batch 146 -> 119 ms. A table has at least twice (positions) or 4/3 (edges) as many slots
@@ -370,47 +370,65 @@ cudaError_t watertight_device(const uint32_t *welded, uint64_t T, void *temp, si
 
 }  // namespace sdfb
 
+// The meshes go through the gate in runs of consecutive ones whose tables fit kGateRoom together (or of one
+// mesh), one run after the other in the same memory: without it the tables of a batch, 48 to 96 B a triangle
+// and 12 to 20 B a vertex, were held all at once. A batch of 10M triangles is one run; another costs three
+// launches and a memset.
+constexpr size_t kGateRoom = size_t(1) << 30;
+
 sdfb_status device_gate(sdfb_ctx *ctx, const std::vector<PlanMesh *> &ms, cudaStream_t st, size_t *bad,
                         const std::function<sdfb_status()> &meanwhile) {
-  // Records first (uploaded), then everything that starts at ~0, then the slots of the vertices.
+  // Records first (uploaded), then the results and bounds and the tables, which start at ~0, and the slots of
+  // the vertices.
   const size_t n = ms.size();
   if (n == 0) return SDFB_OK;
+  struct Run {
+    size_t first, count, cleared;  // meshes, bytes of their tables
+    uint32_t vblocks, tblocks;
+  };
   std::vector<GateRec> recs(n);
-  uint64_t vblocks = 0, tblocks = 0;
+  std::vector<Run> runs;
   const size_t o_result = align256(n * sizeof(GateRec)), o_bounds = o_result + align256(n * 24);
-  size_t at = o_bounds + align256(n * 24);
-  for (size_t m = 0; m < n; ++m) {
-    const PlanMesh &p = *ms[m];
-    GateRec &r = recs[m];
-    r.verts = p.verts;
-    r.idx = p.idx;
-    r.V = p.V;
-    r.T = p.T;
-    r.vblock = static_cast<uint32_t>(vblocks);
-    r.tblock = static_cast<uint32_t>(tblocks);
-    vblocks += (uint64_t(p.V) + kVertsPerBlock - 1) / kVertsPerBlock;
-    tblocks += (uint64_t(p.T) + kTrisPerBlock - 1) / kTrisPerBlock;
-    const uint64_t vs = weld_slots(p.V), es = edge_slots(p.T);
-    if (vblocks >= (1ull << 31) || tblocks >= (1ull << 31))
-      return ctx_fail(ctx, SDFB_ERR_INVALID_ARGUMENT, "batch too large");
-    r.vmask = static_cast<uint32_t>(vs - 1);
-    r.emask = es - 1;
-    auto take = [&](size_t bytes) {
-      const size_t o = at;
-      at += align256(bytes);
-      return reinterpret_cast<char *>(o);  // an offset until the buffer is known
-    };
-    r.ekeys = reinterpret_cast<unsigned long long *>(take(es * 8));
-    r.ecount = reinterpret_cast<uint32_t *>(take(es * 4));
-    r.vtab = reinterpret_cast<uint32_t *>(take(vs * 4));
+  const size_t o_tables = o_bounds + align256(n * 24);
+  size_t total = o_tables;
+  for (size_t first = 0; first < n;) {
+    uint64_t vblocks = 0, tblocks = 0;
+    size_t end = first, tables = 0, slots = 0;
+    for (; end < n; ++end) {
+      const PlanMesh &p = *ms[end];
+      GateRec &r = recs[end];
+      const uint64_t vs = weld_slots(p.V), es = edge_slots(p.T);
+      const uint64_t vb = vblocks + (uint64_t(p.V) + kVertsPerBlock - 1) / kVertsPerBlock;
+      const uint64_t tb = tblocks + (uint64_t(p.T) + kTrisPerBlock - 1) / kTrisPerBlock;
+      const size_t need = align256(es * 8) + align256(es * 4) + align256(vs * 4);
+      const size_t need_slots = align256(size_t(p.V) * 4);
+      if (end > first && (tables + need + slots + need_slots > kGateRoom || vb >= (1ull << 31) || tb >= (1ull << 31))) break;
+      r.verts = p.verts;
+      r.idx = p.idx;
+      r.V = p.V;
+      r.T = p.T;
+      r.vblock = static_cast<uint32_t>(vblocks);
+      r.tblock = static_cast<uint32_t>(tblocks);
+      r.vmask = static_cast<uint32_t>(vs - 1);
+      r.emask = es - 1;
+      // offsets until the buffer is known
+      r.ekeys = reinterpret_cast<unsigned long long *>(o_tables + tables);
+      r.ecount = reinterpret_cast<uint32_t *>(o_tables + tables + align256(es * 8));
+      r.vtab = reinterpret_cast<uint32_t *>(o_tables + tables + align256(es * 8) + align256(es * 4));
+      r.slot = reinterpret_cast<uint32_t *>(slots);  // past the run's tables
+      tables += need;
+      slots += need_slots;
+      vblocks = vb;
+      tblocks = tb;
+    }
+    for (size_t m = first; m < end; ++m)
+      recs[m].slot = reinterpret_cast<uint32_t *>(reinterpret_cast<size_t>(recs[m].slot) + o_tables + tables);
+    runs.push_back(Run{first, end - first, tables, static_cast<uint32_t>(vblocks), static_cast<uint32_t>(tblocks)});
+    total = std::max(total, o_tables + tables + slots);
+    first = end;
   }
-  const size_t cleared = at - o_result;
-  for (size_t m = 0; m < n; ++m) {
-    recs[m].slot = reinterpret_cast<uint32_t *>(at);
-    at += align256(size_t(ms[m]->V) * 4);
-  }
-  if (!ctx->weld_tmp.ensure(at))
-    return ctx_fail(ctx, SDFB_ERR_OUT_OF_MEMORY, "cannot allocate %zu bytes of device memory", at);
+  if (!ctx->weld_tmp.ensure(total))
+    return ctx_fail(ctx, SDFB_ERR_OUT_OF_MEMORY, "cannot allocate %zu bytes of device memory", total);
   if (!ctx->gate_pin.ensure(n * sizeof(GateRec) + n * 24)) return ctx_fail(ctx, SDFB_ERR_OUT_OF_MEMORY, "pinned staging");
   char *d = static_cast<char *>(ctx->weld_tmp.p);
   auto fix = [&](auto *&p) { p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(d + reinterpret_cast<size_t>(p)); };
@@ -425,18 +443,22 @@ sdfb_status device_gate(sdfb_ctx *ctx, const std::vector<PlanMesh *> &ms, cudaSt
   }
   std::memcpy(ctx->gate_pin.p, recs.data(), n * sizeof(GateRec));
   unsigned long long *h = reinterpret_cast<unsigned long long *>(static_cast<char *>(ctx->gate_pin.p) + n * sizeof(GateRec));
-  const GateRec *dr = reinterpret_cast<const GateRec *>(d);
-  const int k = static_cast<int>(n);
   cudaError_t e = cudaMemcpyAsync(d, ctx->gate_pin.p, n * sizeof(GateRec), cudaMemcpyHostToDevice, st);
-  if (e == cudaSuccess) e = cudaMemsetAsync(d + o_result, 0xff, cleared, st);
-  if (e != cudaSuccess) return ctx_cuda(ctx, e, "gate set-up");
-  k_gate_bounds<<<static_cast<unsigned>(vblocks), kThreads, 0, st>>>(dr, k);
-  note_launch();
-  k_gate_weld<<<static_cast<unsigned>(vblocks), kThreads, 0, st>>>(dr, k);
-  note_launch();
-  k_gate_edges<<<static_cast<unsigned>(tblocks), kThreads, 0, st>>>(dr, k);
-  note_launch();
-  e = cudaGetLastError();
+  for (const Run &run : runs) {
+    const GateRec *dr = reinterpret_cast<const GateRec *>(d) + run.first;
+    const int k = static_cast<int>(run.count);
+    // The first memset takes the results and bounds of all meshes with it.
+    const size_t at = run.first == 0 ? o_result : o_tables;
+    if (e == cudaSuccess) e = cudaMemsetAsync(d + at, 0xff, o_tables + run.cleared - at, st);
+    if (e != cudaSuccess) return ctx_cuda(ctx, e, "gate set-up");
+    k_gate_bounds<<<run.vblocks, kThreads, 0, st>>>(dr, k);
+    note_launch();
+    k_gate_weld<<<run.vblocks, kThreads, 0, st>>>(dr, k);
+    note_launch();
+    k_gate_edges<<<run.tblocks, kThreads, 0, st>>>(dr, k);
+    note_launch();
+    e = cudaGetLastError();
+  }
   if (e == cudaSuccess) e = cudaMemcpyAsync(h, d + o_result, n * 24, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaEventRecord(ctx->gate_done, st);
   const sdfb_status early = meanwhile && e == cudaSuccess ? meanwhile() : SDFB_OK;

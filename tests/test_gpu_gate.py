@@ -60,3 +60,35 @@ def test_gate_bad_index(ctx):
     with pytest.raises(sdfb.SdfbError) as e:
         ctx.bake_batch([(v, f), (v, bad)], [g, g], sdfb.make_opts())
     assert e.value.status == sdfb.ERR_BAD_MESH and "mesh 1" in str(e.value)
+
+
+def test_batch_gate_in_runs():
+    """A batch whose tables do not fit the gate's share of memory together: the meshes go through it in runs,
+    which reuse one buffer, and every mesh gets its own verdict (a closed mesh's sign would be wrong for the
+    open one, in the columns below its hole)."""
+    import sdfb
+    import torch
+    from sdfb import meshgen as mg
+    v, f = mg.displaced_torus(1025, 512, 0.28, 0.1, 3)  # just past 2^20 triangles: 111 MB of tables
+    c = v[f].mean(axis=1)
+    g = np.ascontiguousarray(f[~((c[:, 2] > 0.0) & (np.abs(c[:, 1]) < 0.15) & (c[:, 0] > 0))])
+    dv = torch.as_tensor(v).cuda()
+    df, dg = torch.as_tensor(f.astype(np.int32)).cuda(), torch.as_tensor(g.astype(np.int32)).cuda()
+    closed = (dv.data_ptr(), len(v), df.data_ptr(), len(f))
+    opened = (dv.data_ptr(), len(v), dg.data_ptr(), len(g))
+    meshes = [opened if k % 5 == 2 else closed for k in range(24)]
+    grid = sdfb.make_grid((-0.5,) * 3, 1.0 / 24, (24,) * 3)
+    dist = torch.empty(24, *grid.shape, device="cuda")
+    occ = torch.empty(24, *grid.shape, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    at = [d.data_ptr() for d in dist], [o.data_ptr() for o in occ]
+    with sdfb.Context(0) as ctx:
+        # Occupancy with statistics: the gate's tables are nearly all that the call allocates.
+        ctx.bake_batch_device(meshes, [grid] * 24, None, None, at[1], stats=sdfb.Stats())
+        assert ctx.device_bytes() < 1.6 * 2 ** 30
+        ctx.bake_batch_device(meshes, [grid] * 24, None, *at)
+        lone = {m: ctx.bake(v, i, grid)[0] for m, i in ((closed, f), (opened, g))}
+        wrong = ctx.bake(v, g, grid, sdfb.make_opts(sign_mode=sdfb.SIGN_PARITY))[0]
+    assert (np.signbit(wrong) != np.signbit(lone[opened])).sum() > 10
+    for d, m in zip(dist.cpu().numpy(), meshes):
+        assert np.array_equal(np.signbit(d), np.signbit(lone[m]))
