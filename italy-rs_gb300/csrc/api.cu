@@ -249,12 +249,6 @@ sdfb_status device_caps(sdfb_ctx *ctx, cudaStream_t st, std::vector<PlanMesh> &m
   return SDFB_OK;
 }
 
-// Waits for what a failed call has enqueued early: it reads and writes the caller's buffers.
-static void settle(sdfb_ctx *ctx, cudaStream_t st) {
-  cudaStreamSynchronize(ctx->gate_stream);
-  cudaStreamSynchronize(st);
-}
-
 sdfb_status device_signs(sdfb_ctx *ctx, const sdfb_opts &o, PlanMesh *ms, size_t count, bool needed, cudaStream_t st,
                          size_t *bad, const std::function<sdfb_status()> &meanwhile) {
   size_t at = 0;
@@ -266,7 +260,6 @@ sdfb_status device_signs(sdfb_ctx *ctx, const sdfb_opts &o, PlanMesh *ms, size_t
     if (meanwhile) {
       if ((s = fork_gate(ctx, st)) != SDFB_OK) return s;
       s = device_gate(ctx, v, ctx->gate_stream, bad ? bad : &at, meanwhile);
-      if (s != SDFB_OK) settle(ctx, st);
     } else {
       s = device_gate(ctx, v, st, bad ? bad : &at);
     }
@@ -378,6 +371,7 @@ sdfb_status sdfb_bake_device(sdfb_ctx *ctx, const float *d_verts, uint32_t num_v
   cudaSetDevice(ctx->device);
   const sdfb_opts o = opts_or_default(opts);
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
+  Settle settle(ctx, st);
   std::vector<PlanMesh> ms(1);
   PlanMesh &p = ms[0];
   p.verts = d_verts;
@@ -392,9 +386,8 @@ sdfb_status sdfb_bake_device(sdfb_ctx *ctx, const float *d_verts, uint32_t num_v
   if (p.dist && !stats) tree = [&] { return early_tree(ctx, st, ms, o); };
   sdfb_status s = device_signs(ctx, o, &p, 1, p.dist || !p.occ || stats, st, nullptr, tree);
   if (s != SDFB_OK) return s;
-  if ((s = device_caps(ctx, st, ms)) == SDFB_OK) s = run_batch(ctx, st, ms, o, false, stats, p.bvh != nullptr);
-  if (s != SDFB_OK && p.bvh) settle(ctx, st);
-  return s;
+  if ((s = device_caps(ctx, st, ms)) != SDFB_OK) return s;
+  return settle.end(run_batch(ctx, st, ms, o, false, stats, p.bvh != nullptr));
 }
 
 sdfb_status sdfb_bake(sdfb_ctx *ctx, const float *verts, uint32_t num_verts, const uint32_t *idx, uint32_t num_tris,
@@ -408,6 +401,7 @@ sdfb_status sdfb_bake(sdfb_ctx *ctx, const float *verts, uint32_t num_verts, con
   cudaSetDevice(ctx->device);
   const sdfb_opts o = opts_or_default(opts);
   const cudaStream_t st = ctx->stream;
+  Settle settle(ctx, st);
   std::vector<PlanMesh> ms(1);
   PlanMesh &p = ms[0];
   const uint64_t cells = uint64_t(grid->nx) * grid->ny * grid->nz;
@@ -431,16 +425,13 @@ sdfb_status sdfb_bake(sdfb_ctx *ctx, const float *verts, uint32_t num_verts, con
   float *const direct_dist =
       (want_dist && p.sign != kSignGwn) ? static_cast<float *>(mapped_host(dist_out)) : nullptr;
   p.dist = want_dist ? (direct_dist ? direct_dist : static_cast<float *>(ctx->out_dist.p)) : nullptr;
-  if ((s = device_caps(ctx, st, ms)) == SDFB_OK) s = run_batch(ctx, st, ms, o, false, stats, p.bvh != nullptr);
-  if (s != SDFB_OK) {
-    if (p.bvh) settle(ctx, st);
-    return s;
-  }
+  if ((s = device_caps(ctx, st, ms)) != SDFB_OK) return s;
+  if ((s = run_batch(ctx, st, ms, o, false, stats, p.bvh != nullptr)) != SDFB_OK) return s;
   if (want_dist && !direct_dist)
     CK(cudaMemcpyAsync(dist_out, ctx->out_dist.p, cells * 4, cudaMemcpyDeviceToHost, st));
   if (want_occ) CK(cudaMemcpyAsync(occ_out, ctx->out_occ.p, cells, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
-  return SDFB_OK;
+  return settle.end();
 }
 
 sdfb_status sdfb_bake_soup(sdfb_ctx *ctx, const float *positions, uint32_t num_tris, const float bounds_min[3],
@@ -459,6 +450,7 @@ sdfb_status sdfb_bake_soup(sdfb_ctx *ctx, const float *positions, uint32_t num_t
   const sdfb_opts o = opts_or_default(opts);
   const uint32_t V = 3 * num_tris;
   const cudaStream_t st = ctx->stream;
+  Settle settle(ctx, st);
   const uint64_t cells = uint64_t(grid_out->nx) * grid_out->ny * grid_out->nz;
   const bool want_dist = dist_out && !o.no_distance, want_occ = occ_out && !o.no_occupancy;
   ENSURE(ctx->in_verts, size_t(V) * 12);
@@ -506,10 +498,7 @@ sdfb_status sdfb_bake_soup(sdfb_ctx *ctx, const float *positions, uint32_t num_t
     if (beside) {
       p.dist = static_cast<float *>(ctx->out_dist.p);
       p.occ = want_occ ? static_cast<uint8_t *>(ctx->out_occ.p) : nullptr;
-      if ((s = early_tree(ctx, st, ms, o)) != SDFB_OK) {
-        settle(ctx, st);
-        return s;
-      }
+      if ((s = early_tree(ctx, st, ms, o)) != SDFB_OK) return s;
     }
     CK(cudaEventSynchronize(ctx->gate_done));
     U = static_cast<uint32_t>(h[0]);
@@ -530,26 +519,19 @@ sdfb_status sdfb_bake_soup(sdfb_ctx *ctx, const float *positions, uint32_t num_t
     p.pidx = d_welded;
     p.pV = U;
     p.pT = num_tris;
-    if ((s = device_caps(ctx, st, ms)) != SDFB_OK) {
-      if (p.bvh) settle(ctx, st);
-      return s;
-    }
+    if ((s = device_caps(ctx, st, ms)) != SDFB_OK) return s;
   } else if (p.sign == kSignParity && want_dist) {
     p.pverts = static_cast<const float *>(ctx->in_verts2.p);
     p.pidx = static_cast<const uint32_t *>(ctx->in_idx2.p);
     p.pV = U;
     p.pT = num_tris;
   }
-  s = run_batch(ctx, st, ms, o, false, stats, p.bvh != nullptr);
-  if (s != SDFB_OK) {
-    if (p.bvh) settle(ctx, st);
-    return s;
-  }
+  if ((s = run_batch(ctx, st, ms, o, false, stats, p.bvh != nullptr)) != SDFB_OK) return s;
   if (want_dist && !direct_dist)
     CK(cudaMemcpyAsync(dist_out, ctx->out_dist.p, cells * 4, cudaMemcpyDeviceToHost, st));
   if (want_occ) CK(cudaMemcpyAsync(occ_out, ctx->out_occ.p, cells, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
-  return SDFB_OK;
+  return settle.end();
 }
 
 sdfb_status sdfb_weld_device(sdfb_ctx *ctx, const float *d_positions, uint32_t num_positions,
@@ -647,6 +629,7 @@ sdfb_status voxelize_sparse_run(sdfb_ctx *ctx, const float *positions, uint32_t 
   const uint32_t V = 3 * num_tris;
   const size_t cells = size_t(resolution) * resolution * resolution;
   const cudaStream_t st = ctx->stream;
+  Settle settle(ctx, st);
   ENSURE(ctx->in_verts, size_t(V) * 12);
   ENSURE(ctx->in_idx, size_t(V) * 4);
   ENSURE(ctx->out_occ, cells);
@@ -690,7 +673,7 @@ sdfb_status voxelize_sparse_run(sdfb_ctx *ctx, const float *positions, uint32_t 
   CK(sparse_count(static_cast<const uint8_t *>(ctx->out_occ.p), cells, ctx->sparse_tmp.p, ctx->sparse_tmp.cap, &total,
                   st));
   *count = total;
-  if (total == 0) return SDFB_OK;
+  if (total == 0) return settle.end();
   const size_t counted = ctx->sparse_tmp.cap;
   ENSURE(ctx->sparse_tmp, sparse_temp_bytes(cells, total));
   ENSURE(ctx->out_dist, total * 4);
@@ -714,7 +697,7 @@ sdfb_status voxelize_sparse_run(sdfb_ctx *ctx, const float *positions, uint32_t 
     CK(cudaMemcpyAsync(cells_out, ctx->sparse_xyz.p, n * 12, cudaMemcpyDeviceToHost, st));
   }
   CK(cudaStreamSynchronize(st));
-  return SDFB_OK;
+  return settle.end();
 }
 
 extern "C" {
@@ -730,6 +713,7 @@ sdfb_status sdfb_bake_batch_device(sdfb_ctx *ctx, uint32_t count, const sdfb_mes
   cudaSetDevice(ctx->device);
   const sdfb_opts o = opts_or_default(opts);
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
+  Settle settle(ctx, st);
   std::vector<PlanMesh> ms(count);
   for (uint32_t m = 0; m < count; ++m) {
     const sdfb_mesh_desc &d = meshes[m];
@@ -752,7 +736,7 @@ sdfb_status sdfb_bake_batch_device(sdfb_ctx *ctx, uint32_t count, const sdfb_mes
     return ctx_fail(ctx, s, "mesh %zu: %s", bad, e.c_str());
   }
   if (s != SDFB_OK || (s = device_caps(ctx, st, ms)) != SDFB_OK) return s;
-  return run_batch(ctx, st, ms, o, true, stats);
+  return settle.end(run_batch(ctx, st, ms, o, true, stats));
 }
 
 sdfb_status sdfb_bake_batch(sdfb_ctx *ctx, uint32_t count, const sdfb_mesh_desc *meshes, const sdfb_grid_desc *grids,
@@ -764,6 +748,7 @@ sdfb_status sdfb_bake_batch(sdfb_ctx *ctx, uint32_t count, const sdfb_mesh_desc 
   cudaSetDevice(ctx->device);
   const sdfb_opts o = opts_or_default(opts);
   const cudaStream_t st = ctx->stream;
+  Settle settle(ctx, st);
   size_t nv = 0, ni = 0;
   for (uint32_t m = 0; m < count; ++m) {
     if (!meshes[m].verts || !meshes[m].idx || !grid_ok(&grids[m]))
@@ -835,7 +820,7 @@ sdfb_status sdfb_bake_batch(sdfb_ctx *ctx, uint32_t count, const sdfb_mesh_desc 
     if (ms[m].occ && !direct_occ[m]) CK(cudaMemcpyAsync(occ_outs[m], ms[m].occ, cells, cudaMemcpyDeviceToHost, st));
   }
   CK(cudaStreamSynchronize(st));
-  return SDFB_OK;
+  return settle.end();
 }
 
 }  // extern "C"

@@ -171,6 +171,26 @@ struct sdfb_ctx {
   uint64_t device_bytes() const;
 };
 
+// Waits, when a call fails half way, for what it has enqueued on its stream and the gate's: that reads and
+// writes the caller's buffers, which are the caller's again once the call returns.
+struct Settle {
+  sdfb_ctx *ctx;
+  cudaStream_t st;
+  bool done = false;
+  Settle(sdfb_ctx *c, cudaStream_t s) : ctx(c), st(s) {}
+  Settle(const Settle &) = delete;
+  ~Settle() {
+    if (done) return;
+    if (ctx->gate_stream) cudaStreamSynchronize(ctx->gate_stream);
+    cudaStreamSynchronize(st);
+  }
+  // The call's last status: after SDFB_OK nothing is left to wait for.
+  sdfb_status end(sdfb_status s = SDFB_OK) {
+    done = s == SDFB_OK;
+    return s;
+  }
+};
+
 int bucket_tris(uint64_t T);
 int bucket_grid(const sdfb_grid_desc &g);
 

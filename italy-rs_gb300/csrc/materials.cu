@@ -359,6 +359,7 @@ extern "C" sdfb_status sdfb_bake_materials(sdfb_ctx *ctx, const float *positions
   if (ms != SDFB_OK) return ms;
   cudaSetDevice(ctx->device);
   const cudaStream_t st = ctx->stream;
+  Settle settle(ctx, st);
   const uint64_t cells = uint64_t(grid->nx) * grid->ny * grid->nz;
   ENSURE(ctx->mat_cells, align256(cells * 12) + 2 * align256(cells * 4));
   float *color = static_cast<float *>(ctx->mat_cells.p);
@@ -393,7 +394,7 @@ extern "C" sdfb_status sdfb_bake_materials(sdfb_ctx *ctx, const float *positions
   if (metallic_out) CK(cudaMemcpyAsync(metallic_out, metal, cells * 4, cudaMemcpyDeviceToHost, st));
   if (roughness_out) CK(cudaMemcpyAsync(roughness_out, rough, cells * 4, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
-  return SDFB_OK;
+  return settle.end();
 }
 
 extern "C" sdfb_status sdfb_voxelize_sparse_colors(sdfb_ctx *ctx, const float *positions, uint32_t num_tris,
@@ -414,6 +415,7 @@ extern "C" sdfb_status sdfb_voxelize_sparse_colors(sdfb_ctx *ctx, const float *p
   const uint64_t n_out = std::min<uint64_t>(*count, cap);
   if (n_out == 0) return SDFB_OK;
   const cudaStream_t st = ctx->stream;
+  Settle settle(ctx, st);
   BatchDev B;
   if ((s = soup_batch(ctx, positions, num_tris, g, st, B)) != SDFB_OK) return s;
   if ((s = triangle_materials(ctx, *materials, num_tris, st)) != SDFB_OK) return s;
@@ -430,5 +432,5 @@ extern "C" sdfb_status sdfb_voxelize_sparse_colors(sdfb_ctx *ctx, const float *p
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(colors_out, ctx->mat_cells.p, n_out * 12, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
-  return SDFB_OK;
+  return settle.end();
 }
