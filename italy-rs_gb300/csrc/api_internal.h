@@ -182,7 +182,10 @@ struct Settle {
   ~Settle() {
     if (done) return;
     if (ctx->gate_stream) cudaStreamSynchronize(ctx->gate_stream);
-    cudaStreamSynchronize(st);
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;  // a wait would end the caller's capture
+    if (cudaStreamIsCapturing(st, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone)
+      cudaStreamSynchronize(st);
+    cudaGetLastError();  // the call reports its own error; the next one starts from a clean state
   }
   // The call's last status: after SDFB_OK nothing is left to wait for.
   sdfb_status end(sdfb_status s = SDFB_OK) {

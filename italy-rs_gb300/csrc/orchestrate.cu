@@ -661,6 +661,12 @@ sdfb_status run_batch(sdfb_ctx *ctx, cudaStream_t st, std::vector<PlanMesh> &ms,
 // 64^3 and 97 x 61 x 43 cells 239 -> 209, 398 -> 354 and 457 -> 404 us.
 
 sdfb_status fork_gate(sdfb_ctx *ctx, cudaStream_t st) {
+  // A stream under capture is refused here, as the gate's wait would: its event would draw the gate's stream
+  // into the capture, and other bakes of the context would fail until the capture ends.
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  CK(cudaStreamIsCapturing(st, &capture));
+  if (capture != cudaStreamCaptureStatusNone)
+    return ctx_fail(ctx, SDFB_ERR_CUDA, "the stream is being captured, and a bake with an automatic sign waits for it");
   CK(cudaEventRecord(ctx->gate_fork, st));
   CK(cudaStreamWaitEvent(ctx->gate_stream, ctx->gate_fork, 0));
   return SDFB_OK;

@@ -59,3 +59,34 @@ def test_same_refusals(ctx, fault, want_occ):
             ctx.bake(w, h, g, want_occ=want_occ, stats=stats)
         assert e.value.status == sdfb.ERR_BAD_MESH
         assert np.array_equal(*(ctx.bake(v, f, g, stats=s)[0] for s in (None, sdfb.Stats())))  # nothing is left behind
+
+
+@pytest.mark.parametrize("sign", ["auto", "parity"])
+def test_stream_under_capture(ctx, sign):
+    """A bake on a stream that is being captured is refused, and leaves the context to other streams meanwhile."""
+    import sdfb
+    import torch
+    v, f = _mesh("closed")
+    g = sdfb.make_grid((-0.5,) * 3, 1.0 / 21, (21, 22, 23))
+    dv, df = torch.as_tensor(v).cuda(), torch.as_tensor(f.astype(np.int32)).cuda()
+    d, o = torch.zeros(g.shape, device="cuda"), torch.zeros(g.shape, dtype=torch.uint8, device="cuda")
+    opts = sdfb.make_opts(sign_mode=sdfb.SIGN_AUTO if sign == "auto" else sdfb.SIGN_PARITY)
+
+    def bake(stream):
+        ctx.bake_device(dv.data_ptr(), len(v), df.data_ptr(), len(f), g, opts, d.data_ptr(), o.data_ptr(), stream)
+
+    torch.cuda.synchronize()
+    bake(0)
+    want = d.cpu().numpy()
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    with torch.cuda.stream(stream):
+        graph.capture_begin(capture_error_mode="relaxed")
+        with pytest.raises(sdfb.SdfbError) as e:
+            bake(stream.cuda_stream)
+        assert e.value.status == sdfb.ERR_CUDA
+        bake(0)  # on the context's own stream
+        try:
+            graph.capture_end()
+        except RuntimeError:
+            pass  # a wait inside the capture ended it
+    assert np.array_equal(d.cpu().numpy(), want)
