@@ -122,7 +122,9 @@ typedef struct sdfb_stats {
   uint64_t triangles;
   uint64_t sat_tests;      /* triangle/box tests run by the occupancy kernel */
   uint64_t crossings;      /* parity crossings found */
-  uint64_t box_tests;      /* count_work: tree children measured against a whole tile */
+  uint64_t box_tests;      /* count_work: tree children measured against a whole tile (in all four
+                              counts cells that stand in for ones beyond the grid's edge count; the
+                              searches for a block to start a tile from do not) */
   uint64_t tri_tests;      /* count_work: exact point-triangle distances */
   double flops_distance;   /* count_work: FP32 flops of the distance tests as executed, terms a lane
                               shares between its cells counted once (FMA = 2) */

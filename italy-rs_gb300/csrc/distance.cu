@@ -370,7 +370,7 @@ struct Walker {
         const uint32_t was = atomicMin(best + (e & 127), __float_as_uint(d2));
         if ((e & 127) == kMiddle && __float_as_uint(d2) < was) m.seed = blk;
       }
-      if (COUNT) ws.tri_tests += kWarp;
+      if (COUNT) ws.tri_tests += min(np - base, kWarp >> lb) << lb;
     }
     __syncwarp();
 #pragma unroll
@@ -547,7 +547,7 @@ struct Walker {
       d2 = ex * ex + ey * ey + ez * ez;
       kept = near(c.w, copysignf(ex, tx), copysignf(ey, ty), copysignf(ez, tz), d2, fx * fx + fy * fy + fz * fz,
                   ax + ay + az + be.x + be.y + be.z);
-      if (COUNT) ws.box_tests += kWarp;
+      if (COUNT) ws.box_tests += __popc(__ballot_sync(kFull, valid));
     } else {
       const float4 *o = tree_obb(m.t.obb, valid ? child : 0);
       const float4 o0 = __ldg(o), o1 = __ldg(o + kObbPlane), o2 = __ldg(o + 2 * kObbPlane),
@@ -563,7 +563,7 @@ struct Walker {
       kept = near(c.w, fmaf(e2, o3.x, fmaf(e1, o2.x, e0 * o1.x)), fmaf(e2, o3.y, fmaf(e1, o2.y, e0 * o1.y)),
                   fmaf(e2, o3.z, fmaf(e1, o2.z, e0 * o1.z)), d2, f0 * f0 + f1 * f1 + f2 * f2,
                   a0 + a1 + a2 + o0.w + o1.w + o2.w);
-      if (COUNT) ws.plane_tests += kWarp;
+      if (COUNT) ws.plane_tests += __popc(__ballot_sync(kFull, valid));
     }
     return kept && valid;
   }

@@ -76,3 +76,17 @@ def test_block_pass_with_more_nodes_than_it_keeps(ctx, oracle, leaf):
             ref = d
             assert np.abs(d.reshape(-1) - d64).max() <= TOL * 0.8  # the sphere's diameter, not the grid's
         assert np.array_equal(d, ref), (tile, budget)
+
+
+@pytest.mark.parametrize("T, leaf, blocks", [(1, 2, 1), (5, 2, 3), (5, 4, 2), (9, 8, 2), (64, 2, 32)])
+def test_counted_work(ctx, T, leaf, blocks):
+    """The counts are of tests that a lane had work for: one node with fewer than 32 blocks, seen by one tile."""
+    import sdfb
+    v, i = soup(T, T)
+    st = sdfb.Stats()
+    g = sdfb.make_grid((-0.5,) * 3, 0.25, (4, 4, 2))
+    ctx.bake(v, i, g, sdfb.make_opts(sign_mode=sdfb.SIGN_NONE, leaf_size=leaf, tile=1, step_budget=-1, count_work=True,
+                                     no_occupancy=True), want_occ=False, stats=st)
+    assert (st.box_tests, st.plane_tests) == (0, blocks)
+    assert st.rect_tests <= 32 * blocks and st.rect_tests % 32 == 0
+    assert 32 * leaf <= st.tri_tests <= 32 * leaf * (1 + blocks) and st.tri_tests % leaf == 0
