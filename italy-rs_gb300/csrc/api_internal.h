@@ -62,7 +62,6 @@ struct ResidentBvh {
   sdfb::PTreeRec tree{};              // distance
   const sdfb::Node *nodes = nullptr;  // winding number: the caps
   const sdfb::TriRec *tris = nullptr;
-  const uint32_t *leaf_order = nullptr;
   const float4 *node_moment = nullptr;
   int num_nodes = 0, num_inner = 0, num_tris = 0, root = 0;
 };

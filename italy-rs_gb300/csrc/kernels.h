@@ -108,7 +108,6 @@ struct MeshRec {
   const Node *cap_nodes;
   const TriRec *cap_trec;
   const float4 *cap_moment;  // per inner cap node: (area-weighted normal sum, total area)
-  const uint32_t *cap_order;
 };
 
 // Prefix tables of a batch (device): starts[m] of each numbering, starts[M] = total.
@@ -153,7 +152,6 @@ cudaError_t ptree_build(const BatchDev &batch, const PTreeRec *trees, const uint
 struct BvhDev {
   TriRec *tris = nullptr;          // T_total records in leaf order
   Node *nodes = nullptr;           // (T_total - 1) inner nodes + M virtual roots
-  uint32_t *leaf_order = nullptr;  // local (per-mesh) triangle index of each record
   uint32_t *bounds = nullptr;      // 6 ordered-uint words per mesh: centroid min xyz, max xyz
   float4 *node_moment = nullptr;   // per inner node: (sum of area x unit normal over its triangles,
                                    // their total area)
@@ -194,8 +192,8 @@ struct DistanceArgs {
   unsigned long long *tile_counter;   // pass A's chunk counter, zero before the launch
   unsigned long long chunk_tiles;     // tiles per chunk (set by the launcher)
   unsigned long long *work_counters;  // optional: [0] box, [1] triangle, [3] plane, [4] rectangle tests (lanes)
-  // Deferral of long tiles (none when defer_list is null or step_budget <= 0): every step_budget
-  // pairs of children measured a walk checks whether all tiles have been handed out and, if so, defers its
+  // Deferral of long tiles (none when defer_list is null or step_budget <= 0): every step_budget steps
+  // (sdfb_opts) a walk checks whether all tiles have been handed out and, if so, defers its
   // tile. The list holds defer_capacity tile indices; defer_counters[0] counts deferred tiles (it
   // may pass the capacity), [1] is the second pass's tile counter. Both are zero before the launch.
   unsigned long long *defer_list;

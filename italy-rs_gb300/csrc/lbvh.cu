@@ -381,14 +381,10 @@ __global__ void k_roots(BatchDev B, int num_inner, const uint32_t *__restrict__ 
   store_node(nodes, num_inner + m, box, refs);
 }
 
-__global__ __launch_bounds__(kThreads) void k_gather(BatchDev B, const uint32_t *__restrict__ vals,
-                                                     const TriRec *__restrict__ rec, TriRec *__restrict__ out,
-                                                     uint32_t *__restrict__ order) {
+__global__ __launch_bounds__(kThreads) void k_gather(uint64_t T, const uint32_t *__restrict__ vals,
+                                                     const TriRec *__restrict__ rec, TriRec *__restrict__ out) {
   const uint64_t k = uint64_t(blockIdx.x) * kThreads + threadIdx.x;
-  if (k >= B.total_tris) return;
-  const uint32_t t = vals[k];
-  out[k] = rec[t];
-  order[k] = static_cast<uint32_t>(t - B.tri_starts[find_mesh(B.tri_starts, B.num_meshes, t)]);
+  if (k < T) out[k] = rec[vals[k]];
 }
 
 // Far-field moments of every inner node, bottom-up like k_refit: (sum of a_i n_i, sum of a_i)
@@ -424,8 +420,8 @@ size_t lbvh_temp_bytes(uint64_t total_tris, int num_meshes) { return temp_layout
 
 size_t lbvh_bytes(uint64_t T, int M) {
   const size_t n = std::max<uint64_t>(T, 1), m = std::max<uint64_t>(T, 2) - 1;
-  return align256(n * sizeof(TriRec)) + align256((m + M) * sizeof(Node)) + align256(n * 4) +
-         align256(size_t(M) * 6 * 4) + align256(m * sizeof(float4));
+  return align256(n * sizeof(TriRec)) + align256((m + M) * sizeof(Node)) + align256(size_t(M) * 6 * 4) +
+         align256(m * sizeof(float4));
 }
 
 void lbvh_bind(BvhDev &b, void *mem, uint64_t T, int M) {
@@ -435,8 +431,6 @@ void lbvh_bind(BvhDev &b, void *mem, uint64_t T, int M) {
   p += align256(n * sizeof(TriRec));
   b.nodes = reinterpret_cast<Node *>(p);
   p += align256((m + M) * sizeof(Node));
-  b.leaf_order = reinterpret_cast<uint32_t *>(p);
-  p += align256(n * 4);
   b.bounds = reinterpret_cast<uint32_t *>(p);
   p += align256(size_t(M) * 6 * 4);
   b.node_moment = reinterpret_cast<float4 *>(p);
@@ -488,7 +482,7 @@ cudaError_t lbvh_build(const BatchDev &B, BvhDev &b, void *temp, size_t temp_byt
   }
   k_roots<<<(M + 127) / 128, 128, 0, st>>>(B, b.num_inner, vals, t.lo, t.hi, t.ilo, t.ihi, t.subtree, b.nodes, err);
   note_launch();
-  k_gather<<<blocks_for(T), kThreads, 0, st>>>(B, vals, t.rec, b.tris, b.leaf_order);
+  k_gather<<<blocks_for(T), kThreads, 0, st>>>(T, vals, t.rec, b.tris);
   note_launch();
   if (T >= 2) {
     if ((e = cudaMemsetAsync(t.visits, 0, sizeof(int) * (T - 1), st)) != cudaSuccess) return e;

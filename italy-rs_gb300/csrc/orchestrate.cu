@@ -257,7 +257,6 @@ void make_layout(sdfb_ctx *ctx, const std::vector<PlanMesh> &ms, const sdfb_opts
         r.cap_nodes = p.caps->nodes;
         r.cap_trec = p.caps->tris;
         r.cap_moment = p.caps->node_moment;
-        r.cap_order = p.caps->leaf_order;
         r.cap_nodes_n = p.caps->num_nodes;
         r.cap_inner_n = p.caps->num_inner;
         r.cap_recs_n = p.caps->num_tris;
@@ -317,7 +316,6 @@ void bind_built(Layout &L, char *trees, const BvhDev *caps) {
       r.cap_nodes = caps->nodes;
       r.cap_trec = caps->tris;
       r.cap_moment = caps->node_moment;
-      r.cap_order = caps->leaf_order;
       r.cap_nodes_n = caps->num_nodes;
       r.cap_inner_n = caps->num_inner;
       r.cap_recs_n = static_cast<int>(L.cap_total);
@@ -583,7 +581,7 @@ sdfb_status finish_batch(sdfb_ctx *ctx, Workspace &ws, cudaStream_t st, const Ba
     return ctx_fail(ctx, SDFB_ERR_BUSY, "crossing list resized; enqueue again");
   }
   if (h_err & kErrStackOverflow)
-    return ctx_fail(ctx, SDFB_ERR_OVERFLOW, "BVH traversal stack overflow (depth > %d)", S.stack);
+    return ctx_fail(ctx, SDFB_ERR_OVERFLOW, "BVH traversal stack overflow");
   if (h_err & kErrCorruptTree)
     return ctx_fail(ctx, SDFB_ERR_INTERNAL, "BVH walk met an invalid reference or ran past its step limit");
   if (h_err & kErrDispatch) return ctx_fail(ctx, SDFB_ERR_INTERNAL, "distance tile dispatch timed out");
@@ -647,7 +645,7 @@ sdfb_status run_batch(sdfb_ctx *ctx, cudaStream_t st, std::vector<PlanMesh> &ms,
     s = finish_batch(ctx, ctx->ws, st, S, ms, stats);
     if (s == SDFB_ERR_BUSY) continue;  // crossing list resized
     if (s == SDFB_ERR_OVERFLOW && S.stack < 64) {
-      oo.stack_depth = 64;  // the tuned shallow stack was too small for this tree
+      oo.stack_depth = 64;  // only fault injection makes a stack too small: it spares this one
       continue;
     }
     return s;
@@ -768,7 +766,6 @@ sdfb_status build_resident(sdfb_ctx *ctx, Workspace &ws, cudaStream_t st, const 
     CK(lbvh_build(batch(&d->caps, d->cap_tris, p.cT), b, ws.build_tmp.p, ws.build_tmp.cap, d_err, st));
     cap_out.nodes = b.nodes;
     cap_out.tris = b.tris;
-    cap_out.leaf_order = b.leaf_order;
     cap_out.node_moment = b.node_moment;
     cap_out.num_nodes = b.num_nodes;
     cap_out.num_inner = b.num_inner;
