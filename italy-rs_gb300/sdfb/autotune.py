@@ -9,12 +9,13 @@ Three parameters of the distance pass trade against each other with the mesh and
   * step budget (work steps between a tile's looks at whether it should be handed to the
     block-per-tile second pass, or never): a small budget moves more tiles into the pass that splits
     a tile's walk over a block, which pays on small grids (fewer tiles than the GPU holds warps).
-The table also holds a traversal stack depth, 32 or 64; every tree fits either.
+The table also holds a traversal stack depth, 32 or 64, which only fault injection looks at: every tree fits
+either. It is written as 64; the batch mode tries both.
 
 For each (log2 triangles, log2 grid edge) bucket of a sweep of displaced spheres and grids, the tuner
 times device-buffer bakes (the bake's own device time, median of `reps`; the geometric mean over a cubic
 and a ragged grid of the bucket, whose tiles the GPU holds in different numbers) under a
-coordinate descent over the four parameters, then fills every bucket of the table from the
+coordinate descent over the three parameters, then fills every bucket of the table from the
 nearest measured one and writes "tri_bucket grid_bucket leaf tile stack budget" lines (tile
 0-based, budget 0 = never) that
 the library reads at context creation (tuning/gb300.tsv beside lib/, or the file SDFB_TUNING names).
@@ -193,7 +194,7 @@ def _time_bake(ctx, sdfb, dev, grids, params, reps: int) -> float:
 
 
 def tune_case(ctx, sdfb, dev, grids, reps: int, log=print):
-    """Coordinate descent: tile, leaf, stack, budget, then tile again. Returns (params, ms)."""
+    """Coordinate descent: tile, leaf, budget, then tile again. Returns (params, ms)."""
     cache = {}
 
     def t(p):
@@ -202,14 +203,14 @@ def tune_case(ctx, sdfb, dev, grids, reps: int, log=print):
         return cache[p]
 
     best = START
-    for axis, values in ((1, TILES), (0, LEAVES), (2, STACKS), (3, BUDGETS), (1, TILES)):
+    for axis, values in ((1, TILES), (0, LEAVES), (3, BUDGETS), (1, TILES)):
         for v in values:
             p = list(best)
             p[axis] = v
             p = tuple(p)
             if t(p) < t(best):
                 best = p
-    log(f"    {len(cache)} configurations, best leaf {best[0]} tile {best[1]} stack {best[2]} budget {best[3]}: "
+    log(f"    {len(cache)} configurations, best leaf {best[0]} tile {best[1]} budget {best[3]}: "
         f"{t(best):.3f} ms "
         f"(defaults {t(START):.3f} ms)")
     return best, t(best)

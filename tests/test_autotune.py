@@ -50,3 +50,10 @@ def test_tune_batch_descends_and_keeps_the_table_when_nothing_is_faster():
     assert best[:2] == (5, 32) and best_ms == 90.0 and table_ms == 100.0
     best, best_ms, table_ms = autotune.tune_batch(lambda p: 100.0 if p is None else 120.0, log=lambda *a: None)
     assert best is None and best_ms == table_ms == 100.0
+
+
+def test_tune_case_leaves_the_stack_depth(monkeypatch):
+    # noise would decide between two depths that run the same code
+    monkeypatch.setattr(autotune, "_time_bake", lambda ctx, sdfb, dev, grids, p, reps: 100.0 - p[1] - (p[2] == 32))
+    best, ms = autotune.tune_case(None, None, None, [], 1, log=lambda *a: None)
+    assert best == (2, 6, 64, 2048) and ms == 94.0
