@@ -12,7 +12,8 @@
 //                      distance to its oriented box; the cells that it could improve become
 //                      (block, cell) pairs in shared memory;
 //   lanes = triangles  pairs are taken 32 / n at a time, n lanes computing the exact distances to a
-//                      block's n triangles; the minimum goes to the cell's bound in shared memory.
+//                      block's n triangles; the minimum goes to the cell's bound in shared memory. A block
+//                      that most cells want is measured by all of them instead, lanes = cells.
 //
 // Before, all lanes were cells throughout: every node and triangle was tested by 128 cells although
 // most die on the first one's answer, 50-70 instructions a triangle. Testing children by lanes costs
@@ -79,6 +80,12 @@ constexpr int kMaxLevels = 8;        // 2^31 triangles in blocks of 2 make 6 lev
 constexpr int kStackSize = 32 * kMaxLevels;  // a node leaves at most 31 siblings behind on its level
 constexpr int kFlushAt = 16;                 // surviving blocks measured against the cells together
 constexpr int kSurvivors = kFlushAt + kWarp;
+// Cells of a tile of 128 from which on a block is measured by all of them rather than in pairs. Large
+// triangles, pairs alone and with 64, 48 and 32 cells: a box of 12 at 256^3 0.32 ms, 0.30 each; 80 at 256^3
+// 0.86, 0.68, 0.67, 0.66; 2,000 as large as their box at 128^3 2.8, 1.46, 1.46, 1.45; 82k small ones at 256^3
+// 4.38, 4.14, 4.08, 4.07. Smaller tiles keep to pairs: they belong to grids that leave the GPU underfilled, where
+// the pairs' shorter chain of loads counts (1,280 triangles at 32^3 59.5 us, 62.3 with 24 of 32 cells).
+constexpr uint32_t kDirectCells = 48;
 constexpr int kDrainAt = 64;                 // pairs that start a round of exact tests
 // Steps of work as sdfb_opts.step_budget counts them, about 8 instructions each.
 constexpr int kStepsPerVisit = 16, kStepsPerBlock = 10, kStepsPerRound = 12;
@@ -186,6 +193,7 @@ struct WarpMem {
   uint32_t blocks[kSurvivors];  // surviving blocks; blocks[0] is the nearest of its node
   uint32_t mesh;                // the mesh that t is of
   uint32_t seed;                // the block that last improved the middle cell of the tile at seed_at
+  uint32_t started;             // the block that the tile's bounds were started from
   float seed_at[3];
   uint16_t pairs[kDrainAt + kWarp * 4];  // (index into blocks << 7) | (v << 5) | lane
 };
@@ -250,7 +258,7 @@ struct Walker {
     }
     if (lane == 0) {
       m.t = tree;
-      m.seed = kNoSeed;
+      m.seed = m.started = kNoSeed;
       *const_cast<volatile uint32_t *>(&m.mesh) = mesh;
     }
     __syncwarp();
@@ -379,8 +387,33 @@ struct Walker {
     np = 0;
   }
 
-  // Measures the surviving blocks against every cell, runs the pairs, refits the planes.
-  __device__ __forceinline__ void flush(int &nb) {
+  // Exact distances of a block's triangles to every cell, lanes = cells: for a block that most cells want.
+  __device__ __forceinline__ void direct(uint32_t blk) {
+    const int lb = m.t.block_log2;
+    float b[VPL];
+#pragma unroll
+    for (int v = 0; v < VPL; ++v) b[v] = kInf;
+    for (int k = 0; k < (1 << lb); ++k) {
+      const float4 *tri = tree_tri(m.t.tri, (size_t(blk) << lb) + k);
+      const float4 q0 = __ldg(tri), q1 = __ldg(tri + kTriPlane), q2 = __ldg(tri + 2 * kTriPlane),
+                   q3 = __ldg(tri + 3 * kTriPlane), q4 = __ldg(tri + 4 * kTriPlane);
+#pragma unroll
+      for (int v = 0; v < VPL; ++v) b[v] = fminf(b[v], tri_dist2(q0, q1, q2, q3, q4, px, py, pz[v]));
+      if (COUNT) ws.tri_tests += kWarp * VPL;
+    }
+#pragma unroll
+    for (int v = 0; v < VPL; ++v) {
+      const uint32_t was = atomicMin(best + v * kWarp + lane, __float_as_uint(b[v]));
+      keep[v] = fminf(b[v], __uint_as_float(was)) * kKeep;
+      if (v * kWarp + lane == kMiddle && __float_as_uint(b[v]) < was) m.seed = blk;
+    }
+    steps += (3 + 5 * VPL) << lb;
+    __syncwarp();
+  }
+
+  // Measures the surviving blocks against every cell, runs the pairs, refits the planes (not the last time:
+  // no node is left that they could drop).
+  __device__ __forceinline__ void flush(int &nb, bool last) {
     int np = 0;
     bool any_pair = false;
     const float4 *obb = m.t.obb;
@@ -402,9 +435,19 @@ struct Walker {
       if (COUNT) ws.rect_tests += kWarp * VPL;
       if (!__any_sync(kFull, some)) continue;
       any_pair = true;
+      uint32_t masks[VPL], cells = 0;
 #pragma unroll
       for (int v = 0; v < VPL; ++v) {
-        const uint32_t mask = __ballot_sync(kFull, want[v]);
+        masks[v] = __ballot_sync(kFull, want[v]);
+        cells += __popc(masks[v]);
+      }
+      if (VPL >= 4 && cells >= kDirectCells) {
+        direct(m.blocks[i]);
+        continue;
+      }
+#pragma unroll
+      for (int v = 0; v < VPL; ++v) {
+        const uint32_t mask = masks[v];
         if (want[v])
           m.pairs[np + __popc(mask & ((1u << lane) - 1u))] = static_cast<uint16_t>((i << 7) | (v << 5) | lane);
         np += __popc(mask);
@@ -415,7 +458,7 @@ struct Walker {
     __syncwarp();
     steps += nb * kStepsPerBlock;
     nb = 0;
-    if (any_pair) fit();
+    if (any_pair && !last) fit();
   }
 
   // Finds the block to start from: of the blocks nearest to the middle of the last tiles of the
@@ -529,6 +572,7 @@ struct Walker {
 #pragma unroll
     for (int v = 0; v < VPL; ++v) best[v * kWarp + lane] = __float_as_uint(b[v]);
     if (lane < 3) m.seed_at[lane] = lane == 0 ? m.centre.x : (lane == 1 ? m.centre.y : m.centre.z);
+    if (lane == 3) m.started = m.seed;
     __syncwarp();
   }
 
@@ -565,7 +609,7 @@ struct Walker {
                   a0 + a1 + a2 + o0.w + o1.w + o2.w);
       if (COUNT) ws.plane_tests += __popc(__ballot_sync(kFull, valid));
     }
-    return kept && valid;
+    return kept && valid && (level > 0 || child != m.started);
   }
 
   // Takes the kept blocks into the list, the nearest first.
@@ -575,7 +619,6 @@ struct Walker {
     if (kept) m.blocks[nb + (lane == nl ? 0 : rank + 1)] = child;
     nb += __popc(mask);
     __syncwarp();
-    if (nb >= kFlushAt) flush(nb);
   }
 
   // Walks below node `cur` ((level << 28) | node). Returns false when the tail check stopped it with
@@ -619,11 +662,11 @@ struct Walker {
         }
         take_blocks(kept, child, mask, d2, nb);
       }
-      if (sp == 0) break;
+      const bool last = sp == 0;
+      if (nb >= kFlushAt || (last && nb > 0)) flush(nb, last);
+      if (last) return true;
       cur = m.stack[--sp];
     }
-    if (nb > 0) flush(nb);
-    return true;
   }
 };
 
@@ -744,29 +787,32 @@ __global__ __launch_bounds__(kThreadsA, kMinBlocksA) void k_distance(DistanceArg
       w.pick_seed(s_mem, kWarpsPerBlockA);
     }
     w.start();
-    w.fit();
-    bool done = w.walk(w.root(), tail, lim);
-    // The tile's indices are located again rather than kept in registers across the walk.
-    typename W::Cells c;
-    c.locate(B, tile);
-    if (!done) {
+    bool listed = false;
+    for (TailCheck check = tail;; check = never) {
+      w.fit();
+      if (w.walk(w.root(), check, lim)) break;
       unsigned long long slot = 0;
       if (lane == 0) slot = atomicAdd(a.defer_counters, 1ull);
       slot = __shfl_sync(kFull, slot, 0);
       if (slot < a.defer_capacity) {
         if (lane == 0) a.defer_list[slot] = tile;
-#pragma unroll
-        for (int v = 0; v < VPL; ++v)
-          if (c.active(lane, v))
-            c.M->dist[c.cell(lane, v)] = __uint_as_float(w.best[v * kWarp + lane]);  // pass B starts from these
-        continue;
+        listed = true;
+        break;
       }
-      // The list is full: finish the tile here, from the bounds found so far.
-      w.fit();
-      w.walk(w.root(), never, lim);
+      // The list is full: the tile is finished here, from the bounds found so far.
     }
+    // The tile's indices are located again rather than kept in registers across the walk.
+    typename W::Cells c;
+    c.locate(B, tile);
     __syncwarp();
-    store_cells<TX, TY, TZ>(a, c, lane, w.best);
+    if (listed) {
+#pragma unroll
+      for (int v = 0; v < VPL; ++v)
+        if (c.active(lane, v))
+          c.M->dist[c.cell(lane, v)] = __uint_as_float(w.best[v * kWarp + lane]);  // pass B starts from these
+    } else {
+      store_cells<TX, TY, TZ>(a, c, lane, w.best);
+    }
     __syncwarp();
   }
   flush_stats<COUNT>(a, w.ws, lane);
@@ -830,6 +876,7 @@ __global__ __launch_bounds__(kThreads, kMinBlocksB) void k_distance_deferred(Dis
         if (!mask) continue;
         if (level == 1) {
           w.take_blocks(kept, child, mask, d2, nb);
+          if (nb >= kFlushAt) w.flush(nb, false);
           continue;
         }
         uint32_t at = 0;
@@ -848,7 +895,7 @@ __global__ __launch_bounds__(kThreads, kMinBlocksB) void k_distance_deferred(Dis
       }
       __syncthreads();
     }
-    if (nb > 0) w.flush(nb);
+    if (nb > 0) w.flush(nb, true);
     __syncthreads();
     if (warp == 0) store_cells<TX, TY, TZ>(a, c, lane, s_best);
     __syncthreads();

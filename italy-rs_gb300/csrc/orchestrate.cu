@@ -662,7 +662,7 @@ sdfb_status fork_gate(sdfb_ctx *ctx, cudaStream_t st) {
   // A stream under capture is refused here, as the gate's wait would: its event would draw the gate's stream
   // into the capture, and other bakes of the context would fail until the capture ends.
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  CK(cudaStreamIsCapturing(st, &capture));
+  if (st != ctx->stream) CK(cudaStreamIsCapturing(st, &capture));
   if (capture != cudaStreamCaptureStatusNone)
     return ctx_fail(ctx, SDFB_ERR_CUDA, "the stream is being captured, and a bake with an automatic sign waits for it");
   CK(cudaEventRecord(ctx->gate_fork, st));

@@ -90,3 +90,25 @@ def test_counted_work(ctx, T, leaf, blocks):
     assert (st.box_tests, st.plane_tests) == (0, blocks)
     assert st.rect_tests <= 32 * blocks and st.rect_tests % 32 == 0
     assert 32 * leaf <= st.tri_tests <= 32 * leaf * (1 + blocks) and st.tri_tests % leaf == 0
+
+
+@pytest.mark.parametrize("T", [2, 12, 70, 600])
+def test_large_triangles(ctx, oracle, T):
+    """Triangles as large as the grid: most of a tile's cells want the blocks that survive, and are measured
+    against them directly. Every block size, tile and pass gives the same bits."""
+    import sdfb
+    rng = np.random.default_rng(T)
+    v = rng.uniform(-0.6, 0.6, (3 * T, 3)).astype(np.float32)
+    i = np.arange(3 * T, dtype=np.uint32).reshape(-1, 3)
+    n, origin, voxel = (30, 17, 26), (-0.5, -0.3, -0.45), 1.0 / 30
+    g = sdfb.make_grid(origin, voxel, n)
+    d64 = oracle.distance(v, i, origin, voxel, n)
+    ref = None
+    for leaf in (2, 4, 8):
+        for tile, budget in [(t, b) for t in range(1, 7) for b in (-1, 64)]:
+            d, _ = ctx.bake(v, i, g, sdfb.make_opts(sign_mode=sdfb.SIGN_NONE, leaf_size=leaf, tile=tile,
+                                                    step_budget=budget, no_occupancy=True), want_occ=False)
+            if ref is None:
+                ref = d
+                assert np.abs(d.reshape(-1) - d64).max() <= TOL * 1.2 * 3 ** 0.5  # the triangles' box
+            assert np.array_equal(d, ref), (leaf, tile, budget)
