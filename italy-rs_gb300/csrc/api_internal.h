@@ -95,6 +95,7 @@ struct GwnInput {
   const int8_t *col_s;
   float band_voxels;
   uint32_t *err;
+  uint64_t capacity;   // crossings that col_z and col_s hold; col_start may pass it (the bake is then repeated)
   uint64_t gwn_cells;  // cells of the winding-number meshes (refine list capacity)
   uint32_t most_caps;  // cap triangles of the mesh that has most
 };

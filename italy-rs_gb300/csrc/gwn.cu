@@ -126,6 +126,7 @@ struct GwnArgs {
   const uint64_t *col_start;
   const float *col_z;
   const int8_t *col_s;
+  uint64_t capacity;  // of col_z and col_s
   float band_voxels;
   TileCells *tiles;  // pass 1 -> pass 2 (coarse): tiles' parts with cells to refine
   unsigned long long *listed_tiles, *refine_count;  // their number, and their cells'
@@ -144,10 +145,19 @@ struct GwnArgs {
 constexpr unsigned long long kDirectWork = 1 << 21;  // caps times cells
 __device__ __forceinline__ bool few(const GwnArgs &a) { return *a.cell_count * a.most_caps <= kDirectWork; }
 
+// A column's crossings in the lists: [s0, s1). Where the lists are too short for all crossings the columns'
+// starts pass their end: what is beyond it was not written, and is not read (the bake is repeated).
+__device__ __forceinline__ void column_list(const GwnArgs &a, const MeshRec &M, int vx, int vy, uint64_t &s0,
+                                            uint64_t &s1) {
+  const uint64_t col = M.col_base + uint64_t(vy) * M.g.nx + vx;
+  s0 = __ldg(a.col_start + col);
+  s1 = min(__ldg(a.col_start + col + 1), a.capacity);
+}
+
 // Signed crossings of the column above height pz (the integer winding number of mesh + caps).
 __device__ __forceinline__ int column_winding(const GwnArgs &a, const MeshRec &M, int vx, int vy, float pz) {
-  const uint64_t col = M.col_base + uint64_t(vy) * M.g.nx + vx;
-  const uint64_t s0 = __ldg(a.col_start + col), s1 = __ldg(a.col_start + col + 1);
+  uint64_t s0, s1;
+  column_list(a, M, vx, vy, s0, s1);
   int w = 0;
   for (uint64_t k = s0; k < s1; ++k)
     if (__ldg(a.col_z + k) > pz) w += __ldg(a.col_s + k);
@@ -158,8 +168,8 @@ __device__ __forceinline__ int column_winding(const GwnArgs &a, const MeshRec &M
 template <int V>
 __device__ __forceinline__ void column_windings(const GwnArgs &a, const MeshRec &M, int vx, int vy,
                                                 const float (&pz)[V], int (&w)[V]) {
-  const uint64_t col = M.col_base + uint64_t(vy) * M.g.nx + vx;
-  const uint64_t s0 = __ldg(a.col_start + col), s1 = __ldg(a.col_start + col + 1);
+  uint64_t s0, s1;
+  column_list(a, M, vx, vy, s0, s1);
 #pragma unroll
   for (int v = 0; v < V; ++v) w[v] = 0;
   for (uint64_t k = s0; k < s1; ++k) {
@@ -649,6 +659,7 @@ cudaError_t gwn_enqueue(const GwnInput &in, void *temp, int num_sms, cudaStream_
   a.col_start = in.col_start;
   a.col_z = in.col_z;
   a.col_s = in.col_s;
+  a.capacity = in.capacity;
   a.band_voxels = in.band_voxels;
   a.tile_counter = counters;
   a.refine_count = counters + 1;

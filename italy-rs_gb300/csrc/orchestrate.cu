@@ -453,6 +453,7 @@ sdfb_status enqueue_batch(sdfb_ctx *ctx, Workspace &ws, cudaStream_t st, std::ve
   gi.batch = B;
   gi.col_start = static_cast<const uint64_t *>(ws.col_start.p);
   gi.col_z = static_cast<const float *>(ws.col_z.p);
+  gi.capacity = S.capacity;
   gi.col_s = static_cast<const int8_t *>(ws.col_s.p);
   gi.band_voxels = o.band_voxels;
   gi.err = d_err;

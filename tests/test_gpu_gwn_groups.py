@@ -55,3 +55,25 @@ def test_cells_left_by_the_coarse_pass(ctx, oracle, level, direct):
     d64 = oracle.distance(v, f, origin, voxel, dims, samples=samples)
     sure = (np.abs(np.abs(w) - 0.5) > 1e-6) & (d64 > 1e-6)
     assert np.array_equal(d.reshape(-1)[samples][sure] < 0, np.abs(w[sure]) > 0.5)
+
+
+def test_more_crossings_than_the_lists_hold(oracle):
+    """Many large triangles on a small grid: the first pass over the columns finds far more crossings than the lists
+    were made for. The winding number then reads what they hold, and the bake is repeated with longer ones."""
+    import sdfb
+    rng = np.random.default_rng(3)
+    T, n, voxel, origin = 3000, (24, 22, 20), 0.05, (-0.6, -0.55, -0.5)
+    v = rng.uniform(-0.7, 0.7, (3 * T, 3)).astype(np.float32)
+    f = np.arange(3 * T, dtype=np.uint32).reshape(-1, 3)
+    g = sdfb.make_grid(origin, voxel, n)
+    opts = sdfb.make_opts(sign_mode=sdfb.SIGN_GWN)
+    with sdfb.Context(0) as ctx:  # a fresh one: lists at their least
+        d, _ = ctx.bake(v, f, g, opts)
+        st = sdfb.Stats()
+        again, _ = ctx.bake(v, f, g, opts, stats=st)
+    assert st.crossings > 4 * (4 * n[0] * n[1] + 2 * 4 * T)  # mesh and caps: the least, several times over
+    assert np.array_equal(d, again)
+    w = oracle.gwn(v, f, origin, voxel, n)
+    d64 = oracle.distance(v, f, origin, voxel, n)
+    sure = (np.abs(np.abs(w) - 0.5) > 1e-5) & (d64 > 1e-5)
+    assert sure.mean() > 0.9 and np.array_equal(d.reshape(-1)[sure] < 0, np.abs(w[sure]) > 0.5)
