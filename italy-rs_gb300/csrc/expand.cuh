@@ -4,7 +4,8 @@
 // counts its items, the block scans the counts in shared memory, and its threads take the items in order, each
 // finding the owner by binary search in the shared starts and reading the triangle from shared
 // memory. A triangle with more than kWarpItems items goes to a list instead; a second kernel gives each
-// of those a warp, one with more than kBlockItems a block and one with more than kGridItems the grid.
+// of those a warp, one with more than kBlockItems a block, or several while there are few, and one with more than
+// kGridItems the grid.
 // (A block takes as long as its triangles have items: with the list from 4096 items on, the occupancy
 // stage of 1280 triangles at 128^3 and 256^3 took 179 and 891 us, now 27 and 45.)
 //
@@ -35,6 +36,13 @@ constexpr int kExpandThreads = 256;
 // meshes 43 -> 49 us), from 512 to a block (2048: 320 triangles at 128^3 31 -> 48 us).
 constexpr uint64_t kWarpItems = 48, kBlockItems = 512, kGridItems = 1 << 18;
 constexpr uint64_t kGridList = 1024;
+// The triangles for a block are cut into parts where they are fewer than twice the blocks, so that none of
+// the blocks is idle and none holds the others up. One block a triangle, parts for one, two, four times the
+// blocks, and a device-wide scan of all items as it was once: occupancy stage of a turned box of 12 triangles at
+// 128^3 387, 43, 45, 47 and 52 us, of 80 triangles at 256^3 191, 69, 63, 62 and 76, of 200 as large as the grid
+// at 128^3 439, 235, 166, 143 and 164, of 320 at 128^3 31, 29, 30, 33 and 29; crossings of the box at 400^3 127,
+// 25, 27, 29 and 54.
+constexpr unsigned long long kBlockShare = 2;
 
 // Triangles left to the second kernel: those for a warp from the front of `tris`, those for a block from
 // its end, those for the grid in a list of their own (as far as it holds them). counts: zero before the
@@ -118,11 +126,13 @@ __global__ __launch_bounds__(kExpandThreads) void k_expand_big(BatchDev B, BigLi
     for (uint64_t k = lane; k < c; k += kWarp) op.item(B, tri, k);
     if (lane == 0) items += c;
   }
-  for (unsigned long long i = blockIdx.x; i < nblock; i += gridDim.x) {
+  const unsigned long long share = nblock ? max(1ull, kBlockShare * gridDim.x / nblock) : 1;
+  for (unsigned long long i = blockIdx.x; i < nblock * share; i += gridDim.x) {
+    const unsigned long long t = i / share, part = i - t * share;
     typename Op::Tri tri;
-    const uint64_t c = op.setup(B, big.tris[big.n - 1 - i], tri);
-    for (uint64_t k = threadIdx.x; k < c; k += kExpandThreads) op.item(B, tri, k);
-    if (threadIdx.x == 0) items += c;
+    const uint64_t c = op.setup(B, big.tris[big.n - 1 - t], tri);
+    for (uint64_t k = part * kExpandThreads + threadIdx.x; k < c; k += share * kExpandThreads) op.item(B, tri, k);
+    if (threadIdx.x == 0 && part == 0) items += c;
   }
   for (unsigned long long i = 0; i < ngrid; ++i) {
     typename Op::Tri tri;

@@ -70,3 +70,24 @@ def test_more_grid_wide_triangles_than_listed(ctx):
         _, o = ctx.bake(v, np.arange(3 * n, dtype=np.uint32).reshape(-1, 3), g, sdfb.make_opts(), want_dist=False)
         occ.append(o)
     assert occ[0].any() and np.array_equal(*occ)
+
+
+@pytest.mark.parametrize("T", [1, 12, 150, 700, 1500])
+def test_few_large_triangles(ctx, oracle, T):
+    """Triangles of 513 to some 100k candidate cells, each by several thread blocks, by one, or more of them than
+    blocks: occupancy and parity of the oracle, and all cells tested once."""
+    import sdfb
+    rng = np.random.default_rng(T)
+    dims, voxel = (75, 61, 66), 1.0 / 64
+    v = (rng.uniform(0.1, 0.9, (T, 1, 3)) + rng.normal(0, 0.25, (T, 3, 3))).astype(np.float32).reshape(-1, 3)
+    f = np.arange(3 * T, dtype=np.uint32).reshape(-1, 3)
+    st = sdfb.Stats()
+    d, occ = ctx.bake(v, f, sdfb.make_grid((0, 0, 0), voxel, dims), sdfb.make_opts(sign_mode=sdfb.SIGN_PARITY), stats=st)
+    p = v.reshape(-1, 3, 3) * 64
+    lo = np.clip(np.floor(p.min(axis=1)), 0, np.array(dims) - 1)
+    hi = np.clip(np.floor(p.max(axis=1)), 0, np.array(dims) - 1)
+    assert st.sat_tests == int((hi - lo + 1).prod(axis=1).sum())
+    assert np.array_equal(occ.reshape(-1), oracle.occupancy(v, f, (0, 0, 0), voxel, dims))
+    s = np.asarray(oracle.sign_parity(v, f, (0, 0, 0), voxel, dims)).reshape(-1)
+    away = d.reshape(-1) > 1e-5 if T == 1 else np.abs(d.reshape(-1)) > 1e-5
+    assert np.array_equal((d.reshape(-1) < 0)[away], (s < 0)[away])
