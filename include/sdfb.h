@@ -71,7 +71,9 @@ typedef struct sdfb_grid_desc {
 typedef struct sdfb_opts {
   uint32_t struct_size;
   int32_t sign_mode;      /* sdfb_sign_mode, default AUTO */
-  float band_voxels;      /* GWN: width in voxels of the FP64 band around the surface, default 1 */
+  float band_voxels;      /* GWN: width in voxels of the band around the surface whose signs are summed in
+                             FP64, default 1. Near caps' solid angles enter in FP32 with a bound on their
+                             error; a sign that the bounds do not prove gets FP64 ones */
   int32_t leaf_size;      /* 1..16: the tree's blocks hold the largest of 2, 4, 8 triangles not above
                              it, at least 2; default: autotuned table */
   int32_t tile;           /* distance tile shape 1..6 (4x4x2, 8x4x1, 4x4x4, 8x4x2, 4x4x8, 8x4x4
@@ -103,7 +105,7 @@ typedef struct sdfb_opts {
 #define SDFB_FAULT_STACK_ALL 8     /* every traversal stack holds 2 entries -> OVERFLOW */
 
 /* Per-call statistics, filled when the pointer is non-null. Times are CUDA-event times on the
- * bake stream (ms); counts are exact. A single-mesh call that asks for them runs its stages one after
+ * bake stream (ms); counts are exact, of what they say they count. A single-mesh call that asks for them runs its stages one after
  * another; one that does not builds the tree and tests occupancy while the sign is being found. */
 typedef struct sdfb_stats {
   uint32_t struct_size;
@@ -129,7 +131,7 @@ typedef struct sdfb_stats {
   double flops_distance;   /* count_work: FP32 flops of the distance tests as executed, terms a lane
                               shares between its cells counted once (FMA = 2) */
   uint64_t kernel_launches; /* kernels this call launched */
-  uint64_t gwn_fp64_cells;  /* GWN: cells whose winding number was evaluated in FP64 (band + ambiguous) */
+  uint64_t gwn_fp64_cells;  /* GWN: cells whose winding number was summed in FP64 (band + ambiguous) */
   uint64_t graph_replayed;  /* 1 when the launch sequence was replayed from a CUDA graph */
   uint64_t tiles_deferred;  /* distance tiles that exceeded the step budget and were finished by a
                                whole block in the second distance pass */

@@ -17,6 +17,7 @@
 namespace sdfb {
 namespace {
 
+// The 64-bit finalizer of MurmurHash3 (Appleby).
 inline uint64_t mix64(uint64_t x) {
   x ^= x >> 33;
   x *= 0xff51afd7ed558ccdULL;

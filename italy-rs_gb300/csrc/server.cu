@@ -66,6 +66,7 @@ struct Hash2 {
   uint64_t a = 0xcbf29ce484222325ull, b = 0x6a09e667f3bcc909ull;
 };
 
+// The 64-bit finalizer of MurmurHash3 (Appleby).
 inline uint64_t avalanche(uint64_t h) {
   h ^= h >> 33;
   h *= 0xff51afd7ed558ccdull;

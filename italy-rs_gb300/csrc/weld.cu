@@ -51,6 +51,7 @@ inline uint64_t pow2_at_least(uint64_t n) {
   return p;
 }
 
+// The 64-bit finalizer of MurmurHash3 (Appleby).
 __device__ __forceinline__ uint64_t mix64(uint64_t x) {
   x ^= x >> 33;
   x *= 0xff51afd7ed558ccdull;
